@@ -1,56 +1,209 @@
 // True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores: IEEE float32
 // multiply-add, no TF32, no reduced-precision staging.  It serves the float32 path of the
-// whole model, whose purpose is to show faults that bfloat16 rounding hides, so it favours a
-// fixed summation order over speed: every output element adds its K products in the same
-// order whatever M is, hence a token's logits do not depend on what else is in the batch.
+// whole model, whose purpose is to show faults that bfloat16 rounding hides, so the summation
+// order is fixed: K is cut into segments by a rule on N and K alone; in a segment every output
+// element adds its products over the even k and over the odd k in ascending order and then those
+// two sums, and the segments' sums are added in order.  Neither M nor the tile that computes an
+// element changes a bit, hence a token's logits do not depend on what else is in the batch.
 // (The reference reaches float32 by running its library path with DTYPE=float32 on the CPU,
 // tests/test_batching.py:57; it has no float32 GPU path.)
+//
+// Bound by the float32 FMA rate (74 TFLOP/s) for many rows, by the weight's bytes for few.  The
+// packed two-float multiply-add of this architecture does two neighbouring k per instruction:
+// both operands lie along K as they are stored, so tiles go to shared memory untransposed by
+// cp.async (16 bytes, or 4 where rows do not start on 16) and pairs need no shuffling.  Rows are
+// padded by 16 bytes: the eight rows that a quarter warp reads lie in different banks.  501 rows,
+// N x K = 6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728: 482, 334, 1,357, 672 us (32 to
+// 37 TFLOP/s; a 64 x 64 tile with scalar multiply-adds and no pipeline took 862, 737, 2,366, 1,727).
+// The packed multiply-add pipe is active 59 % of the time; tiles of 8 x 4 or 4 x 8 a thread with twice
+// the warps, steps of 16 of K, and scalar multiply-adds (33 TFLOP/s at 3,000 rows against 37) are slower.
 #include "common.cuh"
 
-constexpr int BM = 64, BN = 64, BK = 16;
+namespace {
 
-__global__ void __launch_bounds__(256) gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W,
-                                                          float* __restrict__ C, int ldc, int M, int N, int K) {
-    __shared__ float As[BK][BM + 4], Ws[BK][BN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int i = threadIdx.x; i < BM * BK; i += 256) {
-            const int r = i / BK, c = i % BK;
-            const int m = m0 + r, n = n0 + r, k = k0 + c;
-            As[c][r] = (m < M && k < K) ? A[(size_t)m * lda + k] : 0.f;
-            Ws[c][r] = (n < N && k < K) ? W[(size_t)n * K + k] : 0.f;
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp4(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" :: "r"(dst), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
+
+constexpr int BK_MAX = 64;
+
+// A warp's lanes are 4 (rows) x 8 (columns); a lane owns TM x TN outputs, rows 4 apart, columns 8 apart, so a warp covers
+// 4 TM x 8 TN and the block WM x WN of those.
+template <int TM, int TN, int WM, int WN, int BK, int STAGES>
+struct Tile {
+    static constexpr int BM = 4 * TM * WM, BN = 8 * TN * WN, THREADS = 32 * WM * WN, LD = BK + 4;
+    static constexpr int STAGE = (BM + BN) * LD, SMEM = STAGES * STAGE * 4;
+};
+
+// grid (column tiles, row tiles, segments of K); segment z writes out + z * M * ldc
+template <int TM, int TN, int WM, int WN, int BK, int STAGES, bool VEC>
+__global__ void __launch_bounds__(32 * WM * WN) gemm_f32_nt_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W,
+                                                                   float* __restrict__ out, int ldc, int M, int N, int K, int segment) {
+    using L = Tile<TM, TN, WM, WN, BK, STAGES>;
+    extern __shared__ __align__(16) float smem[];
+    const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * L::BM, n0 = blockIdx.x * L::BN;
+    const int row_a = (warp / WN) * 4 * TM + (lane >> 3), row_b = (warp % WN) * 8 * TN + (lane & 7);
+    const int k_first = blockIdx.z * segment, k_end = min(K, k_first + segment);
+    const int steps = (k_end - k_first + BK - 1) / BK;
+
+    auto load = [&](int step) {
+        const uint32_t dst = s0 + (step % STAGES) * L::STAGE * 4;
+        const int k0 = k_first + step * BK;
+        constexpr int PIECE = VEC ? 4 : 1, PER_ROW = BK / PIECE;
+        for (int id = tid; id < (L::BM + L::BN) * PER_ROW; id += L::THREADS) {
+            const int r = id / PER_ROW, k = k0 + id % PER_ROW * PIECE;
+            const bool is_a = r < L::BM;
+            const int g = is_a ? m0 + r : n0 + r - L::BM;
+            const bool ok = k < k_end && g < (is_a ? M : N);
+            const float* src = !ok ? A : is_a ? A + (size_t)g * lda + k : W + (size_t)g * K + k;
+            const uint32_t at = dst + (r * L::LD + id % PER_ROW * PIECE) * 4;
+            if (VEC) cp16(at, src, ok); else cp4(at, src, ok);
         }
-        __syncthreads();
+    };
+    float2 acc[TM][TN];
 #pragma unroll
-        for (int k = 0; k < BK; ++k) {
-            float a[4], b[4];
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { a[i] = As[k][ty * 4 + i]; b[i] = Ws[k][tx * 4 + i]; }
+        for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < steps) load(s);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;\n" :: "n"(STAGES - 2) : "memory");
+        __syncthreads();                       // the stage is there for everyone, and everyone is done with the one loaded next
+        if (step + STAGES - 1 < steps) load(step + STAGES - 1);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const float* a_s = smem + (step % STAGES) * L::STAGE + row_a * L::LD;
+        const float* b_s = smem + (step % STAGES) * L::STAGE + (L::BM + row_b) * L::LD;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
+        for (int kk = 0; kk < BK; kk += 4) {
+            float4 b[TN];
+#pragma unroll
+            for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(b_s + 8 * j * L::LD + kk);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(a_s + 4 * i * L::LD + kk);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = __ffma2_rn(make_float2(a.x, a.y), make_float2(b[j].x, b[j].y), acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] = __ffma2_rn(make_float2(a.z, a.w), make_float2(b[j].z, b[j].w), acc[i][j]);
+            }
+        }
+    }
+    out += (size_t)blockIdx.z * M * ldc;
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + row_a + 4 * i;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n < N) C[(size_t)m * ldc + n] = acc[i][j];
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + row_b + 8 * j;
+            if (n < N) out[(size_t)m * ldc + n] = acc[i][j].x + acc[i][j].y;
         }
     }
 }
 
-MI_EXPORT int mi_gemm_f32_nt(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K,
+// C = the segments' sums, added in order; ws [S, M, N]
+__global__ void add_segments_kernel(const float* __restrict__ ws, float* __restrict__ C, int ldc, int M, int N, int S) {
+    const size_t plane = (size_t)M * N;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += (size_t)gridDim.x * blockDim.x) {
+        float v = ws[i];
+        for (int s = 1; s < S; ++s) v += ws[s * plane + i];
+        C[i / N * ldc + i % N] = v;
+    }
+}
+
+template <int TM, int TN, int WM, int WN, int BK, int STAGES>
+int launch(const float* A, int lda, const float* W, float* out, int ldc, int M, int N, int K, int S, int segment, cudaStream_t stream) {
+    using L = Tile<TM, TN, WM, WN, BK, STAGES>;
+    static_assert(BK_MAX % BK == 0, "a segment is a whole number of every tile's steps");
+    const dim3 grid((N + L::BN - 1) / L::BN, (M + L::BM - 1) / L::BM, S);
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+    auto kernel = vec ? gemm_f32_nt_kernel<TM, TN, WM, WN, BK, STAGES, true> : gemm_f32_nt_kernel<TM, TN, WM, WN, BK, STAGES, false>;
+    static bool configured[2] = {false, false};
+    if (!configured[vec]) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+        if (e != cudaSuccess) return (int)e;
+        configured[vec] = true;
+    }
+    kernel<<<grid, L::THREADS, L::SMEM, stream>>>(A, lda, W, out, ldc, M, N, K, segment);
+    return (int)cudaGetLastError();
+}
+
+// Narrow products have few column tiles: their K is cut until a row tile alone gives about one block per SM, in pieces of at least
+// 1,024 (501 rows, N 2,560, K 9,728 in one segment: 80 blocks of 128 x 128, 1,093 us; in 8: 672 us).
+int segments(int N, int K, int* segment) {
+    const int tiles = (N + 127) / 128;
+    int S = K / 1024 < 8 ? K / 1024 : 8;
+    if (S > 160 / tiles) S = 160 / tiles;
+    if (S < 1) S = 1;
+    *segment = K < BK_MAX ? BK_MAX : ((K + S - 1) / S + BK_MAX - 1) / BK_MAX * BK_MAX;
+    return (K + *segment - 1) / *segment > 1 ? (K + *segment - 1) / *segment : 1;
+}
+
+constexpr int ROWS_AT_ONCE = 1024;             // rows per pass of a product that is cut along K: bounds its workspace
+
+// The tile whose last wave wastes least, by the area an SM works through (relative rates measured with every SM full).
+int pick_tile(int M, int N, int S) {
+    static const int bm[5] = {128, 64, 64, 32, 16}, bn[5] = {128, 128, 64, 64, 16};
+    static const float rate[5] = {1.f, 1.f, 0.94f, 0.8f, 0.3f};
+    int best = 0;
+    float least = 0.f;
+    const int sms = mi::device_sms();
+    for (int t = 0; t < 5; ++t) {
+        const long long blocks = (long long)((M + bm[t] - 1) / bm[t]) * ((N + bn[t] - 1) / bn[t]) * S;
+        const float cost = (float)((blocks + sms - 1) / sms) * bm[t] * bn[t] / rate[t];
+        if (t == 0 || cost < least) { least = cost; best = t; }
+    }
+    return best;
+}
+
+int run_tile(const float* A, int lda, const float* W, float* out, int ldc, int M, int N, int K, int S, int segment, int tile, cudaStream_t stream) {
+    switch (tile) {
+        case 0: return launch<8, 8, 4, 2, 32, 3>(A, lda, W, out, ldc, M, N, K, S, segment, stream);
+        case 1: return launch<8, 8, 2, 2, 32, 3>(A, lda, W, out, ldc, M, N, K, S, segment, stream);
+        case 2: return launch<8, 8, 2, 1, 32, 3>(A, lda, W, out, ldc, M, N, K, S, segment, stream);
+        case 3: return launch<8, 4, 1, 2, 32, 4>(A, lda, W, out, ldc, M, N, K, S, segment, stream);
+        default: return launch<2, 2, 2, 1, 64, 6>(A, lda, W, out, ldc, M, N, K, S, segment, stream);
+    }
+}
+
+}  // namespace
+
+// floats of workspace that a product of this shape needs (0: none)
+MI_EXPORT long long mi_gemm_f32_workspace(int M, int N, int K) {
+    int segment;
+    const int S = segments(N, K, &segment);
+    return S > 1 ? (long long)S * (M < ROWS_AT_ONCE ? M : ROWS_AT_ONCE) * N : 0;
+}
+
+// tile < 0: chosen here (every tile gives the same bits)
+MI_EXPORT int mi_gemm_f32_nt(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, float* ws, int tile,
                              cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-    gemm_f32_nt_kernel<<<grid, 256, 0, stream>>>(A, lda, W, C, ldc, M, N, K);
-    return (int)cudaGetLastError();
+    int segment;
+    const int S = segments(N, K, &segment);
+    if (S > 1 && !ws) return -2;
+    const int step = S > 1 ? ROWS_AT_ONCE : M;
+    for (int m = 0; m < M; m += step) {
+        const int rows = M - m < step ? M - m : step;
+        const int t = tile >= 0 ? tile : pick_tile(rows, N, S);
+        const int rc = run_tile(A + (size_t)m * lda, lda, W, S > 1 ? ws : C + (size_t)m * ldc, S > 1 ? N : ldc, rows, N, K, S, segment, t, stream);
+        if (rc) return rc;
+        if (S > 1) {
+            const size_t n = (size_t)rows * N;
+            const int blocks = (int)((n + 1023) / 1024 < 148 * 8 ? (n + 1023) / 1024 : 148 * 8);
+            add_segments_kernel<<<blocks, 256, 0, stream>>>(ws, C + (size_t)m * ldc, ldc, rows, N, S);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return (int)e;
+        }
+    }
+    return 0;
 }

@@ -26,6 +26,7 @@ def load_library():
         from .build import build
         path = build()
         _LIB = ctypes.CDLL(path)
+        _LIB.mi_gemm_f32_workspace.restype = ctypes.c_longlong
     return _LIB
 
 
@@ -247,8 +248,7 @@ class CudaOps:
             N = w.shape[0]
             assert x.stride(1) == 1 and w.is_contiguous() and w.dtype == torch.float32
             out = torch.empty((M, N), dtype=torch.float32, device=x.device)
-            _check(self.lib.mi_gemm_f32_nt(_p(x), x.stride(0), _p(w), _p(out), N, M, N, K, self._stream()), "gemm_f32")
-            self.launches += 1
+            self._gemm_f32(x, x.stride(0), w, out, N, M, N, K)
             return out
         M, K = x.shape
         if (self._use_tc(M, w.shape[0], K) and K % 64 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
@@ -278,6 +278,14 @@ class CudaOps:
             if err != -2:
                 _check(err, "gemm_skinny")
         return self._library_linear(x, w, out_dtype)
+
+    def _gemm_f32(self, x, ldx, w, out, ldc, M, N, K, tile=-1):
+        """out [M, N] (rows ldc apart) = x [M, K] (rows ldx apart) @ w [N, K].T in float32; narrow products are cut along K by a rule on N
+        and K alone, their partial sums pass a workspace.  tile: a tile of csrc/gemm_f32.cu instead of its own choice (same bits)."""
+        n = self.lib.mi_gemm_f32_workspace(M, N, K)
+        ws = torch.empty(n, dtype=torch.float32, device=x.device) if n else None
+        _check(self.lib.mi_gemm_f32_nt(_p(x), ldx, _p(w), _p(out), ldc, M, N, K, _p(ws), tile, self._stream()), "gemm_f32")
+        self.launches += 2 if n else 1
 
     @staticmethod
     def _library_linear(x, w, out_dtype):
@@ -569,6 +577,8 @@ class CudaOps:
                 _p(meta.seg_q_start), _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D,
                 meta.page_size, meta.tile, _c.c_float(scale), win, self._stream()), "attn_prefill_mma")
             self.launches += 1
+        elif num_tiles and self._f32_tiles(q, D, D, meta):
+            self._prefill_f32(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
         elif num_tiles:
             _check(self.lib.mi_attn_prefill_generic(
                 _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles,
@@ -612,6 +622,20 @@ class CudaOps:
                 H, KV, D, meta.page_size, S, _c.c_float(scale), win, code, self._stream()), "attn_decode")
             self.launches += 2 if S > 1 else 1
         return out
+
+    def _f32_tiles(self, q, D, V, meta):
+        """Whether the float32 prompt attention with tiles takes these rows: heads of 64 or 128 that start on 16 bytes, tiles of 64 rows."""
+        return (self.fast_attention and q.dtype == torch.float32 and D == V and D in (64, 128) and meta.tile == 64 and q.stride(0) % 4 == 0
+                and q.data_ptr() % 16 == 0)
+
+    def _prefill_f32(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias=None, bias_last=0,
+                     slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):
+        _check(self.lib.mi_attn_prefill_f32(
+            _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), meta.prefill_tiles.shape[0], _p(meta.seg_q_start),
+            _p(meta.seg_pos0), _p(meta.block_table), _p(getattr(meta, "table_rows", None)), meta.max_pages, H, KV, D, meta.page_size, meta.tile,
+            _c.c_float(scale), block, window, sink, _p(sink_values), _p(bias), bias_last, _p(slopes), _c.c_float(cap), keep, _p(gate), gate_stride,
+            self._stream()), "attn_prefill_f32")
+        self.launches += 1
 
     # ---------------------------------------------------------------- float32 stream, scalar norms, polynomial norm
     def embed_scaled_norm(self, ids, table, g, eps, out_dtype):
@@ -732,8 +756,7 @@ class CudaOps:
         if not side_by_side:
             out = torch.empty((H, T, N), dtype=torch.float32, device=x.device)
         for h in range(H):
-            _check(self.lib.mi_gemm_f32_nt(_p(xs[h]), xs.stride(1), _p(w[h]), _p(out[h]), out.stride(1), T, N, K, self._stream()), "gemm_f32")
-        self.launches += H
+            self._gemm_f32(xs[h], xs.stride(1), w[h], out[h], out.stride(1), T, N, K)
         return rows if side_by_side else out
 
     def latent_prepare(self, p, q_abs, H, D, R, C, norm_w, eps, inv_freq, meta, cache, q_rows=None, dkv_col=None, half_pairs=False):
@@ -935,6 +958,9 @@ class CudaOps:
             else:                                          # a slope per head times the distance, beside (or instead of) the table
                 _check(self.lib.mi_attn_prefill_mma_sloped(*args, _p(slopes), self._stream()), "attn_prefill_mma_sloped")
             self.launches += 1
+        elif num_tiles and self._f32_tiles(q, D, V, meta):
+            self._prefill_f32(q, k_cache, v_cache, out, meta, H, KV, D, scale, blk, win, int(bool(sink)), sink_values, distance_bias, bias_last,
+                              slopes, cap, keep, gate, gate_stride)
         elif num_tiles:
             _check(self.lib.mi_masked_prefill(
                 _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),
