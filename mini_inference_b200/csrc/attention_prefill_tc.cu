@@ -18,6 +18,13 @@
 //            at the end divide by the row sum and store.
 // Two blocks fit on an SM (256 tensor-memory columns and 96 KB of shared memory each), so one
 // block's softmax overlaps the other's MMAs.  Every mbarrier wait is bounded.
+//
+// FORM other than PLAIN: masks and softmax terms of csrc/attention_masked.cu, and every softmax weight enters P V as TWO
+// bfloat16 numbers, its rounding and what the rounding left (16 mantissa bits, summed in float32): 64 float32 scores take
+// 64 columns, 64 weights as two packed halves take 32 + 32, so both halves replace the scores they came from and P V is
+// issued twice on the same values.  MASKED: blocks of positions, window, sink (score 0 or learned).  BIASED adds the distance
+// table and slopes; EXTENDED the cap, the kept first keys and the output gate (no sink, no blocks).  2,048 tokens, 16 heads of
+// 128, with the products around it: 208 -> 109 us against the mma.sync form of this kernel (149 us of the 208 were attention).
 #include "sm100.cuh"
 #include <map>
 #include <mutex>
@@ -51,15 +58,31 @@ MI_EXPORT int mi_attn_tc_timing(unsigned long long* out, int reset) {
 namespace {
 
 constexpr int BQ = 128, BKV = 64;
+constexpr int PLAIN = 0, MASKED = 1, BIASED = 2, EXTENDED = 3;
+constexpr float LOG2E = 1.4426950408889634f;
+
+struct Terms {
+    int block, sink, keep, bias_last, gate_stride;
+    float cap;
+    const float *sink_values, *bias_t, *slopes;       // [H]; [H, bias_last + 1]; [H]; each or null
+    const __nv_bfloat16* gate;                        // [T, H D], rows gate_stride apart, or null
+};
+
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
 constexpr int ATT_THREADS = 224;      // warp 0: Q and K loads, 1: MMA issue, 2-5: softmax, 6: V loads
 
-template <int D>
+template <int D, int FORM>
 __global__ void __launch_bounds__(ATT_THREADS, 2)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap,
                        const __grid_constant__ CUtensorMap vmap, __nv_bfloat16* __restrict__ out,
                        const int* __restrict__ tiles, const int* __restrict__ seg_q_start,
                        const int* __restrict__ seg_pos0, const int* __restrict__ block_table,
-                       const int* __restrict__ table_rows, int table_stride, int H, int KV, int ps, float scale_log2, int window, int* __restrict__ error_word) {
+                       const int* __restrict__ table_rows, int table_stride, int H, int KV, int ps, float scale_log2, int window, int* __restrict__ error_word,
+                       const __grid_constant__ Terms terms) {
+    constexpr bool SPLIT = FORM != PLAIN;
     constexpr int HALVES = D / 64;                       // 64-element (128-byte) column blocks of a head
     constexpr int Q_BYTES = BQ * D * 2, KV_BYTES = BKV * D * 2;
     constexpr int TMEM_COLS = 256;                       // S0: 64, S1: 64 (P overwrites the first 32 columns of its S), O: D
@@ -82,9 +105,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
     const int qs = seg_q_start[seg], n = seg_q_start[seg + 1] - qs, pos0 = seg_pos0[seg];
     const int rows = min(BQ, n - r0);
     const int p_first = pos0 + r0, p_last = pos0 + r0 + rows - 1;
-    const int kt_lo = window > 0 ? max(0, p_first - window + 1) / BKV : 0;
+    auto first_key = [&](int p) {
+        int lo = window > 0 ? max(0, p - window + 1) : 0;
+        if constexpr (FORM == MASKED || FORM == BIASED) { if (terms.block > 0) lo = max(lo, p / terms.block * terms.block); }
+        return lo;
+    };
+    const int kt_lo = first_key(p_first) / BKV;
     const int kt_hi = p_last / BKV;
-    const int nt = kt_hi - kt_lo + 1;
+    // the tiles of the kept keys come first (those that the window's tiles do not hold anyway)
+    const int kept_tiles = FORM == EXTENDED && window > 0 ? min((terms.keep + BKV - 1) / BKV, kt_lo) : 0;
+    const int nt = kt_hi - kt_lo + 1 + kept_tiles;
+    auto kt_of = [&](int i) { return FORM == EXTENDED && i < kept_tiles ? i : kt_lo + i - kept_tiles; };
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -121,7 +152,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         const CUtensorMap* map = is_v ? &vmap : &kmap;
         bool ok = true;
         for (int i = 0; i < nt; ++i) {
-            const int s = i & 1, kt = kt_lo + i;
+            const int s = i & 1, kt = kt_of(i);
             if (lane == 0) {
                 if (i >= 2 && !mbar_wait(empty + 8 * s, ((i >> 1) - 1) & 1)) { atomicExch(error_word, 21); ok = false; }
                 if (ok) mbar_expect_tx(full + 8 * s, KV_BYTES);
@@ -175,6 +206,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
                 for (int kk = 0; kk < BKV / 16; ++kk) {
                     const uint32_t b = sV + s * KV_BYTES + kk * (16 * 128);
                     umma_ts(tmem + O_COL, tmem + S_COL + 64 * s + kk * 8, umma_desc_sw128(b, BKV * 128, 1024), idesc_o, (i | kk) != 0);
+                    if (SPLIT) umma_ts(tmem + O_COL, tmem + S_COL + 64 * s + 32 + kk * 8, umma_desc_sw128(b, BKV * 128, 1024), idesc_o, true);
                 }
                 umma_commit(v_empty + 8 * s);                  // the values of this stage are free once these finish
                 umma_commit(pv_done);                          // and O holds tile i
@@ -186,10 +218,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
         const int row = lg * 32 + lane;                        // row of the tile
         const int p_row = pos0 + r0 + row;
         const uint32_t lane_addr = tmem + ((uint32_t)(lg * 32) << 16);
-        float m_ref = -INFINITY, l = 0.f;
+        const int lo_row = first_key(p_row);
+        float m_ref = -INFINITY, l = 0.f;                      // a sink's term: a running maximum that starts at its score, a sum at 1
+        if constexpr (FORM == MASKED || FORM == BIASED) {
+            if (terms.sink) { m_ref = terms.sink_values ? terms.sink_values[h] * LOG2E : 0.f; l = 1.f; }
+        }
+        const float slope_log2 = FORM == BIASED && terms.slopes ? terms.slopes[h] * LOG2E : 0.f;
+        const float* __restrict__ bias_row = FORM == BIASED && terms.bias_t ? terms.bias_t + (size_t)h * (terms.bias_last + 1) : nullptr;
+        // cap * tanh(s / cap) = cap - 2 cap / (1 + e^(2 s / cap)), in base 2
+        const float cap_log2 = FORM == EXTENDED ? terms.cap * LOG2E : 0.f, cap_rate = FORM == EXTENDED && terms.cap > 0.f ? 2.f * scale_log2 / terms.cap : 0.f;
+        const bool capped = FORM == EXTENDED && terms.cap > 0.f;
+        const float row_scale = FORM == BIASED || capped ? 1.f : scale_log2;      // what the values in r[] still have to be multiplied by
         bool ok = true;
         for (int i = 0; i < nt && ok; ++i) {
-            const int kt = kt_lo + i;
+            const int kt = kt_of(i);
             const uint32_t s_col = S_COL + 64 * (i & 1);
             TICK(t0);
             if (!mbar_spin(s_full + 8 * (i & 1), (i >> 1) & 1)) { atomicExch(error_word, 25); ok = false; break; }
@@ -202,12 +244,39 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
             TICK(ta);
             // Scores stay unscaled in r[]; the scale is folded into the exponent's multiply-add.  Only tiles
             // that touch the diagonal (or the window's edge) for some row of the warp pay for masking.
-            const bool inside = kt * BKV + BKV - 1 <= p_row && (window <= 0 || kt * BKV > p_row - window);
+            if constexpr (FORM == BIASED) {
+                const int d0 = p_row - kt * BKV;                     // distance to the tile's first key (negative ones are masked below)
+                if (bias_row != nullptr) {
+                    if (__all_sync(0xffffffffu, d0 - (BKV - 1) >= terms.bias_last)) {
+                        const float far = bias_row[terms.bias_last] * LOG2E;
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) r[c] = __float_as_uint(fmaf(__uint_as_float(r[c]), scale_log2, fmaf(-slope_log2, (float)(d0 - c), far)));
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 64; ++c) {
+                            const float b = bias_row[max(0, min(d0 - c, terms.bias_last))] * LOG2E;
+                            r[c] = __float_as_uint(fmaf(__uint_as_float(r[c]), scale_log2, fmaf(-slope_log2, (float)(d0 - c), b)));
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 64; ++c) r[c] = __float_as_uint(fmaf(__uint_as_float(r[c]), scale_log2, -slope_log2 * (float)(d0 - c)));
+                }
+            }
+            if constexpr (FORM == EXTENDED) {
+                if (capped) {
+#pragma unroll
+                    for (int c = 0; c < 64; ++c)
+                        r[c] = __float_as_uint(cap_log2 - __fdividef(2.f * cap_log2, 1.f + fast_exp2(__uint_as_float(r[c]) * cap_rate)));
+                }
+            }
+            const bool kept = FORM == EXTENDED && kt * BKV + BKV <= terms.keep;
+            const bool inside = kt * BKV + BKV - 1 <= p_row && (kt * BKV >= lo_row || kept);
             if (!__all_sync(0xffffffffu, inside)) {
 #pragma unroll
                 for (int c = 0; c < 64; ++c) {
                     const int j = kt * BKV + c;
-                    const bool vis = j <= p_row && (window <= 0 || j > p_row - window);
+                    const bool vis = j <= p_row && (j >= lo_row || (FORM == EXTENDED && j < terms.keep));
                     if (!vis) r[c] = 0xff800000u;                     // -inf
                 }
             }
@@ -219,7 +288,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
 #pragma unroll
                 for (int q = 0; q < 4; ++q) mxs[q] = max3(mxs[q], __uint_as_float(r[c + 2 * q]), __uint_as_float(r[c + 2 * q + 1]));
             }
-            const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * scale_log2;   // scale > 0
+            const float mx = fmaxf(fmaxf(mxs[0], mxs[1]), fmaxf(mxs[2], mxs[3])) * row_scale;   // scale > 0
             // keep the exponent offset unless the maximum grew by more than 2^8: rescaling O is then rare
             float alpha = 1.f;
             bool rescale = false;
@@ -232,21 +301,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
             const float off = m_ref == -INFINITY ? 0.f : m_ref;
             TICK(tb);
             uint32_t pk[32];
-            const float2 scale2 = make_float2(scale_log2, scale_log2), noff2 = make_float2(-off, -off);
+            const float2 scale2 = make_float2(row_scale, row_scale), noff2 = make_float2(-off, -off);
             float2 sums[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
                 const float2 arg = __ffma2_rn(make_float2(__uint_as_float(r[2 * c]), __uint_as_float(r[2 * c + 1])), scale2, noff2);
                 const float2 p = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
                 sums[c & 3] = __fadd2_rn(sums[c & 3], p);
-                __nv_bfloat162 hh = __floats2bfloat162_rn(p.x, p.y);
-                pk[c] = *reinterpret_cast<uint32_t*>(&hh);
+                pk[c] = pack_bf16(p.x, p.y);
+                if (SPLIT) {                                      // what the rounding leaves takes the place of a score that is done with
+                    const float2 back = make_float2(__uint_as_float(pk[c] << 16), __uint_as_float(pk[c] & 0xffff0000u));
+                    const float2 left = __ffma2_rn(back, make_float2(-1.f, -1.f), p);
+                    r[c] = pack_bf16(left.x, left.y);
+                }
             }
             const float2 s01 = __fadd2_rn(sums[0], sums[1]), s23 = __fadd2_rn(sums[2], sums[3]);
             const float sum = (s01.x + s01.y) + (s23.x + s23.y);
             l += sum;
             TICK(tc);
             tmem_st32(lane_addr + s_col, pk);                  // P takes the place of the scores it came from
+            if (SPLIT) tmem_st32(lane_addr + s_col + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
             TICK(t2);
             // Every thread follows pv_done phase by phase (a parity wait can only tell the current phase
             // from the one before it); O holds tile i-1 completely after this.
@@ -261,6 +335,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
 #pragma unroll
                     for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * alpha);
                     tmem_st32(lane_addr + O_COL + c * 32, o);
+                }
+            }
+            if (i == nt - 1 && ok) {                               // values behind the last row's key may be anything, and 0 * inf is no 0
+                const int first = p_last - kt * BKV + 1;
+                if (first < BKV) {
+                    if (!mbar_spin(v_full + 8 * (i & 1), (i >> 1) & 1)) { atomicExch(error_word, 29); ok = false; }
+                    else {
+                        unsigned char* v = base + Q_BYTES + 2 * KV_BYTES + (i & 1) * KV_BYTES;
+                        for (int id = row; id < (BKV - first) * HALVES * 8; id += BQ) {
+                            const int chunk = id % 8, hb = id / 8 % HALVES, vr = first + id / (8 * HALVES);
+                            *reinterpret_cast<uint4*>(v + hb * (BKV * 128) + vr * 128 + chunk * 16) = make_uint4(0, 0, 0, 0);
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    }
                 }
             }
             tmem_wait_st();
@@ -284,6 +372,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_co
                 tmem_ld32(lane_addr + O_COL + c * 32, o);
                 tmem_wait_ld();
                 if (row < rows) {
+                    if (FORM == EXTENDED && terms.gate) {
+                        const __nv_bfloat162* grow = reinterpret_cast<const __nv_bfloat162*>(terms.gate + (size_t)(qs + r0 + row) * terms.gate_stride + h * D + c * 32);
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            const float2 gv = __bfloat1622float2(grow[e]);
+                            o[2 * e] = __float_as_uint(__fdividef(__uint_as_float(o[2 * e]), 1.f + fast_exp2(-LOG2E * gv.x)));
+                            o[2 * e + 1] = __float_as_uint(__fdividef(__uint_as_float(o[2 * e + 1]), 1.f + fast_exp2(-LOG2E * gv.y)));
+                        }
+                    }
 #pragma unroll
                     for (int v4 = 0; v4 < 4; ++v4) {
                         uint4 w;
@@ -323,31 +420,58 @@ bool cache_map(const void* cache, long long rows, int D, int ps, CUtensorMap* ou
 
 }  // namespace
 
-// tiles: (entry, first row) of 128-row tiles.  cache_rows = pages (with the null page) * KV * page_size.
-MI_EXPORT int mi_attn_prefill_tc(const void* q, int q_stride, int num_tokens, const void* k_cache, const void* v_cache,
-                                 long long cache_rows, void* out, const int* tiles, int num_tiles, const int* seg_q_start,
-                                 const int* seg_pos0, const int* block_table, const int* table_rows, int table_stride, int H,
-                                 int KV, int D, int ps, int tile_rows, float scale, int window, int* error_word, cudaStream_t stream) {
+template <int FORM>
+static int prefill_tc_launch(const void* q, int q_stride, int num_tokens, const void* k_cache, const void* v_cache,
+                             long long cache_rows, void* out, const int* tiles, int num_tiles, const int* seg_q_start,
+                             const int* seg_pos0, const int* block_table, const int* table_rows, int table_stride, int H,
+                             int KV, int D, int ps, int tile_rows, float scale, int window, int* error_word, const Terms& terms, cudaStream_t stream) {
     if (num_tiles == 0) return 0;
     if ((D != 64 && D != 128) || H % KV || tile_rows != BQ || q_stride % 8 || ps % 8 || BKV % ps || ((uintptr_t)q % 16)) return -2;
     CUtensorMap qmap, kmap, vmap;
     if (!sm100_host::make_map_bf16(&qmap, q, num_tokens, (uint64_t)H * D, q_stride, BQ, 64)) return -5;
     if (!cache_map(k_cache, cache_rows, D, ps, &kmap) || !cache_map(v_cache, cache_rows, D, ps, &vmap)) return -5;
     const size_t smem = (size_t)BQ * D * 2 + 4 * (size_t)BKV * D * 2 + 13 * 8 + 16 + 1024;
-    const float scale_log2 = scale * 1.4426950408889634f;
+    const float scale_log2 = scale * LOG2E;
     dim3 grid(H, num_tiles);
-#define LAUNCH(DD, IDX) do { \
+#define LAUNCH(DD) do { \
         static bool configured = false; \
         if (!configured) { \
-            cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<DD, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (e != cudaSuccess) return (int)e; \
             configured = true; \
         } \
-        return (int)launch_pdl(attn_prefill_tc_kernel<DD>, grid, dim3(ATT_THREADS), smem, stream, qmap, kmap, vmap, \
+        return (int)launch_pdl(attn_prefill_tc_kernel<DD, FORM>, grid, dim3(ATT_THREADS), smem, stream, qmap, kmap, vmap, \
                                (__nv_bfloat16*)out, tiles, seg_q_start, seg_pos0, block_table, table_rows, table_stride, H, KV, ps, \
-                               scale_log2, window, error_word); \
+                               scale_log2, window, error_word, terms); \
     } while (0)
-    if (D == 128) LAUNCH(128, 0);
-    LAUNCH(64, 1);
+    if (D == 128) LAUNCH(128);
+    LAUNCH(64);
 #undef LAUNCH
+}
+
+// tiles: (entry, first row) of 128-row tiles.  cache_rows = pages (with the null page) * KV * page_size.
+MI_EXPORT int mi_attn_prefill_tc(const void* q, int q_stride, int num_tokens, const void* k_cache, const void* v_cache,
+                                 long long cache_rows, void* out, const int* tiles, int num_tiles, const int* seg_q_start,
+                                 const int* seg_pos0, const int* block_table, const int* table_rows, int table_stride, int H,
+                                 int KV, int D, int ps, int tile_rows, float scale, int window, int* error_word, cudaStream_t stream) {
+    return prefill_tc_launch<PLAIN>(q, q_stride, num_tokens, k_cache, v_cache, cache_rows, out, tiles, num_tiles, seg_q_start, seg_pos0, block_table,
+                                    table_rows, table_stride, H, KV, D, ps, tile_rows, scale, window, error_word, Terms{}, stream);
+}
+
+// The forms with split weights.  sink_values [H] (null: score 0), bias_t [H, bias_last + 1] or null, slopes [H] or null; cap <= 0: none;
+// gate (4-byte aligned rows) or null.  A cap, kept keys or a gate exclude blocks, a sink and distance terms.
+MI_EXPORT int mi_attn_prefill_tc_split(const void* q, int q_stride, int num_tokens, const void* k_cache, const void* v_cache,
+                                       long long cache_rows, void* out, const int* tiles, int num_tiles, const int* seg_q_start,
+                                       const int* seg_pos0, const int* block_table, const int* table_rows, int table_stride, int H,
+                                       int KV, int D, int ps, int tile_rows, float scale, int window, int* error_word, int block, int sink,
+                                       const float* sink_values, const float* bias_t, int bias_last, const float* slopes, float cap, int keep,
+                                       const void* gate, int gate_stride, cudaStream_t stream) {
+    const Terms terms{block, sink, keep, bias_last, gate_stride, cap, sink_values, bias_t, slopes, (const __nv_bfloat16*)gate};
+    const bool extended = cap > 0.f || keep > 0 || gate, distances = bias_t || slopes;
+    if (extended && (block > 0 || sink || distances || (gate && ((uintptr_t)gate % 4 || gate_stride % 2)))) return -2;
+#define RUN(FORM) prefill_tc_launch<FORM>(q, q_stride, num_tokens, k_cache, v_cache, cache_rows, out, tiles, num_tiles, seg_q_start, seg_pos0, \
+                                          block_table, table_rows, table_stride, H, KV, D, ps, tile_rows, scale, window, error_word, terms, stream)
+    if (extended) return RUN(EXTENDED);
+    return distances ? RUN(BIASED) : RUN(MASKED);
+#undef RUN
 }

@@ -546,8 +546,8 @@ class CudaOps:
 
     def paged_attention(self, q, k_cache, v_cache, meta, H, KV, D, scale, window, split_weights=False):
         """split_weights: the tensor-core kernels take every softmax weight into the P V product as TWO bfloat16 numbers (its
-        rounding and the rest: 16 mantissa bits, float32 sums) instead of one; the tcgen05 prompt kernel, which has no such
-        form, is left out.  The float32 kernels behind them compute the weights in float32 anyway.
+        rounding and the rest: 16 mantissa bits, float32 sums) instead of one.  The float32 kernels behind them compute the
+        weights in float32 anyway.
         meta: the step's arrays for this cache group.  seg_q_start, seg_pos0, seg_kv_len per entry; decode_segs (entries
         that feed one token), prefill_tiles / prefill_tiles2 ((entry, first row) per tile of meta.tile / 2 * meta.tile query
         rows); block_table [rows, max_pages] with entry i reading row table_rows[i] (row i when table_rows is None)."""
@@ -562,8 +562,10 @@ class CudaOps:
         fast = (self.fast_attention and q.dtype == torch.bfloat16 and D in (64, 128) and q.stride(0) % 8 == 0
                 and q.data_ptr() % 16 == 0)
         tc = (fast and self.tc_attention and num_tiles and meta.tile == 64 and meta.page_size % 8 == 0
-              and 64 % meta.page_size == 0 and num_tiles2 and not split_weights)
-        if tc:
+              and 64 % meta.page_size == 0 and num_tiles2)
+        if tc and split_weights:
+            self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
+        elif tc:
             rc = self.lib.mi_attn_prefill_tc(
                 _p(q), q.stride(0), T, _p(k_cache), _p(v_cache), _c.c_longlong(k_cache.shape[0] * KV * meta.page_size),
                 _p(out), _p(tiles2), num_tiles2, _p(meta.seg_q_start), _p(meta.seg_pos0),
@@ -622,6 +624,17 @@ class CudaOps:
                 H, KV, D, meta.page_size, S, _c.c_float(scale), win, code, self._stream()), "attn_decode")
             self.launches += 2 if S > 1 else 1
         return out
+
+    def _prefill_tc_split(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias_t=None, bias_last=0,
+                          slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):
+        """The tcgen05 prompt kernel with split weights and the terms of masked_attention; bias_t [H, bias_last + 1]."""
+        _check(self.lib.mi_attn_prefill_tc_split(
+            _p(q), q.stride(0), q.shape[0], _p(k_cache), _p(v_cache), _c.c_longlong(k_cache.shape[0] * KV * meta.page_size), _p(out),
+            _p(meta.prefill_tiles2), meta.prefill_tiles2.shape[0], _p(meta.seg_q_start), _p(meta.seg_pos0), _p(meta.block_table),
+            _p(getattr(meta, "table_rows", None)), meta.max_pages, H, KV, D, meta.page_size, 128, _c.c_float(scale), window, _p(self._stream_error),
+            block, sink, _p(sink_values), _p(bias_t), bias_last, _p(slopes), _c.c_float(cap), keep, _p(gate), gate_stride, self._stream()),
+            "attn_prefill_tc_split")
+        self.launches += 1
 
     def _f32_tiles(self, q, D, V, meta):
         """Whether the float32 prompt attention with tiles takes these rows: heads of 64 or 128 that start on 16 bytes, tiles of 64 rows."""
@@ -929,7 +942,17 @@ class CudaOps:
             assert sink_values is None or (sink and sink_values.dtype == torch.float32 and sink_values.numel() == H)
             assert distance_bias is None or (distance_bias.dtype == torch.float32 and distance_bias.is_contiguous() and distance_bias.shape[1] == H)
         bias_last = 0 if distance_bias is None else distance_bias.shape[0] - 1
-        if (num_tiles and tc_ext and self.fast_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
+        tiles2 = getattr(meta, "prefill_tiles2", None)
+        # heads of 64 or 128, pages that divide a tile of 64 keys into TMA boxes of at least 8 rows: the tcgen05 kernel (2,048 tokens, 16 heads of
+        # 128: 149 us on the mma.sync kernel); other page sizes keep the mma.sync forms, other heads the float32 kernels
+        tc = (num_tiles and self.fast_attention and self.tc_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
+              and tiles2 is not None and tiles2.shape[0] and meta.page_size % 8 == 0 and 64 % meta.page_size == 0 and tc_form
+              and (plain or self.biased_attention_tc) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
+        if tc:
+            bias_t = None if distance_bias is None and distance_bias_by_head is None else self._bias_rows_by_head(distance_bias, distance_bias_by_head)
+            self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, blk, win, int(bool(sink)), sink_values, bias_t,
+                                   0 if bias_t is None else bias_t.shape[1] - 1, slopes, cap, keep, gate, gate_stride)
+        elif (num_tiles and tc_ext and self.fast_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
                 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0):
             _check(self.lib.mi_attn_prefill_mma_capped(
                 _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),

@@ -49,6 +49,10 @@ def test_prompt_attention_forms(ops, dtype, H, KV, D, page, form):      # noqa: 
     g = torch.Generator().manual_seed(1)
     q = torch.randn(T, (H + 1) * D, generator=g).to(dtype).to(DEV)[:, :H * D]           # rows of a wider tensor
     k, v = (torch.randn(121, KV, page, D, generator=g).to(dtype).to(DEV) for _ in range(2))
+    for i, (pos0, n) in enumerate(segs[:4]):                    # what a page holds behind a prompt's last key must not matter
+        last = pos0 + n - 1
+        page_id = meta.block_table[meta.rows[i], last // page].long()
+        k[page_id, :, last % page + 1:], v[page_id, :, last % page + 1:] = float("nan"), float("inf")
     args = form_arguments(form, H, D, T, dtype)
     got = ops.masked_attention(q, k, v, meta, H, KV, D, D, D ** -0.5, **args)
     ops.check_errors()
