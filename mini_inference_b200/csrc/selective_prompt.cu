@@ -1,0 +1,200 @@
+// Selective state-space scan for steps that bring prompt portions: per channel c and state n, token by token,
+//     S[c, n] <- exp(step_c A[c, n]) S[c, n] + step_c x_c B_n;   y_c = sum_n S[c, n] C_n + D_c x_c;   out = y * silu(z),
+// step = softplus(dt + dt_b).  All float32; the slot's first I N floats are S.
+//
+// Instruction issue bounds it: per token, channel and state one exponential and four more operations, 134 M of each for 2,048 tokens x
+// 4,096 channels x 16 states.  Only the update itself is a chain from token to token.  Eight lanes share a channel and hold
+// two states each in one packed pair (N = 16), so 4,096 channels are 1,024 warps, two per scheduler; exponentials run on the
+// FMA pipe, two at a time.  A block is 32 channels: eight warps walk the tokens, eight more make the next chunk of 32 tokens ready (steps, inputs, B, C to
+// shared memory) and finish the previous one (skip term, gate, store), so neither softplus nor a load is waited for; one barrier a chunk.
+// Eight tokens' partial sums are added up over the eight lanes together (seven shuffles instead of 24).  2,048 tokens: 541 -> 141 us.  The kernel in
+// which all warps do everything in turn (recurrent.cu) stays for decode steps, where there is one token a request, and for other N.
+#include "common.cuh"
+#include <math.h>
+
+using namespace mi;
+
+namespace {
+
+constexpr int TC = 32, CB = 32, HELPERS = 256;
+
+// e^v of two numbers at once for v <= 0: n = round(v / ln 2), e^v = 2^n e^(v - n ln 2), the second factor as 1 + f + f^2 P(f) with P of degree
+// 3 fitted to (e^f - 1 - f) / f^2 on |f| <= ln 2 / 2.  The largest relative error is 1.1e-7 at |f| = ln 2 / 2 and falls with f^2 towards
+// 1, where a decay acts hundreds of times in a row (ex2.approx is 2 ulp off there and the states' error was three times as large).
+__device__ __forceinline__ float2 exp_neg2(float2 v) {
+    v = make_float2(fmaxf(v.x, -87.f), fmaxf(v.y, -87.f));
+    const float2 big = make_float2(12582912.f, 12582912.f);        // 1.5 * 2^23: the sum's low bits are the rounded integer
+    const float2 t = __ffma2_rn(v, make_float2(1.4426950408889634f, 1.4426950408889634f), big);
+    const float2 n = __fadd2_rn(t, make_float2(-12582912.f, -12582912.f));
+    const float2 f = __ffma2_rn(n, make_float2(-0.69314718055994531f, -0.69314718055994531f), v);
+    float2 p = make_float2(0.0083124945f, 0.0083124945f);
+    p = __ffma2_rn(p, f, make_float2(0.041890331f, 0.041890331f));
+    p = __ffma2_rn(p, f, make_float2(0.16667116f, 0.16667116f));
+    p = __ffma2_rn(p, f, make_float2(0.49999231f, 0.49999231f));
+    const float2 one = make_float2(1.f, 1.f);
+    p = __ffma2_rn(__ffma2_rn(p, f, one), f, one);
+    return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)), __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
+}
+
+// z / (1 + e^-z); fast forms (a few units in the last place of float32) where the result is rounded to bfloat16
+template <typename T> __device__ __forceinline__ float silu_for(float z) { return z / (1.f + expf(-z)); }
+template <> __device__ __forceinline__ float silu_for<__nv_bfloat16>(float z) { return __fdividef(z, 1.f + __expf(-z)); }
+
+// grid (entries, ceil(I / 32)); L lanes of NS states each, N = L NS
+template <typename T, int L, int NS>
+__global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
+    const T* __restrict__ x, const float* __restrict__ dt, const float* __restrict__ dt_b, const float* __restrict__ A,
+    const T* __restrict__ B, int ldb, const T* __restrict__ Cm, int ldc, const float* __restrict__ Dv, const T* __restrict__ z, int ldz,
+    float* __restrict__ state, long long state_stride, T* __restrict__ out, const int* __restrict__ seg_q_start,
+    const int* __restrict__ seg_slot, int I) {
+    constexpr int N = L * NS;
+    __shared__ __align__(16) float Bs[2][TC][N], Cs[2][TC][N], ys[2][TC][CB];
+    __shared__ __align__(16) float2 in[2][TC][CB];                  // step, step * x
+    const int seg = blockIdx.x, qs = seg_q_start[seg], n = seg_q_start[seg + 1] - qs, c0 = blockIdx.y * CB;
+    const int chunks = (n + TC - 1) / TC;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp >= L) {
+        // ---------------- helpers: a warp takes 32 channels of a token; what an iteration works on was requested an iteration earlier
+        const int ht = threadIdx.x - CB * L, hw = ht >> 5, cc = c0 + lane;
+        const bool live = cc < I;
+        const float bias = live ? dt_b[cc] : 0.f, skip = live ? Dv[cc] : 0.f;
+        constexpr int HW = HELPERS / 32, R = TC / HW, RB = (TC * N + HELPERS - 1) / HELPERS;
+        float rs[R];
+        T rx[R], rB[RB], rC[RB], fx[R], fz[R];
+        auto request = [&](int k) {                                 // chunk k for making ready, chunk k - 2 for finishing
+            const int ta = k * TC, tb = ta - 2 * TC;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int tt = hw + HW * r;
+                if (live && ta + tt < n) {
+                    rs[r] = dt[(size_t)(qs + ta + tt) * I + cc];
+                    rx[r] = x[(size_t)(qs + ta + tt) * I + cc];
+                }
+                if (live && tb >= 0 && tb + tt < n) {
+                    fx[r] = x[(size_t)(qs + tb + tt) * I + cc];
+                    fz[r] = z[(size_t)(qs + tb + tt) * ldz + cc];
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RB; ++r) {
+                const int i = ht + HELPERS * r, tt = i / N, nn = i % N;
+                if (tt < TC && ta + tt < n) {
+                    rB[r] = B[(size_t)(qs + ta + tt) * ldb + nn];
+                    rC[r] = Cm[(size_t)(qs + ta + tt) * ldc + nn];
+                }
+            }
+        };
+        request(0);
+        for (int k = -1; k <= chunks; ++k) {                        // makes chunk k + 1 ready, finishes chunk k - 1
+            if (k >= 0) __syncthreads();
+            const int ta = (k + 1) * TC, tb = (k - 1) * TC, b = (k + 1) & 1;        // chunks k - 1 and k + 1 use the same buffers
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const int tt = hw + HW * r;
+                if (live && tb >= 0 && tb + tt < n) {
+                    const float xv = to_f32(fx[r]), zv = to_f32(fz[r]);
+                    out[(size_t)(qs + tb + tt) * I + cc] = from_f32<T>((ys[b][tt][lane] + skip * xv) * silu_for<T>(zv));
+                }
+            }
+            if (ta < n) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {                       // tokens behind the entry's last: a step of 0 changes no state
+                    const int tt = hw + HW * r;
+                    float2 v = make_float2(0.f, 0.f);
+                    if (live && ta + tt < n) {
+                        const float d = rs[r] + bias;
+                        v.x = d > 20.f ? d : log1pf(expf(d));
+                        v.y = v.x * to_f32(rx[r]);
+                    }
+                    in[b][tt][lane] = v;
+                }
+#pragma unroll
+                for (int r = 0; r < RB; ++r) {
+                    const int i = ht + HELPERS * r, tt = i / N, nn = i % N;
+                    if (tt < TC) {
+                        const bool ok = ta + tt < n;
+                        Bs[b][tt][nn] = ok ? to_f32(rB[r]) : 0.f;
+                        Cs[b][tt][nn] = ok ? to_f32(rC[r]) : 0.f;
+                    }
+                }
+            }
+            request(k + 2);
+        }
+        return;
+    }
+    // ---------------- the scan: lane l of L holds the states NS l .. NS l + NS - 1
+    constexpr int CW = 32 / L;                                      // channels of a warp
+    const int l = lane % L, cl = warp * CW + lane / L, c = c0 + cl;
+    const bool live = c < I;
+    float* S = state + (long long)seg_slot[seg] * state_stride + (size_t)(live ? c : 0) * N + l * NS;
+    float2 s[NS / 2], a[NS / 2];
+#pragma unroll
+    for (int g = 0; g < NS / 2; ++g) {
+        s[g] = a[g] = make_float2(0.f, 0.f);
+        if (live) {
+            s[g] = make_float2(S[2 * g], S[2 * g + 1]);
+            const float* ar = A + (size_t)c * N + l * NS + 2 * g;
+            a[g] = make_float2(ar[0], ar[1]);
+        }
+    }
+    for (int k = 0; k <= chunks; ++k) {
+        __syncthreads();
+        if (k == chunks) break;                                     // the helpers finish the last chunk
+        const int b = k & 1;
+#pragma unroll 1
+        for (int t0 = 0; t0 < TC; t0 += L) {
+            float y[L];
+            float2 decay[L][NS / 2];                                // not part of the chain from token to token: made side by side
+#pragma unroll
+            for (int e = 0; e < L; ++e) {
+                const float step = in[b][t0 + e][cl].x;
+#pragma unroll
+                for (int g = 0; g < NS / 2; ++g) decay[e][g] = exp_neg2(__fmul2_rn(make_float2(step, step), a[g]));
+            }
+#pragma unroll
+            for (int e = 0; e < L; ++e) {
+                const float sx = in[b][t0 + e][cl].y;
+                float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int g = 0; g < NS / 2; ++g) {
+                    const float2 bv = *reinterpret_cast<const float2*>(&Bs[b][t0 + e][l * NS + 2 * g]);
+                    const float2 cv = *reinterpret_cast<const float2*>(&Cs[b][t0 + e][l * NS + 2 * g]);
+                    s[g] = __ffma2_rn(decay[e][g], s[g], __fmul2_rn(make_float2(sx, sx), bv));
+                    sum = __ffma2_rn(s[g], cv, sum);
+                }
+                y[e] = sum.x + sum.y;
+            }
+            // L sums over L lanes together: half of what is left changes hands at every step, lane l ends with token t0 + l
+#pragma unroll
+            for (int w = 1; w < L; w <<= 1)
+#pragma unroll
+                for (int e = 0; e < L; e += 2 * w) {
+                    const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
+                    y[e] = (l & w ? y[e + w] : y[e]) + got;
+                }
+            ys[b][t0 + l][cl] = y[0];
+        }
+    }
+    if (live) {
+#pragma unroll
+        for (int g = 0; g < NS / 2; ++g) { S[2 * g] = s[g].x; S[2 * g + 1] = s[g].y; }
+    }
+}
+
+}  // namespace
+
+// x [T, I] and out [T, I] contiguous in the run's type; dt float32 [T, I] (before bias and softplus); B, C, z: strided views; A float32
+// [I, N], N one of 8, 16, 32.
+MI_EXPORT int mi_selective_prompt(const void* x, const float* dt, const float* dt_b, const float* A, const void* B, int ldb, const void* C, int ldc,
+                                  const float* Dv, const void* z, int ldz, float* state, long long state_stride, void* out,
+                                  const int* seg_q_start, const int* seg_slot, int num_segs, int I, int N, int dtype, cudaStream_t stream) {
+    if (num_segs == 0 || I == 0) return 0;
+    const dim3 grid(num_segs, (I + CB - 1) / CB);
+#define GO(T, L, NS) selective_prompt_kernel<T, L, NS><<<grid, CB * L + HELPERS, 0, stream>>>((const T*)x, dt, dt_b, A, (const T*)B, ldb, (const T*)C, ldc, Dv, \
+                                                                              (const T*)z, ldz, state, state_stride, (T*)out, seg_q_start, seg_slot, I)
+#define PICK(T) do { if (N == 16) GO(T, 8, 2); else if (N == 8) GO(T, 4, 2); else if (N == 32) GO(T, 8, 4); else return -2; } while (0)
+    if (dtype == MI_BF16) PICK(__nv_bfloat16); else PICK(float);
+#undef PICK
+#undef GO
+    return (int)cudaGetLastError();
+}
