@@ -1337,6 +1337,13 @@ class CudaOps:
             dt = dt.float()
         assert dt.is_contiguous()
         out = torch.empty((T, I), dtype=out_dtype, device=x.device)
+        if T > batch.num_segs and N in (8, 16, 32):          # a step with prompt portions (one token a request: the kernel below)
+            _check(self.lib.mi_selective_prompt(
+                _p(x), _p(dt), _p(dt_b), _p(A), _p(B), B.stride(0), _p(C), C.stride(0), _p(Dv), _p(z), z.stride(0), _p(state),
+                _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, I, N, _code(x.dtype),
+                self._stream()), "selective_prompt")
+            self.launches += 1
+            return out
         _check(self.lib.mi_selective_scan(_p(x), _p(dt), _p(dt_b), _p(A), _p(B), B.stride(0), _p(C), C.stride(0), _p(Dv), _p(z), z.stride(0),
                                           _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), T,
                                           batch.num_segs, I, N, _code(x.dtype), self._stream()), "selective_scan")
