@@ -26,7 +26,7 @@ def load_library():
         from .build import build
         path = build()
         _LIB = ctypes.CDLL(path)
-        _LIB.mi_gemm_f32_workspace.restype = ctypes.c_longlong
+        _LIB.mi_gemm_f32_workspace.restype = _LIB.mi_octet_floats.restype = ctypes.c_longlong
     return _LIB
 
 
@@ -706,12 +706,29 @@ class CudaOps:
         return y
 
     # ---------------------------------------------------------------- matrix-state recurrences
+    @staticmethod
+    def _takes_octets(rows, batch, D, V, state):
+        """Whether a step's recurrence goes eight tokens at a time (csrc/state_octets.cu): steps with prompts, keys of 64 or 128, values in blocks
+        of 16 columns, states of an even number of floats, rows whose heads start on 16 bytes."""
+        return (rows.shape[0] > 4 * batch.num_segs and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
+                and rows.stride(0) % 4 == 0 and rows.data_ptr() % 16 == 0)
+
+    def _octet_scratch(self, T, batch, H, D, V, delta):
+        return torch.empty(self.lib.mi_octet_floats(T, batch.num_segs, H, D, V, int(delta)), dtype=torch.float32, device=self.device)
+
     def lightning_scan(self, p, H, D, V, decay, state, batch):
         """p [T, >= 2 H D + H V] = q | k | v before silu; state float32 [slots, H D V] (an entry continues from its slot's
         state and leaves the new one there).  Returns float32 [T, H V]."""
         T = p.shape[0]
         assert p.stride(1) == 1 and state.dtype == torch.float32 and state.is_contiguous()
         out = torch.empty((T, H * V), dtype=torch.float32, device=p.device)
+        if self._takes_octets(p, batch, D, V, state):
+            scratch = self._octet_scratch(T, batch, H, D, V, False)
+            _check(self.lib.mi_lightning_octets(_p(p), p.stride(0), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
+                                                _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error),
+                                                _code(p.dtype), self._stream()), "lightning_octets")
+            self.launches += 2
+            return out
         prep = torch.empty((T, 2 * H * D + H * V), dtype=torch.float32, device=p.device)      # silu(q | k | v), what the scan stages
         _check(self.lib.mi_lightning_scan(_p(p), p.stride(0), _p(prep), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
                                           _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _code(p.dtype),
@@ -740,6 +757,12 @@ class CudaOps:
         """S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q per head, token by token.  float32 [T, H V]."""
         T = prep.shape[0]
         out = torch.empty((T, H * V), dtype=torch.float32, device=prep.device)
+        if self._takes_octets(prep, batch, D, V, state):
+            scratch = self._octet_scratch(T, batch, H, D, V, True)
+            _check(self.lib.mi_delta_octets(_p(prep), prep.stride(0), _p(scratch), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
+                                            _p(batch.seg_slot), T, batch.num_segs, H, KV, D, V, _p(self._stream_error), self._stream()), "delta_octets")
+            self.launches += 2
+            return out
         _check(self.lib.mi_delta_scan(_p(prep), prep.stride(0), _p(state), _c.c_longlong(state.stride(0)), _p(out),
                                       _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, KV, D, V, self._stream()),
                "delta_scan")
