@@ -15,7 +15,9 @@
 // are made together, lane l ends with sum l; u goes around through shared memory.  One more warp brings the records by bulk copies into
 // a ring, two octets at a time: a head's records lie one behind the other, and so do its values of the block's columns.  (A record
 // and a row of values per token took the copying thread 480 ns for four tokens, whatever the compute warps did.)
-// MEASURED
+// Scan with its octet_kernel, 16 heads of 128 x 128: 2,048 tokens 556 -> 237 us (delta), 291 -> 164 us (constant, silu included); 1,300 + 517 + 231
+// tokens 539 -> 248 and 282 -> 164 us; 16 x 64 tokens 216 -> 107 and 117 -> 75 us.  One warp a scheduler issues every 2.4 clocks: what is left
+// is the latency of one warp's own instructions.
 #include "sm100.cuh"
 #include <math.h>
 
@@ -25,7 +27,7 @@ using namespace mi::sm100;
 namespace {
 
 constexpr int C = 8, NC = 4, WARPS = 4, COLS = NC * WARPS;      // tokens at a time; columns of a warp, warps and columns of a block
-constexpr int GROUP = 2, STAGES = 3, SCALARS = 2 * C * C + C + 8;      // octets per copy;      // N [8][8] | B [8][8] | beta [8] | d^8 - 1 | unused
+constexpr int GROUP = 1, STAGES = 6, SCALARS = 2 * C * C + C + 8;      // octets per copy, copies in flight; N [8][8] | B [8][8] | beta [8] | d^8 - 1 | unused
 constexpr int B_OFF = C * C, BETA_OFF = 2 * C * C, D8_OFF = BETA_OFF + C;
 
 template <bool DELTA> __host__ __device__ constexpr int vectors() { return DELTA ? 3 * C + 1 : 2 * C; }
@@ -109,13 +111,18 @@ __global__ void __launch_bounds__(128) octet_kernel(const T* __restrict__ in, co
             if (!ok) { q[i][r] = k[i][r] = 0.f; g[i][r] = 1.f; }
         }
     }
-    for (int c = 2 * lane; c < V; c += 64)                          // values: [head][column block][slot][8][COLS] float32
+    for (int c = 2 * lane; c < V; c += 64) {                        // values: [head][column block][slot][8][COLS] float32, zeros behind the last token
+        float t[C][2];
+#pragma unroll
         for (int i = 0; i < C; ++i) {
-            float t[2] = {0.f, 0.f};
-            if (t0 + i < n) load_n<2>(in + (size_t)(qs + t0 + i) * L.ld + L.v + h * V + c, t);
-            if (!DELTA) { t[0] = silu(t[0]); t[1] = silu(t[1]); }
-            *reinterpret_cast<float2*>(v_out + ((((size_t)h * (V / COLS) + c / COLS) * gridDim.x + slot) * C + i) * COLS + c % COLS) = make_float2(t[0], t[1]);
+            t[i][0] = t[i][1] = 0.f;
+            if (t0 + i < n) load_n<2>(in + (size_t)(qs + t0 + i) * L.ld + L.v + h * V + c, t[i]);
         }
+        float* to = v_out + (((size_t)h * (V / COLS) + c / COLS) * gridDim.x + slot) * C * COLS + c % COLS;
+#pragma unroll
+        for (int i = 0; i < C; ++i)
+            *reinterpret_cast<float2*>(to + i * COLS) = DELTA ? make_float2(t[i][0], t[i][1]) : make_float2(silu(t[i][0]), silu(t[i][1]));
+    }
     float* o = rec + ((size_t)h * gridDim.x + slot) * record_floats<DELTA>(D);
     float* kd = o;                                                  // DELTA: k_i G_i
     float* qd = o + (DELTA ? C * D : 0);
@@ -173,9 +180,9 @@ __global__ void __launch_bounds__(128) octet_kernel(const T* __restrict__ in, co
     }
 }
 
-// grid (entries, heads, V / COLS); WARPS compute warps and one that copies
+// grid (V / COLS, heads, entries); WARPS compute warps and one that copies
 template <bool DELTA, int D>
-__global__ void __launch_bounds__(32 * WARPS + 32, 1) scan_kernel(const float* __restrict__ rec, const float* __restrict__ v, int slots, float* __restrict__ state,
+__global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(const float* __restrict__ rec, const float* __restrict__ v, int slots, float* __restrict__ state,
                                                                   long long state_stride, float* __restrict__ out, const int* __restrict__ seg_q_start,
                                                                   const int* __restrict__ seg_slot, int H, int V, int* __restrict__ error_word) {
     constexpr int RF = record_floats<DELTA>(D), STAGE = GROUP * (RF + C * COLS), R = D / 32, RP = R / 2, NV = C * NC;
@@ -184,7 +191,7 @@ __global__ void __launch_bounds__(32 * WARPS + 32, 1) scan_kernel(const float* _
     float* around = sm + STAGES * STAGE;                            // [2][WARPS][C][NC]: w (delta), two octets in turn
     uint64_t* bars = reinterpret_cast<uint64_t*>(around + 2 * WARPS * NV);
     const uint32_t full = smem_u32(bars), empty = smem_u32(bars + STAGES);
-    const int seg = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * COLS;
+    const int seg = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * COLS;
     const int qs = seg_q_start[seg], n = seg_q_start[seg + 1] - qs, octets = (n + C - 1) / C;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -196,7 +203,7 @@ __global__ void __launch_bounds__(32 * WARPS + 32, 1) scan_kernel(const float* _
         // ---------------- copies: GROUP octets' records, and their tokens' COLS values each
         if (lane == 0) {
             const float* src = rec + ((size_t)h * slots + first_slot(qs, seg)) * RF;
-            const float* vs = v + (((size_t)h * (V / COLS) + blockIdx.z) * slots + first_slot(qs, seg)) * C * COLS;
+            const float* vs = v + (((size_t)h * (V / COLS) + blockIdx.x) * slots + first_slot(qs, seg)) * C * COLS;
             for (int k = 0; k < octets; k += GROUP) {
                 const int turn = k / GROUP, s = turn % STAGES, m = min(GROUP, octets - k);
                 if (turn >= STAGES && !mbar_wait(empty + 8 * s, (turn / STAGES - 1) & 1)) { atomicExch(error_word, 41); break; }
@@ -350,7 +357,7 @@ int run_scan(const float* rec, const float* values, int slots, float* state, lon
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    scan_kernel<DELTA, D><<<dim3(num_segs, H, V / COLS), 32 * WARPS + 32, bytes, stream>>>(rec, values, slots, state, state_stride, out, seg_q_start, seg_slot,
+    scan_kernel<DELTA, D><<<dim3(V / COLS, H, num_segs), 32 * WARPS + 32, bytes, stream>>>(rec, values, slots, state, state_stride, out, seg_q_start, seg_slot,
                                                                                         H, V, error_word);
     return (int)cudaGetLastError();
 }
@@ -359,7 +366,7 @@ template <typename T, bool DELTA>
 int run(const T* in, const Source& L, const float* decay, float* rec, float* values, float* state, long long state_stride, float* out,
         const int* seg_q_start, const int* seg_slot, int T_, int num_segs, int H, int KV, int D, int V, int* error_word, cudaStream_t stream) {
     if (num_segs == 0 || T_ == 0) return 0;
-    if ((D != 64 && D != 128) || V % COLS || H > 65535 || H % KV || state_stride % 2 || (uintptr_t)state % 8) return -2;
+    if ((D != 64 && D != 128) || V % COLS || H > 65535 || num_segs > 65535 || H % KV || state_stride % 2 || (uintptr_t)state % 8) return -2;
     if (L.ld % 4 || (uintptr_t)in % 16 || (uintptr_t)values % 16 || (uintptr_t)rec % 16) return -2;       // every head starts on a multiple of 16 entries
     const int slots = T_ / C + num_segs;
     const dim3 ogrid(slots, (H + 3) / 4);

@@ -64,3 +64,81 @@ def test_prompt_attention_forms(ops, dtype, H, KV, D, page, form):      # noqa: 
     # float32: sums of up to 365 products in another order.  bfloat16: the output's own rounding, half of 2^-8 of the value, may fall differently
     err, limit = (got.float() - want.float()).abs().max().item(), want.float().abs().max().item()
     assert err < (4e-6 if dtype == torch.float32 else 2 ** -8) * limit, (form, err / limit)
+
+
+class Entries:
+    """A step's entries as the recurrences see them."""
+
+    def __init__(self, lens):
+        q = [0]
+        for n in lens:
+            q.append(q[-1] + n)
+        self.num_segs = len(lens)
+        self.seg_q_start = torch.tensor(q, dtype=torch.int32, device=DEV)
+        self.seg_slot = torch.arange(len(lens), 0, -1, dtype=torch.int32, device=DEV)
+
+
+def rows_error(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+@pytest.mark.parametrize("lens", [(9, 1, 8, 40), (129,), (7, 63), (15, 1, 1, 16)])
+@pytest.mark.parametrize("H,KV,D,V", [(4, 2, 128, 48), (3, 3, 64, 32), (5, 1, 128, 128)])
+def test_recurrences_eight_tokens_at_a_time(ops, lens, H, KV, D, V):        # noqa: F811
+    """The delta rule with channel decays and the constant decay against their token-by-token kernels: whole octets, remainders, single tokens
+    beside prompts, decays down to 0, states that start non-zero, slots out of order."""
+    T, batch, g = sum(lens), Entries(lens), torch.Generator().manual_seed(sum(lens) + D)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
+    C = 2 * KV * D + H * V
+    prep = torch.zeros(T, (C + H * D + H + 3) // 4 * 4, device=DEV)
+    qk = r(T, 2 * KV, D)
+    prep[:, :2 * KV * D] = (qk / qk.norm(dim=-1, keepdim=True)).reshape(T, -1)
+    prep[:, 2 * KV * D:C] = r(T, H * V)
+    decay = torch.rand(T, H * D, generator=g).to(DEV) ** 0.2
+    decay[:, ::7], decay[:, 1::7] = 1.0, 0.0
+    prep[:, C:C + H * D] = decay
+    prep[:, C + H * D:C + H * D + H] = torch.rand(T, H, generator=g).to(DEV)
+    state = r(len(lens) + 1, H * D * V + 6)
+    p = r(T, 2 * H * D + H * V + 8).to(torch.bfloat16)
+    constant = torch.tensor([1.0 - 2.0 ** -(1 + 2 * h) for h in range(H)], device=DEV)
+    runs = {"delta": lambda s: ops.delta_scan(prep, H, KV, D, V, s, batch), "constant": lambda s: ops.lightning_scan(p, H, D, V, constant, s, batch)}
+    for name, run in runs.items():
+        a, b = state.clone(), state.clone()
+        taken = ops._takes_octets
+        assert taken(prep, batch, D, V, a) == (T > 4 * len(lens))
+        got = run(a)
+        ops._takes_octets = lambda *args: False
+        try:
+            want = run(b)
+        finally:
+            del ops._takes_octets
+        ops.check_errors()
+        # two float32 orders of sums over up to 129 tokens and 128 rows
+        assert rows_error(got, want) < 3e-6 and rows_error(a, b) < 3e-6, name
+        assert torch.equal(a[:, H * D * V:], state[:, H * D * V:]) and torch.equal(a[0], state[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,inner,N", [((33, 1, 64), 40, 16), ((5, 100), 96, 8), ((31, 2), 33, 32), ((70,), 64, 16)])
+def test_selective_scan_of_prompts(ops, dtype, lens, inner, N):         # noqa: F811
+    """Chunks of 32 tokens and channels with remainders, against the same tokens one at a time (decode steps take the other kernel)."""
+    T, g = sum(lens), torch.Generator().manual_seed(sum(lens))
+    r = lambda *s: torch.randn(*s, generator=g)                 # noqa: E731
+    x, z, B, C = (r(T, w).to(dtype).to(DEV) for w in (inner, inner, N, N))
+    dt, dt_b, Dv = r(T, inner).to(DEV), r(inner).to(DEV), r(inner).to(DEV)
+    A = -torch.exp(r(inner, N)).to(DEV)
+    A[:, 0] = -300.0                                             # a decay of e^-87 and less is 0
+    state = r(len(lens) + 1, inner * N + 4).to(DEV)
+    a, b = state.clone(), state.clone()
+    batch = Entries(lens)
+    got = ops.selective_scan(x, dt, dt_b, A, B, C, Dv, z, a, batch, dtype)
+    want = torch.empty_like(got)
+    starts = batch.seg_q_start.tolist()
+    for i, n in enumerate(lens):
+        one = Entries((1,))
+        one.seg_slot = batch.seg_slot[i:i + 1]
+        for t in range(starts[i], starts[i] + n):
+            row = slice(t, t + 1)
+            want[row] = ops.selective_scan(x[row].contiguous(), dt[row].contiguous(), dt_b, A, B[row], C[row], Dv, z[row], b, one, dtype)
+    assert rows_error(a, b) < 3e-6
+    assert rows_error(got, want) < (3e-6 if dtype == torch.float32 else 4e-3)        # bfloat16: the output's own rounding may fall differently
