@@ -436,6 +436,92 @@ __global__ void delta_prepare_kernel(const T* __restrict__ p, int ldp, const T* 
     }
 }
 
+// The same for prompts whose heads have up to 128 entries in whole quads: a warp takes a unit of eight neighbouring tokens, four channels a
+// lane (8- or 16-byte loads and stores), its taps in registers, every sum inside the warp.  What bounds it is the float32 rows written; 2,048
+// tokens of 16 heads: MEASURED (the kernel above reads and computes every q and k entry twice, an entry a thread, with two
+// block-wide barriers a token).
+template <typename T> __device__ __forceinline__ float4 quad_at(const T* p) {
+    if constexpr (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
+    else {
+        const uint2 t = *reinterpret_cast<const uint2*>(p);
+        return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u), __uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
+    }
+}
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(128) delta_prepare_warp_kernel(const T* __restrict__ p, int ldp, const T* __restrict__ a, int lda,
+                                     const float* __restrict__ conv, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
+                                     const float* __restrict__ state, long long state_stride, long long hist_off,
+                                     float* __restrict__ out, int ldo, const int* __restrict__ token_seg,
+                                     const int* __restrict__ seg_q_start, const int* __restrict__ seg_slot,
+                                     int H, int KV, int D, int V, float unit_eps, int T_) {
+    constexpr int TOKS = 8;
+    const int unit = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, t0 = blockIdx.x * TOKS;
+    const int C = 2 * KV * D + H * V, toks = min(TOKS, T_ - t0);
+    if (unit > 2 * KV + 2 * H) return;
+    if (unit == 2 * KV + 2 * H) {                                   // beta
+        for (int i = lane; i < toks * H; i += 32) {
+            const size_t t = t0 + i / H;
+            out[t * ldo + C + H * D + i % H] = sigmoidf(to_f32(p[t * ldp + C + i % H]));
+        }
+        return;
+    }
+    if (unit >= 2 * KV + H) {                                       // decays
+        const int hh = unit - 2 * KV - H, d = 4 * lane;
+        if (d >= D) return;
+        const float rate = expf(A_log[hh]);
+        const float4 b = *reinterpret_cast<const float4*>(dt_bias + hh * D + d);
+        float4 x[TOKS];
+#pragma unroll
+        for (int k = 0; k < TOKS; ++k) if (k < toks) x[k] = quad_at<T>(a + (size_t)(t0 + k) * lda + hh * D + d);
+        auto g = [&](float v) { const float sp = v > 20.f ? v : log1pf(expf(v)); return expf(-rate * sp); };
+#pragma unroll
+        for (int k = 0; k < TOKS; ++k)
+            if (k < toks)
+                *reinterpret_cast<float4*>(out + (size_t)(t0 + k) * ldo + C + hh * D + d) = make_float4(g(x[k].x + b.x), g(x[k].y + b.y), g(x[k].z + b.z), g(x[k].w + b.w));
+        return;
+    }
+    const bool is_v = unit >= 2 * KV;
+    const int n = is_v ? V : D, c = (is_v ? 2 * KV * D + (unit - 2 * KV) * V : unit * D) + 4 * lane;
+    const bool live = 4 * lane < n;
+    float w[4][TAPS];
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) w[e][j] = live ? conv[(size_t)(c + e) * TAPS + j] : 0.f;
+    // the tokens' rows and the TAPS - 1 before them, whatever entry those belong to: requested together
+    float4 x[TOKS + TAPS - 1];
+#pragma unroll
+    for (int i = 0; i < TOKS + TAPS - 1; ++i) {
+        const int t = t0 - (TAPS - 1) + i;
+        x[i] = live && t >= 0 && t < T_ ? quad_at<T>(p + (size_t)t * ldp + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float scale = unit < KV ? rsqrtf((float)D) : 1.f;
+#pragma unroll
+    for (int k = 0; k < TOKS; ++k) {
+        if (k >= toks) break;
+        const int seg = token_seg[t0 + k], r = t0 + k - seg_q_start[seg];
+        float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {
+            float4 v = x[k + j];
+            const int off = r - (TAPS - 1 - j);
+            if (off < 0) {                                          // before the entry's first token: the slot's inputs
+                if (live) {
+                    const float* hist = state + (long long)seg_slot[seg] * state_stride + hist_off + (size_t)(TAPS - 1 + off) * C + c;
+                    v = make_float4(hist[0], hist[1], hist[2], hist[3]);
+                }
+            }
+            y.x = fmaf(w[0][j], v.x, y.x); y.y = fmaf(w[1][j], v.y, y.y); y.z = fmaf(w[2][j], v.z, y.z); y.w = fmaf(w[3][j], v.w, y.w);
+        }
+        y = make_float4(silu(y.x), silu(y.y), silu(y.z), silu(y.w));
+        if (!is_v) {
+            const float inv = 1.f / sqrtf(warp_sum(live ? y.x * y.x + y.y * y.y + y.z * y.z + y.w * y.w : 0.f) + unit_eps) * scale;
+            y = make_float4(y.x * inv, y.y * inv, y.z * inv, y.w * inv);
+        }
+        if (live) *reinterpret_cast<float4*>(out + (size_t)(t0 + k) * ldo + c) = y;
+    }
+}
+
 // hist[j] <- input at (entry's end - (taps - 1) + j), j = 0 .. taps - 2; a thread owns a channel and goes up in j, so an
 // entry shorter than taps - 1 shifts its own rows safely.
 template <typename T>
@@ -502,21 +588,17 @@ __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int l
         qs_[k] = seg_q_start[seg];
         slot_[k] = seg_slot[seg];
     }
-    // the block's weights pass through shared memory: read from w in order, then each thread takes its own 8 TAPS numbers
-    // (rows of 8 TAPS + 1 floats keep the threads on different banks)
-    constexpr int ROW = 8 * TAPS + 1;
-    __shared__ float wsm[256 * ROW];
-    const int cb = blockIdx.y * blockDim.x * 8;                                   // the block's first channel
-    const int mine = min((int)blockDim.x * 8, C - cb) * TAPS;
-    for (int i = threadIdx.x; i < mine; i += blockDim.x) wsm[(i / (8 * TAPS)) * ROW + i % (8 * TAPS)] = w[(size_t)cb * TAPS + i];
-    __syncthreads();
-    const int c = cb + threadIdx.x * 8;
+    // a thread's 8 TAPS weights are neighbours: 16-byte loads that a warp's lanes use whole lines of (staged through shared memory behind a
+    // barrier, once per eight tokens, they were most of the kernel's time: 2,048 tokens x 4,096 channels 40 us)
+    const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
     if (c >= C) return;
     float wreg[8][TAPS], breg[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
+    for (int i = 0; i < 2 * TAPS; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(w + (size_t)c * TAPS + 4 * i);
+        const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) wreg[e][j] = wsm[threadIdx.x * ROW + e * TAPS + j];
+        for (int e = 0; e < 4; ++e) wreg[(4 * i + e) / TAPS][(4 * i + e) % TAPS] = f[e];
     }
     if (bias) {
         const float4 a = *reinterpret_cast<const float4*>(bias + c), b = *reinterpret_cast<const float4*>(bias + c + 4);
@@ -965,7 +1047,18 @@ MI_EXPORT int mi_delta_prepare(const void* p, int ldp, const void* a, int lda, c
     if (units > 65535) return -2;
     const int toks = T_ >= 1024 ? 8 : 1;
     dim3 pgrid((T_ + toks - 1) / toks, units);
-    if (dtype == MI_BF16)
+    const int el = dtype == MI_BF16 ? 2 : 4;
+    const bool warps = T_ >= 64 && taps >= 2 && taps <= 4 && D % 4 == 0 && V % 4 == 0 && D <= 128 && V <= 128 && ldp % 4 == 0 && lda % 4 == 0 && ldo % 4 == 0 &&
+                       ((uintptr_t)p | (uintptr_t)a) % (4 * el) == 0 && ((uintptr_t)out | (uintptr_t)dt_bias) % 16 == 0;
+    if (warps) {
+        const dim3 wgrid((T_ + 7) / 8, (units + 3) / 4);
+#define GO(T, TAPS) delta_prepare_warp_kernel<T, TAPS><<<wgrid, 128, 0, stream>>>((const T*)p, ldp, (const T*)a, lda, conv, A_log, dt_bias, state, state_stride, \
+                                                                                 hist_off, out, ldo, token_seg, seg_q_start, seg_slot, H, KV, D, V, unit_eps, T_)
+#define PICK(T) do { if (taps == 2) GO(T, 2); else if (taps == 3) GO(T, 3); else GO(T, 4); } while (0)
+        if (dtype == MI_BF16) PICK(__nv_bfloat16); else PICK(float);
+#undef PICK
+#undef GO
+    } else if (dtype == MI_BF16)
         delta_prepare_kernel<__nv_bfloat16><<<pgrid, 128, 0, stream>>>((const __nv_bfloat16*)p, ldp, (const __nv_bfloat16*)a, lda, conv, A_log, dt_bias,
                                                                        state, state_stride, hist_off, out, ldo, token_seg, seg_q_start, seg_slot,
                                                                        H, KV, D, V, taps, unit_eps, T_, toks);
@@ -992,7 +1085,7 @@ MI_EXPORT int mi_short_conv(const void* h, int ldh, const float* w, const float*
     const int shift = (T_ == num_segs && T_ < 256) ? 1 : 0;      // a step of single tokens: one kernel filters and moves the slot's inputs
     // prompt portions only: a decode step's few tokens are done sooner by the kernel that needs no staging of weights
     const bool vec = dtype == MI_BF16 && T_ >= 256 && taps >= 1 && taps <= 4 && C % 8 == 0 && ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)out % 16 == 0 &&
-                     (taps == 1 || (state_stride % 4 == 0 && hist_off % 4 == 0 && (uintptr_t)state % 16 == 0)) && (!bias || (uintptr_t)bias % 16 == 0);
+                     (taps == 1 || (state_stride % 4 == 0 && hist_off % 4 == 0 && (uintptr_t)state % 16 == 0)) && (uintptr_t)w % 16 == 0 && (!bias || (uintptr_t)bias % 16 == 0);
     if (vec) {
         const int tok = T_ >= 1024 ? 8 : 2, threads = min(256, (C / 8 + 31) / 32 * 32);
         dim3 vgrid((T_ + tok - 1) / tok, (C / 8 + threads - 1) / threads);

@@ -707,6 +707,12 @@ class CudaOps:
 
     # ---------------------------------------------------------------- matrix-state recurrences
     @staticmethod
+    def _takes_step(T, batch, D, V, state):
+        """Whether a step's recurrence has a whole state in a block's registers (csrc/state_step.cu): one token per entry, sizes of 64 or 128,
+        states on 16 bytes."""
+        return T == batch.num_segs and D in (64, 128) and V in (64, 128) and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0
+
+    @staticmethod
     def _takes_octets(rows, batch, D, V, state):
         """Whether a step's recurrence goes eight tokens at a time (csrc/state_octets.cu): steps with prompts, keys of 64 or 128, values in blocks
         of 16 columns, states of an even number of floats, rows whose heads start on 16 bytes."""
@@ -722,6 +728,11 @@ class CudaOps:
         T = p.shape[0]
         assert p.stride(1) == 1 and state.dtype == torch.float32 and state.is_contiguous()
         out = torch.empty((T, H * V), dtype=torch.float32, device=p.device)
+        if self._takes_step(T, batch, D, V, state):
+            _check(self.lib.mi_lightning_step(_p(p), p.stride(0), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
+                                              _p(batch.seg_slot), T, H, D, V, _code(p.dtype), self._stream()), "lightning_step")
+            self.launches += 1
+            return out
         if self._takes_octets(p, batch, D, V, state):
             scratch = self._octet_scratch(T, batch, H, D, V, False)
             _check(self.lib.mi_lightning_octets(_p(p), p.stride(0), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
@@ -757,6 +768,11 @@ class CudaOps:
         """S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q per head, token by token.  float32 [T, H V]."""
         T = prep.shape[0]
         out = torch.empty((T, H * V), dtype=torch.float32, device=prep.device)
+        if self._takes_step(T, batch, D, V, state):
+            _check(self.lib.mi_delta_step(_p(prep), prep.stride(0), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
+                                          _p(batch.seg_slot), T, H, KV, D, V, self._stream()), "delta_step")
+            self.launches += 1
+            return out
         if self._takes_octets(prep, batch, D, V, state):
             scratch = self._octet_scratch(T, batch, H, D, V, True)
             _check(self.lib.mi_delta_octets(_p(prep), prep.stride(0), _p(scratch), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
