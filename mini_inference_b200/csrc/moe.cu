@@ -119,12 +119,26 @@ __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) route_topk_kernel(const
     float* sc = hs + (size_t)TOK * hidden;             // [TOK][3][EA]: logits -> scores, choice scores, group scratch
     const int t0 = blockIdx.x * TOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int nt = min(TOK, T_ - t0);
-    for (int i = threadIdx.x; i < TOK * hidden; i += blockDim.x) {
-        const int tk = i / hidden, c = i % hidden;
-        hs[i] = tk < nt ? to_f32(h[(size_t)(t0 + tk) * ldh + c]) : 0.f;
+    const bool vec = hidden % 4 == 0 && ((uintptr_t)router % 16) == 0;
+    constexpr int VN = Vec16<T>::N;
+    if (hidden % VN == 0 && ldh % VN == 0 && (uintptr_t)h % 16 == 0) {        // rows in 16-byte pieces, a token's all at once
+#pragma unroll
+        for (int tk = 0; tk < TOK; ++tk)
+            for (int c = threadIdx.x * VN; c < hidden; c += blockDim.x * VN) {
+                float v[VN];
+#pragma unroll
+                for (int e = 0; e < VN; ++e) v[e] = 0.f;
+                if (tk < nt) load16(h + (size_t)(t0 + tk) * ldh + c, v);
+#pragma unroll
+                for (int e = 0; e < VN; e += 4) *reinterpret_cast<float4*>(hs + (size_t)tk * hidden + c + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+            }
+    } else {
+        for (int i = threadIdx.x; i < TOK * hidden; i += blockDim.x) {
+            const int tk = i / hidden, c = i % hidden;
+            hs[i] = tk < nt ? to_f32(h[(size_t)(t0 + tk) * ldh + c]) : 0.f;
+        }
     }
     __syncthreads();
-    const bool vec = hidden % 4 == 0 && ((uintptr_t)router % 16) == 0;
     if (TOK == 8 && vec) {
         // four experts at a time: a token's entries are read from shared memory once for the four (a 16-byte load of a warp takes four
         // clocks of that memory's pipe, four multiply-adds one each: with an expert at a time the loads were the bound).  The 32

@@ -495,11 +495,16 @@ __global__ void __launch_bounds__(128) delta_prepare_warp_kernel(const T* __rest
         const int t = t0 - (TAPS - 1) + i;
         x[i] = live && t >= 0 && t < T_ ? quad_at<T>(p + (size_t)t * ldp + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
+    int seg_[TOKS], first_[TOKS];                                   // looked up together as well
+#pragma unroll
+    for (int k = 0; k < TOKS; ++k) seg_[k] = token_seg[min(t0 + k, T_ - 1)];
+#pragma unroll
+    for (int k = 0; k < TOKS; ++k) first_[k] = seg_q_start[seg_[k]];
     const float scale = unit < KV ? rsqrtf((float)D) : 1.f;
 #pragma unroll
     for (int k = 0; k < TOKS; ++k) {
         if (k >= toks) break;
-        const int seg = token_seg[t0 + k], r = t0 + k - seg_q_start[seg];
+        const int seg = seg_[k], r = t0 + k - first_[k];
         float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < TAPS; ++j) {
@@ -573,6 +578,7 @@ __global__ void short_conv_kernel(const T* __restrict__ h, int ldh, const float*
 
 // The same for bfloat16 rows whose channels come in multiples of eight: a thread owns eight channels (16-byte loads and stores), keeps
 // their TAPS weights in registers and walks TOK neighbouring tokens (each looks its own entry up: an entry may end between them).
+// silu with the fast exponential and quotient (a few units in the last place of float32): the result is rounded to bfloat16
 template <int TAPS, int TOK>
 __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int ldh, const float* __restrict__ w, const float* __restrict__ bias,
                                       const float* __restrict__ state, long long state_stride, long long hist_off, __nv_bfloat16* __restrict__ out,
@@ -625,7 +631,7 @@ __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int l
                 acc[e] = breg[e];
 #pragma unroll
                 for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wreg[e][j], entry(k + j, e), acc[e]);
-                if (act == 1) acc[e] = silu(acc[e]);
+                if (act == 1) acc[e] = __fdividef(acc[e], 1.f + __expf(-acc[e]));
                 if (residual) acc[e] += entry(k + TAPS - 1, e);
             }
             uint4 o;
@@ -665,7 +671,7 @@ __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int l
         __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            if (act == 1) acc[e] = silu(acc[e]);
+            if (act == 1) acc[e] = __fdividef(acc[e], 1.f + __expf(-acc[e]));
             if (residual) acc[e] += x[e];                    // x holds the last tap's input: the token's own
         }
 #pragma unroll
@@ -1048,7 +1054,7 @@ MI_EXPORT int mi_delta_prepare(const void* p, int ldp, const void* a, int lda, c
     const int toks = T_ >= 1024 ? 8 : 1;
     dim3 pgrid((T_ + toks - 1) / toks, units);
     const int el = dtype == MI_BF16 ? 2 : 4;
-    const bool warps = T_ >= 64 && taps >= 2 && taps <= 4 && D % 4 == 0 && V % 4 == 0 && D <= 128 && V <= 128 && ldp % 4 == 0 && lda % 4 == 0 && ldo % 4 == 0 &&
+    const bool warps = T_ > num_segs && T_ >= 64 && taps >= 2 && taps <= 4 && D % 4 == 0 && V % 4 == 0 && D <= 128 && V <= 128 && ldp % 4 == 0 && lda % 4 == 0 && ldo % 4 == 0 &&
                        ((uintptr_t)p | (uintptr_t)a) % (4 * el) == 0 && ((uintptr_t)out | (uintptr_t)dt_bias) % 16 == 0;
     if (warps) {
         const dim3 wgrid((T_ + 7) / 8, (units + 3) / 4);
@@ -1087,11 +1093,11 @@ MI_EXPORT int mi_short_conv(const void* h, int ldh, const float* w, const float*
     const bool vec = dtype == MI_BF16 && T_ >= 256 && taps >= 1 && taps <= 4 && C % 8 == 0 && ldh % 8 == 0 && (uintptr_t)h % 16 == 0 && (uintptr_t)out % 16 == 0 &&
                      (taps == 1 || (state_stride % 4 == 0 && hist_off % 4 == 0 && (uintptr_t)state % 16 == 0)) && (uintptr_t)w % 16 == 0 && (!bias || (uintptr_t)bias % 16 == 0);
     if (vec) {
-        const int tok = T_ >= 1024 ? 8 : 2, threads = min(256, (C / 8 + 31) / 32 * 32);
+        const int tok = T_ >= 1024 ? 4 : 2, threads = min(128, (C / 8 + 31) / 32 * 32);
         dim3 vgrid((T_ + tok - 1) / tok, (C / 8 + threads - 1) / threads);
 #define GO(TAPS, TOK) short_conv_vec_kernel<TAPS, TOK><<<vgrid, threads, 0, stream>>>((const __nv_bfloat16*)h, ldh, w, bias, state, state_stride, hist_off, \
                           (__nv_bfloat16*)out, token_seg, seg_q_start, seg_slot, T_, C, residual, act)
-#define PICK(TAPS) do { if (tok == 8) GO(TAPS, 8); else GO(TAPS, 2); } while (0)
+#define PICK(TAPS) do { if (tok == 4) GO(TAPS, 4); else GO(TAPS, 2); } while (0)
         if (taps == 1) PICK(1); else if (taps == 2) PICK(2); else if (taps == 3) PICK(3); else PICK(4);
 #undef PICK
 #undef GO

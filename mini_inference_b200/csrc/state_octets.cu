@@ -13,7 +13,7 @@
 // shared memory once per four columns.  A 16-byte load of a warp takes the shared-memory pipe four clocks even where lanes read the same
 // words, so with 8 lanes to a pair of columns the loads were 65 % of that pipe's time.  The 32 sums over lanes (eight tokens, four columns)
 // are made together, lane l ends with sum l; u goes around through shared memory.  One more warp brings the records by bulk copies into
-// a ring, two octets at a time: a head's records lie one behind the other, and so do its values of the block's columns.  (A record
+// a ring: a head's records lie one behind the other, and so do its values of the block's columns, so an octet is two copies.  (A record
 // and a row of values per token took the copying thread 480 ns for four tokens, whatever the compute warps did.)
 // Scan with its octet_kernel, 16 heads of 128 x 128: 2,048 tokens 556 -> 237 us (delta), 291 -> 164 us (constant, silu included); 1,300 + 517 + 231
 // tokens 539 -> 248 and 282 -> 164 us; 16 x 64 tokens 216 -> 107 and 117 -> 75 us.  One warp a scheduler issues every 2.4 clocks: what is left
@@ -27,7 +27,7 @@ using namespace mi::sm100;
 namespace {
 
 constexpr int C = 8, NC = 4, WARPS = 4, COLS = NC * WARPS;      // tokens at a time; columns of a warp, warps and columns of a block
-constexpr int GROUP = 1, STAGES = 6, SCALARS = 2 * C * C + C + 8;      // octets per copy, copies in flight; N [8][8] | B [8][8] | beta [8] | d^8 - 1 | unused
+constexpr int STAGES = 6, SCALARS = 2 * C * C + C + 8;      // N [8][8] | B [8][8] | beta [8] | d^8 - 1 | unused
 constexpr int B_OFF = C * C, BETA_OFF = 2 * C * C, D8_OFF = BETA_OFF + C;
 
 template <bool DELTA> __host__ __device__ constexpr int vectors() { return DELTA ? 3 * C + 1 : 2 * C; }
@@ -185,7 +185,7 @@ template <bool DELTA, int D>
 __global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(const float* __restrict__ rec, const float* __restrict__ v, int slots, float* __restrict__ state,
                                                                   long long state_stride, float* __restrict__ out, const int* __restrict__ seg_q_start,
                                                                   const int* __restrict__ seg_slot, int H, int V, int* __restrict__ error_word) {
-    constexpr int RF = record_floats<DELTA>(D), STAGE = GROUP * (RF + C * COLS), R = D / 32, RP = R / 2, NV = C * NC;
+    constexpr int RF = record_floats<DELTA>(D), STAGE = RF + C * COLS, R = D / 32, RP = R / 2, NV = C * NC;
     static_assert(NV == 32, "a lane per sum");
     extern __shared__ __align__(128) float sm[];
     float* around = sm + STAGES * STAGE;                            // [2][WARPS][C][NC]: w (delta), two octets in turn
@@ -200,17 +200,17 @@ __global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(co
     }
     __syncthreads();
     if (warp == WARPS) {
-        // ---------------- copies: GROUP octets' records, and their tokens' COLS values each
+        // ---------------- copies: an octet's record, and its values of the block's columns
         if (lane == 0) {
             const float* src = rec + ((size_t)h * slots + first_slot(qs, seg)) * RF;
             const float* vs = v + (((size_t)h * (V / COLS) + blockIdx.x) * slots + first_slot(qs, seg)) * C * COLS;
-            for (int k = 0; k < octets; k += GROUP) {
-                const int turn = k / GROUP, s = turn % STAGES, m = min(GROUP, octets - k);
-                if (turn >= STAGES && !mbar_wait(empty + 8 * s, (turn / STAGES - 1) & 1)) { atomicExch(error_word, 41); break; }
-                const uint32_t dst = smem_u32(sm + s * STAGE);
-                mbar_expect_tx(full + 8 * s, m * (RF + C * COLS) * 4);
-                bulk_load(dst, src + (size_t)k * RF, m * RF * 4, full + 8 * s);
-                bulk_load(dst + GROUP * RF * 4, vs + (size_t)k * C * COLS, m * C * COLS * 4, full + 8 * s);
+            for (int k = 0; k < octets; ++k) {
+                const int st = k % STAGES;
+                if (k >= STAGES && !mbar_wait(empty + 8 * st, (k / STAGES - 1) & 1)) { atomicExch(error_word, 41); break; }
+                const uint32_t dst = smem_u32(sm + st * STAGE);
+                mbar_expect_tx(full + 8 * st, STAGE * 4);
+                bulk_load(dst, src + (size_t)k * RF, RF * 4, full + 8 * st);
+                bulk_load(dst + RF * 4, vs + (size_t)k * C * COLS, C * COLS * 4, full + 8 * st);
             }
         }
         return;
@@ -249,18 +249,20 @@ __global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(co
                 y[i * NC + c] = a.x + a.y;
             }
     };
+    bool there = false;                                             // the next record was there when this one was begun
     for (int k = 0; k < octets; ++k) {
-        const int turn = k / GROUP, j = k % GROUP, st = turn % STAGES;
-        if (j == 0 && !mbar_spin(full + 8 * st, (turn / STAGES) & 1)) { if (lane == 0) atomicExch(error_word, 42); break; }
-        const float* r = sm + st * STAGE + j * RF + R * lane;
-        const float* sc = sm + st * STAGE + j * RF + vectors<DELTA>() * D;
-        const float* vv = sm + st * STAGE + GROUP * RF + j * C * COLS + cw;
+        const int st = k % STAGES, st1 = (k + 1) % STAGES;
+        if (!there && !mbar_spin(full + 8 * st, (k / STAGES) & 1)) { if (lane == 0) atomicExch(error_word, 42); break; }
+        const float* r = sm + st * STAGE + R * lane;
+        const float* sc = sm + st * STAGE + vectors<DELTA>() * D;
+        const float* vv = sm + st * STAGE + RF + cw;
         float2 x[C][RP], xq[C][RP], u[C][NC / 2];                    // u[i][c / 2]: two columns
         float z[NV], own[C];                                         // own: u of this lane's column
         if constexpr (DELTA) {
             float2 dec[RP];
             fetch(x, r, 0);
             fetch(xq, r, C);
+            there = k + 1 < octets && mbar_test(full + 8 * st1, ((k + 1) / STAGES) & 1);
             float y[NV];
             dots(x, y);
             fetch(x, r, 2 * C);
@@ -303,6 +305,7 @@ __global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(co
         } else {
             fetch(xq, r, 0);
             fetch(x, r, C);
+            there = k + 1 < octets && mbar_test(full + 8 * st1, ((k + 1) / STAGES) & 1);
             const float d8 = sc[D8_OFF];                             // d^8 - 1
 #pragma unroll
             for (int i = 0; i < C; ++i) {
@@ -333,10 +336,8 @@ __global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(co
         o = fmaf(b0.w, own[3], o) + o2;
         if (C * k + my_i < n) *out_at = o;
         out_at += (size_t)C * H * V;
-        if (j == GROUP - 1) {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(empty + 8 * st);
-        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + 8 * st);
     }
 #pragma unroll
     for (int p = 0; p < RP; ++p)
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(32 * WARPS + 32, DELTA ? 2 : 3) scan_kernel(co
 template <bool DELTA, int D>
 int run_scan(const float* rec, const float* values, int slots, float* state, long long state_stride, float* out, const int* seg_q_start, const int* seg_slot,
              int num_segs, int H, int V, int* error_word, cudaStream_t stream) {
-    constexpr int bytes = (STAGES * GROUP * (record_floats<DELTA>(D) + C * COLS) + 2 * WARPS * C * NC) * 4 + 2 * STAGES * 8;
+    constexpr int bytes = (STAGES * (record_floats<DELTA>(D) + C * COLS) + 2 * WARPS * C * NC) * 4 + 2 * STAGES * 8;
     static bool configured = false;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(scan_kernel<DELTA, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
