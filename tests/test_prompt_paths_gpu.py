@@ -142,3 +142,33 @@ def test_selective_scan_of_prompts(ops, dtype, lens, inner, N):         # noqa: 
             want[row] = ops.selective_scan(x[row].contiguous(), dt[row].contiguous(), dt_b, A, B[row], C[row], Dv, z[row], b, one, dtype)
     assert rows_error(a, b) < 3e-6
     assert rows_error(got, want) < (3e-6 if dtype == torch.float32 else 4e-3)        # bfloat16: the output's own rounding may fall differently
+
+
+@pytest.mark.parametrize("H,KV,D", [(16, 8, 128), (3, 1, 64), (5, 5, 128)])
+@pytest.mark.parametrize("form", ["unit", "weights_rotated", "all_rotated", "temperature_keys", "blend", "plain"])
+def test_unit_heads_of_prompts(ops, H, KV, D, form):            # noqa: F811
+    """Normed, rotated and cached heads of 300 tokens at once, against the same tokens in pieces that the other kernel takes."""
+    T, page, g = 300, 16, torch.Generator().manual_seed(H + D)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
+    keys = form == "temperature_keys"
+    p = r(T, (H + KV) * D + (0 if keys else KV * D)).to(torch.bfloat16)
+    qw, kw = (r(D).abs() + 0.5 for _ in range(2))
+    freq = torch.rand(D // 2, generator=g).to(DEV) * 0.1
+    args = {"unit": {}, "plain": {}, "weights_rotated": dict(q_weight=qw, k_weight=kw, inv_freq=freq[:D // 4].contiguous()), "all_rotated": dict(inv_freq=freq),
+            "temperature_keys": dict(q_weight=qw, k_weight=kw, q_temp=(0.1, 64), values_are_keys=True), "blend": {}}[form]
+    source = r(T, 2 * KV * D).to(torch.bfloat16)[:, KV * D:] if form == "blend" else None
+    lam = torch.tensor([0.3], device=DEV) if form == "blend" else None
+    slots = torch.randperm(T, generator=g).to(torch.int32).to(DEV) + page
+    positions = torch.arange(7, 7 + T, dtype=torch.int32, device=DEV)
+    results = []
+    for piece in (T, 100):
+        rows, k = p.clone(), torch.zeros((T + page) // page + 2, KV, page, D, dtype=torch.bfloat16, device=DEV)
+        v = torch.zeros_like(k)
+        for a in range(0, T, piece):
+            meta = type("Meta", (), dict(slots=slots[a:a + piece].contiguous(), positions=positions[a:a + piece].contiguous(), page_size=page))
+            part = rows[a:a + piece]
+            ops.unit_qk_cache(part, H, KV, D, D, None if form == "plain" else 1e-6, lam, None if source is None else source[a:a + piece], meta, k, v, **args)
+        results.append((rows, k, v))
+    for a, b in zip(*results):                                  # one bfloat16 rounding of values that differ in their last float32 bits
+        assert (a.float() - b.float()).abs().max().item() <= 2 ** -8 * b.float().abs().max().item()
+        assert (a != b).float().mean().item() < 1e-2
