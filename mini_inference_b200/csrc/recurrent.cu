@@ -1020,20 +1020,24 @@ MI_EXPORT int mi_lightning_scan(const void* p, int ldp, float* prep, const float
     return launch_scan<0>(prep, L, decay, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H, D, V, stream);
 }
 
-// p [T, ldp] = q | k | v as projected; inv_freq: half frequencies (nullptr or half = 0: no rotation).  Otherwise as mi_lightning_scan.
-MI_EXPORT int mi_retention_scan(const void* p, int ldp, float* prep, const int* positions, const float* inv_freq, int half, float k_scale,
-                                const float* decay, float* state, long long state_stride, float* out, const int* seg_q_start,
-                                const int* seg_slot, int T_, int num_segs, int H, int D, int V, int dtype, cudaStream_t stream) {
-    if (num_segs == 0 || T_ == 0) return 0;
+// out [T, 2 H D + H V] float32 = q | k | v of p [T, ldp] as the recurrence takes them: q and k rotated (inv_freq: half frequencies; nullptr or
+// half = 0: not), k times k_scale
+MI_EXPORT int mi_retention_rows(const void* p, int ldp, float* out, const int* positions, const float* inv_freq, int half, float k_scale, int T_, int H, int D,
+                                int V, int dtype, cudaStream_t stream) {
+    if (T_ == 0) return 0;
     if (2 * half > D) return -2;
     const int n = 2 * H * D + H * V;
     dim3 pgrid(T_, T_ >= 256 ? 1 : min(8, (n + 255) / 256));
-    if (dtype == MI_BF16) rotate_f32_kernel<__nv_bfloat16><<<pgrid, 256, 0, stream>>>((const __nv_bfloat16*)p, ldp, prep, positions, inv_freq, inv_freq ? half : 0, k_scale, H, D, V);
-    else rotate_f32_kernel<float><<<pgrid, 256, 0, stream>>>((const float*)p, ldp, prep, positions, inv_freq, inv_freq ? half : 0, k_scale, H, D, V);
-    int err = (int)cudaGetLastError();
-    if (err) return err;
-    ScanLayout L{n, 0, H * D, 2 * H * D, 0, 0, 0, 0};
-    return launch_scan<0>(prep, L, decay, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H, D, V, stream);
+    if (dtype == MI_BF16) rotate_f32_kernel<__nv_bfloat16><<<pgrid, 256, 0, stream>>>((const __nv_bfloat16*)p, ldp, out, positions, inv_freq, inv_freq ? half : 0, k_scale, H, D, V);
+    else rotate_f32_kernel<float><<<pgrid, 256, 0, stream>>>((const float*)p, ldp, out, positions, inv_freq, inv_freq ? half : 0, k_scale, H, D, V);
+    return (int)cudaGetLastError();
+}
+
+// rows [T, 2 H D + H V] float32 as mi_retention_rows leaves them; out float32 [T, H V]
+MI_EXPORT int mi_retention_scan(const float* rows, const float* decay, float* state, long long state_stride, float* out, const int* seg_q_start,
+                                const int* seg_slot, int T_, int num_segs, int H, int D, int V, cudaStream_t stream) {
+    const ScanLayout L{2 * H * D + H * V, 0, H * D, 2 * H * D, 0, 0, 0, 0};
+    return launch_scan<0>(rows, L, decay, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H, D, V, stream);
 }
 
 MI_EXPORT int mi_delta_scan(const float* prep, int ld, float* state, long long state_stride, float* out, const int* seg_q_start,

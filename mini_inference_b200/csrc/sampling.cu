@@ -84,11 +84,17 @@ __global__ void sample_split_kernel(const float* __restrict__ logits, int ld, in
     const uint32_t seed = draw ? seeds[r] : 0u, counter = draw ? counters[r] : 0u;
     unsigned long long key = 0;
     const int base = blockIdx.y * NT * PER_THREAD;
+    float vals[PER_THREAD];                              // fetched together: between the branches below each load waited for the one before
+#pragma unroll
+    for (int k = 0; k < PER_THREAD; ++k) {
+        const int i = base + k * NT + threadIdx.x;
+        vals[k] = i < vocab ? row[i] : 0.f;
+    }
 #pragma unroll
     for (int k = 0; k < PER_THREAD; ++k) {
         const int i = base + k * NT + threadIdx.x;
         if (i < vocab) {
-            float v = row[i];
+            float v = vals[k];
             if (draw) v = v * inv_t + gumbel(seed, counter, (uint32_t)i);
             const unsigned long long cand = score_key(v, i);
             key = cand > key ? cand : key;
@@ -120,7 +126,7 @@ MI_EXPORT int mi_sample_split(const float* logits, int ld, int rows, int vocab, 
                               const uint32_t* seeds, const uint32_t* counters, int* out,
                               unsigned long long* slots, int* arrivals, cudaStream_t stream) {
     if (rows == 0) return 0;
-    constexpr int NT = 256, PER = 16;
+    constexpr int NT = 256, PER = 8;
     const int chunks = (vocab + NT * PER - 1) / (NT * PER);
     return (int)mi::launch_pdl(sample_split_kernel<NT, PER>, dim3(rows, chunks), dim3(NT), 0, stream, logits, ld, vocab,
                                temps, seeds, counters, out, slots, arrivals);

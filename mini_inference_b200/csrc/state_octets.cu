@@ -83,7 +83,7 @@ struct Source {                 // where a token's numbers are: q, k, g (+ head 
 };
 
 // grid (slots, heads / 4), 4 warps: a warp owns one octet of one head.  DELTA: in is the float32 prologue's rows; else the rows as projected.
-template <typename T, bool DELTA, int D>
+template <typename T, bool DELTA, bool SILU, int D>
 __global__ void __launch_bounds__(128) octet_kernel(const T* __restrict__ in, const Source L, const float* __restrict__ decay, float* __restrict__ rec,
                                                    float* __restrict__ v_out, const int* __restrict__ seg_q_start, int num_segs, int H, int KV, int V) {
     constexpr int R = D / 32;                                       // neighbouring rows a lane owns
@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(128) octet_kernel(const T* __restrict__ in, co
         if (DELTA) load_n<R>(row + L.g + h * D + lane * R, g[i]);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            if (!DELTA) { q[i][r] = silu(q[i][r]); k[i][r] = silu(k[i][r]); g[i][r] = d1; }
+            if (SILU) { q[i][r] = silu(q[i][r]); k[i][r] = silu(k[i][r]); }
+            if (!DELTA) g[i][r] = d1;
             if (!ok) { q[i][r] = k[i][r] = 0.f; g[i][r] = 1.f; }
         }
     }
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(128) octet_kernel(const T* __restrict__ in, co
         float* to = v_out + (((size_t)h * (V / COLS) + c / COLS) * gridDim.x + slot) * C * COLS + c % COLS;
 #pragma unroll
         for (int i = 0; i < C; ++i)
-            *reinterpret_cast<float2*>(to + i * COLS) = DELTA ? make_float2(t[i][0], t[i][1]) : make_float2(silu(t[i][0]), silu(t[i][1]));
+            *reinterpret_cast<float2*>(to + i * COLS) = SILU ? make_float2(silu(t[i][0]), silu(t[i][1])) : make_float2(t[i][0], t[i][1]);
     }
     float* o = rec + ((size_t)h * gridDim.x + slot) * record_floats<DELTA>(D);
     float* kd = o;                                                  // DELTA: k_i G_i
@@ -364,7 +365,7 @@ int run_scan(const float* rec, const float* values, int slots, float* state, lon
     return (int)cudaGetLastError();
 }
 
-template <typename T, bool DELTA>
+template <typename T, bool DELTA, bool SILU>
 int run(const T* in, const Source& L, const float* decay, float* rec, float* values, float* state, long long state_stride, float* out,
         const int* seg_q_start, const int* seg_slot, int T_, int num_segs, int H, int KV, int D, int V, int* error_word, cudaStream_t stream) {
     if (num_segs == 0 || T_ == 0) return 0;
@@ -372,8 +373,8 @@ int run(const T* in, const Source& L, const float* decay, float* rec, float* val
     if (L.ld % 4 || (uintptr_t)in % 16 || (uintptr_t)values % 16 || (uintptr_t)rec % 16) return -2;       // every head starts on a multiple of 16 entries
     const int slots = T_ / C + num_segs;
     const dim3 ogrid(slots, (H + 3) / 4);
-    if (D == 128) octet_kernel<T, DELTA, 128><<<ogrid, 128, 0, stream>>>(in, L, decay, rec, values, seg_q_start, num_segs, H, KV, V);
-    else octet_kernel<T, DELTA, 64><<<ogrid, 128, 0, stream>>>(in, L, decay, rec, values, seg_q_start, num_segs, H, KV, V);
+    if (D == 128) octet_kernel<T, DELTA, SILU, 128><<<ogrid, 128, 0, stream>>>(in, L, decay, rec, values, seg_q_start, num_segs, H, KV, V);
+    else octet_kernel<T, DELTA, SILU, 64><<<ogrid, 128, 0, stream>>>(in, L, decay, rec, values, seg_q_start, num_segs, H, KV, V);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
     if (D == 128) return run_scan<DELTA, 128>(rec, values, slots, state, state_stride, out, seg_q_start, seg_slot, num_segs, H, V, error_word, stream);
@@ -392,8 +393,16 @@ MI_EXPORT int mi_delta_octets(const float* prep, int ld, float* scratch, float* 
                               const int* seg_slot, int T_, int num_segs, int H, int KV, int D, int V, int* error_word, cudaStream_t stream) {
     const int channels = 2 * KV * D + H * V;
     float* values = scratch + (size_t)(T_ / C + num_segs) * H * record_floats<true>(D);
-    return run<float, true>(prep, Source{ld, 0, KV * D, 2 * KV * D, channels, channels + H * D}, nullptr, scratch, values, state, state_stride, out, seg_q_start,
+    return run<float, true, false>(prep, Source{ld, 0, KV * D, 2 * KV * D, channels, channels + H * D}, nullptr, scratch, values, state, state_stride, out, seg_q_start,
                             seg_slot, T_, num_segs, H, KV, D, V, error_word, stream);
+}
+
+// rows [T, 2 H D + H V] float32 = q | k | v as they enter the recurrence; decay [H]; otherwise as mi_delta_octets
+MI_EXPORT int mi_constant_octets(const float* rows, float* scratch, const float* decay, float* state, long long state_stride, float* out, const int* seg_q_start,
+                                 const int* seg_slot, int T_, int num_segs, int H, int D, int V, int* error_word, cudaStream_t stream) {
+    float* values = scratch + (size_t)(T_ / C + num_segs) * H * record_floats<false>(D);
+    return run<float, false, false>(rows, Source{2 * H * D + H * V, 0, H * D, 2 * H * D, 0, 0}, decay, scratch, values, state, state_stride, out, seg_q_start,
+                                    seg_slot, T_, num_segs, H, H, D, V, error_word, stream);
 }
 
 // p [T, ldp] = q | k | v before silu; decay [H]; otherwise as mi_delta_octets
@@ -403,8 +412,8 @@ MI_EXPORT int mi_lightning_octets(const void* p, int ldp, float* scratch, const 
     const Source L{ldp, 0, H * D, 2 * H * D, 0, 0};
     float* values = scratch + (size_t)(T_ / C + num_segs) * H * record_floats<false>(D);
     if (dtype == MI_BF16)
-        return run<__nv_bfloat16, false>((const __nv_bfloat16*)p, L, decay, scratch, values, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H,
+        return run<__nv_bfloat16, false, true>((const __nv_bfloat16*)p, L, decay, scratch, values, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H,
                                          D, V, error_word, stream);
-    return run<float, false>((const float*)p, L, decay, scratch, values, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H, D, V, error_word,
+    return run<float, false, true>((const float*)p, L, decay, scratch, values, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H, D, V, error_word,
                              stream);
 }

@@ -1102,10 +1102,16 @@ class CudaOps:
         out = torch.empty((T, H * V), dtype=torch.float32, device=p.device)
         prep = torch.empty((T, 2 * H * D + H * V), dtype=torch.float32, device=p.device)
         half = 0 if inv_freq is None else inv_freq.numel()
-        _check(self.lib.mi_retention_scan(_p(p), p.stride(0), _p(prep), _p(batch.positions), _p(inv_freq), half, _c.c_float(k_scale),
-                                          _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                          _p(batch.seg_slot), T, batch.num_segs, H, D, V, _code(p.dtype), self._stream()),
-               "retention_scan")
+        _check(self.lib.mi_retention_rows(_p(p), p.stride(0), _p(prep), _p(batch.positions), _p(inv_freq), half, _c.c_float(k_scale), T, H, D, V,
+                                          _code(p.dtype), self._stream()), "retention_rows")
+        if self._takes_octets(prep, batch, D, V, state):
+            scratch = self._octet_scratch(T, batch, H, D, V, False)
+            _check(self.lib.mi_constant_octets(_p(prep), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
+                                               _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error), self._stream()), "constant_octets")
+            self.launches += 3
+            return out
+        _check(self.lib.mi_retention_scan(_p(prep), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
+                                          _p(batch.seg_slot), T, batch.num_segs, H, D, V, self._stream()), "retention_scan")
         self.launches += 2
         return out
 

@@ -100,8 +100,11 @@ def test_recurrences_eight_tokens_at_a_time(ops, lens, H, KV, D, V):        # no
     prep[:, C + H * D:C + H * D + H] = torch.rand(T, H, generator=g).to(DEV)
     state = r(len(lens) + 1, H * D * V + 6)
     p = r(T, 2 * H * D + H * V + 8).to(torch.bfloat16)
+    batch.positions = torch.arange(T, dtype=torch.int32, device=DEV)
+    freq = torch.rand(D // 4, generator=g).to(DEV)
     constant = torch.tensor([1.0 - 2.0 ** -(1 + 2 * h) for h in range(H)], device=DEV)
-    runs = {"delta": lambda s: ops.delta_scan(prep, H, KV, D, V, s, batch), "constant": lambda s: ops.lightning_scan(p, H, D, V, constant, s, batch)}
+    runs = {"delta": lambda s: ops.delta_scan(prep, H, KV, D, V, s, batch), "constant": lambda s: ops.lightning_scan(p, H, D, V, constant, s, batch),
+            "rotated": lambda s: ops.retention_scan(p, H, D, V, freq, D ** -0.5, constant, s, batch)}
     for name, run in runs.items():
         a, b = state.clone(), state.clone()
         taken = ops._takes_octets
