@@ -563,9 +563,9 @@ class CudaOps:
                 and q.data_ptr() % 16 == 0)
         tc = (fast and self.tc_attention and num_tiles and meta.tile == 64 and meta.page_size % 8 == 0
               and 64 % meta.page_size == 0 and num_tiles2)
-        if tc and split_weights:
+        if tc and split_weights and meta.max_kv_len >= self.SPLIT_TC_KEYS:
             self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
-        elif tc:
+        elif tc and not split_weights:
             rc = self.lib.mi_attn_prefill_tc(
                 _p(q), q.stride(0), T, _p(k_cache), _p(v_cache), _c.c_longlong(k_cache.shape[0] * KV * meta.page_size),
                 _p(out), _p(tiles2), num_tiles2, _p(meta.seg_q_start), _p(meta.seg_pos0),
@@ -624,6 +624,10 @@ class CudaOps:
                 H, KV, D, meta.page_size, S, _c.c_float(scale), win, code, self._stream()), "attn_decode")
             self.launches += 2 if S > 1 else 1
         return out
+
+    # Prompts whose longest request sees fewer keys stay on the mma.sync forms: both kernels' time is hidden behind the host's launches there, and the
+    # query's tensor map costs 2 us of those (192 keys: 51 against 53 us a mixer; 2,516 keys: 159 against 70).
+    SPLIT_TC_KEYS = 256
 
     def _prefill_tc_split(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias_t=None, bias_last=0,
                           slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):
@@ -714,13 +718,16 @@ class CudaOps:
 
     @staticmethod
     def _takes_octets(rows, batch, D, V, state):
-        """Whether a step's recurrence goes eight tokens at a time (csrc/state_octets.cu): steps with prompts, keys of 64 or 128, values in blocks
-        of 16 columns, states of an even number of floats, rows whose heads start on 16 bytes."""
-        return (rows.shape[0] > 4 * batch.num_segs and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
+        """Whether a step's recurrence goes eight tokens at a time (csrc/state_octets.cu): keys of 64 or 128, values in blocks of 16 columns, states
+        of an even number of floats, rows whose heads start on 16 bytes, and steps of at least 128 tokens: with 96 the token-by-token kernel's
+        26 us are hidden behind the host's launches and the second launch costs 7 us, with 192 the mixer takes 87 us instead of 100."""
+        return (rows.shape[0] >= max(128, 4 * batch.num_segs + 1) and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
                 and rows.stride(0) % 4 == 0 and rows.data_ptr() % 16 == 0)
 
     def _octet_scratch(self, T, batch, H, D, V, delta):
-        return torch.empty(self.lib.mi_octet_floats(T, batch.num_segs, H, D, V, int(delta)), dtype=torch.float32, device=self.device)
+        """Per octet and head its record (25 or 16 vectors of D, 144 numbers) and eight tokens' values (csrc/state_octets.cu: mi_octet_floats)."""
+        floats = (T // 8 + batch.num_segs) * H * ((25 if delta else 16) * D + 144 + 8 * V)
+        return torch.empty(floats, dtype=torch.float32, device=self.device)
 
     def lightning_scan(self, p, H, D, V, decay, state, batch):
         """p [T, >= 2 H D + H V] = q | k | v before silu; state float32 [slots, H D V] (an entry continues from its slot's
@@ -986,7 +993,7 @@ class CudaOps:
         # 128: 149 us on the mma.sync kernel); other page sizes keep the mma.sync forms, other heads the float32 kernels
         tc = (num_tiles and self.fast_attention and self.tc_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
               and tiles2 is not None and tiles2.shape[0] and meta.page_size % 8 == 0 and 64 % meta.page_size == 0 and tc_form
-              and (plain or self.biased_attention_tc) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
+              and (plain or self.biased_attention_tc) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and meta.max_kv_len >= self.SPLIT_TC_KEYS)
         if tc:
             bias_t = None if distance_bias is None and distance_bias_by_head is None else self._bias_rows_by_head(distance_bias, distance_bias_by_head)
             self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, blk, win, int(bool(sink)), sink_values, bias_t,

@@ -82,7 +82,7 @@ def rows_error(a, b):
     return ((a.double() - b.double()).norm() / b.double().norm()).item()
 
 
-@pytest.mark.parametrize("lens", [(9, 1, 8, 40), (129,), (7, 63), (15, 1, 1, 16)])
+@pytest.mark.parametrize("lens", [(9, 1, 8, 120), (129,), (7, 63, 58), (1, 1, 16, 1, 111)])
 @pytest.mark.parametrize("H,KV,D,V", [(4, 2, 128, 48), (3, 3, 64, 32), (5, 1, 128, 128)])
 def test_recurrences_eight_tokens_at_a_time(ops, lens, H, KV, D, V):        # noqa: F811
     """The delta rule with channel decays and the constant decay against their token-by-token kernels: whole octets, remainders, single tokens
@@ -108,7 +108,9 @@ def test_recurrences_eight_tokens_at_a_time(ops, lens, H, KV, D, V):        # no
     for name, run in runs.items():
         a, b = state.clone(), state.clone()
         taken = ops._takes_octets
-        assert taken(prep, batch, D, V, a) == (T > 4 * len(lens))
+        assert taken(prep, batch, D, V, a)
+        for delta in (0, 1):
+            assert ops.lib.mi_octet_floats(T, len(lens), H, D, V, delta) == ops._octet_scratch(T, batch, H, D, V, delta).numel()
         got = run(a)
         ops._takes_octets = lambda *args: False
         try:
