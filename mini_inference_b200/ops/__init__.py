@@ -719,9 +719,11 @@ class CudaOps:
     @staticmethod
     def _takes_octets(rows, batch, D, V, state):
         """Whether a step's recurrence goes eight tokens at a time (csrc/state_octets.cu): keys of 64 or 128, values in blocks of 16 columns, states
-        of an even number of floats, rows whose heads start on 16 bytes, and steps of at least 128 tokens: with 96 the token-by-token kernel's
-        26 us are hidden behind the host's launches and the second launch costs 7 us, with 192 the mixer takes 87 us instead of 100."""
-        return (rows.shape[0] >= max(128, 4 * batch.num_segs + 1) and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
+        of an even number of floats, rows whose heads start on 16 bytes, and a prompt of at least 128 tokens (with 96 the token-by-token kernel's
+        26 us are hidden behind the host's launches and the second launch costs 7 us, with 192 the mixer takes 87 us instead of 100) or 512
+        tokens in all (16 prompts of 64: 107 us instead of 216)."""
+        T = rows.shape[0]
+        return (T > 4 * batch.num_segs and (T >= 512 or getattr(batch, "max_q_len", T) >= 128) and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
                 and rows.stride(0) % 4 == 0 and rows.data_ptr() % 16 == 0)
 
     def _octet_scratch(self, T, batch, H, D, V, delta):
@@ -847,7 +849,7 @@ class CudaOps:
             return o.view(T, H, C + R)[:, :, :C].permute(1, 0, 2)
         num_decode, num_tiles = meta.decode_segs.shape[0], meta.prefill_tiles.shape[0]
         code, Dk = _code(q.dtype), C + R
-        # Cached rows of 64 or 128 entries, bfloat16: the paged tensor-core kernels (mma.sync forms) with the pool as keys AND values
+        # Cached rows of 64 or 128 entries, bfloat16: the paged tensor-core kernels with the pool as keys AND values
         # of one shared kv head and every softmax weight split into two bfloat16 numbers for the P V product, which keeps the
         # weights' precision where the design wants it; their output has C + R columns per head, of which the first C count.
         if (q.dtype == torch.bfloat16 and Dk in (64, 128) and meta.tile == 64 and self.fast_attention and meta.page_size % 16 == 0
@@ -988,12 +990,11 @@ class CudaOps:
             assert sink_values is None or (sink and sink_values.dtype == torch.float32 and sink_values.numel() == H)
             assert distance_bias is None or (distance_bias.dtype == torch.float32 and distance_bias.is_contiguous() and distance_bias.shape[1] == H)
         bias_last = 0 if distance_bias is None else distance_bias.shape[0] - 1
-        tiles2 = getattr(meta, "prefill_tiles2", None)
         # heads of 64 or 128, pages that divide a tile of 64 keys into TMA boxes of at least 8 rows: the tcgen05 kernel (2,048 tokens, 16 heads of
         # 128: 149 us on the mma.sync kernel); other page sizes keep the mma.sync forms, other heads the float32 kernels
-        tc = (num_tiles and self.fast_attention and self.tc_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
-              and tiles2 is not None and tiles2.shape[0] and meta.page_size % 8 == 0 and 64 % meta.page_size == 0 and tc_form
-              and (plain or self.biased_attention_tc) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and meta.max_kv_len >= self.SPLIT_TC_KEYS)
+        tc = (num_tiles and meta.max_kv_len >= self.SPLIT_TC_KEYS and self.fast_attention and self.tc_attention and q.dtype == torch.bfloat16 and D == V
+              and D in (64, 128) and meta.tile == 64 and getattr(meta, "prefill_tiles2", None) is not None and meta.prefill_tiles2.shape[0] and meta.page_size % 8 == 0 and 64 % meta.page_size == 0 and tc_form
+              and (plain or self.biased_attention_tc) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
         if tc:
             bias_t = None if distance_bias is None and distance_bias_by_head is None else self._bias_rows_by_head(distance_bias, distance_bias_by_head)
             self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, blk, win, int(bool(sink)), sink_values, bias_t,
