@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(TOK == 1 ? 1024 : 256) route_topk_kernel(const
     __syncthreads();
     if (TOK == 8 && vec) {
         // four experts at a time: a token's entries are read from shared memory once for the four (a 16-byte load of a warp takes four
-        // clocks of that memory's pipe, four multiply-adds one each: with an expert at a time the loads were the bound).  The 32
+        // clocks of that memory's pipe, four multiply-adds one each: with an expert at a time the loads were the bound; 2,048 tokens, 32 experts: 63 -> 21 us with the rows staged in 16-byte pieces).  The 32
         // sums over lanes are made together, in the order of warp_sum (16, 8, .. 1 lanes apart): the same bits.
         for (int e0 = warp * 4; e0 < EA; e0 += nw * 4) {
             float dot[32];
@@ -617,7 +617,7 @@ MI_EXPORT int mi_moe_combine(const void* rows, const float* weights, const void*
                              int top, int dtype, cudaStream_t stream) {
     if (T_ == 0) return 0;
     const int vn = dtype == MI_BF16 ? 8 : 4;
-    if (hidden % vn == 0 && ((uintptr_t)rows | (uintptr_t)shared | (uintptr_t)out) % 16 == 0) {        // 2,048 x 4 rows of 2,048: 31 -> 10 us
+    if (hidden % vn == 0 && ((uintptr_t)rows | (uintptr_t)shared | (uintptr_t)out) % 16 == 0) {        // 2,048 x 4 rows of 2,048: 31 -> 11 us
         const dim3 vgrid(T_, T_ >= 512 ? 1 : min(8, (hidden / vn + 63) / 64));
         const int nt = T_ >= 512 ? min(256, (hidden / vn + 31) / 32 * 32) : 64;
         if (dtype == MI_BF16)
