@@ -12,6 +12,7 @@
 // without visible keys changes no bit (its weights are zeros, the factor that rescales is one).
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 
 using namespace mi;
 
@@ -119,10 +120,13 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int q_stride, const float* 
             }
         }
         // ---- terms, mask, online softmax; the weights go to this warp's rows of P
+        const int p_warp = p_first + warp * 16;                // a key that a row does not see may hold anything, and 0 * inf is no 0: its weight is marked
+        const bool whole = kt * BK + BK - 1 <= p_warp && (kt * BK >= first_key(p_warp + 15) || (!PLAIN && kt * BK + BK <= t.keep));
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int p = p_first + row0 + 4 * i, lo = first_key(p);
             float s[4], mx = -INFINITY;
+            bool seen[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int key = kt * BK + ln + 8 * j;
@@ -133,8 +137,8 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int q_stride, const float* 
                     if (slope != 0.f) s[j] -= slope * (float)dist;
                     if (t.cap > 0.f) s[j] = t.cap * tanhf(s[j] / t.cap);
                 }
-                const bool seen = key <= p && (key >= lo || (!PLAIN && key < t.keep));
-                s[j] = seen ? s[j] : -INFINITY;
+                seen[j] = key <= p && (key >= lo || (!PLAIN && key < t.keep));
+                s[j] = seen[j] ? s[j] : -INFINITY;
                 mx = fmaxf(mx, s[j]);
             }
 #pragma unroll
@@ -146,7 +150,7 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int q_stride, const float* 
             for (int j = 0; j < 4; ++j) {
                 const float w = expf(s[j] - z);
                 sum += w;
-                smem[L::P + (row0 + 4 * i) * L::LP + ln + 8 * j] = w;
+                smem[L::P + (row0 + 4 * i) * L::LP + ln + 8 * j] = seen[j] ? w : -1.f;
             }
 #pragma unroll
             for (int x = 1; x < 8; x <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
@@ -156,30 +160,34 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int q_stride, const float* 
             for (int c = 0; c < 2 * DV; ++c) o[i][c] = make_float2(o[i][c].x * alpha, o[i][c].y * alpha);
         }
         __syncwarp();
-        // ---- the weighted sum
+        // ---- the weighted sum; a tile that some row of the warp does not see whole leaves the marked weights out
         const float* pp = smem + L::P + row0 * L::LP;
         const float* vp = smem + L::V + buf * BK * D + 4 * ln;
+        auto add_values = [&](auto marked) {
 #pragma unroll 2
-        for (int k = 0; k < BK; k += 4) {
-            float w[4][4];
+            for (int k = 0; k < BK; k += 4) {
+                float w[4][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 v = *reinterpret_cast<const float4*>(pp + 4 * i * L::LP + k);
-                w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-#pragma unroll
-                for (int c = 0; c < DV; ++c) {
-                    const float4 v = *reinterpret_cast<const float4*>(vp + (k + e) * D + 32 * c);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float2 ww = make_float2(w[i][e], w[i][e]);
-                        o[i][2 * c] = __ffma2_rn(ww, make_float2(v.x, v.y), o[i][2 * c]);
-                        o[i][2 * c + 1] = __ffma2_rn(ww, make_float2(v.z, v.w), o[i][2 * c + 1]);
-                    }
+                for (int i = 0; i < 4; ++i) {
+                    const float4 v = *reinterpret_cast<const float4*>(pp + 4 * i * L::LP + k);
+                    w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
                 }
-        }
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int c = 0; c < DV; ++c) {
+                        const float4 v = *reinterpret_cast<const float4*>(vp + (k + e) * D + 32 * c);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (decltype(marked)::value && w[i][e] < 0.f) continue;
+                            const float2 ww = make_float2(w[i][e], w[i][e]);
+                            o[i][2 * c] = __ffma2_rn(ww, make_float2(v.x, v.y), o[i][2 * c]);
+                            o[i][2 * c + 1] = __ffma2_rn(ww, make_float2(v.z, v.w), o[i][2 * c + 1]);
+                        }
+                    }
+            }
+        };
+        if (whole) add_values(std::false_type{}); else add_values(std::true_type{});
         __syncwarp();
     }
 #pragma unroll

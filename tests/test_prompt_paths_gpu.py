@@ -66,6 +66,34 @@ def test_prompt_attention_forms(ops, dtype, H, KV, D, page, form):      # noqa: 
     assert err < (4e-6 if dtype == torch.float32 else 2 ** -8) * limit, (form, err / limit)
 
 
+@pytest.mark.parametrize("D,page", [(128, 16), (64, 24)])
+@pytest.mark.parametrize("form", ["plain", "causal", "window", "blocks_sink", "cap_keep_gate", "window_keep_narrow"])
+def test_float32_prompt_attention_reads_visible_keys_only(ops, D, page, form):      # noqa: F811
+    """A key or value that is no number is met by the rows that see it and by no other, although their tiles of keys hold it as well."""
+    H, KV, segs, at = 2, 1, [(40, 300), (0, 70)], 133            # key 133 of the first request, which feeds the positions 40 .. 339
+    T = sum(n for _, n in segs)
+    meta, g = make_meta(page, segs, 60, 4), torch.Generator().manual_seed(2)
+    q = torch.randn(T, H * D, generator=g).to(DEV)
+    k, v = (torch.randn(61, KV, page, D, generator=g).to(DEV) for _ in range(2))
+    args = None if form == "plain" else form_arguments(form, H, D, T, torch.float32)
+
+    def call(k, v):
+        return ops.paged_attention(q, k, v, meta, H, KV, D, D ** -0.5, None) if args is None else ops.masked_attention(q, k, v, meta, H, KV, D, D, D ** -0.5, **args)
+
+    want, bad_k, bad_v, place = call(k, v), k.clone(), v.clone(), (meta.block_table[0, at // page].long(), 0, at % page)
+    bad_v[place], bad_k[place] = float("inf"), float("nan")
+    pos = torch.arange(40, 340)
+    mask = args or {}
+    lo = torch.zeros_like(pos) if not mask.get("block_size") else pos // mask["block_size"] * mask["block_size"]
+    lo = torch.maximum(lo, pos - mask["window"] + 1) if mask.get("window") else lo
+    sees = (pos >= at) & ((lo <= at) | (at < mask.get("keep_first", 0)))
+    sees = torch.cat([sees, torch.zeros(70, dtype=torch.bool)]).to(DEV)
+    assert sees.any() and not sees.all()
+    for got in (call(k, bad_v), call(bad_k, v)):
+        assert torch.equal(got[~sees], want[~sees]), form
+        assert not got[sees].isfinite().any(), form
+
+
 class Entries:
     """A step's entries as the recurrences see them."""
 
