@@ -217,7 +217,7 @@ MI_EXPORT int mi_attn_prefill_f32(const float* q, int q_stride, const float* k_c
                                   const float* sink_values, const float* bias, int bias_last, const float* slopes, float cap, int keep,
                                   const float* gate, int gate_stride, cudaStream_t stream) {
     if (num_tiles == 0) return 0;
-    if ((D != 64 && D != 128) || H % KV || tile_rows != BQ || q_stride % 4 || (uintptr_t)q % 16) return -2;
+    if ((D != 64 && D != 128) || H % KV || tile_rows != BQ || q_stride % 4 || ((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16) return -2;
     const Terms t{block, window, sink, window > 0 ? keep : 0, bias_last, gate_stride, cap, sink_values, bias, slopes, gate};
     const bool plain = block <= 0 && !sink && !bias && !slopes && cap <= 0.f && t.keep <= 0 && !gate;
     const dim3 grid(H, num_tiles);

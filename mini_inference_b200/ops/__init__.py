@@ -579,7 +579,7 @@ class CudaOps:
                 _p(meta.seg_q_start), _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D,
                 meta.page_size, meta.tile, _c.c_float(scale), win, self._stream()), "attn_prefill_mma")
             self.launches += 1
-        elif num_tiles and self._f32_tiles(q, D, D, meta):
+        elif num_tiles and self._f32_tiles(q, D, D, meta, k_cache, v_cache):
             self._prefill_f32(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
         elif num_tiles:
             _check(self.lib.mi_attn_prefill_generic(
@@ -640,10 +640,11 @@ class CudaOps:
             "attn_prefill_tc_split")
         self.launches += 1
 
-    def _f32_tiles(self, q, D, V, meta):
-        """Whether the float32 prompt attention with tiles takes these rows: heads of 64 or 128 that start on 16 bytes, tiles of 64 rows."""
+    def _f32_tiles(self, q, D, V, meta, k_cache, v_cache):
+        """Whether the float32 prompt attention with tiles takes these rows: heads of 64 or 128, tiles of 64 rows; queries, keys and values start
+        on 16 bytes (it copies 16 bytes at a time)."""
         return (self.fast_attention and q.dtype == torch.float32 and D == V and D in (64, 128) and meta.tile == 64 and q.stride(0) % 4 == 0
-                and q.data_ptr() % 16 == 0)
+                and (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16 == 0)
 
     def _prefill_f32(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias=None, bias_last=0,
                      slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):
@@ -1028,7 +1029,7 @@ class CudaOps:
             else:                                          # a slope per head times the distance, beside (or instead of) the table
                 _check(self.lib.mi_attn_prefill_mma_sloped(*args, _p(slopes), self._stream()), "attn_prefill_mma_sloped")
             self.launches += 1
-        elif num_tiles and self._f32_tiles(q, D, V, meta):
+        elif num_tiles and self._f32_tiles(q, D, V, meta, k_cache, v_cache):
             self._prefill_f32(q, k_cache, v_cache, out, meta, H, KV, D, scale, blk, win, int(bool(sink)), sink_values, distance_bias, bias_last,
                               slopes, cap, keep, gate, gate_stride)
         elif num_tiles:

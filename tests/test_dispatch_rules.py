@@ -1,0 +1,30 @@
+"""The rules that choose between kernels, on the CPU: what a faster kernel cannot take stays with the general one."""
+import types
+
+import torch
+
+from mini_inference_b200.ops import CudaOps
+
+
+def off_by(floats, *shape):
+    """A contiguous float32 tensor that starts `floats` floats behind a 64-byte boundary."""
+    n = torch.Size(shape).numel()
+    buf = torch.zeros(n + 32)
+    start = (-buf.data_ptr() // 4) % 16 + floats
+    return buf[start:start + n].view(*shape)
+
+
+def step(lens):
+    return types.SimpleNamespace(num_segs=len(lens), max_q_len=max(lens))
+
+
+def test_float32_attention_in_tiles_wants_caches_on_16_bytes():
+    """Its 16-byte copies fault on other addresses; the kernel for any head size loads such keys and values as well."""
+    me, meta = types.SimpleNamespace(fast_attention=True), types.SimpleNamespace(tile=64)
+    q, k, v = off_by(0, 8, 128), off_by(0, 2, 1, 16, 128), off_by(4, 2, 1, 16, 128)
+    assert CudaOps._f32_tiles(me, q, 128, 128, meta, k, v)
+    for floats in (1, 2, 3):
+        odd = off_by(floats, 2, 1, 16, 128)
+        assert not CudaOps._f32_tiles(me, q, 128, 128, meta, odd, v)
+        assert not CudaOps._f32_tiles(me, q, 128, 128, meta, k, odd)
+        assert not CudaOps._f32_tiles(me, off_by(floats, 8, 128), 128, 128, meta, k, v)
