@@ -28,3 +28,11 @@ def test_float32_attention_in_tiles_wants_caches_on_16_bytes():
         assert not CudaOps._f32_tiles(me, q, 128, 128, meta, odd, v)
         assert not CudaOps._f32_tiles(me, q, 128, 128, meta, k, odd)
         assert not CudaOps._f32_tiles(me, off_by(floats, 8, 128), 128, 128, meta, k, v)
+
+
+def test_states_that_start_anywhere_keep_the_general_scan():
+    """The eight-token scan moves states eight bytes at a time (and refuses others); the token-by-token scan takes every start."""
+    rows, one = off_by(0, 600, 3 * 128), step((600,))
+    assert CudaOps._takes_octets(rows, one, 64, 64, off_by(2, 2, 64 * 64))
+    assert not CudaOps._takes_octets(rows, one, 64, 64, off_by(1, 2, 64 * 64))
+    assert not CudaOps._takes_octets(rows, one, 64, 64, off_by(0, 2, 64 * 64 + 1))
