@@ -715,7 +715,7 @@ class CudaOps:
     def _takes_step(T, batch, D, V, state):
         """Whether a step's recurrence has a whole state in a block's registers (csrc/state_step.cu): one token per entry, sizes of 64 or 128,
         states on 16 bytes."""
-        return T == batch.num_segs and D in (64, 128) and V in (64, 128) and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0
+        return T == batch.num_segs and getattr(batch, "max_q_len", 1) == 1 and D in (64, 128) and V in (64, 128) and state.stride(0) % 4 == 0 and state.data_ptr() % 16 == 0
 
     @staticmethod
     def _takes_octets(rows, batch, D, V, state):

@@ -36,3 +36,10 @@ def test_states_that_start_anywhere_keep_the_general_scan():
     assert CudaOps._takes_octets(rows, one, 64, 64, off_by(2, 2, 64 * 64))
     assert not CudaOps._takes_octets(rows, one, 64, 64, off_by(1, 2, 64 * 64))
     assert not CudaOps._takes_octets(rows, one, 64, 64, off_by(0, 2, 64 * 64 + 1))
+
+
+def test_as_many_tokens_as_entries_is_not_one_each():
+    """The kernel for one token per entry reads an entry's first token only."""
+    state = off_by(0, 3, 64 * 64)
+    assert CudaOps._takes_step(2, step((1, 1)), 64, 64, state)
+    assert not CudaOps._takes_step(2, step((2, 0)), 64, 64, state)
