@@ -728,9 +728,8 @@ class CudaOps:
                 and state.data_ptr() % 8 == 0 and rows.stride(0) % 4 == 0 and rows.data_ptr() % 16 == 0)
 
     def _octet_scratch(self, T, batch, H, D, V, delta):
-        """Per octet and head its record (25 or 16 vectors of D, 144 numbers) and eight tokens' values (csrc/state_octets.cu: mi_octet_floats)."""
-        floats = (T // 8 + batch.num_segs) * H * ((25 if delta else 16) * D + 144 + 8 * V)
-        return torch.empty(floats, dtype=torch.float32, device=self.device)
+        """Per octet and head its record and eight tokens' values: as many floats as the kernels' own layout says."""
+        return torch.empty(self.lib.mi_octet_floats(T, batch.num_segs, H, D, V, int(delta)), dtype=torch.float32, device=self.device)
 
     def lightning_scan(self, p, H, D, V, decay, state, batch):
         """p [T, >= 2 H D + H V] = q | k | v before silu; state float32 [slots, H D V] (an entry continues from its slot's
