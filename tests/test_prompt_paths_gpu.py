@@ -205,3 +205,36 @@ def test_unit_heads_of_prompts(ops, H, KV, D, form):            # noqa: F811
     for a, b in zip(*results):                                  # one bfloat16 rounding of values that differ in their last float32 bits
         assert (a.float() - b.float()).abs().max().item() <= 2 ** -8 * b.float().abs().max().item()
         assert (a != b).float().mean().item() < 1e-2
+
+# ---------------------------------------------------------------- kernels that a rule on sizes picks, against the plain statements (tests/ref_ops.py)
+def both_batches(lens, slots):
+    import types
+    qs = [0]
+    for n in lens:
+        qs.append(qs[-1] + n)
+    dev = Entries(lens)
+    dev.seg_slot = torch.tensor(slots, dtype=torch.int32, device=DEV)
+    dev.token_seg = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().to(DEV)
+    dev.max_q_len = max(lens)
+    return types.SimpleNamespace(host={"seg_q_start": qs, "seg_slot": slots}, num_segs=len(lens)), dev
+
+
+@pytest.mark.parametrize("taps", [2, 3, 4])
+@pytest.mark.parametrize("H,KV,D,V", [(4, 2, 128, 128), (3, 1, 64, 48), (2, 2, 12, 20)])
+def test_delta_prologue_of_prompts(ops, taps, H, KV, D, V):     # noqa: F811
+    """A warp takes eight neighbouring tokens: entries that begin and end among them, entries shorter than the taps, the slots' earlier inputs."""
+    from tests.ref_ops import TorchRefOps
+    ref, lens = TorchRefOps(), (5, 1, 2, 97, 60, 35)
+    host, dev = both_batches(lens, [2, 6, 1, 4, 3, 5])
+    T, C, g = sum(lens), 2 * KV * D + H * V, torch.Generator().manual_seed(taps)
+    assert T >= 192                                              # where the kernel's range begins
+    p = torch.randn(T, (C + H + 9) // 4 * 4 + 4, generator=g).to(torch.bfloat16)
+    a = torch.randn(T, 2 * H * D, generator=g).to(torch.bfloat16)
+    conv, A_log, bias = torch.randn(C, taps, generator=g), torch.randn(H, generator=g) * 0.3, torch.randn(H * D, generator=g)
+    state = torch.randn(7, H * D * V + (taps - 1) * C, generator=g)
+    sa, sb = state.clone().to(DEV), state.clone()
+    got = ops.delta_prepare(p.to(DEV), a.to(DEV)[:, :H * D], conv.to(DEV), A_log.to(DEV), bias.to(DEV), H, KV, D, V, taps, 1e-6, sa, dev)
+    want = ref.delta_prepare(p, a[:, :H * D], conv, A_log, bias, H, KV, D, V, taps, 1e-6, sb, host)
+    n = C + H * D + H
+    assert (got[:, :n].cpu() - want[:, :n]).abs().max().item() < 4e-6 * want.abs().max().item()
+    assert torch.equal(sa.cpu(), sb)                             # the newest inputs, copied
