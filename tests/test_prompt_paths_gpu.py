@@ -238,3 +238,20 @@ def test_delta_prologue_of_prompts(ops, taps, H, KV, D, V):     # noqa: F811
     n = C + H * D + H
     assert (got[:, :n].cpu() - want[:, :n]).abs().max().item() < 4e-6 * want.abs().max().item()
     assert torch.equal(sa.cpu(), sb)                             # the newest inputs, copied
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,hidden", [(127, 264), (128, 264), (128, 2050), (600, 2048)])
+def test_weighted_sum_of_experts(ops, dtype, T, hidden):        # noqa: F811
+    """128 tokens or more in 16-byte pieces where rows allow, fewer an entry a thread; with and without weights, a shared expert and its gate."""
+    from mini_inference_b200.ops import _p
+    g, top = torch.Generator().manual_seed(T), 3
+    rows, shared = torch.randn(T * top, hidden, generator=g).to(dtype).to(DEV), torch.randn(T, hidden, generator=g).to(dtype).to(DEV)
+    weights, gate = torch.rand(T, top, generator=g).to(DEV), torch.randn(T, generator=g).to(DEV)
+    for w, s, sg in ((weights, shared, gate), (weights, shared, None), (None, None, None)):
+        out = torch.empty(T, hidden, dtype=dtype, device=DEV)
+        assert ops.lib.mi_moe_combine(_p(rows), _p(w), _p(s), _p(sg), _p(out), T, hidden, top, int(dtype == torch.bfloat16), ops._stream()) == 0
+        want = (rows.double().view(T, top, hidden) * (1.0 if w is None else w.double()[:, :, None])).sum(1)
+        if s is not None:
+            want += s.double() * (1.0 if sg is None else torch.sigmoid(sg.double())[:, None])
+        limit = 1e-6 if dtype == torch.float32 else 2 ** -7
+        assert ((out.double() - want).abs() <= limit * want.abs().clamp_min(0.5)).all()
