@@ -255,3 +255,15 @@ def test_weighted_sum_of_experts(ops, dtype, T, hidden):        # noqa: F811
             want += s.double() * (1.0 if sg is None else torch.sigmoid(sg.double())[:, None])
         limit = 1e-6 if dtype == torch.float32 else 2 ** -7
         assert ((out.double() - want).abs() <= limit * want.abs().clamp_min(0.5)).all()
+
+def test_sampler_forms_agree(ops):                              # noqa: F811
+    """Few scores: eight a thread, fetched together; 4.5 million and more: sixteen, one after the other.  The choices are the same whole numbers."""
+    R, V = 40, 120001
+    g = torch.Generator().manual_seed(0)
+    logits = torch.randn(R, V, generator=g).to(DEV)
+    temps = torch.tensor([0.0, 0.7] * (R // 2), device=DEV)
+    seeds, counters = torch.arange(R, dtype=torch.int32, device=DEV), torch.arange(5, 5 + R, dtype=torch.int32, device=DEV)
+    got = ops.sample(logits, temps, seeds, counters)
+    parts = [ops.sample(logits[a:a + 8], temps[a:a + 8].contiguous(), seeds[a:a + 8].contiguous(), counters[a:a + 8].contiguous()) for a in range(0, R, 8)]
+    assert torch.equal(got, torch.cat(parts))
+    assert torch.equal(got[::2].long(), logits[::2].argmax(-1))
