@@ -578,7 +578,6 @@ __global__ void short_conv_kernel(const T* __restrict__ h, int ldh, const float*
 
 // The same for bfloat16 rows whose channels come in multiples of eight: a thread owns eight channels (16-byte loads and stores), keeps
 // their TAPS weights in registers and walks TOK neighbouring tokens (each looks its own entry up: an entry may end between them).
-// silu with the fast exponential and quotient (a few units in the last place of float32): the result is rounded to bfloat16
 template <int TAPS, int TOK>
 __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int ldh, const float* __restrict__ w, const float* __restrict__ bias,
                                       const float* __restrict__ state, long long state_stride, long long hist_off, __nv_bfloat16* __restrict__ out,
@@ -631,7 +630,7 @@ __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int l
                 acc[e] = breg[e];
 #pragma unroll
                 for (int j = 0; j < TAPS; ++j) acc[e] = fmaf(wreg[e][j], entry(k + j, e), acc[e]);
-                if (act == 1) acc[e] = __fdividef(acc[e], 1.f + __expf(-acc[e]));
+                if (act == 1) acc[e] = silu(acc[e]);
                 if (residual) acc[e] += entry(k + TAPS - 1, e);
             }
             uint4 o;
@@ -671,7 +670,7 @@ __global__ void short_conv_vec_kernel(const __nv_bfloat16* __restrict__ h, int l
         __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            if (act == 1) acc[e] = __fdividef(acc[e], 1.f + __expf(-acc[e]));
+            if (act == 1) acc[e] = silu(acc[e]);
             if (residual) acc[e] += x[e];                    // x holds the last tap's input: the token's own
         }
 #pragma unroll

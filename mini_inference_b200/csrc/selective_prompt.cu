@@ -36,9 +36,7 @@ __device__ __forceinline__ float2 exp_neg2(float2 v) {
     return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)), __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
 }
 
-// z / (1 + e^-z); fast forms (a few units in the last place of float32) where the result is rounded to bfloat16
-template <typename T> __device__ __forceinline__ float silu_for(float z) { return z / (1.f + expf(-z)); }
-template <> __device__ __forceinline__ float silu_for<__nv_bfloat16>(float z) { return __fdividef(z, 1.f + __expf(-z)); }
+__device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
 
 // grid (entries, ceil(I / 32)); L lanes of NS states each, N = L NS
 template <typename T, int L, int NS>
@@ -93,7 +91,7 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
                 const int tt = hw + HW * r;
                 if (live && tb >= 0 && tb + tt < n) {
                     const float xv = to_f32(fx[r]), zv = to_f32(fz[r]);
-                    out[(size_t)(qs + tb + tt) * I + cc] = from_f32<T>((ys[b][tt][lane] + skip * xv) * silu_for<T>(zv));
+                    out[(size_t)(qs + tb + tt) * I + cc] = from_f32<T>((ys[b][tt][lane] + skip * xv) * silu(zv));
                 }
             }
             if (ta < n) {

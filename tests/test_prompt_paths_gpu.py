@@ -177,6 +177,26 @@ def test_selective_scan_of_prompts(ops, dtype, lens, inner, N):         # noqa: 
     assert rows_error(got, want) < (3e-6 if dtype == torch.float32 else 4e-3)        # bfloat16: the output's own rounding may fall differently
 
 
+def test_silu_keeps_its_float32(ops):                           # noqa: F811
+    """The filter's activation and the scan's gate of bfloat16 prompts are float32's silu rounded once, down to inputs where 1 + e^-x is nearly
+    the largest float32: the fast exponential is 4e-4 off at -80 (a tenth of a bfloat16 step) and the fast quotient 0 from -87.4 on."""
+    T, inner, N = 512, 64, 16
+    grid = torch.cat([torch.linspace(-88.5, -60, 220), torch.linspace(-20, 20, 292)]).to(torch.bfloat16).to(DEV)
+    want = (grid.double() / (1 + (-grid.double()).exp())).float().to(torch.bfloat16)
+    rows = grid[:, None].expand(T, inner).contiguous()
+    batch = Entries((T,))
+    batch.token_seg = torch.zeros(T, dtype=torch.int32, device=DEV)
+    conv = ops.short_conv(rows, torch.ones(inner, 1, device=DEV), None, 1, None, 0, batch, act="silu")
+    one, zero = torch.ones(T, inner, dtype=torch.bfloat16, device=DEV), torch.zeros(inner, device=DEV)
+    bc = torch.zeros(T, N, dtype=torch.bfloat16, device=DEV)
+    gate = ops.selective_scan(one, torch.zeros(T, inner, device=DEV), zero, -torch.ones(inner, N, device=DEV), bc, bc, zero + 1, rows,
+                              torch.zeros(2, inner * N, device=DEV), batch, torch.bfloat16)           # (0 + 1 * 1) * silu(z)
+    for got in (conv, gate):
+        # a double rounding may fall the other way where the float32 value lies within its own error of the middle: 2e-7 / 2^-8 of the values
+        assert (got != want[:, None]).float().mean().item() < 5e-3
+        assert ((got.double() / want.double()[:, None] - 1).abs().nan_to_num() <= 2 ** -7).all()
+
+
 @pytest.mark.parametrize("H,KV,D", [(16, 8, 128), (3, 1, 64), (5, 5, 128)])
 @pytest.mark.parametrize("form", ["unit", "weights_rotated", "all_rotated", "temperature_keys", "blend", "plain"])
 def test_unit_heads_of_prompts(ops, H, KV, D, form):            # noqa: F811
