@@ -437,18 +437,15 @@ __global__ void delta_prepare_kernel(const T* __restrict__ p, int ldp, const T* 
 }
 
 // The same for prompts whose heads have up to 128 entries in whole quads: a warp takes a unit of eight neighbouring tokens, four channels a
-// lane (8- or 16-byte loads and stores), its taps in registers, every sum inside the warp.  What bounds it is the float32 rows written; 2,048
+// lane (8-byte loads, 16-byte stores), its taps in registers, every sum inside the warp.  What bounds it is the float32 rows written; 2,048
 // tokens of 16 heads: 107 -> 44 us (the kernel above reads and computes every q and k entry twice, an entry a thread, with two
 // block-wide barriers a token).
-template <typename T> __device__ __forceinline__ float4 quad_at(const T* p) {
-    if constexpr (sizeof(T) == 4) return *reinterpret_cast<const float4*>(p);
-    else {
-        const uint2 t = *reinterpret_cast<const uint2*>(p);
-        return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u), __uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
-    }
+__device__ __forceinline__ float4 quad_at(const __nv_bfloat16* p) {
+    const uint2 t = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u), __uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
 }
-template <typename T, int TAPS>
-__global__ void __launch_bounds__(128) delta_prepare_warp_kernel(const T* __restrict__ p, int ldp, const T* __restrict__ a, int lda,
+template <int TAPS>
+__global__ void __launch_bounds__(128) delta_prepare_warp_kernel(const __nv_bfloat16* __restrict__ p, int ldp, const __nv_bfloat16* __restrict__ a, int lda,
                                      const float* __restrict__ conv, const float* __restrict__ A_log, const float* __restrict__ dt_bias,
                                      const float* __restrict__ state, long long state_stride, long long hist_off,
                                      float* __restrict__ out, int ldo, const int* __restrict__ token_seg,
@@ -472,7 +469,7 @@ __global__ void __launch_bounds__(128) delta_prepare_warp_kernel(const T* __rest
         const float4 b = *reinterpret_cast<const float4*>(dt_bias + hh * D + d);
         float4 x[TOKS];
 #pragma unroll
-        for (int k = 0; k < TOKS; ++k) if (k < toks) x[k] = quad_at<T>(a + (size_t)(t0 + k) * lda + hh * D + d);
+        for (int k = 0; k < TOKS; ++k) if (k < toks) x[k] = quad_at(a + (size_t)(t0 + k) * lda + hh * D + d);
         auto g = [&](float v) { const float sp = v > 20.f ? v : log1pf(expf(v)); return expf(-rate * sp); };
 #pragma unroll
         for (int k = 0; k < TOKS; ++k)
@@ -493,7 +490,7 @@ __global__ void __launch_bounds__(128) delta_prepare_warp_kernel(const T* __rest
 #pragma unroll
     for (int i = 0; i < TOKS + TAPS - 1; ++i) {
         const int t = t0 - (TAPS - 1) + i;
-        x[i] = live && t >= 0 && t < T_ ? quad_at<T>(p + (size_t)t * ldp + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        x[i] = live && t >= 0 && t < T_ ? quad_at(p + (size_t)t * ldp + c) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     int seg_[TOKS], first_[TOKS];                                   // looked up together as well
 #pragma unroll
@@ -1056,18 +1053,15 @@ MI_EXPORT int mi_delta_prepare(const void* p, int ldp, const void* a, int lda, c
     if (units > 65535) return -2;
     const int toks = T_ >= 1024 ? 8 : 1;
     dim3 pgrid((T_ + toks - 1) / toks, units);
-    const int el = dtype == MI_BF16 ? 2 : 4;
     // 192 tokens: a warp walks eight of them, which takes 10 us however few there are (64 tokens 10.1 us against 7.1, 96 10.2 against 8.7, 130 even,
-    // 160 with 30 of them decoded 13.6 against 12.6, 200 10.8 against 14.3)
-    const bool warps = T_ > num_segs && T_ >= 192 && taps >= 2 && taps <= 4 && D % 4 == 0 && V % 4 == 0 && D <= 128 && V <= 128 && ldp % 4 == 0 && lda % 4 == 0 && ldo % 4 == 0 &&
-                       ((uintptr_t)p | (uintptr_t)a) % (4 * el) == 0 && ((uintptr_t)out | (uintptr_t)dt_bias) % 16 == 0;
+    // 160 with 30 of them decoded 13.6 against 12.6, 200 10.8 against 14.3).  bfloat16 rows only: the norms' sums of the two kernels differ in order, and a float32 run's bits must not depend on how many tokens a step has
+    const bool warps = dtype == MI_BF16 && T_ > num_segs && T_ >= 192 && taps >= 2 && taps <= 4 && D % 4 == 0 && V % 4 == 0 && D <= 128 && V <= 128 && ldp % 4 == 0 &&
+                       lda % 4 == 0 && ldo % 4 == 0 && ((uintptr_t)p | (uintptr_t)a) % 8 == 0 && ((uintptr_t)out | (uintptr_t)dt_bias) % 16 == 0;
     if (warps) {
         const dim3 wgrid((T_ + 7) / 8, (units + 3) / 4);
-#define GO(T, TAPS) delta_prepare_warp_kernel<T, TAPS><<<wgrid, 128, 0, stream>>>((const T*)p, ldp, (const T*)a, lda, conv, A_log, dt_bias, state, state_stride, \
-                                                                                 hist_off, out, ldo, token_seg, seg_q_start, seg_slot, H, KV, D, V, unit_eps, T_)
-#define PICK(T) do { if (taps == 2) GO(T, 2); else if (taps == 3) GO(T, 3); else GO(T, 4); } while (0)
-        if (dtype == MI_BF16) PICK(__nv_bfloat16); else PICK(float);
-#undef PICK
+#define GO(TAPS) delta_prepare_warp_kernel<TAPS><<<wgrid, 128, 0, stream>>>((const __nv_bfloat16*)p, ldp, (const __nv_bfloat16*)a, lda, conv, A_log, dt_bias, state, \
+                                                                            state_stride, hist_off, out, ldo, token_seg, seg_q_start, seg_slot, H, KV, D, V, unit_eps, T_)
+        if (taps == 2) GO(2); else if (taps == 3) GO(3); else GO(4);
 #undef GO
     } else if (dtype == MI_BF16)
         delta_prepare_kernel<__nv_bfloat16><<<pgrid, 128, 0, stream>>>((const __nv_bfloat16*)p, ldp, (const __nv_bfloat16*)a, lda, conv, A_log, dt_bias,

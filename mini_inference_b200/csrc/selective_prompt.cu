@@ -8,7 +8,8 @@
 // FMA pipe, two at a time.  A block is 32 channels: eight warps walk the tokens, eight more make the next chunk of 32 tokens ready (steps, inputs, B, C to
 // shared memory) and finish the previous one (skip term, gate, store), so neither softplus nor a load is waited for; one barrier a chunk.
 // Eight tokens' partial sums are added up over the eight lanes together (seven shuffles instead of 24).  2,048 tokens: 541 -> 141 us.  The kernel in
-// which all warps do everything in turn (recurrent.cu) stays for decode steps, where there is one token a request, and for other N.
+// which all warps do everything in turn (recurrent.cu) stays for decode steps, where there is one token a request, for other N, and for
+// float32 runs: it takes every step, so a request's bits there depend on nothing but its own tokens.
 #include "common.cuh"
 #include <math.h>
 
@@ -39,11 +40,11 @@ __device__ __forceinline__ float2 exp_neg2(float2 v) {
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
 
 // grid (entries, ceil(I / 32)); L lanes of NS states each, N = L NS
-template <typename T, int L, int NS>
+template <int L, int NS>
 __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
-    const T* __restrict__ x, const float* __restrict__ dt, const float* __restrict__ dt_b, const float* __restrict__ A,
-    const T* __restrict__ B, int ldb, const T* __restrict__ Cm, int ldc, const float* __restrict__ Dv, const T* __restrict__ z, int ldz,
-    float* __restrict__ state, long long state_stride, T* __restrict__ out, const int* __restrict__ seg_q_start,
+    const __nv_bfloat16* __restrict__ x, const float* __restrict__ dt, const float* __restrict__ dt_b, const float* __restrict__ A,
+    const __nv_bfloat16* __restrict__ B, int ldb, const __nv_bfloat16* __restrict__ Cm, int ldc, const float* __restrict__ Dv, const __nv_bfloat16* __restrict__ z, int ldz,
+    float* __restrict__ state, long long state_stride, __nv_bfloat16* __restrict__ out, const int* __restrict__ seg_q_start,
     const int* __restrict__ seg_slot, int I) {
     constexpr int N = L * NS;
     __shared__ __align__(16) float Bs[2][TC][N], Cs[2][TC][N], ys[2][TC][CB];
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
         const float bias = live ? dt_b[cc] : 0.f, skip = live ? Dv[cc] : 0.f;
         constexpr int HW = HELPERS / 32, R = TC / HW, RB = (TC * N + HELPERS - 1) / HELPERS;
         float rs[R];
-        T rx[R], rB[RB], rC[RB], fx[R], fz[R];
+        __nv_bfloat16 rx[R], rB[RB], rC[RB], fx[R], fz[R];
         auto request = [&](int k) {                                 // chunk k for making ready, chunk k - 2 for finishing
             const int ta = k * TC, tb = ta - 2 * TC;
 #pragma unroll
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
                 const int tt = hw + HW * r;
                 if (live && tb >= 0 && tb + tt < n) {
                     const float xv = to_f32(fx[r]), zv = to_f32(fz[r]);
-                    out[(size_t)(qs + tb + tt) * I + cc] = from_f32<T>((ys[b][tt][lane] + skip * xv) * silu(zv));
+                    out[(size_t)(qs + tb + tt) * I + cc] = __float2bfloat16_rn((ys[b][tt][lane] + skip * xv) * silu(zv));
                 }
             }
             if (ta < n) {
@@ -181,18 +182,16 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
 
 }  // namespace
 
-// x [T, I] and out [T, I] contiguous in the run's type; dt float32 [T, I] (before bias and softplus); B, C, z: strided views; A float32
+// x [T, I] and out [T, I] contiguous bfloat16; dt float32 [T, I] (before bias and softplus); B, C, z: strided bfloat16 views; A float32
 // [I, N], N one of 8, 16, 32.
 MI_EXPORT int mi_selective_prompt(const void* x, const float* dt, const float* dt_b, const float* A, const void* B, int ldb, const void* C, int ldc,
                                   const float* Dv, const void* z, int ldz, float* state, long long state_stride, void* out,
-                                  const int* seg_q_start, const int* seg_slot, int num_segs, int I, int N, int dtype, cudaStream_t stream) {
+                                  const int* seg_q_start, const int* seg_slot, int num_segs, int I, int N, cudaStream_t stream) {
     if (num_segs == 0 || I == 0) return 0;
     const dim3 grid(num_segs, (I + CB - 1) / CB);
-#define GO(T, L, NS) selective_prompt_kernel<T, L, NS><<<grid, CB * L + HELPERS, 0, stream>>>((const T*)x, dt, dt_b, A, (const T*)B, ldb, (const T*)C, ldc, Dv, \
-                                                                              (const T*)z, ldz, state, state_stride, (T*)out, seg_q_start, seg_slot, I)
-#define PICK(T) do { if (N == 16) GO(T, 8, 2); else if (N == 8) GO(T, 4, 2); else if (N == 32) GO(T, 8, 4); else return -2; } while (0)
-    if (dtype == MI_BF16) PICK(__nv_bfloat16); else PICK(float);
-#undef PICK
+#define GO(L, NS) selective_prompt_kernel<L, NS><<<grid, CB * L + HELPERS, 0, stream>>>((const __nv_bfloat16*)x, dt, dt_b, A, (const __nv_bfloat16*)B, ldb, \
+        (const __nv_bfloat16*)C, ldc, Dv, (const __nv_bfloat16*)z, ldz, state, state_stride, (__nv_bfloat16*)out, seg_q_start, seg_slot, I)
+    if (N == 16) GO(8, 2); else if (N == 8) GO(4, 2); else if (N == 32) GO(8, 4); else return -2;
 #undef GO
     return (int)cudaGetLastError();
 }

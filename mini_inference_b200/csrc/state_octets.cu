@@ -405,15 +405,10 @@ MI_EXPORT int mi_constant_octets(const float* rows, float* scratch, const float*
                                     seg_slot, T_, num_segs, H, H, D, V, error_word, stream);
 }
 
-// p [T, ldp] = q | k | v before silu; decay [H]; otherwise as mi_delta_octets
+// p [T, ldp] bfloat16 = q | k | v before silu; decay [H]; otherwise as mi_delta_octets
 MI_EXPORT int mi_lightning_octets(const void* p, int ldp, float* scratch, const float* decay, float* state, long long state_stride, float* out,
-                                  const int* seg_q_start, const int* seg_slot, int T_, int num_segs, int H, int D, int V, int* error_word, int dtype,
-                                  cudaStream_t stream) {
-    const Source L{ldp, 0, H * D, 2 * H * D, 0, 0};
+                                  const int* seg_q_start, const int* seg_slot, int T_, int num_segs, int H, int D, int V, int* error_word, cudaStream_t stream) {
     float* values = scratch + (size_t)(T_ / C + num_segs) * H * record_floats<false>(D);
-    if (dtype == MI_BF16)
-        return run<__nv_bfloat16, false, true>((const __nv_bfloat16*)p, L, decay, scratch, values, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H,
-                                         D, V, error_word, stream);
-    return run<float, false, true>((const float*)p, L, decay, scratch, values, state, state_stride, out, seg_q_start, seg_slot, T_, num_segs, H, H, D, V, error_word,
-                             stream);
+    return run<__nv_bfloat16, false, true>((const __nv_bfloat16*)p, Source{ldp, 0, H * D, 2 * H * D, 0, 0}, decay, scratch, values, state, state_stride, out, seg_q_start,
+                                           seg_slot, T_, num_segs, H, H, D, V, error_word, stream);
 }

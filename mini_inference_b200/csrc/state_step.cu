@@ -109,11 +109,9 @@ MI_EXPORT int mi_delta_step(const float* prep, int ld, float* state, long long s
                             num_segs, H, KV, D, V, stream);
 }
 
-// p [T, ldp] = q | k | v before silu; decay [H]
+// p [T, ldp] bfloat16 = q | k | v before silu; decay [H]
 MI_EXPORT int mi_lightning_step(const void* p, int ldp, const float* decay, float* state, long long state_stride, float* out, const int* seg_q_start,
-                                const int* seg_slot, int num_segs, int H, int D, int V, int dtype, cudaStream_t stream) {
-    const StepSource L{ldp, 0, H * D, 2 * H * D, 0, 0};
-    if (dtype == MI_BF16)
-        return run<__nv_bfloat16, false>((const __nv_bfloat16*)p, L, decay, state, state_stride, out, seg_q_start, seg_slot, num_segs, H, H, D, V, stream);
-    return run<float, false>((const float*)p, L, decay, state, state_stride, out, seg_q_start, seg_slot, num_segs, H, H, D, V, stream);
+                                const int* seg_slot, int num_segs, int H, int D, int V, cudaStream_t stream) {
+    return run<__nv_bfloat16, false>((const __nv_bfloat16*)p, StepSource{ldp, 0, H * D, 2 * H * D, 0, 0}, decay, state, state_stride, out, seg_q_start, seg_slot,
+                                     num_segs, H, H, D, V, stream);
 }

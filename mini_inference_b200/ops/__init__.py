@@ -78,6 +78,7 @@ class CudaOps:
     prefill_tile = 64
     deferred = True                          # linear(..., defer=True) may answer with a DeferredSum
     takes_hints = True                       # add_rmsnorm(..., next_weight=) is understood
+    exact_scans = True                       # delta_scan(..., exact=) is understood
     MAX_ROWS = 4096                          # decode rows x kv heads that the attention merge counters cover
 
     def __init__(self, device):
@@ -711,6 +712,9 @@ class CudaOps:
         return y
 
     # ---------------------------------------------------------------- matrix-state recurrences
+    # bfloat16 runs take the kernel that suits the step (one token per entry; eight tokens at a time; token by token).  Those add in different
+    # orders, and which one runs depends on everything in the step, so float32 runs keep the token-by-token kernels: there a request's bits do
+    # not depend on where its prompt is cut or on what runs beside it.
     @staticmethod
     def _takes_step(T, batch, D, V, state):
         """Whether a step's recurrence has a whole state in a block's registers (csrc/state_step.cu): one token per entry, sizes of 64 or 128,
@@ -737,16 +741,17 @@ class CudaOps:
         T = p.shape[0]
         assert p.stride(1) == 1 and state.dtype == torch.float32 and state.is_contiguous()
         out = torch.empty((T, H * V), dtype=torch.float32, device=p.device)
-        if self._takes_step(T, batch, D, V, state):
+        wide = p.dtype == torch.bfloat16
+        if wide and self._takes_step(T, batch, D, V, state):
             _check(self.lib.mi_lightning_step(_p(p), p.stride(0), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                              _p(batch.seg_slot), T, H, D, V, _code(p.dtype), self._stream()), "lightning_step")
+                                              _p(batch.seg_slot), T, H, D, V, self._stream()), "lightning_step")
             self.launches += 1
             return out
-        if self._takes_octets(p, batch, D, V, state):
+        if wide and self._takes_octets(p, batch, D, V, state):
             scratch = self._octet_scratch(T, batch, H, D, V, False)
             _check(self.lib.mi_lightning_octets(_p(p), p.stride(0), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
                                                 _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error),
-                                                _code(p.dtype), self._stream()), "lightning_octets")
+                                                self._stream()), "lightning_octets")
             self.launches += 2
             return out
         prep = torch.empty((T, 2 * H * D + H * V), dtype=torch.float32, device=p.device)      # silu(q | k | v), what the scan stages
@@ -773,16 +778,17 @@ class CudaOps:
         self.launches += 2 if taps > 1 and not (T == batch.num_segs and T < 256) else 1
         return out
 
-    def delta_scan(self, prep, H, KV, D, V, state, batch):
-        """S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q per head, token by token.  float32 [T, H V]."""
+    def delta_scan(self, prep, H, KV, D, V, state, batch, exact=False):
+        """S <- diag(g) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q per head.  float32 [T, H V].  exact: token by token, as float32
+        runs want it."""
         T = prep.shape[0]
         out = torch.empty((T, H * V), dtype=torch.float32, device=prep.device)
-        if self._takes_step(T, batch, D, V, state):
+        if not exact and self._takes_step(T, batch, D, V, state):
             _check(self.lib.mi_delta_step(_p(prep), prep.stride(0), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
                                           _p(batch.seg_slot), T, H, KV, D, V, self._stream()), "delta_step")
             self.launches += 1
             return out
-        if self._takes_octets(prep, batch, D, V, state):
+        if not exact and self._takes_octets(prep, batch, D, V, state):
             scratch = self._octet_scratch(T, batch, H, D, V, True)
             _check(self.lib.mi_delta_octets(_p(prep), prep.stride(0), _p(scratch), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
                                             _p(batch.seg_slot), T, batch.num_segs, H, KV, D, V, _p(self._stream_error), self._stream()), "delta_octets")
@@ -1112,7 +1118,7 @@ class CudaOps:
         half = 0 if inv_freq is None else inv_freq.numel()
         _check(self.lib.mi_retention_rows(_p(p), p.stride(0), _p(prep), _p(batch.positions), _p(inv_freq), half, _c.c_float(k_scale), T, H, D, V,
                                           _code(p.dtype), self._stream()), "retention_rows")
-        if self._takes_octets(prep, batch, D, V, state):
+        if p.dtype == torch.bfloat16 and self._takes_octets(prep, batch, D, V, state):
             scratch = self._octet_scratch(T, batch, H, D, V, False)
             _check(self.lib.mi_constant_octets(_p(prep), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
                                                _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error), self._stream()), "constant_octets")
@@ -1390,10 +1396,10 @@ class CudaOps:
             dt = dt.float()
         assert dt.is_contiguous()
         out = torch.empty((T, I), dtype=out_dtype, device=x.device)
-        if T > batch.num_segs and N in (8, 16, 32):          # a step with prompt portions (one token a request: the kernel below)
+        if x.dtype == torch.bfloat16 and T > batch.num_segs and N in (8, 16, 32):        # a step with prompt portions (one token a request, float32 runs: the kernel below)
             _check(self.lib.mi_selective_prompt(
                 _p(x), _p(dt), _p(dt_b), _p(A), _p(B), B.stride(0), _p(C), C.stride(0), _p(Dv), _p(z), z.stride(0), _p(state),
-                _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, I, N, _code(x.dtype),
+                _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, I, N,
                 self._stream()), "selective_prompt")
             self.launches += 1
             return out

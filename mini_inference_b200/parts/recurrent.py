@@ -144,7 +144,8 @@ class ChannelDeltaRule(Part):
         a, gate = ag[:, :H * D], ag[:, H * D:]
         prep = ops.delta_prepare(p, a, self.conv, self.A_log, self.dt_bias, H, KV, D, V, self.taps, self.unit_eps,
                                  cache.state, ctx.batch)            # float32 q | k | v | beta | g per token; conv tail -> state
-        o = ops.delta_scan(prep, H, KV, D, V, cache.state, ctx.batch)                   # float32 [T, H V]
+        exact = {"exact": True} if p.dtype == torch.float32 and getattr(ops, "exact_scans", False) else {}
+        o = ops.delta_scan(prep, H, KV, D, V, cache.state, ctx.batch, **exact)          # float32 [T, H V]
         rows = ops.group_rmsnorm_gate(o, self.norm, gate, self.eps, H, V, ctx.dtype)
         return rows, self.o
 

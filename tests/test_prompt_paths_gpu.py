@@ -177,6 +177,48 @@ def test_selective_scan_of_prompts(ops, dtype, lens, inner, N):         # noqa: 
     assert rows_error(got, want) < (3e-6 if dtype == torch.float32 else 4e-3)        # bfloat16: the output's own rounding may fall differently
 
 
+def recurrent_part(kind):
+    """One recurrent mixer of a design, float32, with seeded weights, and the context of a step of [(slot, tokens)] over given states."""
+    import types
+    from mini_inference_b200.config.spec import PartSpec
+    from mini_inference_b200.parts.base import build_part
+    base = dict(hidden_size=96, num_heads=2, key_dim=64, value_dim=64, out_norm_eps=1e-6)
+    spec = {"lightning": PartSpec.of("lightning", decay=(0.9, 0.99), **base), "retention": PartSpec.of("retention", decay=(0.9, 0.99), **base),
+            "channel_delta": PartSpec.of("channel_delta", num_kv_heads=1, conv_taps=4, unit_eps=1e-6, decay_rank=16, gate_rank=16, **base),
+            "selective_scan": PartSpec.of("selective_scan", hidden_size=96, inner=64, state=16, dt_rank=8, conv_taps=4)}[kind]
+    part, g = build_part("mixer", spec), torch.Generator().manual_seed(11)
+    part.load({w.name: (torch.randn(w.shape, generator=g) * (0.3 if len(w.shape) > 1 else 0.5)).to(DEV) for w in part.weight_specs()}, torch.float32, DEV)
+    return part, types.SimpleNamespace(rotary_inv_freq=lambda: None)
+
+
+@pytest.mark.parametrize("kind", ["lightning", "retention", "channel_delta", "selective_scan"])
+def test_float32_recurrences_do_not_see_the_batch(ops, kind):   # noqa: F811
+    """A float32 run's outputs and states are the same bits whether a prompt comes whole or in two portions, alone or beside others.  (Steps of
+    more than four tokens an entry: below that the matrix recurrences' scan sums over eight lanes instead of sixteen.)"""
+    import types
+    part, position = recurrent_part(kind)
+    floats = part.cache_need().shape[0]
+    g = torch.Generator().manual_seed(12)
+    h, other = torch.randn(600, 96, generator=g).to(DEV), torch.randn(700, 96, generator=g).to(DEV)
+
+    def step(state, lens, slots, rows, pos0):
+        batch = Entries(lens)
+        batch.seg_slot = torch.tensor(slots, dtype=torch.int32, device=DEV)
+        batch.token_seg = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().to(DEV)
+        batch.positions = torch.cat([torch.arange(p, p + n) for p, n in zip(pos0, lens)]).int().to(DEV)
+        batch.max_q_len = max(lens)
+        ctx = types.SimpleNamespace(ops=ops, batch=batch, dtype=torch.float32)
+        return part.forward(rows, ctx, types.SimpleNamespace(state=state), position)
+
+    whole = torch.zeros(4, floats, device=DEV)
+    want = step(whole, (600,), (1,), h, (0,))
+    cut = torch.zeros(4, floats, device=DEV)
+    got = [step(cut, (45,), (1,), h[:45], (0,)), step(cut, (97, 700, 1), (1, 3, 2), torch.cat([h[45:142], other, h[:1]]), (45, 0, 0))[:97],
+           step(cut, (458, 1), (1, 2), torch.cat([h[142:], h[:1]]), (142, 1))[:458]]
+    assert torch.equal(torch.cat(got), want)
+    assert torch.equal(cut[1], whole[1])
+
+
 def test_silu_keeps_its_float32(ops):                           # noqa: F811
     """The filter's activation and the scan's gate of bfloat16 prompts are float32's silu rounded once, down to inputs where 1 + e^-x is nearly
     the largest float32: the fast exponential is 4e-4 off at -80 (a tenth of a bfloat16 step) and the fast quotient 0 from -87.4 on."""
