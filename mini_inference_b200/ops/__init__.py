@@ -724,11 +724,11 @@ class CudaOps:
     @staticmethod
     def _takes_octets(rows, batch, D, V, state):
         """Whether a step's recurrence goes eight tokens at a time (csrc/state_octets.cu): keys of 64 or 128, values in blocks of 16 columns, states
-        of an even number of floats on 8 bytes, rows whose heads start on 16 bytes, and a prompt of at least 128 tokens (with 96 the token-by-token kernel's
-        26 us are hidden behind the host's launches and the second launch costs 7 us, with 192 the mixer takes 87 us instead of 100) or 512
-        tokens in all (16 prompts of 64: 107 us instead of 216)."""
+        of an even number of floats on 8 bytes, rows whose heads start on 16 bytes, and a prompt of at least 192 tokens (a channel-delta mixer of 150
+        takes 87 us instead of 86, 130 tokens 87 instead of 81: the token-by-token kernel is hidden behind the host's launches there, and this
+        way has one more; with 192 87 us instead of 100) or 512 tokens in all (16 prompts of 64: 107 us instead of 216)."""
         T = rows.shape[0]
-        return (T > 4 * batch.num_segs and (T >= 512 or getattr(batch, "max_q_len", T) >= 128) and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
+        return (T > 4 * batch.num_segs and (T >= 512 or (T >= 128 and getattr(batch, "max_q_len", 192) >= 192)) and D in (64, 128) and V % 16 == 0 and state.stride(0) % 2 == 0
                 and state.data_ptr() % 8 == 0 and rows.stride(0) % 4 == 0 and rows.data_ptr() % 16 == 0)
 
     def _octet_scratch(self, T, batch, H, D, V, delta):

@@ -43,3 +43,11 @@ def test_as_many_tokens_as_entries_is_not_one_each():
     state = off_by(0, 3, 64 * 64)
     assert CudaOps._takes_step(2, step((1, 1)), 64, 64, state)
     assert not CudaOps._takes_step(2, step((2, 0)), 64, 64, state)
+
+
+def test_line_of_the_eight_token_scans():
+    """A prompt of 192 tokens or 512 tokens in all; shorter steps wait for the host, and this way has one launch more."""
+    rows, state = off_by(0, 600, 3 * 128), off_by(0, 2, 64 * 64)
+    takes = lambda *lens: CudaOps._takes_octets(rows[:sum(lens)], step(lens), 64, 64, state)      # noqa: E731
+    assert takes(192) and takes(192, *[1] * 40) and not takes(191) and not takes(64, 64, 64)
+    assert takes(*[64] * 8) and not takes(*[63] * 8)
