@@ -151,6 +151,27 @@ def test_recurrences_eight_tokens_at_a_time(ops, lens, H, KV, D, V):        # no
         assert torch.equal(a[:, H * D * V:], state[:, H * D * V:]) and torch.equal(a[0], state[0])
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_octets_keep_later_tokens_out(ops, value):              # noqa: F811
+    """A value that is no number reaches its own token and the ones after it; the tokens before it in its octet give the bits they give without it."""
+    lens, H, D, V, at = (140, 133), 2, 128, 32, 13               # token 13: the sixth of the first entry's second octet
+    T, batch, g = sum(lens), Entries(lens), torch.Generator().manual_seed(7)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
+    batch.positions = torch.arange(T, dtype=torch.int32, device=DEV)
+    C, constant, state = 2 * H * D + H * V, torch.tensor([0.9, 0.99], device=DEV), r(3, H * D * V)
+    prep = torch.cat([0.05 * r(T, 2 * H * D), r(T, H * V), torch.rand(T, H * D + 4, generator=g).to(DEV)], dim=1)
+    p = r(T, C).to(torch.bfloat16)
+    runs = {"delta": (prep, lambda x, s: ops.delta_scan(x, H, H, D, V, s, batch)), "constant": (p, lambda x, s: ops.lightning_scan(x, H, D, V, constant, s, batch)),
+            "rotated": (p, lambda x, s: ops.retention_scan(x, H, D, V, None, 1.0, constant, s, batch))}
+    for name, (rows, run) in runs.items():
+        assert ops._takes_octets(rows, batch, D, V, state), name
+        spoiled = rows.clone()
+        spoiled[at, 2 * H * D + 3] = value                       # one value of head 0
+        want, got = run(rows, state.clone()), run(spoiled, state.clone())
+        assert torch.equal(got[:at], want[:at]) and torch.equal(got[lens[0]:], want[lens[0]:]), name
+        assert not got[at, 3].isfinite() and torch.equal(got[:, V:], want[:, V:]), name
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("lens,inner,N", [((33, 1, 64), 40, 16), ((5, 100), 96, 8), ((31, 2), 33, 32), ((70,), 64, 16)])
 def test_selective_scan_of_prompts(ops, dtype, lens, inner, N):         # noqa: F811
