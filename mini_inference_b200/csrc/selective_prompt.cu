@@ -12,6 +12,7 @@
 // float32 runs: it takes every step, so a request's bits there depend on nothing but its own tokens.
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 
 using namespace mi;
 
@@ -19,23 +20,27 @@ namespace {
 
 constexpr int TC = 32, CB = 32, HELPERS = 256;
 
-// e^v of two numbers at once for v <= 0: n = round(v / ln 2), e^v = 2^n e^(v - n ln 2), the second factor as 1 + f + f^2 P(f) with P of degree
-// 3 fitted to (e^f - 1 - f) / f^2 on |f| <= ln 2 / 2.  The largest relative error is 1.1e-7 at |f| = ln 2 / 2 and falls with f^2 towards
-// 1, where a decay acts hundreds of times in a row (ex2.approx is 2 ulp off there and the states' error was three times as large).
-__device__ __forceinline__ float2 exp_neg2(float2 v) {
-    v = make_float2(fmaxf(v.x, -87.f), fmaxf(v.y, -87.f));
-    const float2 big = make_float2(12582912.f, 12582912.f);        // 1.5 * 2^23: the sum's low bits are the rounded integer
-    const float2 t = __ffma2_rn(v, make_float2(1.4426950408889634f, 1.4426950408889634f), big);
-    const float2 n = __fadd2_rn(t, make_float2(-12582912.f, -12582912.f));
-    const float2 f = __ffma2_rn(n, make_float2(-0.69314718055994531f, -0.69314718055994531f), v);
-    float2 p = make_float2(0.0083124945f, 0.0083124945f);
-    p = __ffma2_rn(p, f, make_float2(0.041890331f, 0.041890331f));
-    p = __ffma2_rn(p, f, make_float2(0.16667116f, 0.16667116f));
-    p = __ffma2_rn(p, f, make_float2(0.49999231f, 0.49999231f));
-    const float2 one = make_float2(1.f, 1.f);
-    p = __ffma2_rn(__ffma2_rn(p, f, one), f, one);
-    return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(t.x) << 23)), __int_as_float(__float_as_int(p.y) + (__float_as_int(t.y) << 23)));
+// e^(step A) of two states at once.  hi + lo is A log2(e) to twice float32's bits, so the rounded product of step and A enters nowhere:
+// n = round(step hi), f = step hi - n + step lo, e^(step A) = 2^n 2^f, 2^f a polynomial of degree 6 fitted to (2^f - 1) / f on |f| <= 1/2
+// (weighted minimax, 2e-9).  Largest and mean error relative to e^(step A) of the exact product: 9.5e-8 and 2.3e-8 for step A down to -86,
+// falling with f towards 1, where a decay acts hundreds of times in a row (expf(step * A): 1.4e-7 and 3.2e-8 even where the product is
+// exact, up to 4e-6 at -86 where it is not).  Below 2^-125 the exponent stays there: about 2e-38 instead of less.
+// Takes -1000 <= A <= 0 and 0 <= step <= 1e6 (f stays small where n is past the integers that float32 holds): other numbers go to expf.
+__device__ __forceinline__ float2 decay2(float step, float2 hi, float2 lo) {
+    const float2 st = make_float2(step, step), big = make_float2(12582912.f, 12582912.f);        // 1.5 * 2^23: the sum's low bits are the rounded integer
+    const float2 t = __ffma2_rn(st, hi, big);
+    const float2 f = __ffma2_rn(st, lo, __ffma2_rn(st, hi, __ffma2_rn(t, make_float2(-1.f, -1.f), big)));
+    float2 p = make_float2(1.5476350e-4f, 1.5476350e-4f);
+    p = __ffma2_rn(p, f, make_float2(1.3400323e-3f, 1.3400323e-3f));
+    p = __ffma2_rn(p, f, make_float2(9.6180039e-3f, 9.6180039e-3f));
+    p = __ffma2_rn(p, f, make_float2(5.5503275e-2f, 5.5503275e-2f));
+    p = __ffma2_rn(p, f, make_float2(0.24022651f, 0.24022651f));
+    p = __ffma2_rn(p, f, make_float2(0.69314718f, 0.69314718f));
+    p = __ffma2_rn(p, f, make_float2(1.f, 1.f));
+    const float ex = fmaxf(t.x, 12582912.f - 125.f), ey = fmaxf(t.y, 12582912.f - 125.f);
+    return make_float2(__int_as_float(__float_as_int(p.x) + (__float_as_int(ex) << 23)), __int_as_float(__float_as_int(p.y) + (__float_as_int(ey) << 23)));
 }
+constexpr float LEAST_A = -1000.f, MOST_STEP = 1e6f;
 
 __device__ __forceinline__ float silu(float z) { return z / (1.f + expf(-z)); }
 
@@ -84,8 +89,10 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
             }
         };
         request(0);
+        int unusual = 0;                                            // a step of the chunk made ready last is none that decay2 takes
         for (int k = -1; k <= chunks; ++k) {                        // makes chunk k + 1 ready, finishes chunk k - 1
-            if (k >= 0) __syncthreads();
+            if (k >= 0) __syncthreads_or(unusual);
+            unusual = 0;
             const int ta = (k + 1) * TC, tb = (k - 1) * TC, b = (k + 1) & 1;        // chunks k - 1 and k + 1 use the same buffers
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -103,6 +110,7 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
                     if (live && ta + tt < n) {
                         const float d = rs[r] + bias;
                         v.x = d > 20.f ? d : log1pf(expf(d));
+                        if (!(v.x <= MOST_STEP)) unusual = 1;
                         v.y = v.x * to_f32(rx[r]);
                     }
                     in[b][tt][lane] = v;
@@ -126,53 +134,66 @@ __global__ void __launch_bounds__(CB * L + HELPERS, 1) selective_prompt_kernel(
     const int l = lane % L, cl = warp * CW + lane / L, c = c0 + cl;
     const bool live = c < I;
     float* S = state + (long long)seg_slot[seg] * state_stride + (size_t)(live ? c : 0) * N + l * NS;
-    float2 s[NS / 2], a[NS / 2];
+    const float* ar = A + (size_t)(live ? c : 0) * N + l * NS;
+    float2 s[NS / 2], hi[NS / 2], lo[NS / 2];
+    bool usual = true;
 #pragma unroll
     for (int g = 0; g < NS / 2; ++g) {
-        s[g] = a[g] = make_float2(0.f, 0.f);
+        s[g] = hi[g] = lo[g] = make_float2(0.f, 0.f);
         if (live) {
+            constexpr float H = 1.44269504f, R = 1.92596299e-8f;    // log2(e) = H + R
             s[g] = make_float2(S[2 * g], S[2 * g + 1]);
-            const float* ar = A + (size_t)c * N + l * NS + 2 * g;
-            a[g] = make_float2(ar[0], ar[1]);
+            const float2 a = make_float2(ar[2 * g], ar[2 * g + 1]);
+            hi[g] = make_float2(a.x * H, a.y * H);
+            lo[g] = make_float2(fmaf(a.x, R, fmaf(a.x, H, -hi[g].x)), fmaf(a.y, R, fmaf(a.y, H, -hi[g].y)));
+            usual = usual && a.x >= LEAST_A && a.x <= 0.f && a.y >= LEAST_A && a.y <= 0.f;
         }
     }
+    usual = __all_sync(0xffffffffu, usual);
     for (int k = 0; k <= chunks; ++k) {
-        __syncthreads();
+        const bool fast = !__syncthreads_or(0) && usual;
         if (k == chunks) break;                                     // the helpers finish the last chunk
         const int b = k & 1;
+        auto walk = [&](auto usual_numbers) {                       // one loop body each: a branch between decays and chain would keep them from overlapping
 #pragma unroll 1
-        for (int t0 = 0; t0 < TC; t0 += L) {
-            float y[L];
-            float2 decay[L][NS / 2];                                // not part of the chain from token to token: made side by side
+            for (int t0 = 0; t0 < TC; t0 += L) {
+                float y[L];
+                float2 decay[L][NS / 2];                            // not part of the chain from token to token: made side by side
 #pragma unroll
-            for (int e = 0; e < L; ++e) {
-                const float step = in[b][t0 + e][cl].x;
+                for (int e = 0; e < L; ++e) {
+                    const float step = in[b][t0 + e][cl].x;
+                    const bool behind = k * TC + t0 + e >= n;       // a token behind the entry's last: no decay, whatever A is
 #pragma unroll
-                for (int g = 0; g < NS / 2; ++g) decay[e][g] = exp_neg2(__fmul2_rn(make_float2(step, step), a[g]));
-            }
-#pragma unroll
-            for (int e = 0; e < L; ++e) {
-                const float sx = in[b][t0 + e][cl].y;
-                float2 sum = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int g = 0; g < NS / 2; ++g) {
-                    const float2 bv = *reinterpret_cast<const float2*>(&Bs[b][t0 + e][l * NS + 2 * g]);
-                    const float2 cv = *reinterpret_cast<const float2*>(&Cs[b][t0 + e][l * NS + 2 * g]);
-                    s[g] = __ffma2_rn(decay[e][g], s[g], __fmul2_rn(make_float2(sx, sx), bv));
-                    sum = __ffma2_rn(s[g], cv, sum);
+                    for (int g = 0; g < NS / 2; ++g) {
+                        if (decltype(usual_numbers)::value) decay[e][g] = decay2(step, hi[g], lo[g]);
+                        else decay[e][g] = behind ? make_float2(1.f, 1.f) : make_float2(expf(step * ar[2 * g]), expf(step * ar[2 * g + 1]));
+                    }
                 }
-                y[e] = sum.x + sum.y;
-            }
-            // L sums over L lanes together: half of what is left changes hands at every step, lane l ends with token t0 + l
 #pragma unroll
-            for (int w = 1; w < L; w <<= 1)
+                for (int e = 0; e < L; ++e) {
+                    const float sx = in[b][t0 + e][cl].y;
+                    float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
-                for (int e = 0; e < L; e += 2 * w) {
-                    const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
-                    y[e] = (l & w ? y[e + w] : y[e]) + got;
+                    for (int g = 0; g < NS / 2; ++g) {
+                        const float2 bv = *reinterpret_cast<const float2*>(&Bs[b][t0 + e][l * NS + 2 * g]);
+                        const float2 cv = *reinterpret_cast<const float2*>(&Cs[b][t0 + e][l * NS + 2 * g]);
+                        s[g] = __ffma2_rn(decay[e][g], s[g], __fmul2_rn(make_float2(sx, sx), bv));
+                        sum = __ffma2_rn(s[g], cv, sum);
+                    }
+                    y[e] = sum.x + sum.y;
                 }
-            ys[b][t0 + l][cl] = y[0];
-        }
+                // L sums over L lanes together: half of what is left changes hands at every step, lane l ends with token t0 + l
+#pragma unroll
+                for (int w = 1; w < L; w <<= 1)
+#pragma unroll
+                    for (int e = 0; e < L; e += 2 * w) {
+                        const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
+                        y[e] = (l & w ? y[e + w] : y[e]) + got;
+                    }
+                ys[b][t0 + l][cl] = y[0];
+            }
+        };
+        if (fast) walk(std::true_type{}); else walk(std::false_type{});
     }
     if (live) {
 #pragma unroll

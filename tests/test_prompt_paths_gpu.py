@@ -181,7 +181,7 @@ def test_selective_scan_of_prompts(ops, dtype, lens, inner, N):         # noqa: 
     x, z, B, C = (r(T, w).to(dtype).to(DEV) for w in (inner, inner, N, N))
     dt, dt_b, Dv = r(T, inner).to(DEV), r(inner).to(DEV), r(inner).to(DEV)
     A = -torch.exp(r(inner, N)).to(DEV)
-    A[:, 0] = -300.0                                             # a decay of e^-87 and less is 0
+    A[:, 0] = -300.0                                             # decays of e^-87 and less: 2e-38 at most in the one kernel, down to 0 in the other
     state = r(len(lens) + 1, inner * N + 4).to(DEV)
     a, b = state.clone(), state.clone()
     batch = Entries(lens)
@@ -258,6 +258,45 @@ def test_silu_keeps_its_float32(ops):                           # noqa: F811
         # a double rounding may fall the other way where the float32 value lies within its own error of the middle: 2e-7 / 2^-8 of the values
         assert (got != want[:, None]).float().mean().item() < 5e-3
         assert ((got.double() / want.double()[:, None] - 1).abs().nan_to_num() <= 2 ** -7).all()
+
+
+def states_after_one_decay(ops, A, step, N=16):
+    """What a prompt leaves of states that were 1: its first token has the given step, the other 47 a step of 0, and no token adds anything."""
+    T, inner = 48, A.shape[0]
+    dt = torch.full((T, inner), -200.0, device=DEV)              # softplus: 0
+    dt[0] = step                                                # softplus of more than 20: itself
+    z = torch.zeros(T, inner, dtype=torch.bfloat16, device=DEV)
+    bc, zero, state = torch.zeros(T, N, dtype=torch.bfloat16, device=DEV), torch.zeros(inner, device=DEV), torch.ones(2, inner * N, device=DEV)
+    ops.selective_scan(z, dt, zero, A.contiguous(), bc, bc, zero, z, state, Entries((T,)), torch.bfloat16)
+    return state[1].view(inner, N)
+
+
+@pytest.mark.parametrize("step", [32.0, 21.7])
+def test_decays_of_the_selective_scan(ops, step):               # noqa: F811
+    """e^(step A) over its whole range against 64 bits: no worse than expf of the rounded product, which is within 2 units in the last place."""
+    g = torch.Generator().manual_seed(1)
+    for lo, hi in ((1e-4, 1e-2), (1e-2, 0.1), (0.1, 1), (1, 5), (5, 20), (20, 50), (50, 86)):
+        A = (-(torch.rand(2048, 16, generator=g, dtype=torch.float64) * (hi - lo) + lo) / step).float().to(DEV)
+        product = A.double() * torch.tensor(step, device=DEV).float().double()
+        got = (states_after_one_decay(ops, A, step).double() / product.exp() - 1).abs()
+        expf = ((A * step).exp().double() / product.exp() - 1).abs()
+        # half a unit of the result (6e-8 above a power of two) and of the sum before it; expf's own mean is 2.7e-8 to 3.2e-8
+        assert got.max().item() < max(1.0e-7, expf.max().item()) and got.mean().item() <= 1.02 * expf.mean().item(), (lo, hi)
+    far = states_after_one_decay(ops, torch.full((32, 16), -200.0 / step, device=DEV), step)
+    assert 0 <= far.min().item() and far.max().item() < 1e-37
+
+
+def test_unusual_decays_of_the_selective_scan(ops):             # noqa: F811
+    """Rates that are no number, not negative or huge, and steps beyond any softplus of a sane input, go where expf takes them."""
+    nan = float("nan")
+    A = torch.full((96, 16), -0.5, device=DEV)
+    A[3, 2], A[40, 1], A[41, 5], A[70, 0], A[70, 1], A[71, 9] = nan, 1.5, -3e38, 0.0, -1e30, 3.0e3
+    for step in (24.0, 1e9):
+        want = (step * A).exp()
+        got = states_after_one_decay(ops, A, step)
+        assert got[3, 2].isnan() and got[~A.isnan()].allclose(want[~A.isnan()], rtol=3e-7, atol=1e-37)
+    small = torch.full((32, 16), -1e-9, device=DEV)             # a huge step times a tiny rate
+    assert states_after_one_decay(ops, small, 1e9).allclose((small * 1e9).exp(), rtol=3e-7)
 
 
 @pytest.mark.parametrize("H,KV,D", [(16, 8, 128), (3, 1, 64), (5, 5, 128)])
