@@ -1384,6 +1384,15 @@ class CudaOps:
         self.launches += 3 if T == batch.num_segs else 5
         return y
 
+    @staticmethod
+    def _takes_prompt_scan(T, batch):
+        """Whether a step's selective scan takes the kernel for prompts (csrc/selective_prompt.cu).  A block of it has an SM to itself and walks
+        chunks of 32 tokens: about 3 us an entry, however short, and 0.06 a token.  The other kernel takes 0.235 us a token of the longest entry or 0.083
+        a token of the step, whichever is more (4,096 channels).  Prompt kernel / other: 24 tokens 5.4 / 7.0 us, 24 x 4 17 / 12, 100 x 4 42 / 42,
+        260 x 4 87 / 106, 24 x 16 58 / 33, 130 and five decoded 36 / 42, 74 and five 28 / 25, 130 and 30 112 / 52, 1,024 and 63 315 / 345."""
+        S, longest = batch.num_segs, getattr(batch, "max_q_len", T - batch.num_segs + 1)
+        return 47 * longest > 600 * S + 12 * T or T > 130 * S
+
     def selective_scan(self, x, dt, dt_b, A, B, C, Dv, z, state, batch, out_dtype):
         """S[c, n] <- exp(step_c A[c, n]) S[c, n] + step_c x_c B_n, step = softplus(dt + dt_b); y_c = sum_n S[c, n] C_n + Dv_c x_c;
         returns y * silu(z) in out_dtype.  x [T, I] contiguous; dt [T, I] in the run's dtype or float32; B, C [T, N] and z [T, I] may be
@@ -1396,7 +1405,7 @@ class CudaOps:
             dt = dt.float()
         assert dt.is_contiguous()
         out = torch.empty((T, I), dtype=out_dtype, device=x.device)
-        if x.dtype == torch.bfloat16 and T > batch.num_segs and N in (8, 16, 32):        # a step with prompt portions (one token a request, float32 runs: the kernel below)
+        if x.dtype == torch.bfloat16 and N in (8, 16, 32) and self._takes_prompt_scan(T, batch):
             _check(self.lib.mi_selective_prompt(
                 _p(x), _p(dt), _p(dt_b), _p(A), _p(B), B.stride(0), _p(C), C.stride(0), _p(Dv), _p(z), z.stride(0), _p(state),
                 _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, I, N,

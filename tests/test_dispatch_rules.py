@@ -51,3 +51,11 @@ def test_line_of_the_eight_token_scans():
     takes = lambda *lens: CudaOps._takes_octets(rows[:sum(lens)], step(lens), 64, 64, state)      # noqa: E731
     assert takes(192) and takes(192, *[1] * 40) and not takes(191) and not takes(64, 64, 64)
     assert takes(*[64] * 8) and not takes(*[63] * 8)
+
+
+def test_line_of_the_selective_scan():
+    """An entry costs the kernel for prompts about the same however short it is, the other one walks the longest entry at a quarter of the speed."""
+    takes = lambda *lens: CudaOps._takes_prompt_scan(sum(lens), step(lens))      # noqa: E731
+    assert takes(18) and not takes(17) and not takes(1) and not takes(1, 1)
+    assert takes(40, 1) and takes(130, *[1] * 5) and not takes(74, *[1] * 5) and not takes(2, *[1] * 63)
+    assert takes(*[140] * 4) and not takes(*[100] * 4) and not takes(*[24] * 16) and takes(2048, *[1] * 63)

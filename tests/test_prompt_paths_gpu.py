@@ -299,6 +299,13 @@ def test_unusual_decays_of_the_selective_scan(ops):             # noqa: F811
     assert states_after_one_decay(ops, small, 1e9).allclose((small * 1e9).exp(), rtol=3e-7)
 
 
+@pytest.mark.parametrize("lens,inner,N", [((61, 40), 33, 32), ((70, 1, 33), 40, 8)])
+def test_selective_scan_of_prompts_with_other_states(ops, lens, inner, N):      # noqa: F811
+    """The same with 8 and 32 states a channel, in steps whose portions are long enough for the prompt kernel."""
+    assert ops._takes_prompt_scan(sum(lens), Entries(lens))
+    test_selective_scan_of_prompts(ops, torch.bfloat16, lens, inner, N)
+
+
 @pytest.mark.parametrize("H,KV,D", [(16, 8, 128), (3, 1, 64), (5, 5, 128)])
 @pytest.mark.parametrize("form", ["unit", "weights_rotated", "all_rotated", "temperature_keys", "blend", "plain"])
 def test_unit_heads_of_prompts(ops, H, KV, D, form):            # noqa: F811
