@@ -27,6 +27,10 @@ def load_library():
         path = build()
         _LIB = ctypes.CDLL(path)
         _LIB.mi_gemm_f32_workspace.restype = _LIB.mi_octet_floats.restype = ctypes.c_longlong
+        # declared, so that addresses and floats pass as plain numbers: with wrapped ones the call cost the host 22.7 us where the
+        # values are the keys and 17.3 elsewhere, now 16.0 and 16.3 (the mma.sync form 14.5), and a step of few tokens waits for the host
+        p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+        _LIB.mi_attn_prefill_tc_split.argtypes = [p, i, i, p, p, ctypes.c_longlong, p, p, i, p, p, p, p, i, i, i, i, i, i, f, i, p, i, i, p, p, i, p, f, i, p, i, p]
     return _LIB
 
 
@@ -490,7 +494,7 @@ class CudaOps:
         if code != 0:
             self._stream_error.zero_()
             self._tc2_counters.zero_()
-            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21+ attention, 51-55 gemm_tc2, 61-63 grouped expert product, 71-72 delta rule)")
+            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-63 grouped expert product, 71-72 delta rule)")
 
     # ---------------------------------------------------------------- q/k norm, rotation, cache write
     def qk_norm_rope_cache(self, qkv, H, KV, D, q_weight, k_weight, eps, inv_freq, meta, k_cache, v_cache):
@@ -564,7 +568,7 @@ class CudaOps:
                 and q.data_ptr() % 16 == 0)
         tc = (fast and self.tc_attention and num_tiles and meta.tile == 64 and meta.page_size % 8 == 0
               and 64 % meta.page_size == 0 and num_tiles2)
-        if tc and split_weights and meta.max_kv_len >= self.SPLIT_TC_KEYS:
+        if tc and split_weights and self._takes_split_tc(T, meta, self.SPLIT_TC_LATENT):
             self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
         elif tc and not split_weights:
             rc = self.lib.mi_attn_prefill_tc(
@@ -626,19 +630,28 @@ class CudaOps:
             self.launches += 2 if S > 1 else 1
         return out
 
-    # Prompts whose longest request sees fewer keys stay on the mma.sync forms: both kernels' time is hidden behind the host's launches there, and the
-    # query's tensor map costs 2 us of those (192 keys: 51 against 53 us a mixer; 2,516 keys: 159 against 70).
-    SPLIT_TC_KEYS = 256
+    # Where split softmax weights run on tcgen05: the longest request sees (first) so many keys, or 256 in a step of (second) so many tokens.  On the
+    # device that form is the faster one at every point of 2 to 2,048 rows x 256 to 8,192 keys (256 keys: 8 us against 16, 2,048: 40 against 108); but its
+    # call costs the host 1.5 us more (three tensor maps among its arguments), and a mixer of few tokens waits for the host whatever
+    # its attention takes.  Measured with the mixers, mma.sync / tcgen05: rotated heads, 2 to 260 rows, 260 keys 45 to 49 / 48 to 51 us, 400 keys 45 to 54
+    # / 48 to 51, 520 keys 51 to 60 / 48 to 51; latent attention, whose other kernels take the host twice as long, 2 to 520 rows, 700
+    # keys 92 to 98 / 94 to 100, 1,000 keys 93 to 98 / 95 to 101, 1,500 keys 113 to 120 / 96 to 100, 1,000 rows of 1,000 keys 104 / 96.
+    SPLIT_TC_MASKED, SPLIT_TC_LATENT = (512, 768), (1152, 1792)
+
+    @staticmethod
+    def _takes_split_tc(T, meta, line):
+        return meta.max_kv_len >= line[0] or (T >= line[1] and meta.max_kv_len >= 256)
 
     def _prefill_tc_split(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias_t=None, bias_last=0,
                           slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):
         """The tcgen05 prompt kernel with split weights and the terms of masked_attention; bias_t [H, bias_last + 1]."""
+        at = lambda t: None if t is None else t.data_ptr()      # noqa: E731
+        tiles, table_rows = meta.prefill_tiles2, getattr(meta, "table_rows", None)
         _check(self.lib.mi_attn_prefill_tc_split(
-            _p(q), q.stride(0), q.shape[0], _p(k_cache), _p(v_cache), _c.c_longlong(k_cache.shape[0] * KV * meta.page_size), _p(out),
-            _p(meta.prefill_tiles2), meta.prefill_tiles2.shape[0], _p(meta.seg_q_start), _p(meta.seg_pos0), _p(meta.block_table),
-            _p(getattr(meta, "table_rows", None)), meta.max_pages, H, KV, D, meta.page_size, 128, _c.c_float(scale), window, _p(self._stream_error),
-            block, sink, _p(sink_values), _p(bias_t), bias_last, _p(slopes), _c.c_float(cap), keep, _p(gate), gate_stride, self._stream()),
-            "attn_prefill_tc_split")
+            q.data_ptr(), q.stride(0), q.shape[0], k_cache.data_ptr(), v_cache.data_ptr(), k_cache.shape[0] * KV * meta.page_size, out.data_ptr(),
+            tiles.data_ptr(), tiles.shape[0], meta.seg_q_start.data_ptr(), meta.seg_pos0.data_ptr(), meta.block_table.data_ptr(), at(table_rows),
+            meta.max_pages, H, KV, D, meta.page_size, 128, scale, window, self._stream_error.data_ptr(), block, sink, at(sink_values), at(bias_t), bias_last,
+            at(slopes), cap, keep, at(gate), gate_stride, _raw_stream(self._device_index)), "attn_prefill_tc_split")
         self.launches += 1
 
     def _f32_tiles(self, q, D, V, meta, k_cache, v_cache):
@@ -998,7 +1011,7 @@ class CudaOps:
         bias_last = 0 if distance_bias is None else distance_bias.shape[0] - 1
         # heads of 64 or 128, pages that divide a tile of 64 keys into TMA boxes of at least 8 rows: the tcgen05 kernel (2,048 tokens, 16 heads of
         # 128: 149 us on the mma.sync kernel); other page sizes keep the mma.sync forms, other heads the float32 kernels
-        tc = (num_tiles and meta.max_kv_len >= self.SPLIT_TC_KEYS and self.fast_attention and self.tc_attention and q.dtype == torch.bfloat16 and D == V
+        tc = (num_tiles and self._takes_split_tc(T, meta, self.SPLIT_TC_MASKED) and self.fast_attention and self.tc_attention and q.dtype == torch.bfloat16 and D == V
               and D in (64, 128) and meta.tile == 64 and getattr(meta, "prefill_tiles2", None) is not None and meta.prefill_tiles2.shape[0] and meta.page_size % 8 == 0 and 64 % meta.page_size == 0 and tc_form
               and (plain or self.biased_attention_tc) and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
         if tc:

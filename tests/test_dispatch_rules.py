@@ -59,3 +59,11 @@ def test_line_of_the_selective_scan():
     assert takes(18) and not takes(17) and not takes(1) and not takes(1, 1)
     assert takes(40, 1) and takes(130, *[1] * 5) and not takes(74, *[1] * 5) and not takes(2, *[1] * 63)
     assert takes(*[140] * 4) and not takes(*[100] * 4) and not takes(*[24] * 16) and takes(2048, *[1] * 63)
+
+
+def test_lines_of_split_attention_on_tcgen05():
+    """By keys and by tokens: a step that waits for the host anyway keeps the form that costs the host less."""
+    takes = lambda T, keys, line: CudaOps._takes_split_tc(T, types.SimpleNamespace(max_kv_len=keys), line)      # noqa: E731
+    masked, latent = CudaOps.SPLIT_TC_MASKED, CudaOps.SPLIT_TC_LATENT
+    assert takes(2, 520, masked) and takes(780, 260, masked) and not takes(260, 260, masked) and not takes(2000, 200, masked)
+    assert takes(2, 1500, latent) and takes(2048, 512, latent) and not takes(2, 1000, latent) and not takes(500, 700, latent)

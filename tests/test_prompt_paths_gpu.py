@@ -66,6 +66,14 @@ def test_prompt_attention_forms(ops, dtype, H, KV, D, page, form):      # noqa: 
     assert err < (4e-6 if dtype == torch.float32 else 2 ** -8) * limit, (form, err / limit)
 
 
+@pytest.mark.parametrize("H,KV,D,page", [(4, 2, 128, 16), (3, 1, 64, 8)])
+@pytest.mark.parametrize("form", FORMS)
+def test_prompt_attention_forms_on_tcgen05(ops, monkeypatch, H, KV, D, page, form):      # noqa: F811
+    """The same portions on the kernel that steps of more keys or tokens take."""
+    monkeypatch.setattr(ops, "SPLIT_TC_MASKED", (0, 0))
+    test_prompt_attention_forms(ops, torch.bfloat16, H, KV, D, page, form)
+
+
 @pytest.mark.parametrize("D,page", [(128, 16), (64, 24)])
 @pytest.mark.parametrize("form", ["plain", "causal", "window", "blocks_sink", "cap_keep_gate", "window_keep_narrow"])
 def test_float32_prompt_attention_reads_visible_keys_only(ops, D, page, form):      # noqa: F811
