@@ -356,6 +356,30 @@ def both_batches(lens, slots):
     return types.SimpleNamespace(host={"seg_q_start": qs, "seg_slot": slots}, num_segs=len(lens)), dev
 
 
+@pytest.mark.parametrize("D,V", [(64, 64), (64, 128), (128, 64), (128, 128)])
+def test_one_token_per_entry_of_matrix_states(ops, D, V):       # noqa: F811
+    """Decode steps: states in registers, key heads shared by value heads, slots out of order, rows and slots with padding behind them."""
+    from tests.ref_ops import TorchRefOps
+    ref, H, KV, lens = TorchRefOps(), 6, 2, (1,) * 7
+    host, dev = both_batches(lens, [3, 1, 8, 2, 7, 5, 4])
+    g = torch.Generator().manual_seed(D + V)
+    C = 2 * KV * D + H * V
+    prep = torch.randn(7, C + H * D + H + 6, generator=g)
+    prep[:, :2 * KV * D] *= D ** -0.5
+    prep[:, C:] = torch.rand(7, H * D + H + 6, generator=g)
+    state = torch.randn(9, H * D * V + 12, generator=g)
+    p, decay = torch.randn(7, 2 * H * D + H * V + 5, generator=g).to(torch.bfloat16), torch.rand(H, generator=g)
+    runs = {"delta": lambda o, s, b, x: o.delta_scan(x[0], H, KV, D, V, s, b), "constant": lambda o, s, b, x: o.lightning_scan(x[1], H, D, V, x[2], s, b)}
+    for name, run in runs.items():
+        a, b = state.clone().to(DEV), state.clone()
+        assert ops._takes_step(7, dev, D, V, a), name
+        got = run(ops, a, dev, (prep.to(DEV), p.to(DEV), decay.to(DEV)))
+        want = run(ref, b[:, :H * D * V] if name == "constant" else b, host, (prep, p, decay))
+        # float32 sums of up to 128 products in another order
+        assert rows_error(got.cpu(), want) < 2e-6 and rows_error(a[1:].cpu(), b[1:]) < 2e-6, name
+        assert torch.equal(a[:, H * D * V:].cpu(), state[:, H * D * V:]) and torch.equal(a[6].cpu(), state[6]), name
+
+
 @pytest.mark.parametrize("taps", [2, 3, 4])
 @pytest.mark.parametrize("H,KV,D,V", [(4, 2, 128, 128), (3, 1, 64, 48), (2, 2, 12, 20)])
 def test_delta_prologue_of_prompts(ops, taps, H, KV, D, V):     # noqa: F811
@@ -377,6 +401,34 @@ def test_delta_prologue_of_prompts(ops, taps, H, KV, D, V):     # noqa: F811
     assert torch.equal(sa.cpu(), sb)                             # the newest inputs, copied
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("groups,gs", [(1, 516), (2, 1024), (1, 2052), (3, 4096)])
+def test_wide_group_norms(ops, dtype, groups, gs):              # noqa: F811
+    """A group in a block's registers: one to four quads a thread, whole and not; a weight per group, per row or none; a gate that is a view."""
+    from tests.ref_ops import TorchRefOps
+    ref, g, T, n = TorchRefOps(), torch.Generator().manual_seed(gs), 5, groups * gs
+    o, gate = torch.randn(T, n, generator=g), torch.randn(T, n + 10, generator=g).to(dtype)
+    for weight in (None, torch.randn(gs, generator=g), torch.randn(n, generator=g)):
+        for act in ("sigmoid", "silu"):
+            got = ops.group_rmsnorm_gate(o.to(DEV), None if weight is None else weight.to(DEV), gate.to(DEV)[:, 6:6 + n], 1e-6, groups, gs, dtype, act=act).cpu()
+            want = ref.group_rmsnorm_gate(o, weight, gate[:, 6:6 + n], 1e-6, groups, gs, dtype, act=act)
+            limit = 2e-6 if dtype == torch.float32 else 2 ** -7     # bfloat16: the output may round to the neighbouring number
+            assert ((got.float() - want.float()).abs() <= limit * want.float().abs().clamp_min(0.1)).all(), (act, weight is None)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T", [255, 257])
+@pytest.mark.parametrize("H,V", [(5, 64), (16, 8), (3, 136)])
+def test_head_gates_of_prompts(ops, dtype, T, H, V):            # noqa: F811
+    from tests.ref_ops import TorchRefOps
+    ref, g = TorchRefOps(), torch.Generator().manual_seed(T + V)
+    o, gate = torch.randn(H, T, V, generator=g).to(dtype), torch.randn(T, H + 7, generator=g).to(dtype)
+    for w in (gate[:, 3:3 + H], None):
+        got, want = ops.head_gate(o.to(DEV), None if w is None else gate.to(DEV)[:, 3:3 + H], dtype).cpu(), ref.head_gate(o, w, dtype)
+        limit = 3e-7 if dtype == torch.float32 else 2 ** -7
+        assert ((got.float() - want.float()).abs() <= limit * want.float().abs()).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,hidden", [(127, 264), (128, 264), (128, 2050), (600, 2048)])
 def test_weighted_sum_of_experts(ops, dtype, T, hidden):        # noqa: F811
     """128 tokens or more in 16-byte pieces where rows allow, fewer an entry a thread; with and without weights, a shared expert and its gate."""
@@ -392,6 +444,41 @@ def test_weighted_sum_of_experts(ops, dtype, T, hidden):        # noqa: F811
             want += s.double() * (1.0 if sg is None else torch.sigmoid(sg.double())[:, None])
         limit = 1e-6 if dtype == torch.float32 else 2 ** -7
         assert ((out.double() - want).abs() <= limit * want.abs().clamp_min(0.5)).all()
+
+@pytest.mark.parametrize("form", ["causal", "sink", "bias", "gate", "latent"])
+def test_both_halves_of_a_softmax_weight_count(ops, form):      # noqa: F811
+    """Every weight but the first is e^-0.0021, which bfloat16 rounds down by 0.18 %: with the first half alone all outputs are that much too
+    small, far more than their own roundings' mean, which the other half must take away."""
+    H, KV, D, T, page = 2, (1 if form == "latent" else 2), 128, 1200, 16        # as many keys as the tcgen05 forms want
+    meta, g = make_meta(page, [(0, T)], 80, 6), torch.Generator().manual_seed(3)
+    assert ops._takes_split_tc(T, meta, ops.SPLIT_TC_LATENT)
+    q, k = torch.zeros(T, H * D), torch.zeros(T, KV, D)
+    q[:, ::D], k[1:, :, 0] = 1.0, -0.0021
+    v = (0.5 + torch.rand(T, KV, D, generator=g)) * (1 + torch.rand(D, generator=g))
+    if form == "latent":                                        # keys are the values: the scores read a column that is no value
+        v[:, :, 0] = k[:, :, 0]
+    q, k, v = (x.to(torch.bfloat16) for x in (q, k, v))
+    pools = [torch.zeros(81, KV, page, D, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    where = meta.slots.long()
+    for pool, x in zip(pools, (k, v)):
+        pool[where // page, :, where % page] = x.to(DEV)
+    if form == "latent":
+        got = ops.paged_attention(q.to(DEV), pools[1], pools[1], meta, H, KV, D, 1.0, None, split_weights=True)
+    else:
+        args = {"causal": {}, "sink": dict(sink_values=torch.zeros(H, device=DEV)), "bias": dict(distance_bias=torch.zeros(9, H, device=DEV)),
+                "gate": dict(gate=torch.full((T, H * D), 40.0, dtype=torch.bfloat16, device=DEV))}[form]
+        got = ops.masked_attention(q.to(DEV), *pools, meta, H, KV, D, D, 1.0, None, None, form == "sink", **args)
+    ops.check_errors()
+    w = k[:, 0, 0].double().exp().expand(T, T).tril()
+    total = w.sum(1, keepdim=True) + (form == "sink")
+    sums = lambda w: torch.einsum("tk,khd->thd", w, v.double()) / total[:, :, None]      # noqa: E731
+    want, first_half = sums(w), sums(w.float().to(torch.bfloat16).double())
+    pick = lambda x: x[100:, :, 1:]                             # noqa: E731  (rows of many keys)
+    got = got.cpu().double().view(T, H, D)
+    want, first_half = (x.repeat_interleave(H // KV, dim=1) for x in (want, first_half))
+    assert pick(first_half / want - 1).mean().item() < -1.5e-3
+    assert abs(pick(got / want - 1).mean().item()) < 1.5e-4
+
 
 def test_sampler_forms_agree(ops):                              # noqa: F811
     """Few scores: eight a thread, fetched together; 4.5 million and more: sixteen, one after the other.  The choices are the same whole numbers."""
