@@ -74,6 +74,25 @@ def test_prompt_attention_forms_on_tcgen05(ops, monkeypatch, H, KV, D, page, for
     test_prompt_attention_forms(ops, torch.bfloat16, H, KV, D, page, form)
 
 
+@pytest.mark.parametrize("behind", [0, 1300])
+@pytest.mark.parametrize("n", [2, 64, 65, 128, 200])
+def test_values_behind_the_last_key_do_not_count(ops, n, behind):       # noqa: F811
+    """Plain tcgen05 attention (Qwen3): a last tile of keys that is whole or not, one tile or many; what its pages hold behind the last key is no number."""
+    H, KV, D, page, segs = 4, 2, 128, 16, [(behind, n), (behind + 5, n)]
+    meta, g = make_meta(page, segs, 220, 8), torch.Generator().manual_seed(n)
+    q = torch.randn(2 * n, H * D, generator=g).to(torch.bfloat16).to(DEV)
+    k, v = (torch.randn(221, KV, page, D, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
+    want = ops.paged_attention(q, k, v, meta, H, KV, D, D ** -0.5, None)
+    for i, (pos0, m) in enumerate(segs):
+        last = pos0 + m - 1
+        at = meta.block_table[i, last // page].long()
+        k[at, :, last % page + 1:], v[at, :, last % page + 1:] = float("nan"), float("inf")
+    k[0], v[0] = float("nan"), float("inf")                      # the null page, which the loads of a tile's missing pages read
+    got = ops.paged_attention(q, k, v, meta, H, KV, D, D ** -0.5, None)
+    ops.check_errors()
+    assert got.isfinite().all() and torch.equal(got, want)
+
+
 @pytest.mark.parametrize("D,page", [(128, 16), (64, 24)])
 @pytest.mark.parametrize("form", ["plain", "causal", "window", "blocks_sink", "cap_keep_gate", "window_keep_narrow"])
 def test_float32_prompt_attention_reads_visible_keys_only(ops, D, page, form):      # noqa: F811
