@@ -1,9 +1,12 @@
 // Paged attention, generic variant: any head size that is a multiple of 8 (16-byte rows) up to
 // 256, any number of heads and groups, float32 or bfloat16 storage, optional window.  All
-// arithmetic is float32 on the CUDA cores, in an order that depends only on the request's own
-// positions, so the float32 engine gives the same bits however a batch is cut or mixed.
-// The bfloat16 fast paths live in attention_mma.cu; this file is the float32 path, the
-// fall-back for unusual head sizes, and the reference point of the fast kernels' tests.
+// arithmetic is float32 on the CUDA cores.  A prompt's rows add in an order that depends only on
+// the request's own positions (the same bits however a batch is cut or mixed); a decoded token's
+// keys are cut into `splits` pieces, which the caller chooses by the step's size.
+// Prompts with heads of 64 or 128 have kernels of their own (attention_prefill_tc.cu and
+// attention_prefill_mma.cu in bfloat16, attention_prefill_f32.cu in float32), decoded tokens in
+// bfloat16 attention_decode_mma.cu; this file decodes in float32, takes all other head sizes, and
+// is the reference point of the fast kernels' tests.
 //
 // Reference (davidjoyme/mini-inference): prompt portions attend over the gathered context with
 // a causal (offset) mask, engine/core/model_runner.py:161-173; decoded tokens use the split-KV

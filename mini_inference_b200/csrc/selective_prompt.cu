@@ -7,7 +7,7 @@
 // two states each in one packed pair (N = 16), so 4,096 channels are 1,024 warps, two per scheduler; exponentials run on the
 // FMA pipe, two at a time.  A block is 32 channels: eight warps walk the tokens, eight more make the next chunk of 32 tokens ready (steps, inputs, B, C to
 // shared memory) and finish the previous one (skip term, gate, store), so neither softplus nor a load is waited for; one barrier a chunk.
-// Eight tokens' partial sums are added up over the eight lanes together (seven shuffles instead of 24).  2,048 tokens: 541 -> 141 us.  The kernel in
+// Eight tokens' partial sums are added up over the eight lanes together (seven shuffles instead of 24).  2,048 tokens: 490 -> 148 us.  The kernel in
 // which all warps do everything in turn (recurrent.cu) stays for decode steps, where there is one token a request, for other N, and for
 // float32 runs: it takes every step, so a request's bits there depend on nothing but its own tokens.
 #include "common.cuh"

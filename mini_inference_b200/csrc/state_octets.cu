@@ -15,8 +15,8 @@
 // are made together, lane l ends with sum l; u goes around through shared memory.  One more warp brings the records by bulk copies into
 // a ring: a head's records lie one behind the other, and so do its values of the block's columns, so an octet is two copies.  (A record
 // and a row of values per token took the copying thread 480 ns for four tokens, whatever the compute warps did.)
-// Scan with its octet_kernel, 16 heads of 128 x 128: 2,048 tokens 556 -> 237 us (delta), 291 -> 164 us (constant, silu included); 1,300 + 517 + 231
-// tokens 539 -> 248 and 282 -> 164 us; 16 x 64 tokens 216 -> 107 and 117 -> 75 us.  One warp a scheduler issues every 2.4 clocks: what is left
+// Scan with its octet_kernel, 16 heads of 128 x 128: 2,048 tokens 553 -> 234 us (delta), 286 -> 166 us (constant, silu included); 4 x 512
+// tokens 449 -> 198 and 197 -> 135 us; 16 x 64 tokens 212 -> 101 and 113 -> 71 us.  One warp a scheduler issues every 2.4 clocks: what is left
 // is the latency of one warp's own instructions.  (Two groups of 16 lanes with four columns each in a warp need 40 % fewer instructions per
 // column, but half as many warps share one prompt: 297 and 198 us.)
 #include "sm100.cuh"

@@ -362,6 +362,7 @@ def test_unit_heads_of_prompts(ops, H, KV, D, form):            # noqa: F811
         assert (a.float() - b.float()).abs().max().item() <= 2 ** -8 * b.float().abs().max().item()
         assert (a != b).float().mean().item() < 1e-2
 
+
 # ---------------------------------------------------------------- kernels that a rule on sizes picks, against the plain statements (tests/ref_ops.py)
 def both_batches(lens, slots):
     import types
@@ -419,6 +420,7 @@ def test_delta_prologue_of_prompts(ops, taps, H, KV, D, V):     # noqa: F811
     assert (got[:, :n].cpu() - want[:, :n]).abs().max().item() < 4e-6 * want.abs().max().item()
     assert torch.equal(sa.cpu(), sb)                             # the newest inputs, copied
 
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("groups,gs", [(1, 516), (2, 1024), (1, 2052), (3, 4096)])
 def test_wide_group_norms(ops, dtype, groups, gs):              # noqa: F811
@@ -463,6 +465,7 @@ def test_weighted_sum_of_experts(ops, dtype, T, hidden):        # noqa: F811
             want += s.double() * (1.0 if sg is None else torch.sigmoid(sg.double())[:, None])
         limit = 1e-6 if dtype == torch.float32 else 2 ** -7
         assert ((out.double() - want).abs() <= limit * want.abs().clamp_min(0.5)).all()
+
 
 @pytest.mark.parametrize("form", ["causal", "sink", "bias", "gate", "latent"])
 def test_both_halves_of_a_softmax_weight_count(ops, form):      # noqa: F811
