@@ -99,6 +99,8 @@ class StepBatch:
         self.num_tokens, self.num_segs, self.tile = facts.num_tokens, facts.num_entries, facts.tile
         self.num_logit_rows = num_logit_rows
         self.max_kv_len, self.max_q_len = max_kv_len, int(facts.lens.max())
+        prompts = facts.lens > 1                                    # entries that feed more than one token; the most keys one of them sees
+        self.max_prompt_kv_len = int(facts.kv_len[prompts].max()) if prompts.any() else 0
         self.host = {"seg_q_start": facts.q_start, "seg_pos0": facts.pos0, "seg_kv_len": facts.kv_len,
                      "seg_slot": facts.slots.tolist(), "lens": facts.lens}
         for name in ("token_ids", "positions", "token_seg", "seg_q_start", "seg_pos0", "seg_kv_len", "seg_slot", "logit_rows"):

@@ -630,7 +630,7 @@ class CudaOps:
             self.launches += 2 if S > 1 else 1
         return out
 
-    # Where split softmax weights run on tcgen05: the longest request sees (first) so many keys, or 256 in a step of (second) so many tokens.  On the
+    # Where split softmax weights run on tcgen05: a prompt portion sees (first) so many keys, or 256 in a step of (second) so many tokens.  On the
     # device that form is the faster one at every point of 2 to 2,048 rows x 256 to 8,192 keys (256 keys: 8 us against 16, 2,048: 40 against 108); but its
     # call costs the host 1.5 us more (three tensor maps among its arguments), and a mixer of few tokens waits for the host whatever
     # its attention takes.  Measured with the mixers, mma.sync / tcgen05: rotated heads, 2 to 260 rows, 260 keys 45 to 49 / 48 to 51 us, 400 keys 45 to 54
@@ -640,7 +640,9 @@ class CudaOps:
 
     @staticmethod
     def _takes_split_tc(T, meta, line):
-        return meta.max_kv_len >= line[0] or (T >= line[1] and meta.max_kv_len >= 256)
+        keys = getattr(meta, "max_prompt_kv_len", None)             # a decoded token's keys are another kernel's
+        keys = meta.max_kv_len if keys is None else keys
+        return keys >= line[0] or (T >= line[1] and keys >= 256)
 
     def _prefill_tc_split(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias_t=None, bias_last=0,
                           slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):

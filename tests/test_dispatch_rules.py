@@ -67,3 +67,19 @@ def test_lines_of_split_attention_on_tcgen05():
     masked, latent = CudaOps.SPLIT_TC_MASKED, CudaOps.SPLIT_TC_LATENT
     assert takes(2, 520, masked) and takes(780, 260, masked) and not takes(260, 260, masked) and not takes(2000, 200, masked)
     assert takes(2, 1500, latent) and takes(2048, 512, latent) and not takes(2, 1000, latent) and not takes(500, 700, latent)
+
+
+def test_a_decoded_tokens_keys_do_not_count_for_prompt_attention():
+    """Beside a decoded token of 3,000 keys a portion of two tokens behind 500 is a short one."""
+    from mini_inference_b200.engine.batch import BatchLayout, StepBatch, StepFacts
+    fields = [(n, 8) for n in ("token_ids", "positions", "token_seg", "seg_q_start", "seg_pos0", "seg_kv_len", "seg_slot", "logit_rows")]
+    layout = BatchLayout(fields)
+
+    def batch(lens, pos0):
+        facts = StepFacts(lens, pos0, list(range(1, len(lens) + 1)), 64)
+        return StepBatch(layout, torch.zeros(layout.size, dtype=torch.int32), None, facts, {}, 1, int(facts.kv_len.max()), False)
+
+    mixed, decode = batch([2, 1], [500, 3000]), batch([1, 1], [3000, 20])
+    assert mixed.max_kv_len == 3001 and mixed.max_prompt_kv_len == 502 and decode.max_prompt_kv_len == 0
+    assert not CudaOps._takes_split_tc(3, mixed, CudaOps.SPLIT_TC_MASKED)
+    assert CudaOps._takes_split_tc(3, batch([2, 1], [600, 3000]), CudaOps.SPLIT_TC_MASKED)
