@@ -8,7 +8,8 @@
 // (The reference reaches float32 by running its library path with DTYPE=float32 on the CPU,
 // tests/test_batching.py:57; it has no float32 GPU path.)
 //
-// Bound by the float32 FMA rate (74 TFLOP/s) for many rows, by the weight's bytes for few.  The
+// Matrices of a million entries and more go to the tensor cores (gemm_f32_tc.cu: the same precision, an order of its own).  The
+// kernel here is bound by the float32 FMA rate (74 TFLOP/s) for many rows, by the weight's bytes for few.  The
 // packed two-float multiply-add of this architecture does two neighbouring k per instruction:
 // both operands lie along K as they are stored, so tiles go to shared memory untransposed by
 // cp.async (16 bytes, or 4 where rows do not start on 16) and pairs need no shuffling.  Rows are
@@ -18,6 +19,13 @@
 // The packed multiply-add pipe is active 59 % of the time; tiles of 8 x 4 or 4 x 8 a thread with twice
 // the warps, steps of 16 of K, and scalar multiply-adds (33 TFLOP/s at 3,000 rows against 37) are slower.
 #include "common.cuh"
+
+namespace mi {                                  // gemm_f32_tc.cu: the same product on the tensor cores
+long long gemm_f32_tc_parts(int M, int K);
+int gemm_f32_tc_tile(int M, int N, int S);
+int gemm_f32_tc(const float* A, int lda, const float* W, float* out, int ldc, int M, int N, int K, int S, int segment, int nt, void* parts,
+                int* error_word, cudaStream_t stream);
+}
 
 namespace {
 
@@ -110,13 +118,21 @@ __global__ void __launch_bounds__(32 * WM * WN) gemm_f32_nt_kernel(const float* 
     }
 }
 
-// C = the segments' sums, added in order; ws [S, M, N]
+// C = the segments' sums, added in order; ws [S, M, N].  VEC neighbouring columns a thread.
+template <int VEC>
 __global__ void add_segments_kernel(const float* __restrict__ ws, float* __restrict__ C, int ldc, int M, int N, int S) {
     const size_t plane = (size_t)M * N;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += (size_t)gridDim.x * blockDim.x) {
-        float v = ws[i];
-        for (int s = 1; s < S; ++s) v += ws[s * plane + i];
-        C[i / N * ldc + i % N] = v;
+    for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC; i < plane; i += (size_t)gridDim.x * blockDim.x * VEC) {
+        float v[VEC];
+        if constexpr (VEC == 4) mi::load16(ws + i, v); else v[0] = ws[i];
+        for (int s = 1; s < S; ++s) {
+            float u[VEC];
+            if constexpr (VEC == 4) mi::load16(ws + s * plane + i, u); else u[0] = ws[s * plane + i];
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) v[e] += u[e];
+        }
+        float* to = C + i / N * ldc + i % N;
+        if constexpr (VEC == 4) *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]); else *to = v[0];
     }
 }
 
@@ -148,7 +164,29 @@ int segments(int N, int K, int* segment) {
     return (K + *segment - 1) / *segment > 1 ? (K + *segment - 1) / *segment : 1;
 }
 
-constexpr int ROWS_AT_ONCE = 1024;             // rows per pass of a product that is cut along K: bounds its workspace
+constexpr int ROWS_AT_ONCE = 1024;             // rows per pass of a product that needs a workspace: bounds it
+
+// Which products run on the tensor cores: by N and K alone (and that W's rows start on 16 bytes, as TMA reads them), so that a row's bits do not
+// depend on M.  Smaller matrices are a few tiles for 148 blocks and keep the multiply-adds.
+bool on_tensor_cores(int N, int K) { return K % 4 == 0 && K >= 512 && N >= 128 && (long long)N * K >= 1 << 20; }
+
+// Their K is cut until a tile of tokens alone gives about one block per SM, in pieces of at least 512
+int tc_segments(int N, int K, int* segment) {
+    int S = K / 512 < 8 ? K / 512 : 8;
+    if (S > 148 / ((N + 127) / 128)) S = 148 / ((N + 127) / 128);
+    if (S < 1) S = 1;
+    *segment = ((K + S - 1) / S + BK_MAX - 1) / BK_MAX * BK_MAX;
+    return (K + *segment - 1) / *segment;
+}
+
+int add_up(const float* ws, float* C, int ldc, int M, int N, int S, cudaStream_t stream) {
+    const bool vec = N % 4 == 0 && ldc % 4 == 0 && (uintptr_t)C % 16 == 0 && (uintptr_t)ws % 16 == 0;
+    const size_t n = ((size_t)M * N + (vec ? 3 : 0)) / (vec ? 4 : 1);
+    const int blocks = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
+    if (vec) add_segments_kernel<4><<<blocks, 256, 0, stream>>>(ws, C, ldc, M, N, S);
+    else add_segments_kernel<1><<<blocks, 256, 0, stream>>>(ws, C, ldc, M, N, S);
+    return (int)cudaGetLastError();
+}
 
 // The tile whose last wave wastes least, by the area an SM works through (relative rates measured with every SM full).
 int pick_tile(int M, int N, int S) {
@@ -180,30 +218,44 @@ int run_tile(const float* A, int lda, const float* W, float* out, int ldc, int M
 // floats of workspace that a product of this shape needs (0: none)
 MI_EXPORT long long mi_gemm_f32_workspace(int M, int N, int K) {
     int segment;
-    const int S = segments(N, K, &segment);
-    return S > 1 ? (long long)S * (M < ROWS_AT_ONCE ? M : ROWS_AT_ONCE) * N : 0;
+    const int rows = M < ROWS_AT_ONCE ? M : ROWS_AT_ONCE;
+    int S = segments(N, K, &segment);
+    const long long plain = S > 1 ? (long long)S * rows * N : 0;      // also for a W of this shape that does not start on 16 bytes
+    if (!on_tensor_cores(N, K)) return plain;
+    S = tc_segments(N, K, &segment);
+    const long long parts = mi::gemm_f32_tc_parts(rows, K) / 4 + (S > 1 ? (long long)S * rows * N : 0);
+    return parts > plain ? parts : plain;
 }
 
 // tile < 0: chosen here (every tile gives the same bits)
-MI_EXPORT int mi_gemm_f32_nt(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, float* ws, int tile,
+MI_EXPORT int mi_gemm_f32_nt(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, float* ws, int tile, int* error_word,
                              cudaStream_t stream) {
     if (M == 0 || N == 0) return 0;
     int segment;
+    if (on_tensor_cores(N, K) && (uintptr_t)W % 16 == 0) {
+        if (!ws) return -2;
+        static const int tokens[5] = {128, 128, 64, 64, 32};
+        const int S = tc_segments(N, K, &segment);
+        for (int m = 0; m < M; m += ROWS_AT_ONCE) {
+            const int rows = M - m < ROWS_AT_ONCE ? M - m : ROWS_AT_ONCE;
+            float* to = C + (size_t)m * ldc;
+            float* shares = ws + mi::gemm_f32_tc_parts(rows, K) / 4;
+            int rc = mi::gemm_f32_tc(A + (size_t)m * lda, lda, W, S > 1 ? shares : to, S > 1 ? N : ldc, rows, N, K, S, segment,
+                                     tile >= 0 ? tokens[tile] : mi::gemm_f32_tc_tile(rows, N, S), ws, error_word, stream);
+            if (rc == 0 && S > 1) rc = add_up(shares, to, ldc, rows, N, S, stream);
+            if (rc) return rc;
+        }
+        return 0;
+    }
     const int S = segments(N, K, &segment);
     if (S > 1 && !ws) return -2;
     const int step = S > 1 ? ROWS_AT_ONCE : M;
     for (int m = 0; m < M; m += step) {
         const int rows = M - m < step ? M - m : step;
         const int t = tile >= 0 ? tile : pick_tile(rows, N, S);
-        const int rc = run_tile(A + (size_t)m * lda, lda, W, S > 1 ? ws : C + (size_t)m * ldc, S > 1 ? N : ldc, rows, N, K, S, segment, t, stream);
+        int rc = run_tile(A + (size_t)m * lda, lda, W, S > 1 ? ws : C + (size_t)m * ldc, S > 1 ? N : ldc, rows, N, K, S, segment, t, stream);
+        if (rc == 0 && S > 1) rc = add_up(ws, C + (size_t)m * ldc, ldc, rows, N, S, stream);
         if (rc) return rc;
-        if (S > 1) {
-            const size_t n = (size_t)rows * N;
-            const int blocks = (int)((n + 1023) / 1024 < 148 * 8 ? (n + 1023) / 1024 : 148 * 8);
-            add_segments_kernel<<<blocks, 256, 0, stream>>>(ws, C + (size_t)m * ldc, ldc, rows, N, S);
-            const cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) return (int)e;
-        }
     }
     return 0;
 }

@@ -289,7 +289,7 @@ class CudaOps:
         and K alone, their partial sums pass a workspace.  tile: a tile of csrc/gemm_f32.cu instead of its own choice (same bits)."""
         n = self.lib.mi_gemm_f32_workspace(M, N, K)
         ws = torch.empty(n, dtype=torch.float32, device=x.device) if n else None
-        _check(self.lib.mi_gemm_f32_nt(_p(x), ldx, _p(w), _p(out), ldc, M, N, K, _p(ws), tile, self._stream()), "gemm_f32")
+        _check(self.lib.mi_gemm_f32_nt(_p(x), ldx, _p(w), _p(out), ldc, M, N, K, _p(ws), tile, _p(self._stream_error), self._stream()), "gemm_f32")
         self.launches += 2 if n else 1
 
     @staticmethod

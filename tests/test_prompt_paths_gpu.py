@@ -24,6 +24,39 @@ def test_gemm_f32_tiles_give_the_same_bits(ops, M, N, K):       # noqa: F811
     assert torch.equal(ops.linear(x[:1], w), got[:1])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 2048, 512), (32, 1030, 1020), (33, 128, 8192), (65, 2500, 700), (129, 4096, 1100), (257, 300, 4000), (1030, 1100, 964)])
+def test_gemm_f32_on_tensor_cores(ops, M, N, K):                # noqa: F811
+    """Products cut into bfloat16 parts: remainders of a tile's rows of W, tokens and 64 of K, one segment of K and several, strided rows, every tile, and
+    rows that bfloat16 parts cannot hold (infinities, NaN, the ends of float32's range), which must not touch any other row."""
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K + 3, generator=g).to(DEV)[:, :K]
+    w = torch.randn(N, K, generator=g).to(DEV)
+    want = x.double() @ w.double().T
+    got = ops.linear(x, w)
+    # K / 64 sums are added up in float32, rounded to nearest (half of 2^-23 of the sum so far), behind sums of 64 cut off after 2^-23
+    assert ((got.double() - want).norm() / want.norm()).item() < 6e-8 * (K / 64) ** 0.5 + 6e-8
+    for tile in range(5):
+        out = torch.empty_like(got)
+        ops._gemm_f32(x, x.stride(0), w, out, N, M, N, K, tile)
+        assert torch.equal(out, got), tile
+    assert torch.equal(ops.linear(x[-1:], w), got[-1:])
+    x, w = x.contiguous(), w.clone()
+    rows = {0: lambda r: r.fill_(0), M // 2: lambda r: r.mul_(1e-30), M // 3: lambda r: r[7:8].fill_(float("inf")), M // 4: lambda r: r[K - 1:].fill_(float("nan")), M - 1: lambda r: r[3:4].fill_(1e36)}
+    for m, change in rows.items():
+        change(x[m])
+    w[N - 1, 5], w[17, K - 2], w[40] = float("-inf"), 1e30, w[40] * 1e-28
+    got2, want2 = ops.linear(x, w), x.double() @ w.double().T
+    plain_rows = [m for m in range(M) if m not in rows]
+    plain_cols = [n for n in range(N) if n not in (N - 1, 17, 40)]
+    assert torch.equal(got2[plain_rows][:, plain_cols], got[plain_rows][:, plain_cols])
+    assert torch.equal(got2.isnan(), want2.isnan()) and torch.equal(got2.isinf(), want2.isinf())
+    for m in range(M):
+        ok = want2[m].isfinite()
+        if ok.any() and (M < 100 or m in rows):
+            size = x[m].double().norm() * w[ok].double().norm(dim=1)        # what a float32 sum's error goes with
+            assert ((got2[m][ok].double() - want2[m][ok]).abs() <= 2e-6 * size + 1e-37).all(), m
+
+
 FORMS = ["causal", "window", "blocks_sink", "learned_sink_bias", "slopes", "slopes_bias_window", "cap_keep_gate", "window_keep_narrow"]
 
 
