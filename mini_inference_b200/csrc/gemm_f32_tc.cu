@@ -1,8 +1,5 @@
-// True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T on the tensor cores: every float32 is cut exactly into three bfloat16 numbers
-// (x = x0 + x1 + x2: 8 + 8 + 8 significant bits, each the rounding of what the ones before leave), and a product of two of them is the sum of
-//   x0 w0 + (x0 w1 + x1 w0) + (x0 w2 + x1 w1 + x2 w0)
-// What is left out is below 2^-26 of |x w| and of either sign.  (The idea is old: Dekker, "A floating-point technique for extending the available
-// precision", 1971; Ozaki et al. 2012 for matrix products on short formats.)  A bfloat16 product is exact in the tensor core's float32 sum.
+// True 32-bit matrix product C[M,N] = A[M,K] * W[N,K]^T on the tensor cores: every float32 is cut exactly into three bfloat16 numbers, six products of
+// parts stand for one product (split3.cuh).
 //
 // Exactness.  The tensor core cuts off instead of rounding when it adds, so no sum stays there for long: 64 of K (24 instructions, the small
 // products first) go into a fresh accumulator in tensor memory, and the epilogue warps add it in float32, rounded to nearest, to sums that they
@@ -24,15 +21,16 @@
 // 4.1e-7 .. 6.5e-7 -> 1.0e-7 .. 1.4e-7.  At 501 rows the tensor pipe is active 64 % of the time and a fifth of it goes to the last wave; a stage
 // brings 80 KB for 1,536 clocks of products, close to what a block can load (53 bytes a clock).  With one row a stage of W is 1,128 clocks
 // of products (an instruction of 32 tokens takes as long as one of 64).
-#include "sm100.cuh"
+#include "split3.cuh"
 #include <algorithm>
 
 using namespace mi;
 using namespace mi::sm100;
+using namespace mi::split3;
 
 namespace {
 
-constexpr int BN = 128, BK = 64, PARTS = 3;
+constexpr int BN = 128, BK = 64;
 constexpr int W_BOX = BN * 32 * 4, W_STAGE = 2 * W_BOX;         // a box is 32 floats (128 bytes) of 128 rows
 constexpr int THREADS = 32 * 19;
 constexpr int A_COLS = PARTS * BK / 2;                          // tensor-memory columns of a stage of W's parts
@@ -42,27 +40,7 @@ constexpr int w_stages(int nt) { return nt == 128 ? 2 : nt == 64 ? 4 : 5; }
 constexpr int x_stages(int nt) { return nt == 128 ? 3 : nt == 64 ? 3 : 4; }
 constexpr int smem_bytes(int nt) { return 1024 + w_stages(nt) * W_STAGE + x_stages(nt) * x_stage(nt) + 2 * 2 * BN * 4 + 512; }
 
-// a, b -> their first parts side by side; a and b become what is left
-__device__ __forceinline__ uint32_t take_part(float& a, float& b) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(&h);
-    a -= __uint_as_float(w << 16);
-    b -= __uint_as_float(w & 0xffff0000u);
-    return w;
-}
 constexpr float LEAST = 0x1p-60f, MOST = 0x1p60f;               // of a row's largest magnitude
-
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n"
-                 :: "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-                    "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr) : "memory");
-}
 
 // parts[3][M][ldp] of A [M, K]; columns K .. ldp are zeros.  flag[m]: the row does not fit three bfloat16 numbers.  One block a row.
 __global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ A, int lda, __nv_bfloat16* __restrict__ parts, int ldp,
@@ -116,7 +94,7 @@ __device__ __forceinline__ Item item_of(const Shape& sh, int i) {
 template <int NT>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const Shape sh, const float* __restrict__ A,
-                   const float* __restrict__ W, const unsigned char* __restrict__ token_flag, float* __restrict__ out, int* __restrict__ error_word) {
+                   const float* __restrict__ W, const unsigned char* token_flag, float* __restrict__ out, int* __restrict__ error_word) {
     constexpr int WS = w_stages(NT), XS = x_stages(NT), X_STAGE = x_stage(NT), HALF = NT / 2;
     constexpr uint32_t TMEM_COLS = 512, D_COL = 2 * A_COLS;
     extern __shared__ unsigned char smem_raw[];
@@ -193,12 +171,11 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
                     tc_fence_after();
                     const uint32_t d = tmem + D_COL + b * NT, a = tmem + b * A_COLS;
                     const uint64_t x = umma_desc_sw128(sX + xs * X_STAGE, 16, 1024);
-                    constexpr int PW[6] = {2, 1, 0, 1, 0, 0}, PX[6] = {0, 1, 2, 0, 1, 0};       // the small products first
 #pragma unroll
-                    for (int p = 0; p < 6; ++p)
+                    for (int p = 0; p < PRODUCTS; ++p)
 #pragma unroll
                         for (int ks = 0; ks < BK / 16; ++ks)
-                            umma_ts(d, a + PW[p] * (BK / 2) + ks * 8, x + ((PX[p] * NT * 128 + ks * 32) >> 4), idesc, (p | ks) != 0);
+                            umma_ts(d, a + PART_A[p] * (BK / 2) + ks * 8, x + ((PART_B[p] * NT * 128 + ks * 32) >> 4), idesc, (p | ks) != 0);
                     umma_commit(a_empty + 8 * b);
                     umma_commit(x_empty + 8 * xs);
                     umma_commit(d_full + 8 * b);
