@@ -26,7 +26,7 @@ def load_library():
         from .build import build
         path = build()
         _LIB = ctypes.CDLL(path)
-        _LIB.mi_gemm_f32_workspace.restype = _LIB.mi_octet_floats.restype = ctypes.c_longlong
+        _LIB.mi_gemm_f32_workspace.restype = _LIB.mi_octet_floats.restype = _LIB.mi_chunk_floats.restype = ctypes.c_longlong
         # declared, so that addresses and floats pass as plain numbers: with wrapped ones the call cost the host 22.7 us where the
         # values are the keys and 17.3 elsewhere, now 16.0 and 16.3 (the mma.sync form 14.5), and a step of few tokens waits for the host
         p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
@@ -750,6 +750,18 @@ class CudaOps:
         """Per octet and head its record and eight tokens' values: as many floats as the kernels' own layout says."""
         return torch.empty(self.lib.mi_octet_floats(T, batch.num_segs, H, D, V, int(delta)), dtype=torch.float32, device=self.device)
 
+    @staticmethod
+    def _takes_chunks(batch, T, D, V):
+        """Whether a recurrence with a constant decay that _takes_octets goes 128 tokens at a time on the tensor cores instead (csrc/state_chunks.cu): keys
+        of 128, values in blocks of 128 columns, a prompt of at least 320 tokens (three kernels of some 36 us in all against eight tokens at a time:
+        192 tokens 27 us there, 256 31, 400 41, 2,048 167 against 73) and 100 tokens an entry on average, since a short entry takes a whole chunk
+        (16 prompts of 64 tokens 79 us there, 94 here; 192 tokens beside 40 decoded ones 92 and 256)."""
+        return D == 128 and V % 128 == 0 and getattr(batch, "max_q_len", 0) >= 320 and T >= 100 * batch.num_segs
+
+    def _chunk_scratch(self, T, batch, H, D, V):
+        """Per chunk and head what it adds to the state, then the state before it."""
+        return torch.empty(self.lib.mi_chunk_floats(T, batch.num_segs, H, D, V), dtype=torch.float32, device=self.device)
+
     def lightning_scan(self, p, H, D, V, decay, state, batch):
         """p [T, >= 2 H D + H V] = q | k | v before silu; state float32 [slots, H D V] (an entry continues from its slot's
         state and leaves the new one there).  Returns float32 [T, H V]."""
@@ -763,6 +775,12 @@ class CudaOps:
             self.launches += 1
             return out
         if wide and self._takes_octets(p, batch, D, V, state):
+            if self._takes_chunks(batch, T, D, V) and p.stride(0) % 8 == 0:
+                _check(self.lib.mi_lightning_chunks(_p(p), p.stride(0), _p(self._chunk_scratch(T, batch, H, D, V)), _p(decay), _p(state),
+                                                    _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs,
+                                                    H, D, V, _p(self._stream_error), self._stream()), "lightning_chunks")
+                self.launches += 3
+                return out
             scratch = self._octet_scratch(T, batch, H, D, V, False)
             _check(self.lib.mi_lightning_octets(_p(p), p.stride(0), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
                                                 _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error),
@@ -1134,6 +1152,12 @@ class CudaOps:
         _check(self.lib.mi_retention_rows(_p(p), p.stride(0), _p(prep), _p(batch.positions), _p(inv_freq), half, _c.c_float(k_scale), T, H, D, V,
                                           _code(p.dtype), self._stream()), "retention_rows")
         if p.dtype == torch.bfloat16 and self._takes_octets(prep, batch, D, V, state):
+            if self._takes_chunks(batch, T, D, V):
+                _check(self.lib.mi_constant_chunks(_p(prep), _p(self._chunk_scratch(T, batch, H, D, V)), _p(decay), _p(state), _c.c_longlong(state.stride(0)),
+                                                   _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error),
+                                                   self._stream()), "constant_chunks")
+                self.launches += 4
+                return out
             scratch = self._octet_scratch(T, batch, H, D, V, False)
             _check(self.lib.mi_constant_octets(_p(prep), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
                                                _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error), self._stream()), "constant_octets")

@@ -211,6 +211,70 @@ def test_recurrences_eight_tokens_at_a_time(ops, lens, H, KV, D, V):        # no
         assert torch.equal(a[:, H * D * V:], state[:, H * D * V:]) and torch.equal(a[0], state[0])
 
 
+def chunk_inputs(lens, H, V, seed):
+    T, D, g = sum(lens), 128, torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
+    batch = Entries(lens)
+    batch.max_q_len, batch.positions = max(lens), torch.arange(T, dtype=torch.int32, device=DEV)
+    decay = torch.tensor([1.0 - 2.0 ** -(1 + 3 * h % 20) for h in range(H)], device=DEV)
+    return batch, r(T, 2 * H * D + H * V + 8).to(torch.bfloat16), r(len(lens) + 1, H * D * V + 6), decay, torch.rand(D // 4, generator=g).to(DEV)
+
+
+def chunk_runs(ops, H, V, decay, freq, batch):
+    return {"constant": lambda p, s: ops.lightning_scan(p, H, 128, V, decay, s, batch),
+            "rotated": lambda p, s: ops.retention_scan(p, H, 128, V, freq, 128 ** -0.5, decay, s, batch)}
+
+
+@pytest.mark.parametrize("lens,H,V", [((320,), 16, 128), ((384,), 3, 256), ((129, 640, 3, 127), 2, 128), ((700, 1, 1, 1, 513), 5, 128)])
+def test_constant_decay_in_chunks(ops, lens, H, V):             # noqa: F811
+    """128 tokens at a time against the token-by-token kernels: whole chunks, remainders, short entries beside long ones, two blocks of columns."""
+    batch, p, state, decay, freq = chunk_inputs(lens, H, V, sum(lens))
+    for name, run in chunk_runs(ops, H, V, decay, freq, batch).items():
+        a, b = state.clone(), state.clone()
+        assert ops._takes_octets(p, batch, 128, V, a) and ops._takes_chunks(batch, sum(lens), 128, V)
+        got = run(p, a)
+        ops._takes_octets = lambda *args: False
+        try:
+            want = run(p, b)
+        finally:
+            del ops._takes_octets
+        ops.check_errors()
+        # two float32 orders of sums over up to 700 decayed tokens and 128 rows
+        assert rows_error(got, want) < 3e-6 and rows_error(a, b) < 3e-6, name
+        assert torch.equal(a[:, H * 128 * V:], state[:, H * 128 * V:]) and torch.equal(a[0], state[0])
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "state", "huge k", "all tiny"])
+def test_chunks_keep_odd_numbers_in_their_place(ops, what):     # noqa: F811
+    """Numbers that three bfloat16 parts do not hold: the outputs are those of the token-by-token kernel, tokens before the number, other entries and
+    other heads have the bits they have without it."""
+    lens, H, V, at = (330, 320), 2, 128, 150                     # token 150: the 23rd of the first entry's second chunk
+    batch, p, state, decay, freq = chunk_inputs(lens, H, V, 3)
+    for name, run in chunk_runs(ops, H, V, decay, freq, batch).items():
+        spoiled, odd_state = p.clone(), state.clone()
+        if what in "qkv":
+            spoiled[at, {"q": 5, "k": 128 * H + 7, "v": 256 * H + 9}[what]] = float("inf") if what != "k" else float("nan")
+        elif what == "state":
+            odd_state[batch.seg_slot[0].item(), 128 * 30 + 4] = float("inf")
+        elif what == "huge k":
+            spoiled[at, 128 * H + 7] = 1e30
+        else:
+            spoiled[at:at + 9, 128 * H:128 * H + 128] = -90.0 if name == "constant" else 1e-35
+        a, b, c = state.clone(), odd_state.clone(), odd_state.clone()
+        want, got = run(p, a), run(spoiled, b)
+        ops._takes_octets = lambda *args: False
+        try:
+            plain = run(spoiled, c)
+        finally:
+            del ops._takes_octets
+        first = 0 if what == "state" else at
+        assert torch.equal(got[:first], want[:first]) and torch.equal(got[330:], want[330:]) and torch.equal(got[:, V:], want[:, V:]), name
+        assert torch.equal(got.isnan(), plain.isnan()) and torch.equal(got.isinf(), plain.isinf()) and torch.equal(b.isnan(), c.isnan()), name
+        ok = plain.isfinite()
+        ok[at + 30 if what == "huge k" else len(ok):] = False    # what 1e30 has swallowed does not come back when it has decayed
+        assert rows_error(torch.where(ok, got, 0.), torch.where(ok, plain, 0.)) < 3e-6, name
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 def test_octets_keep_later_tokens_out(ops, value):              # noqa: F811
     """A value that is no number reaches its own token and the ones after it; the tokens before it in its octet give the bits they give without it."""
