@@ -130,7 +130,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
                 const Item it = item_of<NT>(sh, i);
                 for (int k = 0; k < it.stages; ++k) {
-                    if (turn > 0 && !mbar_wait(w_empty + 8 * s, (turn - 1) & 1)) { atomicExch(error_word, 51); ok = false; break; }
+                    if (turn > 0 && !mbar_wait(w_empty + 8 * s, (turn - 1) & 1)) { atomicExch(error_word, 81); ok = false; break; }
                     mbar_expect_tx(w_full + 8 * s, W_STAGE);
                     const int x = it.k_first + k * BK;
                     tma_load_2d(sW + s * W_STAGE, &wmap, x, it.n0, w_full + 8 * s);
@@ -147,7 +147,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             for (int i = blockIdx.x; i < items && ok; i += gridDim.x) {
                 const Item it = item_of<NT>(sh, i);
                 for (int k = 0; k < it.stages; ++k) {
-                    if (turn > 0 && !mbar_wait(x_empty + 8 * s, (turn - 1) & 1)) { atomicExch(error_word, 52); ok = false; break; }
+                    if (turn > 0 && !mbar_wait(x_empty + 8 * s, (turn - 1) & 1)) { atomicExch(error_word, 82); ok = false; break; }
                     mbar_expect_tx(x_full + 8 * s, X_STAGE);
 #pragma unroll
                     for (int p = 0; p < PARTS; ++p)
@@ -165,9 +165,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
                 const Item it = item_of<NT>(sh, i);
                 for (int k = 0; k < it.stages; ++k, ++n) {
                     const int b = n & 1;
-                    if (n >= 2 && !mbar_spin(d_empty + 8 * b, ((n >> 1) - 1) & 1)) { atomicExch(error_word, 53); ok = false; break; }
-                    if (!mbar_spin(x_full + 8 * xs, x_turn & 1)) { atomicExch(error_word, 54); ok = false; break; }
-                    if (!mbar_spin(a_full + 8 * b, (n >> 1) & 1)) { atomicExch(error_word, 55); ok = false; break; }
+                    if (n >= 2 && !mbar_spin(d_empty + 8 * b, ((n >> 1) - 1) & 1)) { atomicExch(error_word, 83); ok = false; break; }
+                    if (!mbar_spin(x_full + 8 * xs, x_turn & 1)) { atomicExch(error_word, 84); ok = false; break; }
+                    if (!mbar_spin(a_full + 8 * b, (n >> 1) & 1)) { atomicExch(error_word, 85); ok = false; break; }
                     tc_fence_after();
                     const uint32_t d = tmem + D_COL + b * NT, a = tmem + b * A_COLS;
                     const uint64_t x = umma_desc_sw128(sX + xs * X_STAGE, 16, 1024);
@@ -194,9 +194,9 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             __nv_bfloat162 mx = __floats2bfloat162_rn(0.f, 0.f);
             for (int k = 0; k < it.stages; ++k, ++n) {
                 if ((n & 1) == g) {
-                    if (!mbar_wait(w_full + 8 * s, turn & 1)) { atomicExch(error_word, 56); ok = false; break; }
+                    if (!mbar_wait(w_full + 8 * s, turn & 1)) { atomicExch(error_word, 86); ok = false; break; }
                     if (n >= 2) {
-                        if (!mbar_wait(a_empty + 8 * g, ((n >> 1) - 1) & 1)) { atomicExch(error_word, 57); ok = false; break; }
+                        if (!mbar_wait(a_empty + 8 * g, ((n >> 1) - 1) & 1)) { atomicExch(error_word, 87); ok = false; break; }
                         tc_fence_after();
                     }
                     const unsigned char* at = base + s * W_STAGE + row * 128;
@@ -243,7 +243,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             for (int c = 0; c < HALF; ++c) acc[c] = 0.f;
             for (int k = 0; k < it.stages; ++k, ++n) {
                 const int b = n & 1;
-                if (!mbar_wait(d_full + 8 * b, (n >> 1) & 1)) { atomicExch(error_word, 58); ok = false; break; }
+                if (!mbar_wait(d_full + 8 * b, (n >> 1) & 1)) { atomicExch(error_word, 88); ok = false; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < HALF; c += 16) {
@@ -263,7 +263,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
 #pragma unroll
             for (int c = 0; c < HALF; ++c)
                 if (nrow < sh.N && m_first + c < sh.M) to[(size_t)c * sh.ldc] = acc[c];
-            if (!mbar_wait(m_full + 8 * (turn_of_item & 1), (turn_of_item >> 1) & 1)) { atomicExch(error_word, 59); ok = false; break; }
+            if (!mbar_wait(m_full + 8 * (turn_of_item & 1), (turn_of_item >> 1) & 1)) { atomicExch(error_word, 89); ok = false; break; }
             const float* rm = row_max + (turn_of_item & 1) * 2 * BN + row;
             const float most = fmaxf(rm[0], rm[BN]);
             const bool odd_row = !(most <= MOST) || (most > 0.f && most < LEAST);

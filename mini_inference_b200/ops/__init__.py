@@ -16,7 +16,7 @@ import torch
 
 from ..parts.base import GatedDelta
 
-_LIB = None
+_LIB = _CALLS = None
 _c = ctypes
 
 
@@ -24,14 +24,42 @@ def load_library():
     global _LIB
     if _LIB is None:
         from .build import build
-        path = build()
-        _LIB = ctypes.CDLL(path)
-        _LIB.mi_gemm_f32_workspace.restype = _LIB.mi_octet_floats.restype = _LIB.mi_chunk_floats.restype = ctypes.c_longlong
-        # declared, so that addresses and floats pass as plain numbers: with wrapped ones the call cost the host 22.7 us where the
-        # values are the keys and 17.3 elsewhere, now 16.0 and 16.3 (the mma.sync form 14.5), and a step of few tokens waits for the host
-        p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
-        _LIB.mi_attn_prefill_tc_split.argtypes = [p, i, i, p, p, ctypes.c_longlong, p, p, i, p, p, p, p, i, i, i, i, i, i, f, i, p, i, i, p, p, i, p, f, i, p, i, p]
+        _LIB = ctypes.CDLL(build())
     return _LIB
+
+
+class _Pointer:
+    """What ctypes makes of a pointer argument: a tensor, an address, a wrapped address or None."""
+
+    @staticmethod
+    def from_param(v):
+        return ctypes.c_void_p(v.data_ptr() if hasattr(v, "data_ptr") else getattr(v, "value", v))
+
+
+def load_calls():
+    """The library's entry points as functions that take tensors, numbers and None: those of the extension beside the library (ops/build.py), else
+    the same through ctypes."""
+    global _CALLS
+    if _CALLS is None:
+        import types
+        from .build import INTEGER, POINTER, host_calls, signatures
+        lib, fast, calls = load_library(), host_calls(), types.SimpleNamespace()
+        for name, (ret, args) in signatures().items():
+            fn = getattr(lib, name, None)                        # entry points behind a build flag
+            if fn is None:
+                continue
+            fn.restype = ctypes.c_int if ret == "int" else ctypes.c_longlong
+            if fast is not None:
+                fast.bind(name, ctypes.cast(fn, ctypes.c_void_p).value)
+                fn = getattr(fast, name)
+            else:
+                fn = ctypes.CDLL(lib._name)[name]                # a function object of its own: the library's stays undeclared
+                fn.restype = ctypes.c_int if ret == "int" else ctypes.c_longlong
+                fn.argtypes = [_Pointer if k == POINTER else (ctypes.c_longlong if t == "long long" else ctypes.c_int) if k == INTEGER else ctypes.c_float
+                               for t, k in args]
+            setattr(calls, name, fn)
+        _CALLS = calls
+    return _CALLS
 
 
 _CODES = {torch.float32: 0, torch.bfloat16: 1}
@@ -44,15 +72,12 @@ def _code(dtype):
         raise TypeError(f"dtype {dtype} is not supported by the kernels (float32, bfloat16)") from None
 
 
-def _raw_stream(device_index):
-    getter = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if getter is not None:
-        return getter(device_index)
-    return torch.cuda.current_stream(device_index).cuda_stream
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device_index: torch.cuda.current_stream(device_index).cuda_stream)
 
 
 def _p(t):
-    return _c.c_void_p(0 if t is None else t.data_ptr())
+    """A pointer argument of an entry point: the tensor itself (None: a null pointer)."""
+    return t
 
 
 def _check(err, what):
@@ -90,7 +115,7 @@ class CudaOps:
         if self.device.type != "cuda" or not torch.cuda.is_available():
             raise RuntimeError("mini_inference_b200 runs on a CUDA device only (no CPU path); "
                                f"device '{device}' is not one")
-        self.lib = load_library()
+        self.lib = load_calls()
         self._device_index = self.device.index if self.device.index is not None else torch.cuda.current_device()
         self.NUM_SMS = torch.cuda.get_device_properties(self._device_index).multi_processor_count
         self.force_splits = None             # tests set this to exercise the split merge on short contexts
@@ -150,21 +175,21 @@ class CudaOps:
     def _stream(self):
         # the raw handle of torch's current stream on this device: one C call (torch.cuda.current_stream builds a
         # Stream object every time, which at ~10 launches per layer was a fifth of an eager decode step's host time)
-        return _c.c_void_p(_raw_stream(self._device_index))
+        return _raw_stream(self._device_index)
 
     # ---------------------------------------------------------------- elementwise / norms
     def scatter_i32(self, table, idx, val):
         """table[idx[i]] = val[i]: the block-table entries that changed since the last step (cache/manager.py)."""
         n = idx.shape[0]
         if n:
-            _check(self.lib.mi_scatter_i32(_p(table), _p(idx), _p(val), n, _c.c_longlong(table.numel()), self._stream()),
+            _check(self.lib.mi_scatter_i32(table, idx, val, n, table.numel(), self._stream()),
                    "scatter_i32")
             self.launches += 1
 
     def embedding(self, ids, table):
         T, hidden = ids.shape[0], table.shape[1]
         out = torch.empty((T, hidden), dtype=table.dtype, device=table.device)
-        _check(self.lib.mi_embedding(_p(ids), _p(table), _p(out), T, hidden, table.shape[0], _code(table.dtype),
+        _check(self.lib.mi_embedding(ids, table, out, T, hidden, table.shape[0], _code(table.dtype),
                                      self._stream()), "embedding")
         self.launches += 1
         return out
@@ -179,9 +204,9 @@ class CudaOps:
         if isinstance(delta, DeferredSum):
             if rows is None and x.dtype == torch.bfloat16 and x.is_contiguous() and hidden % 4 == 0 and delta.shape == tuple(x.shape):
                 y = torch.empty_like(x)
-                rc = self.lib.mi_deferred_add_rmsnorm(_p(x), _p(delta.ws), _p(weight), _p(y), delta.M, delta.N, delta.K, delta.grid,
-                                                      delta.max_contrib, delta.tok, _c.c_float(eps), _code(weight.dtype),
-                                                      _p(ahead), _c.c_longlong(ahead_bytes), self._stream())
+                rc = self.lib.mi_deferred_add_rmsnorm(x, delta.ws, weight, y, delta.M, delta.N, delta.K, delta.grid,
+                                                      delta.max_contrib, delta.tok, eps, _code(weight.dtype),
+                                                      ahead, ahead_bytes, self._stream())
                 if rc == 0:
                     self.launches += 1
                     return y
@@ -191,8 +216,8 @@ class CudaOps:
         assert x.is_contiguous() and (delta is None or delta.is_contiguous())
         n = x.shape[0] if rows is None else rows.shape[0]
         y = torch.empty((n, hidden), dtype=x.dtype, device=x.device)
-        _check(self.lib.mi_add_rmsnorm_ahead(_p(x), _p(delta), _p(weight), _p(y), _p(rows), n, hidden, _c.c_float(eps),
-                                             _code(x.dtype), _code(weight.dtype), _p(ahead), _c.c_longlong(ahead_bytes),
+        _check(self.lib.mi_add_rmsnorm_ahead(x, delta, weight, y, rows, n, hidden, eps,
+                                             _code(x.dtype), _code(weight.dtype), ahead, ahead_bytes,
                                              self._stream()), "add_rmsnorm")
         self.launches += 1
         return y
@@ -208,7 +233,7 @@ class CudaOps:
         if (self._use_tc(M, w.shape[0], K) and K % 64 == 0 and inter % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
                 and w.is_contiguous() and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16):
             out = torch.empty((M, inter), dtype=torch.bfloat16, device=x.device)
-            rc = self.lib.mi_gemm_tc2_glu(_p(x), x.stride(0), _p(w), _p(out), M, inter, K, self.GATES[act], *self._tc2_scratch(), _p(self._stream_error), self._stream())
+            rc = self.lib.mi_gemm_tc2_glu(x, x.stride(0), w, out, M, inter, K, self.GATES[act], *self._tc2_scratch(), self._stream_error, self._stream())
             if rc == 0:
                 self.launches += 1
                 return out
@@ -217,7 +242,7 @@ class CudaOps:
         gu = self.linear(x, w, defer=True)
         if isinstance(gu, DeferredSum):          # the few-row product left its partial sums: the activation kernel adds them
             out = torch.empty((M, inter), dtype=torch.bfloat16, device=x.device)
-            rc = self.lib.mi_deferred_glu(_p(gu.ws), _p(out), M, inter, gu.K, gu.grid, gu.max_contrib, gu.tok, self.GATES[act], self._stream())
+            rc = self.lib.mi_deferred_glu(gu.ws, out, M, inter, gu.K, gu.grid, gu.max_contrib, gu.tok, self.GATES[act], self._stream())
             if rc == 0:
                 self.launches += 1
                 return out
@@ -231,7 +256,7 @@ class CudaOps:
         if not isinstance(value, DeferredSum):
             return value
         out = torch.empty((value.M, value.N), dtype=torch.bfloat16, device=value.device)
-        _check(self.lib.mi_deferred_reduce(_p(value.ws), _p(out), value.M, value.N, value.K, value.grid, value.max_contrib,
+        _check(self.lib.mi_deferred_reduce(value.ws, out, value.M, value.N, value.K, value.grid, value.max_contrib,
                                            value.tok, self._stream()), "deferred_reduce")
         self.launches += 1
         return out
@@ -240,7 +265,7 @@ class CudaOps:
         rows, inter = gate_up.shape[0], gate_up.shape[1] // 2
         assert gate_up.is_contiguous()
         out = torch.empty((rows, inter), dtype=gate_up.dtype, device=gate_up.device)
-        _check(self.lib.mi_swiglu(_p(gate_up), _p(out), rows, inter, _code(gate_up.dtype), self._stream()), "swiglu")
+        _check(self.lib.mi_swiglu(gate_up, out, rows, inter, _code(gate_up.dtype), self._stream()), "swiglu")
         self.launches += 1
         return out
 
@@ -276,7 +301,7 @@ class CudaOps:
             N = w.shape[0]
             od = out_dtype or x.dtype
             out = torch.empty((M, N), dtype=od, device=x.device)
-            err = self.lib.mi_gemm_skinny(_p(x), x.stride(0), _p(w), _p(out), N, M, N, K, _code(od), self._stream())
+            err = self.lib.mi_gemm_skinny(x, x.stride(0), w, out, N, M, N, K, _code(od), self._stream())
             if err == 0:
                 self.launches += 1
                 return out
@@ -289,7 +314,7 @@ class CudaOps:
         and K alone, their partial sums pass a workspace.  tile: a tile of csrc/gemm_f32.cu instead of its own choice (same bits)."""
         n = self.lib.mi_gemm_f32_workspace(M, N, K)
         ws = torch.empty(n, dtype=torch.float32, device=x.device) if n else None
-        _check(self.lib.mi_gemm_f32_nt(_p(x), ldx, _p(w), _p(out), ldc, M, N, K, _p(ws), tile, _p(self._stream_error), self._stream()), "gemm_f32")
+        _check(self.lib.mi_gemm_f32_nt(x, ldx, w, out, ldc, M, N, K, ws, tile, self._stream_error, self._stream()), "gemm_f32")
         self.launches += 2 if n else 1
 
     @staticmethod
@@ -444,7 +469,7 @@ class CudaOps:
         plan = self._stream_plans.get((M, N, K))
         if plan is None:
             g, rt, mc = _c.c_int(), _c.c_int(), _c.c_int()
-            rc = self.lib.mi_gemm_stream_plan(M, N, K, _c.byref(g), _c.byref(rt), _c.byref(mc))
+            rc = load_library().mi_gemm_stream_plan(M, N, K, _c.byref(g), _c.byref(rt), _c.byref(mc))
             plan = self._stream_plans[(M, N, K)] = None if rc else (g.value, rt.value, mc.value)
         if not plan:
             return None
@@ -454,7 +479,7 @@ class CudaOps:
         tok = 8 if M <= 8 else 16 if M <= 16 else 32
         workspace = torch.empty(row_tiles * max_contrib * 128 * tok, dtype=torch.float32, device=x.device)
         if defer:
-            rc = self.lib.mi_gemm_stream_deferred(_p(x), x.stride(0), _p(w), M, N, K, _p(workspace), _p(self._stream_error),
+            rc = self.lib.mi_gemm_stream_deferred(x, x.stride(0), w, M, N, K, workspace, self._stream_error,
                                                   self._stream())
             if rc == 0:
                 self.launches += 1
@@ -462,8 +487,8 @@ class CudaOps:
             if rc != -2:
                 _check(rc, "gemm_stream_deferred")
         out = torch.empty((M, N), dtype=od, device=x.device)
-        rc = self.lib.mi_gemm_stream(_p(x), x.stride(0), _p(w), _p(out), N, M, N, K, _code(od), _p(workspace),
-                                     _p(self._stream_counters), _p(self._stream_error), self._stream())
+        rc = self.lib.mi_gemm_stream(x, x.stride(0), w, out, N, M, N, K, _code(od), workspace,
+                                     self._stream_counters, self._stream_error, self._stream())
         if rc == -2:
             return None
         _check(rc, "gemm_stream")
@@ -478,7 +503,7 @@ class CudaOps:
         if od != torch.bfloat16 or N % 8:
             return None
         out = torch.empty((M, N), dtype=od, device=x.device)
-        rc = self.lib.mi_gemm_tc2(_p(x), x.stride(0), _p(w), _p(out), N, M, N, K, *self._tc2_scratch(), _p(self._stream_error), self._stream())
+        rc = self.lib.mi_gemm_tc2(x, x.stride(0), w, out, N, M, N, K, *self._tc2_scratch(), self._stream_error, self._stream())
         if rc == -2:
             return None
         _check(rc, "gemm_tc2")
@@ -486,7 +511,7 @@ class CudaOps:
         return out
 
     def _tc2_scratch(self):
-        return (_p(self._tc2_ws), _c.c_longlong(self._tc2_ws.numel()), _p(self._tc2_counters), self._tc2_counters.numel())
+        return (self._tc2_ws, self._tc2_ws.numel(), self._tc2_counters, self._tc2_counters.numel())
 
     def check_errors(self):
         """Raises if a bounded wait inside a kernel ran out (synchronises the device)."""
@@ -502,8 +527,8 @@ class CudaOps:
         assert qkv.is_contiguous() and qkv.shape[1] == (H + 2 * KV) * D
         w_dtype = q_weight.dtype if q_weight is not None else qkv.dtype
         _check(self.lib.mi_qk_norm_rope_cache(
-            _p(qkv), _p(q_weight), _p(k_weight), _p(inv_freq), _p(meta.positions), _p(meta.slots),
-            _p(k_cache), _p(v_cache), T, H, KV, D, meta.page_size, _c.c_float(eps), _code(qkv.dtype),
+            qkv, q_weight, k_weight, inv_freq, meta.positions, meta.slots,
+            k_cache, v_cache, T, H, KV, D, meta.page_size, eps, _code(qkv.dtype),
             _code(w_dtype), self._stream()), "qk_norm_rope_cache")
         self.launches += 1
         return qkv[:, :H * D]
@@ -572,25 +597,25 @@ class CudaOps:
             self._prefill_tc_split(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
         elif tc and not split_weights:
             rc = self.lib.mi_attn_prefill_tc(
-                _p(q), q.stride(0), T, _p(k_cache), _p(v_cache), _c.c_longlong(k_cache.shape[0] * KV * meta.page_size),
-                _p(out), _p(tiles2), num_tiles2, _p(meta.seg_q_start), _p(meta.seg_pos0),
-                _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, meta.page_size, 128, _c.c_float(scale), win,
-                _p(self._stream_error), self._stream())
+                q, q.stride(0), T, k_cache, v_cache, (k_cache.shape[0] * KV * meta.page_size),
+                out, tiles2, num_tiles2, meta.seg_q_start, meta.seg_pos0,
+                meta.block_table, rows, meta.max_pages, H, KV, D, meta.page_size, 128, scale, win,
+                self._stream_error, self._stream())
             _check(rc, "attn_prefill_tc")
             self.launches += 1
         elif num_tiles and fast and meta.tile == 64:
             _check((self.lib.mi_attn_prefill_mma_split if split_weights else self.lib.mi_attn_prefill_mma)(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles,
-                _p(meta.seg_q_start), _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D,
-                meta.page_size, meta.tile, _c.c_float(scale), win, self._stream()), "attn_prefill_mma")
+                q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, num_tiles,
+                meta.seg_q_start, meta.seg_pos0, meta.block_table, rows, meta.max_pages, H, KV, D,
+                meta.page_size, meta.tile, scale, win, self._stream()), "attn_prefill_mma")
             self.launches += 1
         elif num_tiles and self._f32_tiles(q, D, D, meta, k_cache, v_cache):
             self._prefill_f32(q, k_cache, v_cache, out, meta, H, KV, D, scale, 0, win)
         elif num_tiles:
             _check(self.lib.mi_attn_prefill_generic(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles,
-                _p(meta.seg_q_start), _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D,
-                meta.page_size, meta.tile, _c.c_float(scale), win, code, self._stream()), "attn_prefill")
+                q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, num_tiles,
+                meta.seg_q_start, meta.seg_pos0, meta.block_table, rows, meta.max_pages, H, KV, D,
+                meta.page_size, meta.tile, scale, win, code, self._stream()), "attn_prefill")
             self.launches += 1
         if not num_decode:
             return out
@@ -612,21 +637,21 @@ class CudaOps:
             # without counters the splits stay in o_part / lse for the merge launch below: the cluster merge must be off too
             cluster = int(self.cluster_merge and counters is not None)
             _check((self.lib.mi_attn_decode_mma_rows_split if split_weights else self.lib.mi_attn_decode_mma_rows)(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(o_part), _p(lse), _p(meta.decode_segs),
-                num_decode, _p(meta.seg_q_start), _p(meta.seg_kv_len), _p(meta.block_table), _p(rows), meta.max_pages,
-                H, KV, D, meta.page_size, S, _c.c_float(scale), win, _p(counters),
-                _p(self._stream_error if self.bulk_decode else None), k_cache.shape[0], cluster, self._stream()),
+                q, q.stride(0), k_cache, v_cache, out, o_part, lse, meta.decode_segs,
+                num_decode, meta.seg_q_start, meta.seg_kv_len, meta.block_table, rows, meta.max_pages,
+                H, KV, D, meta.page_size, S, scale, win, counters,
+                (self._stream_error if self.bulk_decode else None), k_cache.shape[0], cluster, self._stream()),
                 "attn_decode_mma")
             self.launches += 1
             if S > 1 and counters is None:
-                _check(self.lib.mi_attn_decode_merge(_p(o_part), _p(lse), _p(out), _p(meta.decode_segs), num_decode,
-                                                     _p(meta.seg_q_start), H, D, S, code, self._stream()), "attn_merge")
+                _check(self.lib.mi_attn_decode_merge(o_part, lse, out, meta.decode_segs, num_decode,
+                                                     meta.seg_q_start, H, D, S, code, self._stream()), "attn_merge")
                 self.launches += 1
         else:
             _check(self.lib.mi_attn_decode_generic(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(o_part), _p(lse), _p(meta.decode_segs),
-                num_decode, _p(meta.seg_q_start), _p(meta.seg_kv_len), _p(meta.block_table), _p(rows), meta.max_pages,
-                H, KV, D, meta.page_size, S, _c.c_float(scale), win, code, self._stream()), "attn_decode")
+                q, q.stride(0), k_cache, v_cache, out, o_part, lse, meta.decode_segs,
+                num_decode, meta.seg_q_start, meta.seg_kv_len, meta.block_table, rows, meta.max_pages,
+                H, KV, D, meta.page_size, S, scale, win, code, self._stream()), "attn_decode")
             self.launches += 2 if S > 1 else 1
         return out
 
@@ -665,9 +690,9 @@ class CudaOps:
     def _prefill_f32(self, q, k_cache, v_cache, out, meta, H, KV, D, scale, block, window, sink=0, sink_values=None, bias=None, bias_last=0,
                      slopes=None, cap=0.0, keep=0, gate=None, gate_stride=0):
         _check(self.lib.mi_attn_prefill_f32(
-            _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), meta.prefill_tiles.shape[0], _p(meta.seg_q_start),
-            _p(meta.seg_pos0), _p(meta.block_table), _p(getattr(meta, "table_rows", None)), meta.max_pages, H, KV, D, meta.page_size, meta.tile,
-            _c.c_float(scale), block, window, sink, _p(sink_values), _p(bias), bias_last, _p(slopes), _c.c_float(cap), keep, _p(gate), gate_stride,
+            q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, meta.prefill_tiles.shape[0], meta.seg_q_start,
+            meta.seg_pos0, meta.block_table, (getattr(meta, "table_rows", None)), meta.max_pages, H, KV, D, meta.page_size, meta.tile,
+            scale, block, window, sink, sink_values, bias, bias_last, slopes, cap, keep, gate, gate_stride,
             self._stream()), "attn_prefill_f32")
         self.launches += 1
 
@@ -676,7 +701,7 @@ class CudaOps:
         """x = g * e / rms(e), e = table[ids]: the start of a residual stream (float32 [T, hidden] when out_dtype says so)."""
         T, hidden = ids.shape[0], table.shape[1]
         x = torch.empty((T, hidden), dtype=out_dtype, device=table.device)
-        _check(self.lib.mi_embed_scaled_norm(_p(ids), _p(table), _p(g), _p(x), T, hidden, table.shape[0], _c.c_float(eps),
+        _check(self.lib.mi_embed_scaled_norm(ids, table, g, x, T, hidden, table.shape[0], eps,
                                              _code(table.dtype), _code(out_dtype), self._stream()), "embed_scaled_norm")
         self.launches += 1
         return x
@@ -688,7 +713,7 @@ class CudaOps:
         hidden = x.shape[-1]
         n = x.shape[0] if rows is None else rows.shape[0]
         y = torch.empty((n, hidden), dtype=out_dtype, device=x.device)
-        _check(self.lib.mi_add_scaled_rmsnorm(_p(x), _p(delta), _p(pre_add), _p(g), _p(y), _p(rows), n, hidden, _c.c_float(eps),
+        _check(self.lib.mi_add_scaled_rmsnorm(x, delta, pre_add, g, y, rows, n, hidden, eps,
                                               _code(delta.dtype if delta is not None else out_dtype), _code(out_dtype),
                                               self._stream()), "add_scaled_rmsnorm")
         self.launches += 1
@@ -698,7 +723,7 @@ class CudaOps:
         """a N(z) + b N(z^2) + c N(z^3) + e per row, N(y) = y / rms(y); coef = float32 (a, b, c, e) on the device."""
         assert z.is_contiguous()
         out = torch.empty_like(z)
-        _check(self.lib.mi_polynorm(_p(z), _p(coef), _p(out), z.shape[0], z.shape[1], _c.c_float(eps), _code(z.dtype), self._stream()),
+        _check(self.lib.mi_polynorm(z, coef, out, z.shape[0], z.shape[1], eps, _code(z.dtype), self._stream()),
                "polynorm")
         self.launches += 1
         return out
@@ -710,8 +735,8 @@ class CudaOps:
         T = o.shape[0]
         assert o.dtype == torch.float32 and o.is_contiguous() and gate.stride(1) == 1 and gate.dtype == out_dtype
         y = torch.empty((T, groups * gs), dtype=out_dtype, device=o.device)
-        _check(self.lib.mi_group_rmsnorm_gate(_p(o), _p(weight), 1 if weight is None else weight.numel(), _p(gate), gate.stride(0), _p(y),
-                                              T, groups, gs, _c.c_float(eps), _code(out_dtype), {"sigmoid": 0, "silu": 1}[act],
+        _check(self.lib.mi_group_rmsnorm_gate(o, weight, 1 if weight is None else weight.numel(), gate, gate.stride(0), y,
+                                              T, groups, gs, eps, _code(out_dtype), {"sigmoid": 0, "silu": 1}[act],
                                               self._stream()), "group_rmsnorm_gate")
         self.launches += 1
         return y
@@ -722,7 +747,7 @@ class CudaOps:
         H, T, V = o.shape
         assert o.is_contiguous() and o.dtype == out_dtype and (gate is None or (gate.stride(1) == 1 and gate.dtype == out_dtype))
         y = torch.empty((T, H * V), dtype=out_dtype, device=o.device)
-        _check(self.lib.mi_head_gate(_p(o), _p(gate), 0 if gate is None else gate.stride(0), _p(y), T, H, V, _code(out_dtype), self._stream()), "head_gate")
+        _check(self.lib.mi_head_gate(o, gate, 0 if gate is None else gate.stride(0), y, T, H, V, _code(out_dtype), self._stream()), "head_gate")
         self.launches += 1
         return y
 
@@ -770,26 +795,26 @@ class CudaOps:
         out = torch.empty((T, H * V), dtype=torch.float32, device=p.device)
         wide = p.dtype == torch.bfloat16
         if wide and self._takes_step(T, batch, D, V, state):
-            _check(self.lib.mi_lightning_step(_p(p), p.stride(0), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                              _p(batch.seg_slot), T, H, D, V, self._stream()), "lightning_step")
+            _check(self.lib.mi_lightning_step(p, p.stride(0), decay, state, state.stride(0), out, batch.seg_q_start,
+                                              batch.seg_slot, T, H, D, V, self._stream()), "lightning_step")
             self.launches += 1
             return out
         if wide and self._takes_octets(p, batch, D, V, state):
             if self._takes_chunks(batch, T, D, V) and p.stride(0) % 8 == 0:
-                _check(self.lib.mi_lightning_chunks(_p(p), p.stride(0), _p(self._chunk_scratch(T, batch, H, D, V)), _p(decay), _p(state),
-                                                    _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs,
-                                                    H, D, V, _p(self._stream_error), self._stream()), "lightning_chunks")
+                _check(self.lib.mi_lightning_chunks(p, p.stride(0), self._chunk_scratch(T, batch, H, D, V), decay, state,
+                                                    state.stride(0), out, batch.seg_q_start, batch.seg_slot, T, batch.num_segs,
+                                                    H, D, V, self._stream_error, self._stream()), "lightning_chunks")
                 self.launches += 3
                 return out
             scratch = self._octet_scratch(T, batch, H, D, V, False)
-            _check(self.lib.mi_lightning_octets(_p(p), p.stride(0), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
-                                                _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error),
+            _check(self.lib.mi_lightning_octets(p, p.stride(0), scratch, decay, state, state.stride(0), out,
+                                                batch.seg_q_start, batch.seg_slot, T, batch.num_segs, H, D, V, self._stream_error,
                                                 self._stream()), "lightning_octets")
             self.launches += 2
             return out
         prep = torch.empty((T, 2 * H * D + H * V), dtype=torch.float32, device=p.device)      # silu(q | k | v), what the scan stages
-        _check(self.lib.mi_lightning_scan(_p(p), p.stride(0), _p(prep), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out),
-                                          _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _code(p.dtype),
+        _check(self.lib.mi_lightning_scan(p, p.stride(0), prep, decay, state, state.stride(0), out,
+                                          batch.seg_q_start, batch.seg_slot, T, batch.num_segs, H, D, V, _code(p.dtype),
                                           self._stream()), "lightning_scan")
         self.launches += 2
         return out
@@ -804,10 +829,10 @@ class CudaOps:
         C = 2 * KV * D + H * V
         assert p.stride(1) == 1 and a.stride(1) == 1 and a.dtype == p.dtype and state.is_contiguous()
         out = torch.empty((T, (C + H * D + H + 3) // 4 * 4), dtype=torch.float32, device=p.device)
-        _check(self.lib.mi_delta_prepare(_p(p), p.stride(0), _p(a), a.stride(0), _p(conv), _p(A_log), _p(dt_bias), _p(state),
-                                         _c.c_longlong(state.stride(0)), _c.c_longlong(H * D * V), _p(out), out.stride(0),
-                                         _p(batch.token_seg), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs,
-                                         H, KV, D, V, taps, _c.c_float(unit_eps), _code(p.dtype), self._stream()), "delta_prepare")
+        _check(self.lib.mi_delta_prepare(p, p.stride(0), a, a.stride(0), conv, A_log, dt_bias, state,
+                                         state.stride(0), (H * D * V), out, out.stride(0),
+                                         batch.token_seg, batch.seg_q_start, batch.seg_slot, T, batch.num_segs,
+                                         H, KV, D, V, taps, unit_eps, _code(p.dtype), self._stream()), "delta_prepare")
         self.launches += 2 if taps > 1 and not (T == batch.num_segs and T < 256) else 1
         return out
 
@@ -817,18 +842,18 @@ class CudaOps:
         T = prep.shape[0]
         out = torch.empty((T, H * V), dtype=torch.float32, device=prep.device)
         if not exact and self._takes_step(T, batch, D, V, state):
-            _check(self.lib.mi_delta_step(_p(prep), prep.stride(0), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                          _p(batch.seg_slot), T, H, KV, D, V, self._stream()), "delta_step")
+            _check(self.lib.mi_delta_step(prep, prep.stride(0), state, state.stride(0), out, batch.seg_q_start,
+                                          batch.seg_slot, T, H, KV, D, V, self._stream()), "delta_step")
             self.launches += 1
             return out
         if not exact and self._takes_octets(prep, batch, D, V, state):
             scratch = self._octet_scratch(T, batch, H, D, V, True)
-            _check(self.lib.mi_delta_octets(_p(prep), prep.stride(0), _p(scratch), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                            _p(batch.seg_slot), T, batch.num_segs, H, KV, D, V, _p(self._stream_error), self._stream()), "delta_octets")
+            _check(self.lib.mi_delta_octets(prep, prep.stride(0), scratch, state, state.stride(0), out, batch.seg_q_start,
+                                            batch.seg_slot, T, batch.num_segs, H, KV, D, V, self._stream_error, self._stream()), "delta_octets")
             self.launches += 2
             return out
-        _check(self.lib.mi_delta_scan(_p(prep), prep.stride(0), _p(state), _c.c_longlong(state.stride(0)), _p(out),
-                                      _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, KV, D, V, self._stream()),
+        _check(self.lib.mi_delta_scan(prep, prep.stride(0), state, state.stride(0), out,
+                                      batch.seg_q_start, batch.seg_slot, T, batch.num_segs, H, KV, D, V, self._stream()),
                "delta_scan")
         self.launches += 1
         return out
@@ -868,9 +893,9 @@ class CudaOps:
         assert p.stride(1) == 1 and q_abs.is_contiguous() and (q_rows is None or (q_rows.stride(1) == 1 and q_rows.dtype == p.dtype))
         q = torch.empty((T, H, C + R), dtype=p.dtype, device=p.device)
         nf = 0 if inv_freq is None else inv_freq.numel()
-        _check(self.lib.mi_latent_prepare(_p(p), p.stride(0), _p(q_rows), 0 if q_rows is None else q_rows.stride(0),
-                                          -1 if dkv_col is None else int(dkv_col), _p(q_abs), _p(q), _p(cache), _p(norm_w), _p(inv_freq), nf,
-                                          _p(meta.positions), _p(meta.slots), T, H, D, R, C, _c.c_float(eps), int(bool(half_pairs)), _code(p.dtype),
+        _check(self.lib.mi_latent_prepare(p, p.stride(0), q_rows, 0 if q_rows is None else q_rows.stride(0),
+                                          -1 if dkv_col is None else int(dkv_col), q_abs, q, cache, norm_w, inv_freq, nf,
+                                          meta.positions, meta.slots, T, H, D, R, C, eps, int(bool(half_pairs)), _code(p.dtype),
                                           self._stream()), "latent_prepare")
         self.launches += 1
         return q
@@ -909,10 +934,10 @@ class CudaOps:
         out = torch.empty((H, T, C), dtype=q.dtype, device=q.device)
         buf, hs, ts = out, T * C, C
         if num_tiles:
-            _check(self.lib.mi_latent_prefill(_p(q), _p(cache), _p(buf), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),
-                                              _p(meta.seg_pos0), _p(meta.block_table), _p(meta.table_rows), meta.max_pages,
-                                              _c.c_longlong(hs), _c.c_longlong(ts), H, C, R, meta.page_size, meta.tile,
-                                              _c.c_float(scale), _p(sink_values), code, self._stream()), "latent_prefill")
+            _check(self.lib.mi_latent_prefill(q, cache, buf, meta.prefill_tiles, num_tiles, meta.seg_q_start,
+                                              meta.seg_pos0, meta.block_table, meta.table_rows, meta.max_pages,
+                                              hs, ts, H, C, R, meta.page_size, meta.tile,
+                                              scale, sink_values, code, self._stream()), "latent_prefill")
             self.launches += 1
         if num_decode:
             S = self.choose_splits(num_decode * math.ceil(H / 4), meta.max_kv_len, 2)
@@ -920,10 +945,10 @@ class CudaOps:
             if S > 1:
                 o_part = torch.empty((num_decode, H, S, C), dtype=torch.float32, device=q.device)
                 lse = torch.empty((num_decode, H, S), dtype=torch.float32, device=q.device)
-            _check(self.lib.mi_latent_decode(_p(q), _p(cache), _p(buf), _p(o_part), _p(lse), _p(meta.decode_segs), num_decode,
-                                             _p(meta.seg_q_start), _p(meta.seg_kv_len), _p(meta.block_table), _p(meta.table_rows),
-                                             meta.max_pages, _c.c_longlong(hs), _c.c_longlong(ts), H, C, R, meta.page_size, S,
-                                             _c.c_float(scale), _p(sink_values), code, self._stream()), "latent_decode")
+            _check(self.lib.mi_latent_decode(q, cache, buf, o_part, lse, meta.decode_segs, num_decode,
+                                             meta.seg_q_start, meta.seg_kv_len, meta.block_table, meta.table_rows,
+                                             meta.max_pages, hs, ts, H, C, R, meta.page_size, S,
+                                             scale, sink_values, code, self._stream()), "latent_decode")
             self.launches += 2 if S > 1 else 1
         return out
 
@@ -935,7 +960,7 @@ class CudaOps:
         x = torch.empty((T, hidden), dtype=torch.float32, device=table.device)
         rows = None if rows_dtype == torch.float32 else torch.empty((T, hidden), dtype=table.dtype, device=table.device)
         assert table.dtype == rows_dtype
-        _check(self.lib.mi_embed_stream(_p(ids), _p(table), _p(x), _p(rows), T, hidden, table.shape[0], _code(table.dtype),
+        _check(self.lib.mi_embed_stream(ids, table, x, rows, T, hidden, table.shape[0], _code(table.dtype),
                                         self._stream()), "embed_stream")
         self.launches += 1
         return x, (x if rows is None else rows)
@@ -943,7 +968,7 @@ class CudaOps:
     def cast_rows(self, x, dtype):
         assert x.dtype == torch.float32 and x.is_contiguous()
         y = torch.empty(x.shape, dtype=dtype, device=x.device)
-        _check(self.lib.mi_cast_rows(_p(x), _p(y), _c.c_longlong(x.numel()), _code(dtype), self._stream()), "cast_rows")
+        _check(self.lib.mi_cast_rows(x, y, x.numel(), _code(dtype), self._stream()), "cast_rows")
         self.launches += 1
         return y
 
@@ -952,8 +977,8 @@ class CudaOps:
         rows_dtype (x itself when that is float32)."""
         assert x.dtype == torch.float32 and x.is_contiguous() and y.is_contiguous() and y.shape == x.shape
         rows = None if rows_dtype == torch.float32 else torch.empty(x.shape, dtype=rows_dtype, device=x.device)
-        _check(self.lib.mi_out_rmsnorm_add(_p(x), _p(y), _p(weight), _p(scale), _c.c_float(mult), _p(rows), x.shape[0], x.shape[1],
-                                           _c.c_float(eps), _code(y.dtype), self._stream()), "out_rmsnorm_add")
+        _check(self.lib.mi_out_rmsnorm_add(x, y, weight, scale, mult, rows, x.shape[0], x.shape[1],
+                                           eps, _code(y.dtype), self._stream()), "out_rmsnorm_add")
         self.launches += 1
         return x if rows is None else rows
 
@@ -967,12 +992,12 @@ class CudaOps:
             d = delta
             assert x.dtype == torch.float32 and x.is_contiguous() and d.y.is_contiguous() and d.logits.is_contiguous() and d.y.dtype == d.logits.dtype
             assert d.y.shape == x.shape and d.logits.shape == x.shape and d.bias.dtype == torch.float32
-            _check(self.lib.mi_stream_rmsnorm_gated(_p(x), _p(d.y), _p(d.logits), _p(d.bias), _p(d.y_bias), _p(weight), _p(y), _p(rows), n, hidden,
-                                                    _c.c_float(eps), _code(d.y.dtype), _code(out_dtype), self._stream()), "stream_rmsnorm_gated")
+            _check(self.lib.mi_stream_rmsnorm_gated(x, d.y, d.logits, d.bias, d.y_bias, weight, y, rows, n, hidden,
+                                                    eps, _code(d.y.dtype), _code(out_dtype), self._stream()), "stream_rmsnorm_gated")
             self.launches += 1
             return y
         assert x.dtype == torch.float32 and x.is_contiguous() and (delta is None or delta.is_contiguous())
-        _check(self.lib.mi_stream_rmsnorm(_p(x), _p(delta), _p(weight), _p(y), _p(rows), n, hidden, _c.c_float(eps),
+        _check(self.lib.mi_stream_rmsnorm(x, delta, weight, y, rows, n, hidden, eps,
                                           _code(delta.dtype if delta is not None else out_dtype), _code(out_dtype), self._stream()),
                "stream_rmsnorm")
         self.launches += 1
@@ -993,11 +1018,11 @@ class CudaOps:
         assert source is None or (source.stride(1) == 1 and source.dtype == p.dtype and lam is not None)
         assert q_weight is None or (q_weight.dtype == k_weight.dtype == torch.float32 and q_weight.numel() == k_weight.numel() == D)
         coef, every = q_temp if q_temp else (0.0, 0)
-        _check(self.lib.mi_normed_qk_cache(_p(p), p.stride(0), _p(source), 0 if source is None else source.stride(0), _p(lam if source is not None else None),
-                                           _p(meta.slots), _p(k_cache), _p(v_cache), T, H, KV, D, V, meta.page_size,
-                                           _c.c_float(eps or 0.0), int(eps is not None), _p(q_weight), _p(k_weight),
-                                           _p(meta.positions if q_temp or inv_freq is not None else None), _c.c_float(coef), int(every),
-                                           int(bool(values_are_keys)), _p(inv_freq), 0 if inv_freq is None else inv_freq.numel(), _code(p.dtype), self._stream()), "unit_qk_cache")
+        _check(self.lib.mi_normed_qk_cache(p, p.stride(0), source, 0 if source is None else source.stride(0), (lam if source is not None else None),
+                                           meta.slots, k_cache, v_cache, T, H, KV, D, V, meta.page_size,
+                                           (eps or 0.0), int(eps is not None), q_weight, k_weight,
+                                           (meta.positions if q_temp or inv_freq is not None else None), coef, int(every),
+                                           int(bool(values_are_keys)), inv_freq, 0 if inv_freq is None else inv_freq.numel(), _code(p.dtype), self._stream()), "unit_qk_cache")
         self.launches += 1
         return p[:, :H * D]
 
@@ -1041,41 +1066,41 @@ class CudaOps:
         elif (num_tiles and tc_ext and self.fast_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
                 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0):
             _check(self.lib.mi_attn_prefill_mma_capped(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),
-                _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, meta.page_size, meta.tile,
-                _c.c_float(scale), win, _c.c_float(cap), keep, _p(gate), gate_stride, self._stream()), "attn_prefill_mma_capped")
+                q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, num_tiles, meta.seg_q_start,
+                meta.seg_pos0, meta.block_table, rows, meta.max_pages, H, KV, D, meta.page_size, meta.tile,
+                scale, win, cap, keep, gate, gate_stride, self._stream()), "attn_prefill_mma_capped")
             self.launches += 1
         elif (num_tiles and plain and not extended and self.fast_attention and q.dtype == torch.bfloat16 and D == V and D in (64, 128) and meta.tile == 64
                 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0):
             # key and value rows of 64 or 128 entries: the mma.sync prompt kernel, every softmax weight entering P V as two
             # bfloat16 numbers (float32 scores and softmax, 16 mantissa bits of each weight, float32 sums)
             _check(self.lib.mi_attn_prefill_mma_masked(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),
-                _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, meta.page_size, meta.tile,
-                _c.c_float(scale), win, blk, int(bool(sink)), self._stream()), "attn_prefill_mma_masked")
+                q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, num_tiles, meta.seg_q_start,
+                meta.seg_pos0, meta.block_table, rows, meta.max_pages, H, KV, D, meta.page_size, meta.tile,
+                scale, win, blk, int(bool(sink)), self._stream()), "attn_prefill_mma_masked")
             self.launches += 1
         elif (num_tiles and not extended and self.fast_attention and self.biased_attention_tc and q.dtype == torch.bfloat16 and D == V and D in (64, 128)
                 and meta.tile == 64 and q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0):
             # the same kernel with the learned sink's score and the distance table (one row per head) in its softmax
             no_table = distance_bias is None and distance_bias_by_head is None        # slopes or a learned sink alone: the kernel reads no table
             bias_t = None if no_table else self._bias_rows_by_head(distance_bias, distance_bias_by_head)
-            args = (_p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),
-                    _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, meta.page_size, meta.tile,
-                    _c.c_float(scale), win, blk, int(bool(sink)), _p(sink_values), _p(bias_t), 0 if no_table else bias_t.shape[1] - 1)
+            args = (q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, num_tiles, meta.seg_q_start,
+                    meta.seg_pos0, meta.block_table, rows, meta.max_pages, H, KV, D, meta.page_size, meta.tile,
+                    scale, win, blk, int(bool(sink)), sink_values, bias_t, 0 if no_table else bias_t.shape[1] - 1)
             if slopes is None:
                 _check(self.lib.mi_attn_prefill_mma_biased(*args, self._stream()), "attn_prefill_mma_biased")
             else:                                          # a slope per head times the distance, beside (or instead of) the table
-                _check(self.lib.mi_attn_prefill_mma_sloped(*args, _p(slopes), self._stream()), "attn_prefill_mma_sloped")
+                _check(self.lib.mi_attn_prefill_mma_sloped(*args, slopes, self._stream()), "attn_prefill_mma_sloped")
             self.launches += 1
         elif num_tiles and self._f32_tiles(q, D, V, meta, k_cache, v_cache):
             self._prefill_f32(q, k_cache, v_cache, out, meta, H, KV, D, scale, blk, win, int(bool(sink)), sink_values, distance_bias, bias_last,
                               slopes, cap, keep, gate, gate_stride)
         elif num_tiles:
             _check(self.lib.mi_masked_prefill(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(meta.prefill_tiles), num_tiles, _p(meta.seg_q_start),
-                _p(meta.seg_pos0), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, V, meta.page_size, meta.tile,
-                _c.c_float(scale), blk, win, int(bool(sink)), _p(sink_values), _p(distance_bias), bias_last, _p(slopes), _c.c_float(cap), keep,
-                _p(gate), gate_stride, code, self._stream()), "masked_prefill")
+                q, q.stride(0), k_cache, v_cache, out, meta.prefill_tiles, num_tiles, meta.seg_q_start,
+                meta.seg_pos0, meta.block_table, rows, meta.max_pages, H, KV, D, V, meta.page_size, meta.tile,
+                scale, blk, win, int(bool(sink)), sink_values, distance_bias, bias_last, slopes, cap, keep,
+                gate, gate_stride, code, self._stream()), "masked_prefill")
             self.launches += 1
         if not num_decode:
             return out
@@ -1094,27 +1119,27 @@ class CudaOps:
                         raise ValueError(f"attn_decode: {num_decode} rows x {KV} kv heads exceed the {self._merge_counters.numel()} "
                                          "merge counters allocated at start-up")
                     counters = self._merge_counters
-            args = (_p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(o_part), _p(lse), _p(meta.decode_segs), num_decode,
-                    _p(meta.seg_q_start), _p(meta.seg_kv_len), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, meta.page_size, S,
-                    _c.c_float(scale), win, _p(counters), _p(self._stream_error if self.bulk_decode else None), k_cache.shape[0],
+            args = (q, q.stride(0), k_cache, v_cache, out, o_part, lse, meta.decode_segs, num_decode,
+                    meta.seg_q_start, meta.seg_kv_len, meta.block_table, rows, meta.max_pages, H, KV, D, meta.page_size, S,
+                    scale, win, counters, (self._stream_error if self.bulk_decode else None), k_cache.shape[0],
                     int(self.cluster_merge and counters is not None), blk, int(bool(sink)))
             if extended:                                   # args without its last two (blocks, sink)
-                _check(self.lib.mi_attn_decode_mma_rows_capped(*args[:-2], _c.c_float(cap), keep, _p(gate), gate_stride, self._stream()),
+                _check(self.lib.mi_attn_decode_mma_rows_capped(*args[:-2], cap, keep, gate, gate_stride, self._stream()),
                        "attn_decode_mma_capped")
             elif plain:
                 _check(self.lib.mi_attn_decode_mma_rows_masked(*args, self._stream()), "attn_decode_mma_masked")
             else:                                          # the learned sink's score and the distance table (one row per head) in the softmax
                 no_table = distance_bias is None and distance_bias_by_head is None             # slopes or a learned sink alone: the kernel reads no table
                 bias_t = None if no_table else self._bias_rows_by_head(distance_bias, distance_bias_by_head)
-                args += (_p(sink_values), _p(bias_t), 0 if no_table else bias_t.shape[1] - 1)
+                args += (sink_values, bias_t, 0 if no_table else bias_t.shape[1] - 1)
                 if slopes is None:
                     _check(self.lib.mi_attn_decode_mma_rows_biased(*args, self._stream()), "attn_decode_mma_biased")
                 else:
-                    _check(self.lib.mi_attn_decode_mma_rows_sloped(*args, _p(slopes), self._stream()), "attn_decode_mma_sloped")
+                    _check(self.lib.mi_attn_decode_mma_rows_sloped(*args, slopes, self._stream()), "attn_decode_mma_sloped")
             self.launches += 1
             if S > 1 and counters is None:
-                _check(self.lib.mi_attn_decode_merge(_p(o_part), _p(lse), _p(out), _p(meta.decode_segs), num_decode,
-                                                     _p(meta.seg_q_start), H, D, S, code, self._stream()), "attn_merge")
+                _check(self.lib.mi_attn_decode_merge(o_part, lse, out, meta.decode_segs, num_decode,
+                                                     meta.seg_q_start, H, D, S, code, self._stream()), "attn_merge")
                 self.launches += 1
             return out
         if num_decode:
@@ -1124,10 +1149,10 @@ class CudaOps:
                 o_part = torch.empty((num_decode, H, S, V), dtype=torch.float32, device=q.device)
                 lse = torch.empty((num_decode, H, S), dtype=torch.float32, device=q.device)
             _check(self.lib.mi_masked_decode(
-                _p(q), q.stride(0), _p(k_cache), _p(v_cache), _p(out), _p(o_part), _p(lse), _p(meta.decode_segs), num_decode,
-                _p(meta.seg_q_start), _p(meta.seg_kv_len), _p(meta.block_table), _p(rows), meta.max_pages, H, KV, D, V,
-                meta.page_size, S, _c.c_float(scale), blk, win, int(bool(sink)), _p(sink_values), _p(distance_bias), bias_last, _p(slopes),
-                _c.c_float(cap), keep, _p(gate), gate_stride, code, self._stream()), "masked_decode")
+                q, q.stride(0), k_cache, v_cache, out, o_part, lse, meta.decode_segs, num_decode,
+                meta.seg_q_start, meta.seg_kv_len, meta.block_table, rows, meta.max_pages, H, KV, D, V,
+                meta.page_size, S, scale, blk, win, int(bool(sink)), sink_values, distance_bias, bias_last, slopes,
+                cap, keep, gate, gate_stride, code, self._stream()), "masked_decode")
             self.launches += 2 if S > 1 else 1
         return out
 
@@ -1149,22 +1174,22 @@ class CudaOps:
         out = torch.empty((T, H * V), dtype=torch.float32, device=p.device)
         prep = torch.empty((T, 2 * H * D + H * V), dtype=torch.float32, device=p.device)
         half = 0 if inv_freq is None else inv_freq.numel()
-        _check(self.lib.mi_retention_rows(_p(p), p.stride(0), _p(prep), _p(batch.positions), _p(inv_freq), half, _c.c_float(k_scale), T, H, D, V,
+        _check(self.lib.mi_retention_rows(p, p.stride(0), prep, batch.positions, inv_freq, half, k_scale, T, H, D, V,
                                           _code(p.dtype), self._stream()), "retention_rows")
         if p.dtype == torch.bfloat16 and self._takes_octets(prep, batch, D, V, state):
             if self._takes_chunks(batch, T, D, V):
-                _check(self.lib.mi_constant_chunks(_p(prep), _p(self._chunk_scratch(T, batch, H, D, V)), _p(decay), _p(state), _c.c_longlong(state.stride(0)),
-                                                   _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error),
+                _check(self.lib.mi_constant_chunks(prep, self._chunk_scratch(T, batch, H, D, V), decay, state, state.stride(0),
+                                                   out, batch.seg_q_start, batch.seg_slot, T, batch.num_segs, H, D, V, self._stream_error,
                                                    self._stream()), "constant_chunks")
                 self.launches += 4
                 return out
             scratch = self._octet_scratch(T, batch, H, D, V, False)
-            _check(self.lib.mi_constant_octets(_p(prep), _p(scratch), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                               _p(batch.seg_slot), T, batch.num_segs, H, D, V, _p(self._stream_error), self._stream()), "constant_octets")
+            _check(self.lib.mi_constant_octets(prep, scratch, decay, state, state.stride(0), out, batch.seg_q_start,
+                                               batch.seg_slot, T, batch.num_segs, H, D, V, self._stream_error, self._stream()), "constant_octets")
             self.launches += 3
             return out
-        _check(self.lib.mi_retention_scan(_p(prep), _p(decay), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                          _p(batch.seg_slot), T, batch.num_segs, H, D, V, self._stream()), "retention_scan")
+        _check(self.lib.mi_retention_scan(prep, decay, state, state.stride(0), out, batch.seg_q_start,
+                                          batch.seg_slot, T, batch.num_segs, H, D, V, self._stream()), "retention_scan")
         self.launches += 2
         return out
 
@@ -1183,9 +1208,9 @@ class CudaOps:
         weights = torch.empty((T, top), dtype=torch.float32, device=h.device)
         extra = torch.empty((T, extra_rows), dtype=torch.float32, device=h.device) if extra_rows else None
         count, keep = groups if groups else (0, 0)
-        _check(self.lib.mi_route_topk(_p(h), h.stride(0), _p(router), _p(correction), _p(chosen), _p(weights), T, h.shape[1], E, top,
-                                      count, keep, int(score == "sigmoid"), extra_rows, _p(extra), int(group_score == "top2_sum"),
-                                      int(bool(renormalise)), _c.c_float(weight_eps), _c.c_float(route_scale), _code(h.dtype), self._stream()),
+        _check(self.lib.mi_route_topk(h, h.stride(0), router, correction, chosen, weights, T, h.shape[1], E, top,
+                                      count, keep, int(score == "sigmoid"), extra_rows, extra, int(group_score == "top2_sum"),
+                                      int(bool(renormalise)), weight_eps, route_scale, _code(h.dtype), self._stream()),
                "route_topk")
         self.launches += 1
         return (chosen, weights) if score is None else (chosen, weights, extra)
@@ -1195,7 +1220,7 @@ class CudaOps:
         rows, inter = gu.shape[0], gu.shape[1] // 2
         assert gu.is_contiguous()
         out = torch.empty((rows, inter), dtype=gu.dtype, device=gu.device)
-        _check(self.lib.mi_clamped_glu(_p(gu), _p(out), rows, inter, _c.c_float(limit), _c.c_float(slope), _c.c_float(1.0), _code(gu.dtype),
+        _check(self.lib.mi_clamped_glu(gu, out, rows, inter, limit, slope, 1.0, _code(gu.dtype),
                                        self._stream()), "clamped_glu")
         self.launches += 1
         return out
@@ -1207,7 +1232,7 @@ class CudaOps:
         nothing returns to the host.  weight_on_input: sum_j expert(weights[t, j] * h[t]) instead (the rows are scaled where they
         are gathered, the sum is unweighted).  shared_gate float32 [T, 1]: shared[t] is multiplied by sigmoid of it."""
         T, top = chosen.shape
-        sh = _c.c_float(up_shift)
+        sh = up_shift
         sum_weights = None if weight_on_input else weights
         sg = None if shared_gate is None else shared_gate.reshape(-1)
         assert sg is None or (sg.dtype == torch.float32 and sg.is_contiguous() and sg.numel() == T and shared is not None)
@@ -1222,24 +1247,24 @@ class CudaOps:
             cap_pos = cap_tiles * 128
             sorted_pair = torch.empty(cap_pos, dtype=torch.int32, device=dev)
             tile_expert = torch.empty(cap_tiles, dtype=torch.int32, device=dev)
-            _check(self.lib.mi_moe_align(_p(chosen), P, E, 128, _p(sorted_pair), cap_pos, _p(tile_expert), cap_tiles, self._stream()), "moe_align")
+            _check(self.lib.mi_moe_align(chosen, P, E, 128, sorted_pair, cap_pos, tile_expert, cap_tiles, self._stream()), "moe_align")
             a = torch.empty((cap_pos, K), dtype=h.dtype, device=dev)
-            _check(self.lib.mi_moe_gather_rows(_p(h), h.stride(0), _p(sorted_pair), top, _p(a), cap_pos, K, _p(weights if weight_on_input else None), self._stream()), "moe_gather_rows")
+            _check(self.lib.mi_moe_gather_rows(h, h.stride(0), sorted_pair, top, a, cap_pos, K, (weights if weight_on_input else None), self._stream()), "moe_gather_rows")
             y = torch.empty((cap_pos, F), dtype=h.dtype, device=dev)
             rows = torch.empty((P, hidden), dtype=h.dtype, device=dev)
-            _check(self.lib.mi_moe_gemm_tcgen05(_p(a), _p(w_in), E, _p(y), F, _p(sorted_pair), _p(tile_expert), cap_tiles, F, K,
-                                                _c.c_float(limit), _c.c_float(slope), sh, 0, _p(self._stream_error), self._stream()), "moe_gemm_tcgen05 (in)")
-            _check(self.lib.mi_moe_gemm_tcgen05(_p(y), _p(w_out), E, _p(rows), hidden, _p(sorted_pair), _p(tile_expert), cap_tiles, hidden, F,
-                                                _c.c_float(limit), _c.c_float(slope), sh, 1, _p(self._stream_error), self._stream()), "moe_gemm_tcgen05 (out)")
+            _check(self.lib.mi_moe_gemm_tcgen05(a, w_in, E, y, F, sorted_pair, tile_expert, cap_tiles, F, K,
+                                                limit, slope, sh, 0, self._stream_error, self._stream()), "moe_gemm_tcgen05 (in)")
+            _check(self.lib.mi_moe_gemm_tcgen05(y, w_out, E, rows, hidden, sorted_pair, tile_expert, cap_tiles, hidden, F,
+                                                limit, slope, sh, 1, self._stream_error, self._stream()), "moe_gemm_tcgen05 (out)")
             out = torch.empty((T, hidden), dtype=h.dtype, device=dev)
             assert shared is None or (shared.is_contiguous() and shared.shape == out.shape)
-            _check(self.lib.mi_moe_combine(_p(rows), _p(sum_weights), _p(shared), _p(sg), _p(out), T, hidden, top, code, self._stream()), "moe_combine")
+            _check(self.lib.mi_moe_combine(rows, sum_weights, shared, sg, out, T, hidden, top, code, self._stream()), "moe_combine")
             self.launches += 5
             return out
         src, src_top = h, top
         if weight_on_input:                                # row p = weights[p] * h[p // top]; the products then see one choice per row
             src = torch.empty((P, K), dtype=h.dtype, device=dev)
-            _check(self.lib.mi_moe_scale_rows(_p(h), h.stride(0), _p(weights), top, _p(src), P, K, code, self._stream()), "moe_scale_rows")
+            _check(self.lib.mi_moe_scale_rows(h, h.stride(0), weights, top, src, P, K, code, self._stream()), "moe_scale_rows")
             src_top = 1
             self.launches += 1
         tc = h.dtype == torch.bfloat16 and self.moe_tc and K % 64 == 0 and F % 64 == 0 and hidden % 2 == 0 and src.stride(0) % 8 == 0
@@ -1248,18 +1273,18 @@ class CudaOps:
         cap_pos = cap_tiles * BM
         sorted_pair = torch.empty(cap_pos, dtype=torch.int32, device=dev)
         tile_expert = torch.empty(cap_tiles, dtype=torch.int32, device=dev)
-        _check(self.lib.mi_moe_align(_p(chosen), P, E, BM, _p(sorted_pair), cap_pos, _p(tile_expert), cap_tiles, self._stream()), "moe_align")
+        _check(self.lib.mi_moe_align(chosen, P, E, BM, sorted_pair, cap_pos, tile_expert, cap_tiles, self._stream()), "moe_align")
         y = torch.empty((cap_pos, F), dtype=h.dtype, device=dev)
         rows = torch.empty((P, hidden), dtype=h.dtype, device=dev)
         gemm = self.lib.mi_moe_gemm_tc if tc else self.lib.mi_moe_gemm_simt
         extra = (BM,) if tc else ()
-        _check(gemm(_p(src), src.stride(0), _p(w_in), _p(y), F, _p(sorted_pair), _p(tile_expert), cap_tiles, src_top, F, K,
-                    _c.c_float(limit), _c.c_float(slope), sh, 0, *extra, code, self._stream()), "moe_gemm (in)")
-        _check(gemm(_p(y), F, _p(w_out), _p(rows), hidden, _p(sorted_pair), _p(tile_expert), cap_tiles, src_top, hidden, F,
-                    _c.c_float(limit), _c.c_float(slope), sh, 1, *extra, code, self._stream()), "moe_gemm (out)")
+        _check(gemm(src, src.stride(0), w_in, y, F, sorted_pair, tile_expert, cap_tiles, src_top, F, K,
+                    limit, slope, sh, 0, *extra, code, self._stream()), "moe_gemm (in)")
+        _check(gemm(y, F, w_out, rows, hidden, sorted_pair, tile_expert, cap_tiles, src_top, hidden, F,
+                    limit, slope, sh, 1, *extra, code, self._stream()), "moe_gemm (out)")
         out = torch.empty((T, hidden), dtype=h.dtype, device=dev)
         assert shared is None or (shared.is_contiguous() and shared.shape == out.shape)
-        _check(self.lib.mi_moe_combine(_p(rows), _p(sum_weights), _p(shared), _p(sg), _p(out), T, hidden, top, code, self._stream()), "moe_combine")
+        _check(self.lib.mi_moe_combine(rows, sum_weights, shared, sg, out, T, hidden, top, code, self._stream()), "moe_combine")
         self.launches += 4
         return out
 
@@ -1271,9 +1296,9 @@ class CudaOps:
         T, hidden = ids.shape[0], table.shape[1]
         assert state.dtype == torch.int32 and state.is_contiguous() and pairs.dtype == table.dtype and pairs.shape == (buckets + 1, hidden)
         x = torch.empty((T, hidden), dtype=torch.float32, device=table.device)
-        _check(self.lib.mi_embed_pair_stream(_p(ids), _p(table), _p(pairs), _p(x), _p(state), _c.c_longlong(state.stride(0)), _p(batch.positions),
-                                             _p(batch.token_seg), _p(batch.seg_q_start), _p(batch.seg_slot), T, hidden, table.shape[0],
-                                             _c.c_longlong(buckets), _c.c_longlong(mul_prev), _c.c_longlong(mul_cur), _code(table.dtype),
+        _check(self.lib.mi_embed_pair_stream(ids, table, pairs, x, state, state.stride(0), batch.positions,
+                                             batch.token_seg, batch.seg_q_start, batch.seg_slot, T, hidden, table.shape[0],
+                                             buckets, mul_prev, mul_cur, _code(table.dtype),
                                              self._stream()), "embed_bigram_stream")
         self.launches += 1
         return x
@@ -1287,8 +1312,8 @@ class CudaOps:
         assert state is None or (state.dtype == torch.float32 and state.is_contiguous())
         assert taps == 1 or state is not None
         out = torch.empty((T, C), dtype=h.dtype, device=h.device)
-        _check(self.lib.mi_short_conv(_p(h), h.stride(0), _p(weight), _p(bias), _p(state), _c.c_longlong(state.stride(0) if state is not None else 0),
-                                      _c.c_longlong(offset), _p(out), _p(batch.token_seg), _p(batch.seg_q_start), _p(batch.seg_slot), T,
+        _check(self.lib.mi_short_conv(h, h.stride(0), weight, bias, state, (state.stride(0) if state is not None else 0),
+                                      offset, out, batch.token_seg, batch.seg_q_start, batch.seg_slot, T,
                                       batch.num_segs, C, taps, int(residual), {"none": 0, "silu": 1}[act], _code(h.dtype), self._stream()),
                "short_conv")
         self.launches += 2 if taps > 1 else 1
@@ -1298,7 +1323,7 @@ class CudaOps:
         """z + bias (float32 [cols]), then act: "none" or "relu2" (the square of relu)."""
         assert z.is_contiguous() and bias.dtype == torch.float32 and bias.numel() == z.shape[-1]
         out = torch.empty_like(z)
-        _check(self.lib.mi_bias_act(_p(z), _p(bias), _p(out), _c.c_longlong(z.numel() // z.shape[-1]), z.shape[-1], {"none": 0, "relu2": 1}[act],
+        _check(self.lib.mi_bias_act(z, bias, out, (z.numel() // z.shape[-1]), z.shape[-1], {"none": 0, "relu2": 1}[act],
                                     _code(z.dtype), self._stream()), "bias_act")
         self.launches += 1
         return out
@@ -1308,7 +1333,7 @@ class CudaOps:
         T, hidden = ids.shape[0], table.shape[1]
         assert table.is_contiguous() and (pos_table is None or (pos_table.is_contiguous() and pos_table.dtype == table.dtype and pos_table.shape[1] == hidden))
         x = torch.empty((T, hidden), dtype=torch.float32, device=table.device)
-        _check(self.lib.mi_embed_scaled_stream(_p(ids), _p(table), _c.c_float(scale), _p(pos_table), _p(positions), _p(x), T, hidden, table.shape[0],
+        _check(self.lib.mi_embed_scaled_stream(ids, table, scale, pos_table, positions, x, T, hidden, table.shape[0],
                                                0 if pos_table is None else pos_table.shape[0], _code(table.dtype), self._stream()), "embed_scaled_stream")
         self.launches += 1
         return x
@@ -1330,8 +1355,8 @@ class CudaOps:
             assert pre_add.dtype == torch.float32 and pre_add.is_contiguous() and pre_add.numel() in (hidden, x.numel())
             stride = hidden if pre_add.dim() == 2 else 0
         first = a if a is not None else b
-        _check(self.lib.mi_stream_rmsnorm_pair(_p(x), _p(a), _p(b), _p(bias), _p(pre_add), _c.c_longlong(stride), _p(weight), _p(y), _p(rows), n, hidden,
-                                               _c.c_float(eps), _code(first.dtype if first is not None else out_dtype), _code(out_dtype), self._stream()),
+        _check(self.lib.mi_stream_rmsnorm_pair(x, a, b, bias, pre_add, stride, weight, y, rows, n, hidden,
+                                               eps, _code(first.dtype if first is not None else out_dtype), _code(out_dtype), self._stream()),
                "stream_rmsnorm_pair")
         self.launches += 1
         return y
@@ -1340,7 +1365,7 @@ class CudaOps:
         """y = weight * x / rms(x) over the rows of x [T, n] (a strided view is allowed); y contiguous, in x's dtype; float32 statistics."""
         assert x.stride(1) == 1 and weight.dtype == torch.float32 and weight.numel() == x.shape[1]
         y = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-        _check(self.lib.mi_rows_rmsnorm(_p(x), _c.c_longlong(x.stride(0)), _p(weight), _p(y), x.shape[0], x.shape[1], _c.c_float(eps), _code(x.dtype),
+        _check(self.lib.mi_rows_rmsnorm(x, x.stride(0), weight, y, x.shape[0], x.shape[1], eps, _code(x.dtype),
                                         self._stream()), "rows_rmsnorm")
         self.launches += 1
         return y
@@ -1350,7 +1375,7 @@ class CudaOps:
         rows, inter = gu.shape[0], gu.shape[1] // 2
         assert gu.is_contiguous() and (bias is None or (bias.dtype == torch.float32 and bias.numel() == 2 * inter))
         out = torch.empty((rows, inter), dtype=gu.dtype, device=gu.device)
-        _check(self.lib.mi_bias_glu(_p(gu), _p(bias), _p(out), rows, inter, self.GATES[act], _code(gu.dtype),
+        _check(self.lib.mi_bias_glu(gu, bias, out, rows, inter, self.GATES[act], _code(gu.dtype),
                                     self._stream()), "bias_glu")
         self.launches += 1
         return out
@@ -1358,14 +1383,14 @@ class CudaOps:
     def scale_logits(self, logits, s):
         """logits <- logits * s, in place (float32)."""
         assert logits.dtype == torch.float32 and logits.is_contiguous()
-        _check(self.lib.mi_scale_f32(_p(logits), _c.c_longlong(logits.numel()), _c.c_float(s), self._stream()), "scale_logits")
+        _check(self.lib.mi_scale_f32(logits, logits.numel(), s, self._stream()), "scale_logits")
         self.launches += 1
         return logits
 
     def softcap(self, logits, cap):
         """logits <- cap * tanh(logits / cap), in place (float32)."""
         assert logits.dtype == torch.float32 and logits.is_contiguous()
-        _check(self.lib.mi_softcap(_p(logits), _c.c_longlong(logits.numel()), _c.c_float(cap), self._stream()), "softcap")
+        _check(self.lib.mi_softcap(logits, logits.numel(), cap, self._stream()), "softcap")
         self.launches += 1
         return logits
 
@@ -1373,8 +1398,8 @@ class CudaOps:
         """sa * wa * a / rms(a) + sb * wb * b / rms(b) over the rows of a and b (same shape and dtype), float32 statistics."""
         assert a.is_contiguous() and b.is_contiguous() and a.shape == b.shape and a.dtype == b.dtype
         out = torch.empty_like(a)
-        _check(self.lib.mi_dual_rmsnorm_mix(_p(a), _p(wa), _c.c_float(sa), _p(b), _p(wb), _c.c_float(sb), _p(out), a.shape[0], a.shape[1],
-                                            _c.c_float(eps), _code(a.dtype), self._stream()), "dual_rmsnorm_mix")
+        _check(self.lib.mi_dual_rmsnorm_mix(a, wa, sa, b, wb, sb, out, a.shape[0], a.shape[1],
+                                            eps, _code(a.dtype), self._stream()), "dual_rmsnorm_mix")
         self.launches += 1
         return out
 
@@ -1386,8 +1411,8 @@ class CudaOps:
         T = p.shape[0]
         assert p.stride(1) == 1 and w2.is_contiguous() and w2.dtype == p.dtype and w2.shape == (H * D, rank)
         out = torch.empty((T, (5 * H * D + H * V + 3) // 4 * 4), dtype=torch.float32, device=p.device)
-        _check(self.lib.mi_general_delta_prepare(_p(p), p.stride(0), _p(w2), _p(w0), _p(a_b), _p(out), out.stride(0), T, H, D, V, rank,
-                                                 _c.c_float(decay_scale), _c.c_float(unit_eps), _code(p.dtype), self._stream()),
+        _check(self.lib.mi_general_delta_prepare(p, p.stride(0), w2, w0, a_b, out, out.stride(0), T, H, D, V, rank,
+                                                 decay_scale, unit_eps, _code(p.dtype), self._stream()),
                "general_delta_prepare")
         self.launches += 1
         return out
@@ -1397,8 +1422,8 @@ class CudaOps:
         T = prep.shape[0]
         assert prep.dtype == torch.float32 and state.dtype == torch.float32 and state.is_contiguous()
         out = torch.empty((T, H * V), dtype=torch.float32, device=prep.device)
-        _check(self.lib.mi_general_delta_scan(_p(prep), prep.stride(0), _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start),
-                                              _p(batch.seg_slot), T, batch.num_segs, H, D, V, self._stream()), "general_delta_scan")
+        _check(self.lib.mi_general_delta_scan(prep, prep.stride(0), state, state.stride(0), out, batch.seg_q_start,
+                                              batch.seg_slot, T, batch.num_segs, H, D, V, self._stream()), "general_delta_scan")
         self.launches += 1
         return out
 
@@ -1416,9 +1441,9 @@ class CudaOps:
         prep = torch.empty((T, (2 * H * D + H * W + H + 3) // 4 * 4), dtype=torch.float32, device=dev)
         full = torch.empty((T, H * W), dtype=torch.float32, device=dev)
         y = torch.empty((T, H * V), dtype=out_dtype, device=dev)
-        _check(self.lib.mi_matrix_memory(_p(p), p.stride(0), _p(gl), _p(gate_bias), _c.c_float(cap or 0.0), int(cap is not None), _c.c_float(den_eps),
-                                         _p(norm), _p(gate), gate.stride(0), _c.c_float(eps), _p(lg), _p(mneg), _p(prep), prep.stride(0), _p(full),
-                                         _p(y), _p(state), _c.c_longlong(state.stride(0)), _p(batch.seg_q_start), _p(batch.seg_slot), T,
+        _check(self.lib.mi_matrix_memory(p, p.stride(0), gl, gate_bias, (cap or 0.0), int(cap is not None), den_eps,
+                                         norm, gate, gate.stride(0), eps, lg, mneg, prep, prep.stride(0), full,
+                                         y, state, state.stride(0), batch.seg_q_start, batch.seg_slot, T,
                                          batch.num_segs, H, D, V, _code(p.dtype), self._stream()), "matrix_memory")
         self.launches += 3 if T == batch.num_segs else 5
         return y
@@ -1446,13 +1471,13 @@ class CudaOps:
         out = torch.empty((T, I), dtype=out_dtype, device=x.device)
         if x.dtype == torch.bfloat16 and N in (8, 16, 32) and self._takes_prompt_scan(T, batch):
             _check(self.lib.mi_selective_prompt(
-                _p(x), _p(dt), _p(dt_b), _p(A), _p(B), B.stride(0), _p(C), C.stride(0), _p(Dv), _p(z), z.stride(0), _p(state),
-                _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, I, N,
+                x, dt, dt_b, A, B, B.stride(0), C, C.stride(0), Dv, z, z.stride(0), state,
+                state.stride(0), out, batch.seg_q_start, batch.seg_slot, batch.num_segs, I, N,
                 self._stream()), "selective_prompt")
             self.launches += 1
             return out
-        _check(self.lib.mi_selective_scan(_p(x), _p(dt), _p(dt_b), _p(A), _p(B), B.stride(0), _p(C), C.stride(0), _p(Dv), _p(z), z.stride(0),
-                                          _p(state), _c.c_longlong(state.stride(0)), _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), T,
+        _check(self.lib.mi_selective_scan(x, dt, dt_b, A, B, B.stride(0), C, C.stride(0), Dv, z, z.stride(0),
+                                          state, state.stride(0), out, batch.seg_q_start, batch.seg_slot, T,
                                           batch.num_segs, I, N, _code(x.dtype), self._stream()), "selective_scan")
         self.launches += 1
         return out
@@ -1462,7 +1487,7 @@ class CudaOps:
         """x (float32 stream, in place) <- weight * N(alpha * x + y), N(z) = z / rms(z).  Returns x's rows in rows_dtype (x itself when that is float32)."""
         assert x.dtype == torch.float32 and x.is_contiguous() and y.is_contiguous() and y.shape == x.shape and weight.dtype == torch.float32
         rows = None if rows_dtype == torch.float32 else torch.empty(x.shape, dtype=rows_dtype, device=x.device)
-        _check(self.lib.mi_sum_rmsnorm(_p(x), _p(y), _p(weight), _p(rows), x.shape[0], x.shape[1], _c.c_float(alpha), _c.c_float(eps), _code(y.dtype),
+        _check(self.lib.mi_sum_rmsnorm(x, y, weight, rows, x.shape[0], x.shape[1], alpha, eps, _code(y.dtype),
                                        self._stream()), "sum_rmsnorm")
         self.launches += 1
         return x if rows is None else rows
@@ -1479,10 +1504,10 @@ class CudaOps:
         assert taps == 1 or (state.dtype == torch.float32 and state.is_contiguous() and state.shape[1] == (taps - 1) * C)
         q = torch.empty((T, H * D), dtype=p.dtype, device=p.device)
         single = T == batch.num_segs
-        _check(self.lib.mi_conv_qkv_cache(_p(p), p.stride(0), _p(bias), _p(conv), taps, _p(q_norm), _p(k_norm if KV else None), _c.c_float(eps), _p(inv_freq),
-                                          0 if inv_freq is None else inv_freq.numel(), _p(state if taps > 1 else None),
-                                          _c.c_longlong(state.stride(0) if taps > 1 else 0), _p(q), _p(k_cache if KV else None), _p(v_cache if KV else None),
-                                          _p(batch.positions), _p(meta.slots), _p(batch.token_seg), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs,
+        _check(self.lib.mi_conv_qkv_cache(p, p.stride(0), bias, conv, taps, q_norm, (k_norm if KV else None), eps, inv_freq,
+                                          0 if inv_freq is None else inv_freq.numel(), (state if taps > 1 else None),
+                                          (state.stride(0) if taps > 1 else 0), q, (k_cache if KV else None), (v_cache if KV else None),
+                                          batch.positions, meta.slots, batch.token_seg, batch.seg_q_start, batch.seg_slot, T, batch.num_segs,
                                           H, KV, D, V, meta.page_size, _code(p.dtype), self._stream()), "conv_qkv_cache")
         self.launches += 1 if taps == 1 or single else 2
         return q
@@ -1495,20 +1520,20 @@ class CudaOps:
         C, off, dev = I + 2 * G * N, H * N * V, p.device
         assert p.stride(1) == 1 and p.shape[1] >= I + C + H and state.dtype == torch.float32 and state.is_contiguous() and state.shape[1] >= off + (taps - 1) * C
         rows = torch.empty((T, I), dtype=p.dtype, device=dev)
-        code, stride = _code(p.dtype), _c.c_longlong(state.stride(0))
+        code, stride = _code(p.dtype), state.stride(0)
         if T == batch.num_segs:                             # every entry brings one token
             y = torch.empty((T, I), dtype=torch.float32, device=dev)
-            _check(self.lib.mi_ssd_step(_p(p), p.stride(0), _p(conv), _p(conv_b), taps, _p(dt_bias), _p(A), _p(Dv), _p(state), stride, _p(y),
-                                        _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, H, V, N, G, code, self._stream()), "ssd_step")
-            _check(self.lib.mi_gated_part_norm(_p(y), _p(None), 0, _p(None), V, _p(p), p.stride(0), _p(norm), _p(rows), T, I, parts, _c.c_float(eps),
-                                               _p(state), stride, _c.c_longlong(off), _p(batch.seg_slot), C, taps, code, self._stream()), "gated_part_norm")
+            _check(self.lib.mi_ssd_step(p, p.stride(0), conv, conv_b, taps, dt_bias, A, Dv, state, stride, y,
+                                        batch.seg_q_start, batch.seg_slot, batch.num_segs, H, V, N, G, code, self._stream()), "ssd_step")
+            _check(self.lib.mi_gated_part_norm(y, None, 0, None, V, p, p.stride(0), norm, rows, T, I, parts, eps,
+                                               state, stride, off, batch.seg_slot, C, taps, code, self._stream()), "gated_part_norm")
             self.launches += 2
             return rows
         xbc = self.short_conv(p[:, I:I + C], conv, conv_b, taps, state, off, batch, act="silu")
         dt = p[:, I + C:I + C + H]
         y = self.state_space_scan(xbc, dt, dt_bias, A, H, V, N, G, state, batch)
-        _check(self.lib.mi_gated_part_norm(_p(y), _p(xbc), xbc.stride(0), _p(Dv), V, _p(p), p.stride(0), _p(norm), _p(rows), T, I, parts, _c.c_float(eps),
-                                           _p(None), _c.c_longlong(0), _c.c_longlong(0), _p(None), 0, 1, code, self._stream()), "gated_part_norm")
+        _check(self.lib.mi_gated_part_norm(y, xbc, xbc.stride(0), Dv, V, p, p.stride(0), norm, rows, T, I, parts, eps,
+                                           None, 0, 0, None, 0, 1, code, self._stream()), "gated_part_norm")
         self.launches += 1
         return rows
 
@@ -1519,18 +1544,18 @@ class CudaOps:
         T, I = xbc.shape[0], H * V
         assert xbc.is_contiguous() and dt.stride(1) == 1 and dt.dtype == xbc.dtype and state.dtype == torch.float32 and state.is_contiguous()
         y = torch.empty((T, I), dtype=torch.float32, device=xbc.device)
-        stride = _c.c_longlong(state.stride(0))
+        stride = state.stride(0)
         if xbc.dtype == torch.bfloat16 and self.chunked_scan:
-            rc = self.lib.mi_ssd_chunk(_p(xbc), xbc.stride(0), _p(dt), dt.stride(0), _p(dt_bias), _p(A), _p(state), stride, _p(y), _p(batch.seg_q_start),
-                                       _p(batch.seg_slot), T, batch.num_segs, H, V, N, G, self._stream())
+            rc = self.lib.mi_ssd_chunk(xbc, xbc.stride(0), dt, dt.stride(0), dt_bias, A, state, stride, y, batch.seg_q_start,
+                                       batch.seg_slot, T, batch.num_segs, H, V, N, G, self._stream())
             if rc == 0:
                 self.launches += 1
                 return y
             if rc != -2:
                 _check(rc, "ssd_chunk")
         prep = torch.empty((T, (2 * G * N + I + H + 3) // 4 * 4), dtype=torch.float32, device=xbc.device)
-        _check(self.lib.mi_state_space_scan(_p(xbc), xbc.stride(0), _p(dt), dt.stride(0), _p(dt_bias), _p(A), _p(prep), prep.stride(0), _p(state), stride,
-                                            _p(y), _p(batch.seg_q_start), _p(batch.seg_slot), T, batch.num_segs, H, V, N, G, _code(xbc.dtype), self._stream()),
+        _check(self.lib.mi_state_space_scan(xbc, xbc.stride(0), dt, dt.stride(0), dt_bias, A, prep, prep.stride(0), state, stride,
+                                            y, batch.seg_q_start, batch.seg_slot, T, batch.num_segs, H, V, N, G, _code(xbc.dtype), self._stream()),
                "state_space_scan")
         self.launches += 2
         return y
@@ -1550,7 +1575,7 @@ class CudaOps:
         if delta is not None:
             y, wy, eps_y = delta.y, delta.weight, delta.eps
             assert y.is_contiguous() and y.shape == x.shape and y.dtype == out_dtype and wy.dtype == torch.float32
-        _check(self.lib.mi_stream_layernorm(_p(x), _p(y), _p(wy), _c.c_float(eps_y), _p(pre_add), _p(weight), _p(out), _p(rows), n, hidden, _c.c_float(eps),
+        _check(self.lib.mi_stream_layernorm(x, y, wy, eps_y, pre_add, weight, out, rows, n, hidden, eps,
                                             int(weight is None), _code(out_dtype), _code(out_dtype), self._stream()), "stream_layernorm")
         self.launches += 1
         return out
@@ -1558,7 +1583,7 @@ class CudaOps:
     def sigmoid_gate(self, rows, gate):
         """rows [T, n] *= sigmoid(gate), in place; gate [T, n] may be a strided view."""
         assert rows.is_contiguous() and gate.shape == rows.shape and gate.stride(1) == 1 and gate.dtype == rows.dtype
-        _check(self.lib.mi_sigmoid_gate(_p(rows), _p(gate), gate.stride(0), rows.shape[0], rows.shape[1], _code(rows.dtype), self._stream()), "sigmoid_gate")
+        _check(self.lib.mi_sigmoid_gate(rows, gate, gate.stride(0), rows.shape[0], rows.shape[1], _code(rows.dtype), self._stream()), "sigmoid_gate")
         self.launches += 1
         return rows
 
@@ -1572,23 +1597,23 @@ class CudaOps:
         T, C, ring = p.shape[0], 2 * KV * D + H * V, H * D * V
         assert p.stride(1) == 1 and p.shape[1] >= C + H * V + 2 * H and conv.dtype == torch.float32 and conv.is_contiguous() and conv.shape == (C, taps)
         assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1] >= ring + (taps * C if taps > 1 else 0)
-        code, stride = _code(p.dtype), (_c.c_longlong(state.stride(0)), _c.c_longlong(ring))
+        code, stride = _code(p.dtype), (state.stride(0), ring)
         if T == batch.num_segs and self.fused_delta_step:   # every entry brings one token
             rows = torch.empty((T, H * V), dtype=p.dtype, device=p.device)
-            rc = self.lib.mi_gated_delta_step(_p(p), p.stride(0), _p(conv), taps, _p(rate), _p(dt_bias), _p(state), *stride, _p(norm), _p(rows), _p(batch.positions),
-                                              _p(batch.seg_q_start), _p(batch.seg_slot), T, H, KV, D, V, _c.c_float(unit_eps), _c.c_float(eps), _p(self._stream_error), code, self._stream())
+            rc = self.lib.mi_gated_delta_step(p, p.stride(0), conv, taps, rate, dt_bias, state, *stride, norm, rows, batch.positions,
+                                              batch.seg_q_start, batch.seg_slot, T, H, KV, D, V, unit_eps, eps, self._stream_error, code, self._stream())
             if rc == 0:
                 self.launches += 1
                 return rows
             if rc != -2:
                 _check(rc, "gated_delta_step")
         prep = torch.empty((T, (C + 3 * H + 3) // 4 * 4), dtype=torch.float32, device=p.device)
-        _check(self.lib.mi_gated_delta_ready(_p(p), p.stride(0), _p(conv), _p(rate), _p(dt_bias), _p(state), *stride, _p(prep), prep.stride(0), _p(batch.positions),
-                                             _p(batch.token_seg), _p(batch.seg_q_start), _p(batch.seg_slot), T, H, KV, D, V, taps, _c.c_float(unit_eps), code,
+        _check(self.lib.mi_gated_delta_ready(p, p.stride(0), conv, rate, dt_bias, state, *stride, prep, prep.stride(0), batch.positions,
+                                             batch.token_seg, batch.seg_q_start, batch.seg_slot, T, H, KV, D, V, taps, unit_eps, code,
                                              self._stream()), "gated_delta_ready")
         o = self.gated_delta_scan(prep, H, KV, D, V, state, batch, chunks if p.dtype == torch.bfloat16 else None)
         if taps > 1:
-            _check(self.lib.mi_gated_delta_ring(_p(p), p.stride(0), _p(state), *stride, _p(batch.positions), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs,
+            _check(self.lib.mi_gated_delta_ring(p, p.stride(0), state, *stride, batch.positions, batch.seg_q_start, batch.seg_slot, batch.num_segs,
                                                 C, taps, code, self._stream()), "gated_delta_ring")
         self.launches += 2 if taps > 1 else 1
         return self.group_rmsnorm_gate(o, norm, p[:, C:C + H * V], eps, H, V, p.dtype, act="silu")
@@ -1599,20 +1624,20 @@ class CudaOps:
         two an entry: in chunks on the tensor cores, every float32 operand as two bfloat16 numbers; otherwise token by token in float32."""
         T = prep.shape[0]
         out = torch.empty((T, H * V), dtype=torch.float32, device=prep.device)
-        stride = _c.c_longlong(state.stride(0))
+        stride = state.stride(0)
         per = int(self.lib.mi_delta_chunk_bytes(D, V)) if chunks is not None and self.chunked_scan and T > 4 * batch.num_segs else -2
         if per > 0:
             lists, first = chunks
             heads = max(1, min(H, self.delta_work_bytes // (lists.shape[0] * per)))
             work = torch.empty(lists.shape[0] * per * heads, dtype=torch.uint8, device=prep.device)
-            rc = self.lib.mi_gated_delta_chunks(_p(prep), prep.stride(0), _p(lists), lists.shape[0], _p(first), _p(work), _c.c_longlong(work.numel()), _p(state), stride,
-                                                _p(out), _p(batch.seg_q_start), _p(batch.seg_slot), batch.num_segs, H, KV, D, V, _p(self._stream_error), self._stream())
+            rc = self.lib.mi_gated_delta_chunks(prep, prep.stride(0), lists, lists.shape[0], first, work, work.numel(), state, stride,
+                                                out, batch.seg_q_start, batch.seg_slot, batch.num_segs, H, KV, D, V, self._stream_error, self._stream())
             if rc == 0:
                 self.launches += 2 * -(-H // heads)
                 return out
             if rc != -2:
                 _check(rc, "gated_delta_chunks")
-        _check(self.lib.mi_gated_delta_scan(_p(prep), prep.stride(0), _p(state), stride, _p(out), _p(batch.seg_q_start), _p(batch.seg_slot),
+        _check(self.lib.mi_gated_delta_scan(prep, prep.stride(0), state, stride, out, batch.seg_q_start, batch.seg_slot,
                                             T, batch.num_segs, H, KV, D, V, self._stream()), "gated_delta_scan")
         self.launches += 1
         return out
@@ -1628,13 +1653,13 @@ class CudaOps:
         R, V = logits.shape
         out = torch.empty((R,), dtype=torch.int32, device=logits.device)
         if V >= 16384 and R <= 4096:                     # several blocks per row
-            _check(self.lib.mi_sample_split(_p(logits), logits.stride(0), R, V, _p(temperatures), _p(seeds), _p(counters),
-                                            _p(out), _p(self._sample_slots), _p(self._sample_arrivals), self._stream()),
+            _check(self.lib.mi_sample_split(logits, logits.stride(0), R, V, temperatures, seeds, counters,
+                                            out, self._sample_slots, self._sample_arrivals, self._stream()),
                    "sample")
             self.launches += 1
             return out
-        _check(self.lib.mi_sample(_p(logits), logits.stride(0), R, V, _p(temperatures), _p(seeds), _p(counters),
-                                  _p(out), self._stream()), "sample")
+        _check(self.lib.mi_sample(logits, logits.stride(0), R, V, temperatures, seeds, counters,
+                                  out, self._stream()), "sample")
         self.launches += 1
         return out
 
