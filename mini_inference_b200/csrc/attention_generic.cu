@@ -4,9 +4,9 @@
 // the request's own positions (the same bits however a batch is cut or mixed); a decoded token's
 // keys are cut into `splits` pieces, which the caller chooses by the step's size.
 // Prompts with heads of 64 or 128 have kernels of their own (attention_prefill_tc.cu and
-// attention_prefill_mma.cu in bfloat16, attention_prefill_f32.cu in float32), decoded tokens in
-// bfloat16 attention_decode_mma.cu; this file decodes in float32, takes all other head sizes, and
-// is the reference point of the fast kernels' tests.
+// attention_prefill_mma.cu in bfloat16, attention_prefill_f32.cu in float32), and so have decoded
+// tokens (attention_decode_mma.cu, attention_decode_f32.cu); this file takes all other head sizes
+// and groups, and is the reference point of the fast kernels' tests.
 //
 // Reference (davidjoyme/mini-inference): prompt portions attend over the gathered context with
 // a causal (offset) mask, engine/core/model_runner.py:161-173; decoded tokens use the split-KV
@@ -15,7 +15,7 @@
 //
 // Cache layout: [pages, KV, page_size, D]; key j of a request lives at
 //   ((table[j / page_size] * KV + kv_head) * page_size + j % page_size) * D.
-#include "common.cuh"
+#include "attention_decode_f32.cuh"
 #include <math.h>
 
 using namespace mi;
@@ -197,10 +197,17 @@ MI_EXPORT int mi_attn_decode_generic(const void* q, int q_stride, const void* k_
     dim3 grid(num_decode, (H + WARPS - 1) / WARPS, splits);
 #define ARGS(T) (const T*)q, q_stride, (const T*)k_cache, (const T*)v_cache, (T*)out, o_part, lse_part, decode_segs, \
         seg_q_start, seg_kv_len, block_table, table_rows, table_stride, H, KV, D, ps, scale, window
-    if (dtype == MI_BF16) attn_decode_split_kernel<__nv_bfloat16><<<grid, WARPS * 32, 0, stream>>>(ARGS(__nv_bfloat16));
-    else attn_decode_split_kernel<float><<<grid, WARPS * 32, 0, stream>>>(ARGS(float));
+    const DecodeF32 f32{(const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out, o_part, lse_part, decode_segs, seg_q_start, seg_kv_len, block_table,
+                        table_rows, q_stride, num_decode, table_stride, H, KV, D, ps, splits, scale, 0, window, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, 0.f};
+    int err = 0;
+    if (dtype == MI_F32 && takes_decode_f32(f32)) {
+        err = decode_f32(f32, stream);
+    } else {
+        if (dtype == MI_BF16) attn_decode_split_kernel<__nv_bfloat16><<<grid, WARPS * 32, 0, stream>>>(ARGS(__nv_bfloat16));
+        else attn_decode_split_kernel<float><<<grid, WARPS * 32, 0, stream>>>(ARGS(float));
+        err = (int)cudaGetLastError();
+    }
 #undef ARGS
-    int err = (int)cudaGetLastError();
     if (err || splits == 1) return err;
     dim3 mgrid(num_decode, H);
     if (dtype == MI_BF16)

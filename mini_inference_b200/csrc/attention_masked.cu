@@ -24,7 +24,7 @@
 // 1 + coef * ln(floor((p + 1) / every) + 1) of its position p (every > 0); v blended with another layer's values of the same
 // token ((1 - lambda) v + lambda v_src), or, with v_is_k, taken from the keys AS PROJECTED (before the norm; there are no v
 // columns then); k and v written to the token's slot of the pages, q written back in place.
-#include "common.cuh"
+#include "attention_decode_f32.cuh"
 #include <math.h>
 
 using namespace mi;
@@ -462,10 +462,18 @@ MI_EXPORT int mi_masked_decode(const void* q, int q_stride, const void* k_cache,
     dim3 grid(num_decode, (H + WARPS - 1) / WARPS, splits);
 #define ARGS(T) (const T*)q, q_stride, (const T*)k_cache, (const T*)v_cache, (T*)out, o_part, lse_part, decode_segs, seg_q_start, seg_kv_len, \
         block_table, table_rows, table_stride, H, KV, D, Dv, ps, scale, block, window, sink, sink_values, bias, bias_last, slopes, cap, keep, (const T*)gate, gate_stride
-    if (dtype == MI_BF16) masked_decode_kernel<__nv_bfloat16><<<grid, WARPS * 32, 0, stream>>>(ARGS(__nv_bfloat16));
-    else masked_decode_kernel<float><<<grid, WARPS * 32, 0, stream>>>(ARGS(float));
+    const DecodeF32 f32{(const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out, o_part, lse_part, decode_segs, seg_q_start, seg_kv_len, block_table,
+                        table_rows, q_stride, num_decode, table_stride, H, KV, D, ps, splits, scale, block, window, sink, bias_last, keep, gate_stride, sink_values, bias,
+                        slopes, (const float*)gate, cap};
+    int err = 0;
+    if (dtype == MI_F32 && D == Dv && takes_decode_f32(f32)) {
+        err = decode_f32(f32, stream);
+    } else {
+        if (dtype == MI_BF16) masked_decode_kernel<__nv_bfloat16><<<grid, WARPS * 32, 0, stream>>>(ARGS(__nv_bfloat16));
+        else masked_decode_kernel<float><<<grid, WARPS * 32, 0, stream>>>(ARGS(float));
+        err = (int)cudaGetLastError();
+    }
 #undef ARGS
-    int err = (int)cudaGetLastError();
     if (err || splits == 1) return err;
     dim3 mgrid(num_decode, H);
     if (dtype == MI_BF16)

@@ -154,6 +154,35 @@ def test_float32_prompt_attention_reads_visible_keys_only(ops, D, page, form):  
         assert not got[sees].isfinite().any(), form
 
 
+@pytest.mark.parametrize("D,page", [(128, 16), (64, 24)])
+@pytest.mark.parametrize("group", [1, 2, 4, 8])
+@pytest.mark.parametrize("form", ["plain"] + FORMS)
+def test_float32_decoded_tokens(ops, form, group, D, page):     # noqa: F811
+    """Eight keys at a time over the warps of a block, one piece of the keys and several: against the general kernel (which takes rows that do not
+    start on 16 bytes), with pages that hold no numbers behind the last key."""
+    KV, lens = 2, (1, 7, 33, 256, 1000, 65)
+    H, T = KV * group, len(lens)
+    meta, g = make_meta(page, [(n - 1, 1) for n in lens], 110, group + D, indirect=True), torch.Generator().manual_seed(group)
+    q = torch.randn(T, H * D + 1, generator=g).to(DEV)
+    k, v = (torch.randn(111, KV, page, D, generator=g).to(DEV) for _ in range(2))
+    for i, n in enumerate(lens):
+        at = meta.block_table[meta.table_rows[i], (n - 1) // page].long()
+        k[at, :, (n - 1) % page + 1:], v[at, :, (n - 1) % page + 1:] = float("nan"), float("inf")
+    args = None if form == "plain" else form_arguments(form, H, D, T, torch.float32)
+
+    def call(q):
+        return ops.paged_attention(q, k, v, meta, H, KV, D, D ** -0.5, None) if args is None else ops.masked_attention(q, k, v, meta, H, KV, D, D, D ** -0.5, **args)
+
+    want = call(q[:, :H * D])
+    try:
+        for splits in (None, 1, 5):
+            ops.force_splits = splits
+            # float32 sums of up to 1,000 weights and 128 products in another order
+            assert rows_error(call(q[:, :H * D].contiguous()), want) < 2e-6, (form, splits)
+    finally:
+        ops.force_splits = None
+
+
 class Entries:
     """A step's entries as the recurrences see them."""
 
