@@ -160,6 +160,7 @@ class CudaOps:
         self.fast_attention = True           # tests clear this to run the generic attention kernels in bfloat16
         self.biased_attention_tc = True      # prompts of attention with a distance table or a learned sink on the tensor cores (bfloat16)
         self.delta_work_bytes = 160 << 20    # scratch of the delta rule's chunks: as many heads at a time as fit
+        self.channel_work_bytes = 640 << 20  # the same with a decay per key channel: 16 heads of 13,000 tokens
         self.fused_delta_step = True         # decode steps of the delta rule with one decay per head in one kernel (tests clear this)
         self.chunked_scan = True             # prompts of a state space or delta rule with one decay per head in chunks on the tensor cores (tests clear this)
         # Latent attention whose cached rows have 64 or 128 entries can run on the tensor-core paged attention kernels.  Those
@@ -783,6 +784,14 @@ class CudaOps:
         (16 prompts of 64 tokens 79 us there, 94 here; 192 tokens beside 40 decoded ones 92 and 256)."""
         return D == 128 and V % 128 == 0 and getattr(batch, "max_q_len", 0) >= 320 and T >= 100 * batch.num_segs
 
+    @staticmethod
+    def _takes_delta_chunks(batch, T, D, V):
+        """Whether a delta rule with channel decays that _takes_octets goes 32 tokens at a time on the tensor cores instead
+        (csrc/channel_chunks.cu): keys of 128, values in blocks of 16 columns, a prompt of at least 192 tokens (29 us here, 31 there) and 40
+        tokens an entry on average, since a short entry takes a whole chunk (500 tokens beside 10 decoded ones 77 us here, 97 there; 300 beside 10
+        68 and 64; 200 beside 40 171 and 98; without a long prompt 8 of 65 tokens 72 and 62, 16 of 64 105 and 107)."""
+        return D == 128 and V % 16 == 0 and getattr(batch, "max_q_len", 0) >= 192 and T >= 40 * batch.num_segs
+
     def _chunk_scratch(self, T, batch, H, D, V):
         """Per chunk and head what it adds to the state, then the state before it."""
         return torch.empty(self.lib.mi_chunk_floats(T, batch.num_segs, H, D, V), dtype=torch.float32, device=self.device)
@@ -847,6 +856,13 @@ class CudaOps:
             self.launches += 1
             return out
         if not exact and self._takes_octets(prep, batch, D, V, state):
+            if self._takes_delta_chunks(batch, T, D, V):
+                per_head = self.lib.mi_channel_chunk_bytes(T, batch.num_segs, V)
+                work = torch.empty(max(per_head, min(H * per_head, self.channel_work_bytes)), dtype=torch.uint8, device=self.device)
+                _check(self.lib.mi_channel_chunks(prep, prep.stride(0), work, work.numel(), state, state.stride(0), out, batch.seg_q_start,
+                                                  batch.seg_slot, T, batch.num_segs, H, KV, D, V, self._stream_error, self._stream()), "channel_chunks")
+                self.launches += 2 * -(-H // min(H, work.numel() // per_head))
+                return out
             scratch = self._octet_scratch(T, batch, H, D, V, True)
             _check(self.lib.mi_delta_octets(prep, prep.stride(0), scratch, state, state.stride(0), out, batch.seg_q_start,
                                             batch.seg_slot, T, batch.num_segs, H, KV, D, V, self._stream_error, self._stream()), "delta_octets")

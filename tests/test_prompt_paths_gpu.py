@@ -304,6 +304,74 @@ def test_chunks_keep_odd_numbers_in_their_place(ops, what):     # noqa: F811
         assert rows_error(torch.where(ok, got, 0.), torch.where(ok, plain, 0.)) < 3e-6, name
 
 
+def delta_inputs(lens, H, KV, V, seed):
+    T, D, g = sum(lens), 128, torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
+    batch, C = Entries(lens), 2 * KV * D + H * V
+    batch.max_q_len = max(lens)
+    prep = torch.zeros(T, (C + H * D + H + 3) // 4 * 4, device=DEV)
+    qk = r(T, 2 * KV, D)
+    prep[:, :2 * KV * D] = (qk / qk.norm(dim=-1, keepdim=True)).reshape(T, -1)
+    prep[:, 2 * KV * D:C] = r(T, H * V)
+    decay = torch.rand(T, H * D, generator=g).to(DEV) ** 0.2
+    decay[:, ::7], decay[:, 1::7] = 1.0, 0.0
+    prep[:, C:C + H * D] = decay
+    prep[:, C + H * D:C + H * D + H] = torch.rand(T, H, generator=g).to(DEV)
+    return batch, prep, r(len(lens) + 1, H * D * V + 6)
+
+
+@pytest.mark.parametrize("heads_at_once", [False, True])
+@pytest.mark.parametrize("lens,H,KV,V", [((192,), 16, 8, 128), ((193, 31), 3, 3, 16), ((1, 256, 33, 7), 4, 2, 144), ((223, 1, 64, 32, 1), 5, 1, 256)])
+def test_channel_decays_in_chunks(ops, monkeypatch, lens, H, KV, V, heads_at_once):     # noqa: F811
+    """32 tokens at a time against the token-by-token kernel: whole chunks, remainders, single tokens beside prompts, more than 128 columns, decays down
+    to 0, with scratch for all heads and for one at a time."""
+    batch, prep, state = delta_inputs(lens, H, KV, V, sum(lens))
+    if heads_at_once:
+        monkeypatch.setattr(ops, "channel_work_bytes", 0)
+    a, b = state.clone(), state.clone()
+    assert ops._takes_octets(prep, batch, 128, V, a) and ops._takes_delta_chunks(batch, sum(lens), 128, V)
+    got, want = ops.delta_scan(prep, H, KV, 128, V, a, batch), ops.delta_scan(prep, H, KV, 128, V, b, batch, exact=True)
+    ops.check_errors()
+    # two float32 orders of sums over up to 256 decayed tokens and 128 rows
+    assert rows_error(got, want) < 3e-6 and rows_error(a, b) < 3e-6
+    assert torch.equal(a[:, H * 128 * V:], state[:, H * 128 * V:]) and torch.equal(a[0], state[0])
+
+
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta", "state", "huge v", "tiny v"])
+def test_channel_chunks_keep_odd_numbers_in_their_place(ops, what):     # noqa: F811
+    """Numbers that three bfloat16 parts do not hold: the outputs are those of the token-by-token kernel, tokens before the number, other entries and
+    other heads have the bits they have without it."""
+    lens, H, V, at = (200, 192), 2, 32, 83                       # token 83: the 20th of the first entry's third chunk
+    batch, prep, state = delta_inputs(lens, H, H, V, 3)
+    C = 4 * 128 + 2 * V
+    spoiled, odd_state = prep.clone(), state.clone()
+    if what == "state":
+        odd_state[batch.seg_slot[0].item(), V * 30 + 4] = float("inf")
+    elif what == "huge v":
+        spoiled[at, 512 + 3] = 1e30
+    elif what == "tiny v":                                       # a head that holds nothing but numbers at the lower end
+        spoiled[:200, 512:512 + V] *= 1e-36
+        odd_state[batch.seg_slot[0].item(), :128 * V] *= 1e-36
+    else:
+        spoiled[at, {"q": 5, "k": 256 + 7, "v": 512 + 9, "decay": C + 11, "beta": C + 256}[what]] = float("nan") if what in ("k", "decay", "beta") else float("inf")
+    a, b, c = state.clone(), odd_state.clone(), odd_state.clone()
+    assert ops._takes_delta_chunks(batch, 392, 128, V)
+    want, got = ops.delta_scan(prep, H, H, 128, V, a, batch), ops.delta_scan(spoiled, H, H, 128, V, b, batch)
+    plain = ops.delta_scan(spoiled, H, H, 128, V, c, batch, exact=True)
+    first = 0 if what in ("state", "tiny v") else at
+    assert torch.equal(got[:first], want[:first]) and torch.equal(got[200:], want[200:]) and torch.equal(got[:, V:], want[:, V:])
+    assert torch.equal(got.isnan(), plain.isnan()) and torch.equal(got.isinf(), plain.isinf()) and torch.equal(b.isnan(), c.isnan())
+    ok = plain.isfinite()
+    if what == "huge v":                                         # what 1e30 has swallowed does not come back when it has decayed
+        ok[at:200] = False
+        assert rows_error(got[at:at + 8, :V], plain[at:at + 8, :V]) < 3e-6
+    scale = 1e36 if what == "tiny v" else 1.0
+    if what == "tiny v":
+        ok[:, V:] = False
+        ok[200:] = False
+    assert rows_error(torch.where(ok, got, 0.) * scale, torch.where(ok, plain, 0.) * scale) < 3e-6
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 def test_octets_keep_later_tokens_out(ops, value):              # noqa: F811
     """A value that is no number reaches its own token and the ones after it; the tokens before it in its octet give the bits they give without it."""
