@@ -520,7 +520,7 @@ class CudaOps:
         if code != 0:
             self._stream_error.zero_()
             self._tc2_counters.zero_()
-            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-63 grouped expert product, 71-72 delta rule)")
+            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-64 grouped expert product, 71-74 delta rule and constant decay in chunks, 81-82 channel decays in chunks)")
 
     # ---------------------------------------------------------------- q/k norm, rotation, cache write
     def qk_norm_rope_cache(self, qkv, H, KV, D, q_weight, k_weight, eps, inv_freq, meta, k_cache, v_cache):
@@ -1258,19 +1258,18 @@ class CudaOps:
         P, code, dev = T * top, _code(h.dtype), h.device
         if (h.dtype == torch.bfloat16 and self.moe_tcgen05 and P > 48 * E and K % 64 == 0 and F % 64 == 0 and hidden % 8 == 0
                 and h.stride(0) % 8 == 0 and h.data_ptr() % 16 == 0):
-            # many rows per expert: tiles of 128 sorted rows on the tcgen05 tensor cores (csrc/moe_grouped_tc.cu)
-            cap_tiles = (P + 127) // 128 + min(E, P)
-            cap_pos = cap_tiles * 128
+            # many rows per expert: tiles of up to 256 sorted rows on the tcgen05 tensor cores (csrc/moe_grouped_tc.cu)
+            cap_pos = self.lib.mi_moe_plan_rows(P, E)
             sorted_pair = torch.empty(cap_pos, dtype=torch.int32, device=dev)
-            tile_expert = torch.empty(cap_tiles, dtype=torch.int32, device=dev)
-            _check(self.lib.mi_moe_align(chosen, P, E, 128, sorted_pair, cap_pos, tile_expert, cap_tiles, self._stream()), "moe_align")
+            plan = torch.empty(self.lib.mi_moe_plan_ints(P, E), dtype=torch.int32, device=dev)
+            _check(self.lib.mi_moe_plan(chosen, P, E, sorted_pair, cap_pos, plan, self._stream()), "moe_plan")
             a = torch.empty((cap_pos, K), dtype=h.dtype, device=dev)
             _check(self.lib.mi_moe_gather_rows(h, h.stride(0), sorted_pair, top, a, cap_pos, K, (weights if weight_on_input else None), self._stream()), "moe_gather_rows")
             y = torch.empty((cap_pos, F), dtype=h.dtype, device=dev)
             rows = torch.empty((P, hidden), dtype=h.dtype, device=dev)
-            _check(self.lib.mi_moe_gemm_tcgen05(a, w_in, E, y, F, sorted_pair, tile_expert, cap_tiles, F, K,
+            _check(self.lib.mi_moe_gemm_tcgen05(a, w_in, E, y, F, sorted_pair, plan, cap_pos, F, K,
                                                 limit, slope, sh, 0, self._stream_error, self._stream()), "moe_gemm_tcgen05 (in)")
-            _check(self.lib.mi_moe_gemm_tcgen05(y, w_out, E, rows, hidden, sorted_pair, tile_expert, cap_tiles, hidden, F,
+            _check(self.lib.mi_moe_gemm_tcgen05(y, w_out, E, rows, hidden, sorted_pair, plan, cap_pos, hidden, F,
                                                 limit, slope, sh, 1, self._stream_error, self._stream()), "moe_gemm_tcgen05 (out)")
             out = torch.empty((T, hidden), dtype=h.dtype, device=dev)
             assert shared is None or (shared.is_contiguous() and shared.shape == out.shape)

@@ -707,3 +707,54 @@ def test_sampler_forms_agree(ops):                              # noqa: F811
     parts = [ops.sample(logits[a:a + 8], temps[a:a + 8].contiguous(), seeds[a:a + 8].contiguous(), counters[a:a + 8].contiguous()) for a in range(0, R, 8)]
     assert torch.equal(got, torch.cat(parts))
     assert torch.equal(got[::2].long(), logits[::2].argmax(-1))
+
+
+def expert_rows(ops, counts, seed):
+    """chosen [T, 1] with counts[e] tokens of expert e, in a random order."""
+    g = torch.Generator().manual_seed(seed)
+    chosen = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    return chosen[torch.randperm(len(chosen), generator=g)].to(torch.int32).to(DEV)[:, None].contiguous(), g
+
+
+@pytest.mark.parametrize("counts", [(1, 31, 0, 32, 33), (255, 256, 257, 0), (512, 513, 7), (0, 0, 700), (3, 16500, 0, 520, 4)])
+def test_plan_of_expert_tiles(ops, counts):                     # noqa: F811
+    """Every pair once, among its expert's rows; an expert's tiles cover its rows in steps of 32, at most 256 each."""
+    chosen, _ = expert_rows(ops, counts, sum(counts))
+    P, E = chosen.shape[0], len(counts)
+    cap = ops.lib.mi_moe_plan_rows(P, E)
+    pairs, plan = torch.full((cap,), -7, dtype=torch.int32, device=DEV), torch.zeros(ops.lib.mi_moe_plan_ints(P, E), dtype=torch.int32, device=DEV)
+    assert ops.lib.mi_moe_plan(chosen, P, E, pairs, cap, plan, ops._stream()) == 0
+    pairs, plan, chosen = pairs.cpu(), plan.cpu(), chosen.cpu()[:, 0]
+    tiles = plan[4:4 + 4 * plan[0].item()].view(-1, 4)
+    assert sorted(pairs[pairs >= 0].tolist()) == list(range(P)) and int(pairs.min()) >= -1
+    end = 0
+    for first, rows, e, _ in tiles.tolist():
+        assert first == end and rows % 32 == 0 and 0 < rows <= 256
+        end = first + rows
+        here = pairs[first:end]
+        assert (chosen[here[here >= 0].long()] == e).all()
+    assert end == sum(-(-n // 32) * 32 for n in counts) and (pairs[end:] == -1).all()
+    assert [sum(t[2] == e for t in tiles.tolist()) for e in range(E)] == [-(-n // 256) for n in counts]
+
+
+@pytest.mark.parametrize("counts,K,F,hidden", [((1, 31, 32, 33, 200), 64, 64, 8), ((255, 257, 0), 192, 192, 264), ((512, 513), 320, 128, 520), ((0, 60, 420, 96), 1088, 704, 1032)])
+def test_expert_products_in_pairs_of_blocks(ops, counts, K, F, hidden):     # noqa: F811
+    """The grouped products against float64, with the activated rows and the rows rounded to bfloat16 where the kernels round them: tiles of 32 to 256
+    rows, experts without rows, outputs and K that are no multiple of a tile's."""
+    chosen, g = expert_rows(ops, counts, K)
+    T, E = chosen.shape[0], len(counts)
+    r = lambda *s, std=1.0: (std * torch.randn(*s, generator=g)).to(torch.bfloat16).to(DEV)      # noqa: E731
+    h, w_in, w_out = r(T, K), r(E, 2 * F, K, std=K ** -0.5), r(E, hidden, F, std=F ** -0.5)
+    weights = torch.rand(T, 1, generator=g).to(DEV)
+    assert T > 48 * E and ops.moe_tcgen05
+    got = ops.expert_ffn(h, chosen, weights, w_in, w_out, 2.0, 1.7, None)
+    ops.check_errors()
+    want = torch.zeros(T, hidden, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        t = (chosen[:, 0] == e).nonzero()[:, 0]
+        x = h[t].double() @ w_in[e].double().T
+        gate, up = x[:, :F].clamp(max=2.0), x[:, F:].clamp(-2.0, 2.0)
+        y = (gate * torch.sigmoid(1.7 * gate) * (up + 1.0)).to(torch.bfloat16).double()
+        want[t] = (y @ w_out[e].double().T).to(torch.bfloat16).double() * weights[t].double()
+    # three roundings to bfloat16 (activated rows and rows on either side of a tie, the sum), each at most 2^-9 of a number
+    assert rows_error(got, want) < 3 * 2.0 ** -9
