@@ -13,11 +13,11 @@
 // mma.sync and not tcgen05: the walk is a chain, and what counts is how many SMs share it.  A tcgen05 product has 128 rows, all columns of a
 // head (16 blocks for one prompt), where 16 columns a block make 128.
 //
-// 16 heads of 128 x 128 on 8 key heads, microseconds by state_octets.cu / here: 2,048 tokens 238 / 162, 1,300 + 517 + 231 249 / 161, 4 x 512 202 / 168,
-// 400 54 / 44, 192 31 / 29.  Of the 162 the first kernel takes 52 (a third of the issue slots: forward substitution and the products between
-// eights), the second 110: 2,600 clocks a chunk, 156 products a warp of 8.5 each (the rate of one scheduler) and half as much again waiting
-// between the operands' cutting, the products and the partial sums' way around.  Error against 64 bits (2-norm, 1,034 tokens): outputs 1.7e-7 there,
-// 1.5e-7 here, states 5.1e-8 and 4.0e-8.
+// 16 heads of 128 x 128 on 8 key heads, microseconds by state_octets.cu / here: 2,048 tokens 238 / 162, 1,300 + 517 + 231 249 / 160, 4 x 512 202 / 151,
+// 8 x 1,024 680 / 508, 16 x 64 105 / 85, 400 54 / 44, 192 31 / 29.  Of the 162 the first kernel takes 52 (a third of the issue slots: forward
+// substitution and the products between eights), the second 110: 2,600 clocks a chunk, 156 products a warp of 8.5 each (the rate of one
+// scheduler) and half as much again waiting between the operands' cutting, the products and the partial sums' way around.  Error against 64 bits
+// (2-norm, 1,034 tokens): outputs 1.7e-7 there, 1.5e-7 here, states 5.1e-8 and 4.0e-8.
 // Measured and left: outputs made by four more warps (as fast: they share the schedulers' product rate and the shared memory), operands cut
 // by the first kernel (6 bytes a number instead of 4: as fast, and half as much scratch again), 32 columns by eight warps (64 blocks for one prompt: 227).
 //
@@ -338,16 +338,27 @@ __global__ void __launch_bounds__(128, 4) chunk_kernel(const Rows L, unsigned ch
 }
 
 // ------------------------------------------------------------------ the walk over an entry's chunks
-constexpr int STAGES = 3, U_BYTES = VC * UPITCH * 4, STAGE = (U_OFF + U_BYTES + 127) / 128 * 128;
+constexpr int U_BYTES = VC * UPITCH * 4;
+// A chunk in shared memory, in pieces that are refilled when they have been read: W, the flag and U_0 | Q | K, B, the decays
+constexpr int P_AT = P_OFF - K_OFF, DEC_AT = DEC_OFF - K_OFF, K_BYTES = ODD_OFF - K_OFF;
+// DEEP: three whole chunks as they lie in memory (all pieces on the first one's barriers) and a block an SM.  Else two of the first piece and one of
+// the others, which a walk waits for a little (0.2 us a chunk), and two blocks an SM, which use each other's waits.
+template <bool DEEP> struct Ring {
+    static constexpr int W = DEEP ? 3 : 2, R = DEEP ? 3 : 1;            // chunks of the first piece, of the others
+    static constexpr int FLAG_AT = DEEP ? ODD_OFF : MATRIX, U_AT = FLAG_AT + 16, W_BYTES = MATRIX + 16 + U_BYTES;
+    static constexpr int W_STEP = (U_AT + U_BYTES + 127) / 128 * 128, R_STEP = DEEP ? W_STEP : 0;
+    static constexpr int Q_AT = DEEP ? Q_OFF : W * W_STEP, K_AT = Q_AT + MATRIX;
+    static constexpr int BYTES = DEEP ? W * W_STEP : (K_AT + K_BYTES + 127) / 128 * 128, BARS = W + 2 * R;
+};
 struct Exchange {
     float4 u_part[4][4][32];                                            // W S of a warp's rows: [warp][tile of 8 tokens][lane]; token by token: the state's columns
     float4 o_part[2][4][4][32];                                         // Q S, two chunks in turn
     float red[256];
     uint2 u[PARTS][4][32];                                              // the parts of U^T as a left operand: [part][tile][lane]
     int odd[2];
-    uint64_t bars[2 * STAGES];
+    uint64_t bars[2 * 9];
 };
-constexpr int PASS_SMEM = STAGES * STAGE + sizeof(Exchange);
+template <bool DEEP> constexpr int PASS_SMEM = Ring<DEEP>::BYTES + sizeof(Exchange);
 
 // The chunk's tokens one after the other for 16 columns, by 128 threads: a thread has 16 rows of a column, the state (before the chunk) in st [D][VC].
 __device__ __noinline__ void by_token(float* st, float* red, const Rows L, const float* first, int n, int from, int h, int kvh, int V, int v0, float* out, int H,
@@ -385,19 +396,21 @@ __device__ __noinline__ void by_token(float* st, float* red, const Rows L, const
 
 // grid (V / 16, heads, entries); four warps and one that copies.  Products are laid where a warp would wait for the others: those of O while the
 // sums of U go round.  The outputs of a chunk are added up when the sums of the next one have met.
-__global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __restrict__ work, int slots, const Rows L, float* __restrict__ state,
+template <bool DEEP>
+__global__ void __launch_bounds__(160, DEEP ? 1 : 2) pass_kernel(const unsigned char* __restrict__ work, int slots, const Rows L, float* __restrict__ state,
                                                       long long state_stride, float* __restrict__ out, const int* __restrict__ seg_q_start,
                                                       const int* __restrict__ seg_slot, int H, int h0, int V, int* __restrict__ error_word) {
+    using G = Ring<DEEP>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    Exchange& ex = *reinterpret_cast<Exchange*>(smem + STAGES * STAGE);
-    const uint32_t full = smem_u32(ex.bars), empty = full + 8 * STAGES, base = smem_u32(smem);
+    Exchange& ex = *reinterpret_cast<Exchange*>(smem + G::BYTES);
+    const uint32_t full = smem_u32(ex.bars), empty = full + 8 * G::BARS, base = smem_u32(smem);
     const int seg = blockIdx.z, h = h0 + blockIdx.y, v0 = blockIdx.x * VC;
     const int qs = seg_q_start[seg], n = seg_q_start[seg + 1] - qs, chunks = (n + C - 1) / C;
     if (chunks == 0) return;
     const size_t step = record_bytes(V);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 4); }
+        for (int s = 0; s < G::BARS; ++s) { mbar_init(full + 8 * s, 1); mbar_init(empty + 8 * s, 4); }
         mbar_init_fence();
         ex.odd[0] = ex.odd[1] = C;
     }
@@ -406,19 +419,30 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
         const unsigned char* rec = work + ((size_t)blockIdx.y * slots + first_slot(qs, seg)) * step;
         if (lane == 0)
             for (int k = 0; k < chunks; ++k, rec += step) {
-                const int st = k % STAGES;
-                if (k >= STAGES && !mbar_wait(empty + 8 * st, (k / STAGES - 1) & 1)) { atomicExch(error_word, 81); break; }
-                const uint32_t dst = base + st * STAGE, bar = full + 8 * st;
-                mbar_expect_tx(bar, U_OFF + U_BYTES);
-                bulk_load(dst, rec, U_OFF, bar);
-                bulk_load(dst + U_OFF, rec + U_OFF + blockIdx.x * U_BYTES, U_BYTES, bar);
+                bool ok = true;
+                for (int i = 0; i < (DEEP ? 1 : 3) && ok; ++i) {
+                    const int depth = i ? G::R : G::W, slot = k % depth, bar_no = i == 0 ? slot : i == 1 ? G::W + slot : G::W + G::R + slot;
+                    const uint32_t bar = full + 8 * bar_no, dst = base + slot * G::W_STEP;
+                    if (k >= depth && !mbar_wait(empty + 8 * bar_no, (k / depth - 1) & 1)) { atomicExch(error_word, 91); ok = false; break; }
+                    mbar_expect_tx(bar, DEEP ? U_OFF + U_BYTES : i == 0 ? G::W_BYTES : i == 1 ? MATRIX : K_BYTES);
+                    if (i == 0) {
+                        bulk_load(dst, rec, DEEP ? U_OFF : MATRIX, bar);
+                        if (!DEEP) bulk_load(dst + G::FLAG_AT, rec + ODD_OFF, 16, bar);
+                        bulk_load(dst + G::U_AT, rec + U_OFF + blockIdx.x * U_BYTES, U_BYTES, bar);
+                    } else if (i == 1) {
+                        bulk_load(base + G::Q_AT, rec + Q_OFF, MATRIX, bar);
+                    } else {
+                        bulk_load(base + G::K_AT, rec + K_OFF, K_BYTES, bar);
+                    }
+                }
+                if (!ok) break;
             }
         return;
     }
     const int g = lane >> 2, c2 = 2 * (lane & 3);
     bool alive = true;
     auto await = [&](uint32_t bar, int phase) {                         // a wait that ran out is recorded once; no further ones follow
-        if (alive && !mbar_spin(bar, phase & 1)) { alive = false; if (lane == 0) atomicExch(error_word, 82); }
+        if (alive && !mbar_spin(bar, phase & 1)) { alive = false; if (lane == 0) atomicExch(error_word, 92); }
     };
     bool there = false;                                                 // the next chunk was there when this one's sums had met
     auto meet = [] { asm volatile("bar.sync 1, 128;\n" ::: "memory"); };
@@ -474,8 +498,9 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
         }
     };
     for (int k = 0; k < chunks; ++k) {
-        const int st = k % STAGES;
-        const unsigned char* stage = smem + st * STAGE;
+        const int ws = k % G::W, wr = k / G::W, rs = k % G::R, rr = k / G::R;       // the pieces' slots, and how often those were filled before
+        const unsigned char *first = smem + ws * G::W_STEP, *queries = smem + G::Q_AT + rs * G::R_STEP, *keys = queries + MATRIX;
+        const int q_bar = 8 * (G::W + rs), k_bar = q_bar + 8 * G::R;
         uint32_t sa[2][PARTS][4];                                       // the accumulators' layout is the left operand's, two tiles at a time
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
@@ -490,21 +515,24 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
                 sa[ks][p][3] = take_part(x[1][2], x[1][3]);
             }
         }
-        if (!there) await(full + 8 * st, k / STAGES);
+        if (!there) await(full + 8 * ws, wr);
         Sums q;
         Right b0, b1;
         {
             Sums x;
             clear(x);
-            fetch_right(b0, stage + W_OFF, 0);
-            fetch_right(b1, stage + W_OFF, 1);
+            const bool q_there = DEEP || mbar_test(full + q_bar, rr & 1);           // (a wait for what is there takes 170 clocks, an answer that is read later none)
+            fetch_right(b0, first, 0);
+            fetch_right(b1, first, 1);
             product(x, sa[0], b0);
-            fetch_right(b0, stage + Q_OFF, 0);
+            if (!q_there) await(full + q_bar, rr);
+            fetch_right(b0, queries, 0);
             product(x, sa[1], b1);
             put(ex.u_part[w], x);
         }
         clear(q);
-        fetch_right(b1, stage + Q_OFF, 1);
+        fetch_right(b1, queries, 1);
+        const bool k_there = DEEP || mbar_test(full + k_bar, rr & 1);
         product(q, sa[0], b0);
         meet();
         {
@@ -514,7 +542,7 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
                 const float4 a = ex.u_part[e][w][lane];
                 u[0] += a.x; u[1] += a.y; u[2] += a.z; u[3] += a.w;
             }
-            const float* u0 = reinterpret_cast<const float*>(stage + U_OFF) + g * UPITCH + OCT * w + c2;
+            const float* u0 = reinterpret_cast<const float*>(first + G::U_AT) + g * UPITCH + OCT * w + c2;
             const float2 ua = *reinterpret_cast<const float2*>(u0), ub = *reinterpret_cast<const float2*>(u0 + 8 * UPITCH);
             u[0] = ua.x - u[0];
             u[1] = ua.y - u[1];
@@ -528,8 +556,9 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
                 t.y = take_part(v[2], v[3]);
                 ex.u[p][w][lane] = t;
             }
+            int odd = *reinterpret_cast<const int*>(first + G::FLAG_AT);
+            if (!DEEP) arrive(empty + 8 * ws);                          // W, U_0 and the flag have been read
             const uint32_t mx = __reduce_max_sync(0xffffffffu, largest(u));
-            int odd = *reinterpret_cast<const int*>(stage + ODD_OFF);
             if (mx > __float_as_uint(MOST)) {
                 const int mine = !(fabsf(u[0]) <= MOST && fabsf(u[2]) <= MOST) ? OCT * w + c2 : !(fabsf(u[1]) <= MOST && fabsf(u[3]) <= MOST) ? OCT * w + c2 + 1 : C;
                 odd = min(odd, __reduce_min_sync(0xffffffffu, mine));
@@ -538,19 +567,21 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
             }
             if (odd < C && lane == 0) atomicMin(&ex.odd[k & 1], odd);
         }
-        fetch_right(b0, stage + K_OFF, 0);
+        if (!DEEP) arrive(empty + q_bar);                               // ... and Q
+        if (!k_there) await(full + k_bar, rr);
+        fetch_right(b0, keys, 0);
         product(q, sa[1], b1);
-        fetch_right(b1, stage + K_OFF, 1);
+        fetch_right(b1, keys, 1);
         uint32_t pb[PARTS][4];
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
-            float4 x = reinterpret_cast<const float4*>(stage + P_OFF)[(2 * w + ks) * 32 + lane];
+            float4 x = reinterpret_cast<const float4*>(keys + P_AT)[(2 * w + ks) * 32 + lane];
 #pragma unroll
             for (int p = 0; p < PARTS; ++p) { pb[p][2 * ks] = take_part(x.x, x.y); pb[p][2 * ks + 1] = take_part(x.z, x.w); }
         }
         if (k) store(k - 1);
         put(ex.o_part[k & 1][w], q);
-        there = k + 1 < chunks && mbar_test(full + 8 * ((k + 1) % STAGES), (k + 1) / STAGES & 1);
+        there = k + 1 < chunks && mbar_test(full + 8 * ((k + 1) % G::W), (k + 1) / G::W & 1);
         meet();
         const int odd = ex.odd[k & 1];
         float so[4][4];                                                 // the state before the chunk
@@ -590,7 +621,7 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
                 for (int p = 0; p < PRODUCTS; ++p) mma16816(p < PRODUCTS - 1 ? small : lead, a[ks][PART_A[p]], pb[PART_B[p]][2 * ks], pb[PART_B[p]][2 * ks + 1]);
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
-                const float2 dec = *reinterpret_cast<const float2*>(stage + DEC_OFF + 4 * (32 * w + 8 * nt + c2));
+                const float2 dec = *reinterpret_cast<const float2*>(keys + DEC_AT + 4 * (32 * w + 8 * nt + c2));
 #pragma unroll
                 for (int e = 0; e < 4; ++e) s[nt][e] = fmaf(s[nt][e], e & 1 ? dec.y : dec.x, x.lead[nt][e] + x.small[nt][e]);
             }
@@ -599,7 +630,7 @@ __global__ void __launch_bounds__(160, 1) pass_kernel(const unsigned char* __res
         }
         left = min(n - k * C, odd);
         if (threadIdx.x == 0) ex.odd[(k + 1) & 1] = C;                  // all have read it: they had this chunk's sums before it
-        arrive(empty + 8 * st);
+        arrive(empty + (DEEP ? 8 * ws : k_bar));
         if (odd < C) {
             float* cols = reinterpret_cast<float*>(&ex.u_part[0][0][0]);
 #pragma unroll
@@ -632,7 +663,7 @@ MI_EXPORT long long mi_channel_chunk_bytes(int T_, int num_segs, int V) { return
 
 // prep [T, ld] float32 = q [KV D] | k [KV D] | v [H V] | g [H D] | beta [H] (rows on 16 bytes); out float32 [T, H V]; work on 16 bytes
 MI_EXPORT int mi_channel_chunks(const float* prep, int ld, void* work, long long work_bytes, float* state, long long state_stride, float* out,
-                                const int* seg_q_start, const int* seg_slot, int T_, int num_segs, int H, int KV, int D_, int V, int* error_word, cudaStream_t stream) {
+                                const int* seg_q_start, const int* seg_slot, int T_, int num_segs, int longest, int H, int KV, int D_, int V, int* error_word, cudaStream_t stream) {
     if (num_segs == 0 || T_ == 0) return 0;
     if (D_ != D || V % VC || H > 65535 || num_segs > 65535 || H % KV || ld % 4 || ((uintptr_t)prep | (uintptr_t)work) % 16) return -2;
     const int slots = T_ / C + num_segs, at_once = (int)std::min<long long>(H, work_bytes / mi_channel_chunk_bytes(T_, num_segs, V));
@@ -640,7 +671,8 @@ MI_EXPORT int mi_channel_chunks(const float* prep, int ld, void* work, long long
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ChunkSmem));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PASS_SMEM);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PASS_SMEM<true>);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, PASS_SMEM<false>);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
@@ -651,8 +683,14 @@ MI_EXPORT int mi_channel_chunks(const float* prep, int ld, void* work, long long
         chunk_kernel<<<dim3(slots, heads), 128, sizeof(ChunkSmem), stream>>>(L, (unsigned char*)work, seg_q_start, num_segs, h0, V);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
-        pass_kernel<<<dim3(V / VC, heads, num_segs), 160, PASS_SMEM, stream>>>((const unsigned char*)work, slots, L, state, state_stride, out, seg_q_start, seg_slot, H,
-                                                                               h0, V, error_word);
+        // A block an SM where every block then has one (2,048 tokens 162 us against 177 with two), or where there are more than two and the longest
+        // entry's walk is two thirds and more of what an SM walks on average (an entry counted as two chunks more than it has: 1,500 + 300 + 200 tokens
+        // 159 and 191, 1,300 + 517 + 231 160 and 176, 300 + 700 + 200 113 and 100, 4 x 512 168 and 151, 900 + 500 125 and 113, 8 x 1,024 556 and 508).
+        const long long blocks = (long long)heads * num_segs * (V / VC), all = (long long)(T_ / C + 2 * num_segs) * heads * (V / VC);
+        const bool deep = blocks <= 148 || (blocks > 2 * 148 && 20ll * 148 * (longest / C + 2) >= 13 * all);
+        auto walk = deep ? pass_kernel<true> : pass_kernel<false>;
+        walk<<<dim3(V / VC, heads, num_segs), 160, deep ? PASS_SMEM<true> : PASS_SMEM<false>, stream>>>((const unsigned char*)work, slots, L, state, state_stride, out, seg_q_start,
+                                                                                                    seg_slot, H, h0, V, error_word);
         e = cudaGetLastError();
         if (e != cudaSuccess) return (int)e;
     }

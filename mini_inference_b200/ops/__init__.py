@@ -520,7 +520,7 @@ class CudaOps:
         if code != 0:
             self._stream_error.zero_()
             self._tc2_counters.zero_()
-            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-64 grouped expert product, 71-74 delta rule and constant decay in chunks, 81-82 channel decays in chunks)")
+            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-64 grouped expert product, 71-74 delta rule and constant decay in chunks, 81-88 float32 product, 91-92 channel decays in chunks)")
 
     # ---------------------------------------------------------------- q/k norm, rotation, cache write
     def qk_norm_rope_cache(self, qkv, H, KV, D, q_weight, k_weight, eps, inv_freq, meta, k_cache, v_cache):
@@ -787,10 +787,11 @@ class CudaOps:
     @staticmethod
     def _takes_delta_chunks(batch, T, D, V):
         """Whether a delta rule with channel decays that _takes_octets goes 32 tokens at a time on the tensor cores instead
-        (csrc/channel_chunks.cu): keys of 128, values in blocks of 16 columns, a prompt of at least 192 tokens (29 us here, 31 there) and 40
-        tokens an entry on average, since a short entry takes a whole chunk (500 tokens beside 10 decoded ones 77 us here, 97 there; 300 beside 10
-        68 and 64; 200 beside 40 171 and 98; without a long prompt 8 of 65 tokens 72 and 62, 16 of 64 105 and 107)."""
-        return D == 128 and V % 16 == 0 and getattr(batch, "max_q_len", 0) >= 192 and T >= 40 * batch.num_segs
+        (csrc/channel_chunks.cu): keys of 128, values in blocks of 16 columns, and 28 tokens an entry on average beside a prompt of at least 192
+        tokens, 64 without one, since a short entry takes a whole chunk (192 tokens 29 us here, 31 there; 300 beside 10 decoded ones 60 and 64, 200
+        beside 40 171 and 98; 16 of 64 tokens 85 and 105, 16 of 48 101 and 87)."""
+        longest = getattr(batch, "max_q_len", 0)
+        return D == 128 and V % 16 == 0 and longest > 0 and T >= (28 if longest >= 192 else 64) * batch.num_segs
 
     def _chunk_scratch(self, T, batch, H, D, V):
         """Per chunk and head what it adds to the state, then the state before it."""
@@ -860,7 +861,7 @@ class CudaOps:
                 per_head = self.lib.mi_channel_chunk_bytes(T, batch.num_segs, V)
                 work = torch.empty(max(per_head, min(H * per_head, self.channel_work_bytes)), dtype=torch.uint8, device=self.device)
                 _check(self.lib.mi_channel_chunks(prep, prep.stride(0), work, work.numel(), state, state.stride(0), out, batch.seg_q_start,
-                                                  batch.seg_slot, T, batch.num_segs, H, KV, D, V, self._stream_error, self._stream()), "channel_chunks")
+                                                  batch.seg_slot, T, batch.num_segs, batch.max_q_len, H, KV, D, V, self._stream_error, self._stream()), "channel_chunks")
                 self.launches += 2 * -(-H // min(H, work.numel() // per_head))
                 return out
             scratch = self._octet_scratch(T, batch, H, D, V, True)

@@ -321,10 +321,10 @@ def delta_inputs(lens, H, KV, V, seed):
 
 
 @pytest.mark.parametrize("heads_at_once", [False, True])
-@pytest.mark.parametrize("lens,H,KV,V", [((192,), 16, 8, 128), ((193, 31), 3, 3, 16), ((1, 256, 33, 7), 4, 2, 144), ((223, 1, 64, 32, 1), 5, 1, 256)])
+@pytest.mark.parametrize("lens,H,KV,V", [((192,), 16, 8, 128), ((193, 31), 3, 3, 16), ((1, 256, 33, 7), 4, 2, 144), ((223, 1, 64, 32, 1), 5, 1, 256), ((64, 33, 96, 192), 8, 4, 128)])
 def test_channel_decays_in_chunks(ops, monkeypatch, lens, H, KV, V, heads_at_once):     # noqa: F811
-    """32 tokens at a time against the token-by-token kernel: whole chunks, remainders, single tokens beside prompts, more than 128 columns, decays down
-    to 0, with scratch for all heads and for one at a time."""
+    """32 tokens at a time against the token-by-token kernel: whole chunks, remainders, single tokens beside prompts, more than 128 columns, a block
+    and two blocks an SM (the last), decays down to 0, with scratch for all heads and for one at a time."""
     batch, prep, state = delta_inputs(lens, H, KV, V, sum(lens))
     if heads_at_once:
         monkeypatch.setattr(ops, "channel_work_bytes", 0)
@@ -337,23 +337,24 @@ def test_channel_decays_in_chunks(ops, monkeypatch, lens, H, KV, V, heads_at_onc
     assert torch.equal(a[:, H * 128 * V:], state[:, H * 128 * V:]) and torch.equal(a[0], state[0])
 
 
+@pytest.mark.parametrize("H", [2, 40])
 @pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta", "state", "huge v", "tiny v"])
-def test_channel_chunks_keep_odd_numbers_in_their_place(ops, what):     # noqa: F811
+def test_channel_chunks_keep_odd_numbers_in_their_place(ops, what, H):  # noqa: F811
     """Numbers that three bfloat16 parts do not hold: the outputs are those of the token-by-token kernel, tokens before the number, other entries and
     other heads have the bits they have without it."""
-    lens, H, V, at = (200, 192), 2, 32, 83                       # token 83: the 20th of the first entry's third chunk
+    lens, V, at = (200, 192), 32, 83                              # token 83: the 20th of the first entry's third chunk
     batch, prep, state = delta_inputs(lens, H, H, V, 3)
-    C = 4 * 128 + 2 * V
+    C = 2 * H * 128 + H * V
     spoiled, odd_state = prep.clone(), state.clone()
     if what == "state":
         odd_state[batch.seg_slot[0].item(), V * 30 + 4] = float("inf")
     elif what == "huge v":
-        spoiled[at, 512 + 3] = 1e30
+        spoiled[at, 256 * H + 3] = 1e30
     elif what == "tiny v":                                       # a head that holds nothing but numbers at the lower end
-        spoiled[:200, 512:512 + V] *= 1e-36
+        spoiled[:200, 256 * H:256 * H + V] *= 1e-36
         odd_state[batch.seg_slot[0].item(), :128 * V] *= 1e-36
     else:
-        spoiled[at, {"q": 5, "k": 256 + 7, "v": 512 + 9, "decay": C + 11, "beta": C + 256}[what]] = float("nan") if what in ("k", "decay", "beta") else float("inf")
+        spoiled[at, {"q": 5, "k": 128 * H + 7, "v": 256 * H + 9, "decay": C + 11, "beta": C + H * 128}[what]] = float("nan") if what in ("k", "decay", "beta") else float("inf")
     a, b, c = state.clone(), odd_state.clone(), odd_state.clone()
     assert ops._takes_delta_chunks(batch, 392, 128, V)
     want, got = ops.delta_scan(prep, H, H, 128, V, a, batch), ops.delta_scan(spoiled, H, H, 128, V, b, batch)
