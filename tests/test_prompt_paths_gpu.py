@@ -57,6 +57,28 @@ def test_gemm_f32_on_tensor_cores(ops, M, N, K):                # noqa: F811
             assert ((got2[m][ok].double() - want2[m][ok]).abs() <= 2e-6 * size + 1e-37).all(), m
 
 
+@pytest.mark.parametrize("M,N,K", [(652, 896, 4100), (700, 896, 4160), (768, 2048, 4100), (1030, 1152, 4132)])
+def test_gemm_f32_whose_last_segment_is_short(ops, M, N, K):    # noqa: F811
+    """K that leaves a last segment of one or two stages, so that a block has several such items in a row: which rows of W bfloat16 parts cannot hold is then
+    handed over faster than anything else (rows of infinities, NaN and 1e30 in every other tile, in the last segment's columns)."""
+    g = torch.Generator().manual_seed(M + K)
+    x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
+    plain = ops.linear(x, w)
+    odd = {n: v for n, v in zip(range(5, N, 256), [float("nan"), float("inf"), 1e30] * N)}
+    for n, v in odd.items():
+        w[n, K - 1] = v
+    rest = [n for n in range(N) if n not in odd]
+    for _ in range(5):
+        got = ops.linear(x, w)
+        ops.check_errors()
+        want = x.double() @ w.double().T
+        assert torch.equal(got[:, rest], plain[:, rest])
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        big = [n for n, v in odd.items() if v == 1e30]
+        if big:                                                  # the sums that a float32 product of 1e30 is added to are lost beside it
+            assert ((got[:, big].double() - want[:, big]).abs() <= 2e-6 * x.double().norm(dim=1, keepdim=True) * 1e30).all()
+
+
 FORMS = ["causal", "window", "blocks_sink", "learned_sink_bias", "slopes", "slopes_bias_window", "cap_keep_gate", "window_keep_narrow"]
 
 
