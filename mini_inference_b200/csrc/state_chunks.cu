@@ -309,8 +309,9 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_state_kernel(const T* __rest
     if (warp == 16) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-// grid (D V / 4 / 256, heads, entries): a thread has four state entries
-__global__ void __launch_bounds__(256) chunk_scan_kernel(float* __restrict__ sums, const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
+// grid (D V / 4 / 256, heads, entries): a thread has four state entries.  No __restrict__ on sums: the kernel ahead writes them while this one already runs,
+// and loads through a pointer that promises to be the only one may be moved ahead of the wait.
+__global__ void __launch_bounds__(256) chunk_scan_kernel(float* sums, const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
                                                          const int* __restrict__ seg_q_start, const int* __restrict__ seg_slot, int slots, int V) {
     pdl_trigger();
     const int seg = blockIdx.z, h = blockIdx.y, at = 4 * (blockIdx.x * 256 + threadIdx.x);
@@ -345,8 +346,7 @@ __global__ void __launch_bounds__(256) chunk_scan_kernel(float* __restrict__ sum
     *reinterpret_cast<float2*>(S + 2) = make_float2(s.z, s.w);
 }
 
-// grid (slots, heads, V / VC); before [head][slot][D][V]: the state before each chunk (no __restrict__: the kernel ahead writes it while this one already
-// runs, and loads of memory that is promised to stay as it is may be moved ahead of the wait).  Tensor memory: Q's parts, then those of the decayed scores; two
+// grid (slots, heads, V / VC); before [head][slot][D][V]: the state before each chunk (no __restrict__ here either).  Tensor memory: Q's parts, then those of the decayed scores; two
 // accumulators.  Shared memory: K, then V; S_0, then the result.
 template <typename T, bool SILU>
 __global__ void __launch_bounds__(THREADS, 1) chunk_out_kernel(const T* __restrict__ in, const Source L, const float* __restrict__ decay, const float* before,
