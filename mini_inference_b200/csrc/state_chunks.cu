@@ -309,37 +309,49 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_state_kernel(const T* __rest
     if (warp == 16) { tc_fence_after(); tmem_dealloc(tmem, 512); }
 }
 
-// grid (D V / 4 / 256, heads, entries): a thread has four state entries.  No __restrict__ on sums: the kernel ahead writes them while this one already runs,
-// and loads through a pointer that promises to be the only one may be moved ahead of the wait.
-__global__ void __launch_bounds__(256) chunk_scan_kernel(float* sums, const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
-                                                         const int* __restrict__ seg_q_start, const int* __restrict__ seg_slot, int slots, int V) {
+// grid (D V / 1024, heads, entries): a thread has four state entries (V is a multiple of 128).  No __restrict__ on sums: the kernel ahead writes them while
+// this one already runs, and loads through a pointer that promises to be the only one may be moved ahead of the wait.
+// Bound by memory: the sums and the states once each way.  Eight blocks an SM, an entry of one chunk without a loop, and the powers by two threads of a
+// block (64-bit products are slow): eight sums in flight a thread left four blocks an SM (64 heads, microseconds there / here: 16 entries of 64 tokens
+// 390 / 59, 2,048 tokens beside 18 single ones 496 / 101, 1,000 + 6 x 100 102 / 35, 2,048 25 / 17).
+__global__ void __launch_bounds__(256, 8) chunk_scan_kernel(float* sums, const float* __restrict__ decay, float* __restrict__ state, long long state_stride,
+                                                            const int* __restrict__ seg_q_start, const int* __restrict__ seg_slot, int slots, int V) {
+    constexpr int AT_ONCE = 4;
+    __shared__ float less_one[2];
     pdl_trigger();
     const int seg = blockIdx.z, h = blockIdx.y, at = 4 * (blockIdx.x * 256 + threadIdx.x);
     const int qs = seg_q_start[seg], n = seg_q_start[seg + 1] - qs, chunks = (n + C - 1) / C;
-    if (chunks == 0 || at >= D * V) return;
+    if (chunks == 0) return;
     // d^m - 1: s + s (d^m - 1) keeps the last bits of a decay near 1 (an infinity stays one)
+    if (threadIdx.x < 2) less_one[threadIdx.x] = (float)(power((double)decay[h], threadIdx.x ? n - (chunks - 1) * C : C) - 1.0);
     const bool lasts = decay[h] > 0.f;
-    auto decayed = [&](float s, float m) { return fabsf(s) == INFINITY && lasts ? s : fmaf(s, m, s); };
-    const float whole = (float)(power((double)decay[h], C) - 1.0), last = (float)(power((double)decay[h], n - (chunks - 1) * C) - 1.0);
+    auto step_on = [&](float4 s, float m, const float4& t) {
+        auto next = [&](float s, float t) { return (fabsf(s) == INFINITY && lasts ? s : fmaf(s, m, s)) + t; };
+        return make_float4(next(s.x, t.x), next(s.y, t.y), next(s.z, t.z), next(s.w, t.w));
+    };
     float* S = state + (long long)seg_slot[seg] * state_stride + (long long)h * D * V + at;
     float* ws = sums + ((size_t)h * slots + first_slot(qs, seg)) * D * V + at;
     const size_t step = (size_t)D * V;
     const float2 s01 = *reinterpret_cast<const float2*>(S), s23 = *reinterpret_cast<const float2*>(S + 2);
     float4 s = make_float4(s01.x, s01.y, s23.x, s23.y);
+    __syncthreads();
+    const float whole = less_one[0], last = less_one[1];
     pdl_wait();
-    for (int c = 0; c < chunks; c += 8) {
-        float4 t[8];
+    if (chunks == 1) {
+        const float4 t = *reinterpret_cast<const float4*>(ws);
+        *reinterpret_cast<float4*>(ws) = s;
+        s = step_on(s, last, t);
+    } else {
+        for (int c = 0; c < chunks; c += AT_ONCE) {
+            float4 t[AT_ONCE];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) if (c + i < chunks) t[i] = *reinterpret_cast<const float4*>(ws + (c + i) * step);
+            for (int i = 0; i < AT_ONCE; ++i) if (c + i < chunks) t[i] = *reinterpret_cast<const float4*>(ws + (c + i) * step);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            if (c + i >= chunks) break;
-            *reinterpret_cast<float4*>(ws + (c + i) * step) = s;
-            const float m = c + i == chunks - 1 ? last : whole;
-            s.x = decayed(s.x, m) + t[i].x;
-            s.y = decayed(s.y, m) + t[i].y;
-            s.z = decayed(s.z, m) + t[i].z;
-            s.w = decayed(s.w, m) + t[i].w;
+            for (int i = 0; i < AT_ONCE; ++i) {
+                if (c + i >= chunks) break;
+                *reinterpret_cast<float4*>(ws + (c + i) * step) = s;
+                s = step_on(s, c + i == chunks - 1 ? last : whole, t[i]);
+            }
         }
     }
     *reinterpret_cast<float2*>(S) = make_float2(s.x, s.y);
