@@ -777,21 +777,43 @@ class CudaOps:
         return torch.empty(self.lib.mi_octet_floats(T, batch.num_segs, H, D, V, int(delta)), dtype=torch.float32, device=self.device)
 
     @staticmethod
-    def _takes_chunks(batch, T, D, V):
+    def _chunks(T, segs, longest, size):
+        """Chunks of `size` tokens of a step: those of its longest entry, and of the others as if they were equally long."""
+        rest = T - longest
+        return -(-longest // size) + ((segs - 1) * max(1, -(-rest // ((segs - 1) * size))) if segs > 1 else 0)
+
+    @staticmethod
+    def _takes_chunks(batch, T, D, V, H=None):
         """Whether a recurrence with a constant decay that _takes_octets goes 128 tokens at a time on the tensor cores instead (csrc/state_chunks.cu): keys
         of 128, values in blocks of 128 columns, a prompt of at least 320 tokens (three kernels of some 36 us in all against eight tokens at a time:
         192 tokens 27 us there, 256 31, 400 41, 2,048 167 against 73) and 100 tokens an entry on average, since a short entry takes a whole chunk
-        (16 prompts of 64 tokens 79 us there, 94 here; 192 tokens beside 40 decoded ones 92 and 256)."""
-        return D == 128 and V % 128 == 0 and getattr(batch, "max_q_len", 0) >= 320 and T >= 100 * batch.num_segs
+        (16 prompts of 64 tokens 73 us there, 89 here; 192 tokens beside 40 decoded ones 92 and 256).  H heads: where the chunks are one wave of blocks
+        that is all; beyond, both sides' times are weighed, a line through 2 to 64 heads of 128 to 512 columns (within a tenth): 64 heads 2,048 tokens 502 us
+        there, 288 here, 1,024 beside 8 single ones 285 and 305, 400 beside 3 121 and 145; 32 heads 330 beside 2 65 and 71, 700 beside 3 125 and 80."""
+        if not (D == 128 and V % 128 == 0 and getattr(batch, "max_q_len", 0) >= 320 and T >= 100 * batch.num_segs):
+            return False
+        if H is None:
+            return True
+        blocks = CudaOps._chunks(T, batch.num_segs, batch.max_q_len, 128) * H * (V // 128)
+        waves = -(-blocks // 148)
+        return waves == 1 or 3 + 28.5 * waves + 0.08 * blocks < 0.97 * (13 + 0.052 * batch.max_q_len + (0.0024 * T + 0.08 * batch.num_segs) * H * (V // 128))
 
     @staticmethod
-    def _takes_delta_chunks(batch, T, D, V):
+    def _takes_delta_chunks(batch, T, D, V, H=None):
         """Whether a delta rule with channel decays that _takes_octets goes 32 tokens at a time on the tensor cores instead
         (csrc/channel_chunks.cu): keys of 128, values in blocks of 16 columns, and 28 tokens an entry on average beside a prompt of at least 192
-        tokens, 64 without one, since a short entry takes a whole chunk (192 tokens 29 us here, 31 there; 300 beside 10 decoded ones 60 and 64, 200
-        beside 40 171 and 98; 16 of 64 tokens 85 and 105, 16 of 48 101 and 87)."""
+        tokens, 64 without one, since a short entry takes a whole chunk (192 tokens 29 us here, 31 there; 200 beside 40 decoded ones 171 and 98;
+        16 of 64 tokens 85 and 105, 16 of 48 101 and 87: 16 heads).  H heads: both sides' times are weighed as well, a line through 1 to 64 heads of 16 to
+        256 columns (within a tenth): 32 heads 300 tokens beside 10 single ones 103 us here, 91 there, 1,000 beside 20 231 and 248; 64 heads of 16 columns
+        4 x 512 212 and 159, 2,048 265 and 276; 2 heads 8 of 64 tokens 19 and 16; 16 heads 300 beside 10 57 and 61."""
         longest = getattr(batch, "max_q_len", 0)
-        return D == 128 and V % 16 == 0 and longest > 0 and T >= (28 if longest >= 192 else 64) * batch.num_segs
+        if not (D == 128 and V % 16 == 0 and longest > 0 and T >= (28 if longest >= 192 else 64) * batch.num_segs):
+            return False
+        if H is None:
+            return True
+        n, g = CudaOps._chunks(T, batch.num_segs, longest, 32), H * V / 128
+        return (14 + 1.2 * -(-longest // 32) + n * (0.033 * H + 0.06 * g) + 0.06 * batch.num_segs * g
+                < 7.3 + 0.0865 * longest + (0.0035 * T + 0.1 * batch.num_segs) * g)
 
     def _chunk_scratch(self, T, batch, H, D, V):
         """Per chunk and head what it adds to the state, then the state before it."""
@@ -810,7 +832,7 @@ class CudaOps:
             self.launches += 1
             return out
         if wide and self._takes_octets(p, batch, D, V, state):
-            if self._takes_chunks(batch, T, D, V) and p.stride(0) % 8 == 0:
+            if self._takes_chunks(batch, T, D, V, H) and p.stride(0) % 8 == 0:
                 _check(self.lib.mi_lightning_chunks(p, p.stride(0), self._chunk_scratch(T, batch, H, D, V), decay, state,
                                                     state.stride(0), out, batch.seg_q_start, batch.seg_slot, T, batch.num_segs,
                                                     H, D, V, self._stream_error, self._stream()), "lightning_chunks")
@@ -857,7 +879,7 @@ class CudaOps:
             self.launches += 1
             return out
         if not exact and self._takes_octets(prep, batch, D, V, state):
-            if self._takes_delta_chunks(batch, T, D, V):
+            if self._takes_delta_chunks(batch, T, D, V, H):
                 per_head = self.lib.mi_channel_chunk_bytes(T, batch.num_segs, V)
                 work = torch.empty(max(per_head, min(H * per_head, self.channel_work_bytes)), dtype=torch.uint8, device=self.device)
                 _check(self.lib.mi_channel_chunks(prep, prep.stride(0), work, work.numel(), state, state.stride(0), out, batch.seg_q_start,
@@ -1194,7 +1216,7 @@ class CudaOps:
         _check(self.lib.mi_retention_rows(p, p.stride(0), prep, batch.positions, inv_freq, half, k_scale, T, H, D, V,
                                           _code(p.dtype), self._stream()), "retention_rows")
         if p.dtype == torch.bfloat16 and self._takes_octets(prep, batch, D, V, state):
-            if self._takes_chunks(batch, T, D, V):
+            if self._takes_chunks(batch, T, D, V, H):
                 _check(self.lib.mi_constant_chunks(prep, self._chunk_scratch(T, batch, H, D, V), decay, state, state.stride(0),
                                                    out, batch.seg_q_start, batch.seg_slot, T, batch.num_segs, H, D, V, self._stream_error,
                                                    self._stream()), "constant_chunks")

@@ -53,6 +53,20 @@ def test_line_of_the_eight_token_scans():
     assert takes(*[64] * 8) and not takes(*[63] * 8)
 
 
+def test_lines_of_recurrences_in_chunks():
+    """By tokens, entries and heads: short entries take whole chunks, which many heads feel and few do not."""
+    takes = lambda H, V, *lens: CudaOps._takes_chunks(step(lens), sum(lens), 128, V, H)       # noqa: E731
+    for H in (1, 2, 16, 64):
+        assert takes(H, 128, 320) and takes(H, 128, 2048) and takes(H, 128, *[512] * 4) and not takes(H, 128, 319) and not takes(H, 128, 330, *[1] * 4)
+    assert takes(16, 128, 700, 1, 1, 1) and takes(32, 128, 700, 1, 1, 1) and takes(16, 128, 330, 1, 1) and takes(16, 128, 2048, *[1] * 18)
+    assert not takes(32, 128, 330, 1, 1) and not takes(64, 128, 1024, *[1] * 8) and not takes(16, 512, 1024, *[1] * 8) and not takes(48, 128, 330, 1)
+    delta = lambda H, V, *lens: CudaOps._takes_delta_chunks(step(lens), sum(lens), 128, V, H)    # noqa: E731
+    for H in (2, 16, 64):
+        assert delta(H, 128, 192) and delta(H, 128, 2048) and delta(H, 128, *[512] * 4) and not delta(H, 128, 192, *[1] * 10)
+    assert delta(16, 128, 300, *[1] * 10) and delta(32, 128, *[64] * 16) and delta(16, 256, *[64] * 16) and delta(4, 16, 192)
+    assert not delta(32, 128, 300, *[1] * 10) and not delta(2, 128, *[64] * 8) and not delta(64, 16, *[512] * 4) and not delta(64, 16, 192)
+
+
 def test_line_of_the_selective_scan():
     """An entry costs the kernel for prompts about the same however short it is, the other one walks the longest entry at a quarter of the speed."""
     takes = lambda *lens: CudaOps._takes_prompt_scan(sum(lens), step(lens))      # noqa: E731
