@@ -167,7 +167,9 @@ int segments(int N, int K, int* segment) {
 constexpr int ROWS_AT_ONCE = 1024;             // rows per pass of a product that needs a workspace: bounds it
 
 // Which products run on the tensor cores: by N and K alone (and that W's rows start on 16 bytes, as TMA reads them), so that a row's bits do not
-// depend on M.  Smaller matrices are a few tiles for 148 blocks and keep the multiply-adds.
+// depend on M.  Smaller matrices are a few tiles for 148 blocks and keep the multiply-adds.  At the low end of N and K a few rows pay for the many
+// (microseconds by multiply-adds / here: 2,048 x 512 one row 8.4 / 14.9, 33 rows 27 / 16, 1,000 rows 63 / 20; 128 x 8,192 18 / 27, 24 / 29, 87 / 38;
+// 1,024 x 1,024 15.0 / 16.5, 17.1 / 17.5, 81 / 23; from 256 x 4,096 on one row is faster here too); the error is a third everywhere.
 bool on_tensor_cores(int N, int K) { return K % 4 == 0 && K >= 512 && N >= 128 && (long long)N * K >= 1 << 20; }
 
 // Their K is cut until a tile of tokens alone gives about one block per SM, in pieces of at least 512
