@@ -14,8 +14,10 @@
 // waiting for the operand before it.  Scores of all 128 columns in one sum in tensor memory cost 2.2e-7 of error, of 32 columns 1.2e-7, the leading
 // products of parts of 32 on their own 8.9e-8.
 //
-// Numbers that the parts do not hold (infinities, NaN, pieces of rows whose largest magnitude is not in [2^-90, 2^60]) are taken out of the products; the
-// outputs from their token on are computed once more token by token in float32, those before it have the bits they have without it.
+// Numbers that the parts do not hold are taken out of the products; the outputs from their token on are computed once more token by token in float32, those
+// before it have the bits they have without it.  These are infinities and NaN; a query (a quarter of it) or a key whose largest magnitude is not in
+// [2^-50, 2^36], so that scores stay where their parts are whole; 8 values beyond [2^-90, 2^36] and 8 entries of a state beyond [2^-90, 2^60].  All else is
+// as exact as float32 sums are against |q| |k| |v| as vectors; what decays below 2^-100 of that may keep fewer bits than it has in float32.
 #include "split3.cuh"
 #include <algorithm>
 
@@ -29,7 +31,8 @@ constexpr int C = 128, D = 128, VC = 128;                       // tokens of a c
 constexpr int WORKERS = 512, THREADS = WORKERS + 32;            // 16 warps, a thread one row and a quarter of its columns; one warp issues the products
 constexpr int BLOCK64 = C * 128, PART_BYTES = 2 * BLOCK64, OPERAND = PARTS * PART_BYTES;      // 128 rows of 64 bfloat16; an operand's part; its parts
 constexpr int ROW_OUT = VC + 4;                                 // floats of a result's row in shared memory
-constexpr float LEAST = 0x1p-90f, MOST = 0x1p60f;
+struct Range { float least, most; };
+constexpr Range SCORED{0x1p-50f, 0x1p36f}, ADDED{0x1p-90f, 0x1p36f}, STATE{0x1p-90f, 0x1p60f};      // q and k; v, and k on its way into the state; the state
 
 // An entry's chunks lie behind floor(first token / 128) + entry slots: entries never share one.
 __host__ __device__ __forceinline__ int first_slot(int qs, int seg) { return qs / C + seg; }
@@ -90,12 +93,15 @@ template <typename T, int N> __device__ __forceinline__ void load_n(const T* p, 
 template <bool SILU, int N> __device__ __forceinline__ void activate(float (&v)[N]) {
     if constexpr (SILU) silu(v);
 }
-// Whether the parts hold these numbers; if not they become zeros
-template <int N> __device__ __forceinline__ bool fits(float (&v)[N]) {
+template <int N> __device__ __forceinline__ float largest(const float (&v)[N]) {       // NaN if there is one
     float mx = 0.f;
 #pragma unroll
     for (int e = 0; e < N; ++e) asm("max.NaN.f32 %0, %0, %1;\n" : "+f"(mx) : "f"(fabsf(v[e])));
-    const bool ok = mx <= MOST && (mx == 0.f || mx >= LEAST);
+    return mx;
+}
+// Whether the parts hold numbers of which this is the largest magnitude; if not they become zeros
+template <int N> __device__ __forceinline__ bool fits(float (&v)[N], float mx, Range range) {
+    const bool ok = mx <= range.most && (mx == 0.f || mx >= range.least);
     if (!ok) clear(v);
     return ok;
 }
@@ -112,8 +118,9 @@ __device__ __forceinline__ void fetch(Tile<T>& t, const T* src, size_t ld, int r
     }
 }
 // ... -> the three parts in shared memory, the 16-byte pieces of a row by 8 threads side by side.  Answers with the first row that does not fit (C: none).
-template <typename T, bool SILU>
-__device__ __forceinline__ int to_shared(unsigned char* operand, const Tile<T>& t) {
+// ROW: judged by the whole row, else by 8 numbers.
+template <typename T, bool SILU, bool ROW = false>
+__device__ __forceinline__ int to_shared(unsigned char* operand, const Tile<T>& t, Range range) {
     int odd = C;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -122,7 +129,12 @@ __device__ __forceinline__ int to_shared(unsigned char* operand, const Tile<T>& 
 #pragma unroll
         for (int j = 0; j < 8 / Vec16<T>::N; ++j) load16(reinterpret_cast<const T*>(&t.w[i][j]), v + j * Vec16<T>::N);
         activate<SILU>(v);
-        if (!fits(v)) odd = min(odd, row);
+        float mx = largest(v);
+        if (ROW) {
+#pragma unroll
+            for (int w = 1; w < 16; w <<= 1) asm("max.NaN.f32 %0, %0, %1;\n" : "+f"(mx) : "f"(__shfl_xor_sync(0xffffffffu, mx, w)));
+        }
+        if (!fits(v, mx, range)) odd = min(odd, row);
         unsigned char* at = operand + (c >> 3) * BLOCK64 + row * 128 + (((c ^ row) & 7) << 4);
 #pragma unroll
         for (int p = 0; p < PARTS; ++p) {
@@ -276,11 +288,11 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_state_kernel(const T* __rest
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = to_f32(*reinterpret_cast<const T*>(rows + (32 * quarter + j) * PITCH<T> + row * sizeof(T)));
         activate<SILU>(v);
-        bool ok = fits(v);
+        bool ok = fits(v, largest(v), ADDED);
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] *= tail.pw[max(0, ch.n - 1 - 32 * quarter - j)];
         to_tensor(lanes, quarter, v);
-        ok &= to_shared<T, SILU>(base, x) == C;
+        ok &= to_shared<T, SILU>(base, x, ADDED) == C;
         if (!ok) tail.first_odd = 0;
         shared_is_written();
         tmem_wait_st();
@@ -408,9 +420,9 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_out_kernel(const T* __restri
         float s[32], o[32];
         load_n(reinterpret_cast<const T*>(sbuf + row * PITCH<T> + 32 * quarter * sizeof(T)), s);
         activate<SILU>(s);
-        int odd = fits(s) ? C : row;
+        int odd = fits(s, largest(s), SCORED) ? C : row;
         to_tensor(lanes, quarter, s);
-        odd = min(odd, to_shared<T, SILU>(base, k));
+        odd = min(odd, to_shared<T, SILU, true>(base, k, SCORED));
         shared_is_written();
         tmem_wait_st();
         tc_fence_before();
@@ -421,12 +433,12 @@ __global__ void __launch_bounds__(THREADS, 1) chunk_out_kernel(const T* __restri
             Tile<float> t;
             fetch(t, S0, V, D);
             workers_meet();                                     // everyone has its row of Q
-            if (to_shared<float, false>(sbuf, t) < C) odd = 0;
+            if (to_shared<float, false>(sbuf, t, STATE) < C) odd = 0;
         }
         shared_is_written();
         mbar_arrive(s_ready);
         bool ok = add_up(d, turn, lanes, quarter, s);           // the scores; K is done with
-        odd = min(odd, to_shared<T, SILU>(base, k));
+        odd = min(odd, to_shared<T, SILU>(base, k, ADDED));
         shared_is_written();
         if (odd < C) atomicMin(&tail.first_odd, odd);
 #pragma unroll

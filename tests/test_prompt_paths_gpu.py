@@ -326,6 +326,34 @@ def test_chunks_keep_odd_numbers_in_their_place(ops, what):     # noqa: F811
         assert rows_error(torch.where(ok, got, 0.), torch.where(ok, plain, 0.)) < 3e-6, name
 
 
+@pytest.mark.parametrize("q,k,v", [(-49, -49, 34), (34, 34, 34), (-85, -80, 40), (-60, -60, 30), (45, 50, 8), (-88, 20, 30), (30, -88, 38), (0, -30, -80), (-49, 34, -60)])
+def test_chunks_near_the_ends_of_the_parts(ops, q, k, v):       # noqa: F811
+    """Queries, keys and values near the ends of what bfloat16 parts hold, and beyond, together: powers of two, against float64."""
+    lens, H, V, D = (330, 320), 2, 128, 128
+    batch, p, state, decay, _ = chunk_inputs(lens, H, V, 5)
+    decay = torch.tensor([0.5, 0.99], device=DEV)
+    sizes = torch.cat([torch.full((H * D,), 2.0 ** q), torch.full((H * D,), 2.0 ** k), torch.full((H * V,), 2.0 ** v), torch.ones(8)]).to(DEV)
+    p = (p * sizes).to(torch.bfloat16)
+    state = state * 2.0 ** (k + v)
+    a = state.clone()
+    assert ops._takes_chunks(batch, sum(lens), D, V, H)
+    got = ops.retention_scan(p, H, D, V, None, 1.0, decay, a, batch).view(-1, H, V)
+    ops.check_errors()
+    first = 0
+    for i, n in enumerate(lens):
+        x = (p[first:first + n, :3 * H * D].double() / sizes[:3 * H * D]).view(n, 3, H, D)
+        slot = batch.seg_slot[i].item()
+        S = (state[slot, :H * D * V].double() / 2.0 ** (k + v)).view(H, D, V)
+        want = torch.empty(n, H, V, dtype=torch.float64, device=DEV)
+        for t in range(n):
+            S = decay.double()[:, None, None] * S + x[t, 1][:, :, None] * x[t, 2][:, None, :]
+            want[t] = torch.einsum("hd,hdv->hv", x[t, 0], S)
+        # float32 sums over up to 330 decayed tokens and 128 rows
+        assert rows_error(got[first:first + n].double() / 2.0 ** (q + k + v), want) < 3e-6
+        assert rows_error(a[slot, :H * D * V].double() / 2.0 ** (k + v), S.reshape(-1)) < 3e-6
+        first += n
+
+
 def delta_inputs(lens, H, KV, V, seed):
     T, D, g = sum(lens), 128, torch.Generator().manual_seed(seed)
     r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
