@@ -21,8 +21,11 @@
 // Measured and left: outputs made by four more warps (as fast: they share the schedulers' product rate and the shared memory), operands cut
 // by the first kernel (6 bytes a number instead of 4: as fast, and half as much scratch again), 32 columns by eight warps (64 blocks for one prompt: 227).
 //
-// Numbers that the parts do not hold (infinities, NaN, the ends of the range) are found where U is cut into parts, or when a chunk is made ready: from
-// the first such token on the chunk is computed token by token, the tokens before it keep their bits.
+// Numbers that the parts do not hold are found where U is cut into parts, or when a chunk is made ready: from the first such token on the chunk is
+// computed token by token, the tokens before it keep their bits.  These are infinities and NaN, W, Q, K, B and U beyond 2^60, a query or a key whose largest
+// magnitude is below 2^-50 (so that B's parts are whole), a token's 16 columns of U that are all below 2^-100.  All else is as exact as float32 sums are
+// against the vectors' norms; what decays below 2^-100 of a query, a key or a state may keep fewer bits than it has in float32, and a query times a state
+// beyond 2^127 is an infinity also where a chunk's later additions would have taken it back.
 #include "split3.cuh"
 #include <math.h>
 #include <algorithm>
@@ -34,7 +37,7 @@ using namespace mi::split3;
 namespace {
 
 constexpr int C = 32, D = 128, OCT = 8, NOCT = C / OCT, VC = 16;        // tokens of a chunk; rows of a state; columns of four warps
-constexpr float LEAST = 0x1p-100f, MOST = 0x1p60f;
+constexpr float LEAST = 0x1p-100f, MOST = 0x1p60f, LEAST_SCORED = 0x1p-50f;
 
 // What chunk_kernel leaves per (chunk, head), float32: W, Q, K and B in the order in which lanes take them as right operands of m16n8k16 (a lane's
 // four numbers of a tile side by side); pass_kernel cuts them into parts
@@ -134,6 +137,14 @@ __global__ void __launch_bounds__(128, 4) chunk_kernel(const Rows L, unsigned ch
         if (tid < C) sm.beta[tid] = tid < n ? first[(size_t)tid * L.ld + L.beta + h] : 0.f;
         if (tid == 0) sm.odd = C;
         __syncthreads();
+        int tiny = C;                                                   // the warp's first token whose query or key is small but for zeros
+#pragma unroll
+        for (int i = OCT - 1; i >= 0; --i) {
+            const float q[4] = {q4[i].x, q4[i].y, q4[i].z, q4[i].w}, k[4] = {k4[i].x, k4[i].y, k4[i].z, k4[i].w};
+            const uint32_t mq = __reduce_max_sync(0xffffffffu, largest(q)), mk = __reduce_max_sync(0xffffffffu, largest(k));
+            if (min(mq - 1, mk - 1) < __float_as_uint(LEAST_SCORED) - 1) tiny = OCT * warp + i;
+        }
+        if (tiny < C && lane == 0) atomicMin(&sm.odd, tiny);
         float y[32], z[32], last[4] = {0.f, 0.f, 0.f, 0.f};             // 28 A_ij at i (i - 1) / 2 + j, 36 B_ij at i (i + 1) / 2 + j
         float G[4] = {1.f, 1.f, 1.f, 1.f}, kh[OCT][4];
 #pragma unroll
@@ -562,8 +573,19 @@ __global__ void __launch_bounds__(160, DEEP ? 1 : 2) pass_kernel(const unsigned 
             if (mx > __float_as_uint(MOST)) {
                 const int mine = !(fabsf(u[0]) <= MOST && fabsf(u[2]) <= MOST) ? OCT * w + c2 : !(fabsf(u[1]) <= MOST && fabsf(u[3]) <= MOST) ? OCT * w + c2 + 1 : C;
                 odd = min(odd, __reduce_min_sync(0xffffffffu, mine));
-            } else if (mx != 0 && mx < __float_as_uint(LEAST)) {
-                odd = min(odd, OCT * w);
+            }
+            uint32_t low = 0xffffffffu;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) low = min(low, __float_as_uint(fabsf(u[e])) - 1);
+            if (__any_sync(0xffffffffu, low < __float_as_uint(LEAST) - 1)) {        // rare: is it the largest of its token's?
+                float t0 = fmaxf(fabsf(u[0]), fabsf(u[2])), t1 = fmaxf(fabsf(u[1]), fabsf(u[3]));
+#pragma unroll
+                for (int x = 4; x < 32; x <<= 1) {
+                    t0 = fmaxf(t0, __shfl_xor_sync(0xffffffffu, t0, x));
+                    t1 = fmaxf(t1, __shfl_xor_sync(0xffffffffu, t1, x));
+                }
+                const int mine = t0 != 0.f && t0 < LEAST ? OCT * w + c2 : t1 != 0.f && t1 < LEAST ? OCT * w + c2 + 1 : C;
+                odd = min(odd, __reduce_min_sync(0xffffffffu, mine));
             }
             if (odd < C && lane == 0) atomicMin(&ex.odd[k & 1], odd);
         }

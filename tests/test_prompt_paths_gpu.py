@@ -423,6 +423,52 @@ def test_channel_chunks_keep_odd_numbers_in_their_place(ops, monkeypatch, what, 
     assert rows_error(torch.where(ok, got, 0.) * scale, torch.where(ok, plain, 0.) * scale) < 3e-6
 
 
+@pytest.mark.parametrize("q,k,v", [(-49, -45, 30), (-85, -60, 40), (-60, -60, 20), (-80, 0, 20), (0, 0, -95), (30, 0, 28), (0, -70, 0), (-45, -3, -40)])
+def test_channel_chunks_near_the_ends_of_the_parts(ops, monkeypatch, q, k, v):       # noqa: F811
+    """Queries, keys and values near the ends of what bfloat16 parts hold, and beyond, together: powers of two, against float64."""
+    lens, H, V, D = (200, 192), 2, 32, 128
+    batch, prep, state = delta_inputs(lens, H, H, V, 6)
+    C = 2 * H * D + H * V
+    sizes = torch.cat([torch.full((H * D,), 2.0 ** q), torch.full((H * D,), 2.0 ** k), torch.full((H * V,), 2.0 ** v)]).to(DEV)
+    prep[:, :C] *= sizes
+    state = state * 2.0 ** (k + v)
+    a = state.clone()
+    monkeypatch.setattr(ops, "_takes_delta_chunks", lambda *args: True)
+    got = ops.delta_scan(prep, H, H, D, V, a, batch).view(-1, H, V)
+    ops.check_errors()
+    first = 0
+    for i, n in enumerate(lens):
+        rows, slot = prep[first:first + n].double(), batch.seg_slot[i].item()
+        part = lambda at, heads, w: rows[:, at:at + heads * w].view(n, heads, w)         # noqa: E731
+        Q, K, U, g, beta = part(0, H, D), part(H * D, H, D), part(2 * H * D, H, V), part(C, H, D), rows[:, C + H * D:C + H * D + H]
+        S, want = state[slot, :H * D * V].double().view(H, D, V), torch.empty(n, H, V, dtype=torch.float64, device=DEV)
+        for t in range(n):
+            S = g[t][:, :, None] * S
+            u = beta[t][:, None] * (U[t] - torch.einsum("hdv,hd->hv", S, K[t]))
+            S = S + K[t][:, :, None] * u[:, None, :]
+            want[t] = torch.einsum("hd,hdv->hv", Q[t], S)
+        # float32 sums over up to 200 decayed tokens and 128 rows
+        assert rows_error(got[first:first + n].double() / 2.0 ** (q + k + v), want / 2.0 ** (q + k + v)) < 3e-6
+        assert rows_error(a[slot, :H * D * V].double() / 2.0 ** (k + v), S.reshape(-1) / 2.0 ** (k + v)) < 3e-6
+        first += n
+
+
+def test_a_later_value_does_not_say_how_tiny_ones_are_computed(ops):    # noqa: F811
+    """Values too small for their parts, with and without an ordinary one behind them in the same eight tokens: the same bits before it."""
+    lens, H, V = (200, 192), 2, 128
+    batch, prep, state = delta_inputs(lens, H, H, V, 8)
+    first = 256 * H
+    prep[:8, first:first + H * V] *= 2.0 ** -116
+    state[batch.seg_slot[0].item()] = 0
+    outs = []
+    for size in (1.0, 2.0 ** 116):
+        rows = prep.clone()
+        rows[7, first:first + H * V] *= size
+        outs.append(ops.delta_scan(rows, H, H, 128, V, state.clone(), batch))
+    assert ops._takes_delta_chunks(batch, sum(lens), 128, V, H)
+    assert torch.equal(outs[0][:7], outs[1][:7]) and not torch.equal(outs[0][7], outs[1][7])
+
+
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 def test_octets_keep_later_tokens_out(ops, value):              # noqa: F811
     """A value that is no number reaches its own token and the ones after it; the tokens before it in its octet give the bits they give without it."""
