@@ -7,6 +7,8 @@
 // token's numbers are the same bits whatever else is in the batch.
 // Values that three bfloat16 numbers do not hold: a row of A or W whose largest magnitude is not in [2^-60, 2^60] (infinities, NaN, numbers near
 // the ends of float32's range; a row of zeros is fine) has its results computed over again by float32 multiply-adds at the end of a tile.
+// The promise is one about vectors: an error of some 2^-23 of |x| |w|, as float32 sums of any order give it.  It is not one about sum |x_k w_k|: a number
+// below 2^-110 in a row that also holds large ones keeps what is above 2^-133 of it.
 //
 // W is the tensor core's A operand (128 of its rows a tile, read from tensor memory), tokens are its N side (NT = 32, 64 or 128 of them):
 //   warp 0       W as it lies, float32, by TMA into a ring of stages of 64 of K (starts before the kernel ahead is done)

@@ -1,6 +1,6 @@
-// A float32 as three bfloat16 numbers: x = x0 + x1 + x2 exactly (8 + 8 + 8 significant bits, each part the rounding of what the parts before it
-// leave).  Six products of parts stand for one float32 product, x0 w0 + (x0 w1 + x1 w0) + (x0 w2 + x1 w1 + x2 w0); what they leave out is below
-// 2^-26 of |x w| and of either sign, and a product of two bfloat16 numbers is exact in the tensor core's float32 sum.  (Dekker, "A floating-point
+// A float32 as three bfloat16 numbers: x = x0 + x1 + x2 exactly from 2^-110 on (8 + 8 + 8 significant bits, each part the rounding of what the parts before
+// it leave; smaller numbers lose what is below 2^-133).  Six products of parts stand for one float32 product, x0 w0 + (x0 w1 + x1 w0) + (x0 w2 + x1 w1 + x2 w0); what they leave out is at most
+// 2^-24 + 2^-34 of |x w| and of either sign (x = w = 1 + 2^-8 - 2^-17; the rounding of one float32 product is as much), and a product of two bfloat16 numbers is exact in the tensor core's float32 sum.  (Dekker, "A floating-point
 // technique for extending the available precision", 1971; Ozaki et al., 2012, for matrix products on short formats.)
 #pragma once
 #include "sm100.cuh"
