@@ -39,7 +39,8 @@ __host__ __device__ __forceinline__ int first_slot(int qs, int seg) { return qs 
 
 __device__ __noinline__ float silu(float x) { return x / (1.f + expf(-x)); }
 // x / (1 + e^-x).  The quotient by one of Newton's steps on its remainder (Markstein, 1990) is a third of a division that also takes 1 + e^-x
-// beyond 2^126; inputs down there go to that division, once for all N numbers.
+// beyond 2^126; inputs down there go to that division, once for all N numbers.  An infinity becomes NaN here: both do not fit, and their tokens are
+// computed again with the division.
 template <int N> __device__ __forceinline__ void silu(float (&v)[N]) {
     float least = INFINITY;
 #pragma unroll

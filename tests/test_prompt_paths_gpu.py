@@ -354,6 +354,36 @@ def test_chunks_near_the_ends_of_the_parts(ops, q, k, v):       # noqa: F811
         first += n
 
 
+def test_silu_of_the_chunks(ops):                               # noqa: F811
+    """The activation alone, over every bfloat16 from -88 to 2^36: with a decay of 0 and queries and keys of one entry of 64 (silu: 64) a token's output is
+    4,096 times its activated values, without a rounding.  Against the division of the same float32 exponential, and against 64 bits."""
+    D = V = 128
+    x = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).float()
+    x = x[(x.abs() >= 2.0 ** -89) & (x >= -60) & (x <= 2.0 ** 36)]      # silu down to 2^-81, which the parts hold
+    far = torch.linspace(-88, -60, 513)[:512].to(torch.bfloat16).float()       # beyond -60 pieces of eight are told apart by their size
+    g = torch.Generator().manual_seed(1)
+    x = torch.cat([x[torch.randperm(x.numel(), generator=g)] for _ in range(2)])       # beside other neighbours each time
+    x = torch.cat([x, far, torch.ones((-(x.numel() + 512)) % V)])
+    T = x.numel() // V
+    p = torch.zeros(T, 3 * D, dtype=torch.bfloat16)
+    p[:, 0] = p[:, D] = 64.0
+    p[:, 2 * D:] = x.view(T, V)
+    batch = Entries((T,))
+    batch.max_q_len = T
+    state = torch.zeros(2, D * V, device=DEV)
+    assert ops._takes_chunks(batch, T, D, V, 1)
+    got = (ops.lightning_scan(p.to(DEV), 1, D, V, torch.zeros(1, device=DEV), state, batch).double() / 4096).view(-1)
+    ops.check_errors()
+    x = x.to(DEV)
+    want = x.double() / (1 + (-x.double()).exp())
+    division = (x / (1 + torch.exp(-x))).double()
+    ulp = 2.0 ** (want.abs().log2().floor() - 23)
+    # expf is within 1 unit (2 where the quotient's unit is half of it), the sum and the quotient half a unit each, the latter once more where it is not rounded
+    # to nearest
+    assert ((got - want).abs() / ulp).max().item() <= 4 and ((got - division).abs() / ulp).max().item() <= 1
+    assert ((got - want).abs() / ulp).mean().item() <= 1.02 * ((division - want).abs() / ulp).mean().item()
+
+
 def delta_inputs(lens, H, KV, V, seed):
     T, D, g = sum(lens), 128, torch.Generator().manual_seed(seed)
     r = lambda *s: torch.randn(*s, generator=g).to(DEV)         # noqa: E731
