@@ -10,6 +10,7 @@ hundred tokens waits for the host.  Where it cannot be built (no Python headers,
 same calls go through ctypes."""
 from __future__ import annotations
 
+import contextlib
 import hashlib
 import json
 import os
@@ -154,15 +155,13 @@ def _host_source() -> str:
 def _build_host_calls() -> None:
     cc = next((c for c in (os.environ.get("CC"), "cc", "gcc", "clang") if c and shutil.which(c)), None)
     include = sysconfig.get_paths()["include"]
-    if os.path.exists(HOST_CALLS):
+    with contextlib.suppress(FileNotFoundError):
         os.remove(HOST_CALLS)                                   # never an older one beside a new library
     if cc is None or not os.path.isfile(os.path.join(include, "Python.h")):
         _log("no C compiler or no Python headers: the entry points are called through ctypes")
         return
-    src, tmp = os.path.join(BUILD, "host_calls.c"), HOST_CALLS + f".tmp{os.getpid()}"
-    with open(src, "w") as f:
-        f.write(_host_source())
-    r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, src, "-o", tmp], capture_output=True, text=True)
+    tmp = HOST_CALLS + f".tmp{os.getpid()}"
+    r = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, "-x", "c", "-", "-o", tmp], input=_host_source(), capture_output=True, text=True)
     if r.returncode != 0:
         _log(f"{cc} failed on host_calls.c, the entry points are called through ctypes:\n{r.stderr[-2000:]}")
         return
@@ -185,7 +184,7 @@ def _sources():
 
 
 def _digest() -> str:
-    h = hashlib.sha256((" ".join(NVCC_FLAGS) + os.path.basename(HOST_CALLS) + _HOST_SOURCE).encode())
+    h = hashlib.sha256((" ".join(NVCC_FLAGS) + os.path.basename(HOST_CALLS) + _host_source()).encode())
     for f in sorted(os.listdir(CSRC)):
         if f.endswith((".cu", ".cuh", ".h")):
             with open(os.path.join(CSRC, f), "rb") as fh:
@@ -211,6 +210,8 @@ def is_current() -> bool:
 def build(force: bool = False, verbose: bool = True) -> str:
     """Compile every .cu under csrc/ (in parallel) and link _kernels.so.  Returns its path."""
     if not force and is_current():
+        if not os.path.isfile(HOST_CALLS):                      # a library that came without it
+            _build_host_calls()
         return LIB
     nvcc = _nvcc()
     os.makedirs(BUILD, exist_ok=True)

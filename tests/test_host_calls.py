@@ -48,3 +48,24 @@ def test_arguments_arrive_as_given():
         with pytest.raises((TypeError, AttributeError)):
             function(*given[:integer], wrong, *given[integer + 1:])
     assert len(seen) == 1                                        # nothing was called with a wrong argument
+
+
+def test_another_conversion_is_another_build(monkeypatch):
+    """What the generator writes around the fixed part is part of the build's digest."""
+    before, source = build._digest(), build._host_source
+    assert build._digest() == before
+    monkeypatch.setattr(build, "_host_source", lambda: source() + "/* another conversion */")
+    assert build._digest() != before
+
+
+def test_a_library_without_its_extension_gets_one(monkeypatch, tmp_path, capsys):
+    """... or a word that it stays on ctypes."""
+    build.build()
+    monkeypatch.setattr(build, "HOST_CALLS", str(tmp_path / "_host_calls.so"))
+    monkeypatch.setattr(build, "is_current", lambda: True)
+    build.build()
+    assert (tmp_path / "_host_calls.so").exists() or "ctypes" in capsys.readouterr().err
+    (tmp_path / "_host_calls.so").unlink(missing_ok=True)
+    monkeypatch.setattr(build.shutil, "which", lambda c: None)
+    build.build()
+    assert build.host_calls() is None and "ctypes" in capsys.readouterr().err
