@@ -229,6 +229,15 @@ MI_EXPORT long long mi_gemm_f32_workspace(int M, int N, int K) {
     return parts > plain ? parts : plain;
 }
 
+// kernels that mi_gemm_f32_nt launches
+MI_EXPORT int mi_gemm_f32_launches(const float* W, int M, int N, int K) {
+    if (M == 0 || N == 0) return 0;
+    int segment;
+    const int passes = (M + ROWS_AT_ONCE - 1) / ROWS_AT_ONCE;
+    if (on_tensor_cores(N, K) && (uintptr_t)W % 16 == 0) return passes * (tc_segments(N, K, &segment) > 1 ? 3 : 2);
+    return segments(N, K, &segment) > 1 ? passes * 2 : 1;
+}
+
 // tile < 0: chosen here (every tile gives the same bits)
 MI_EXPORT int mi_gemm_f32_nt(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, float* ws, int tile, int* error_word,
                              cudaStream_t stream) {

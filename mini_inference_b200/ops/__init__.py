@@ -4,7 +4,8 @@ kernels in csrc/ (built into _kernels.so, called through its C interface).
 There is no CPU path and no silent fall-back: get_ops() raises when there is no CUDA device
 or the library cannot be built or loaded.  Matrix products of the bfloat16 path go to the
 library GEMM, as the reference's do (engine/core/fused_linear.py:29-34); the float32 path
-uses this package's own float32 GEMM kernel, which never uses a reduced-precision mode.
+uses this package's own float32 products (csrc/gemm_f32.cu, gemm_f32_tc.cu), whose error is that
+of float32 sums whether they run as multiply-adds or as bfloat16 parts on the tensor cores.
 """
 from __future__ import annotations
 
@@ -73,11 +74,6 @@ def _code(dtype):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device_index: torch.cuda.current_stream(device_index).cuda_stream)
-
-
-def _p(t):
-    """A pointer argument of an entry point: the tensor itself (None: a null pointer)."""
-    return t
 
 
 def _check(err, what):
@@ -160,7 +156,7 @@ class CudaOps:
         self.fast_attention = True           # tests clear this to run the generic attention kernels in bfloat16
         self.biased_attention_tc = True      # prompts of attention with a distance table or a learned sink on the tensor cores (bfloat16)
         self.delta_work_bytes = 160 << 20    # scratch of the delta rule's chunks: as many heads at a time as fit
-        self.channel_work_bytes = 640 << 20  # the same with a decay per key channel: 16 heads of 13,000 tokens
+        self.channel_work_bytes = 640 << 20  # the same with a decay per key channel: 16 heads of 18,500 tokens (72,208 bytes per 32 tokens and head of 128 columns)
         self.fused_delta_step = True         # decode steps of the delta rule with one decay per head in one kernel (tests clear this)
         self.chunked_scan = True             # prompts of a state space or delta rule with one decay per head in chunks on the tensor cores (tests clear this)
         # Latent attention whose cached rows have 64 or 128 entries can run on the tensor-core paged attention kernels.  Those
@@ -169,7 +165,7 @@ class CudaOps:
         self.latent_tc = os.environ.get("MI_LATENT_TC", "0") == "1"
         # the grouped products of routed experts on mma.sync tensor-core tiles (bfloat16); MI_MOE_TC=0: the CUDA-core form
         self.moe_tc = os.environ.get("MI_MOE_TC", "1") == "1" and hasattr(self.lib, "mi_moe_gemm_tc")
-        # ... and, where an expert gets many rows, on tcgen05 tiles of 128 sorted rows (csrc/moe_grouped_tc.cu); MI_MOE_TCGEN05=0: never
+        # ... and, where an expert gets many rows, on tcgen05 tiles of up to 256 sorted rows (csrc/moe_grouped_tc.cu); MI_MOE_TCGEN05=0: never
         self.moe_tcgen05 = os.environ.get("MI_MOE_TCGEN05", "1") == "1"
         self.launches = 0                    # kernels of this package launched so far
 
@@ -316,7 +312,7 @@ class CudaOps:
         n = self.lib.mi_gemm_f32_workspace(M, N, K)
         ws = torch.empty(n, dtype=torch.float32, device=x.device) if n else None
         _check(self.lib.mi_gemm_f32_nt(x, ldx, w, out, ldc, M, N, K, ws, tile, self._stream_error, self._stream()), "gemm_f32")
-        self.launches += 2 if n else 1
+        self.launches += self.lib.mi_gemm_f32_launches(w, M, N, K)
 
     @staticmethod
     def _library_linear(x, w, out_dtype):

@@ -774,13 +774,12 @@ def test_head_gates_of_prompts(ops, dtype, T, H, V):            # noqa: F811
 @pytest.mark.parametrize("T,hidden", [(127, 264), (128, 264), (128, 2050), (600, 2048)])
 def test_weighted_sum_of_experts(ops, dtype, T, hidden):        # noqa: F811
     """128 tokens or more in 16-byte pieces where rows allow, fewer an entry a thread; with and without weights, a shared expert and its gate."""
-    from mini_inference_b200.ops import _p
     g, top = torch.Generator().manual_seed(T), 3
     rows, shared = torch.randn(T * top, hidden, generator=g).to(dtype).to(DEV), torch.randn(T, hidden, generator=g).to(dtype).to(DEV)
     weights, gate = torch.rand(T, top, generator=g).to(DEV), torch.randn(T, generator=g).to(DEV)
     for w, s, sg in ((weights, shared, gate), (weights, shared, None), (None, None, None)):
         out = torch.empty(T, hidden, dtype=dtype, device=DEV)
-        assert ops.lib.mi_moe_combine(_p(rows), _p(w), _p(s), _p(sg), _p(out), T, hidden, top, int(dtype == torch.bfloat16), ops._stream()) == 0
+        assert ops.lib.mi_moe_combine(rows, w, s, sg, out, T, hidden, top, int(dtype == torch.bfloat16), ops._stream()) == 0
         want = (rows.double().view(T, top, hidden) * (1.0 if w is None else w.double()[:, :, None])).sum(1)
         if s is not None:
             want += s.double() * (1.0 if sg is None else torch.sigmoid(sg.double())[:, None])
@@ -885,3 +884,14 @@ def test_expert_products_in_pairs_of_blocks(ops, counts, K, F, hidden):     # no
         want[t] = (y @ w_out[e].double().T).to(torch.bfloat16).double() * weights[t].double()
     # three roundings to bfloat16 (activated rows and rows on either side of a tie, the sum), each at most 2^-9 of a number
     assert rows_error(got, want) < 3 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("M,N,K,want", [(5, 4096, 2560, 3), (1030, 4096, 2560, 6), (40, 20480, 1024, 2), (3000, 64, 130, 1), (1030, 96, 2048, 4)])
+def test_launches_of_float32_products_are_counted(ops, M, N, K, want):  # noqa: F811
+    """Splitting, product and sum of the segments, per 1,024 rows."""
+    x, w, before = torch.zeros(M, K, device=DEV), torch.zeros(N, K, device=DEV), ops.launches
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ops.linear(x, w)
+        torch.cuda.synchronize()
+    assert ops.launches - before == want
+    assert sum(e.count for e in prof.key_averages() if "gemm_f32" in e.key or "split_rows" in e.key or "add_segments" in e.key) == want
