@@ -16,21 +16,6 @@ namespace {
 
 constexpr int WARPS = 8, NK = 8;                                // warps of a block, keys of a warp's step
 
-// Sums NV values over the lanes of a warp; lane l ends with the sum of value l % NV
-template <int NV>
-__device__ __forceinline__ float sum_spread(float (&y)[NV], int l) {
-#pragma unroll
-    for (int w = 1; w < NV; w <<= 1)
-#pragma unroll
-        for (int e = 0; e < NV; e += 2 * w) {
-            const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
-            y[e] = (l & w ? y[e + w] : y[e]) + got;
-        }
-    float v = y[0];
-#pragma unroll
-    for (int w = NV; w < 32; w <<= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
-    return v;
-}
 template <int N> __device__ __forceinline__ void load_n(const float* p, float (&v)[N]) {
     if constexpr (N == 4) load16(p, v);
     else load2(p, v[0], v[1]);

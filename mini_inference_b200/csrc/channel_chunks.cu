@@ -57,21 +57,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-// Sums NV values over the lanes of a warp; lane l ends with the sum of value l % NV.
-template <int NV>
-__device__ __forceinline__ float sum_spread(float (&y)[NV], int l) {
-#pragma unroll
-    for (int w = 1; w < NV; w <<= 1)
-#pragma unroll
-        for (int e = 0; e < NV; e += 2 * w) {
-            const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
-            y[e] = (l & w ? y[e + w] : y[e]) + got;
-        }
-    float v = y[0];
-#pragma unroll
-    for (int w = NV; w < 32; w <<= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
-    return v;
-}
 // the largest magnitude of N numbers as float bits (NaN above all)
 template <int N> __device__ __forceinline__ uint32_t largest(const float (&x)[N]) {
     float m = 0.f;
@@ -709,7 +694,8 @@ MI_EXPORT int mi_channel_chunks(const float* prep, int ld, void* work, long long
         // entry's walk is two thirds and more of what an SM walks on average (an entry counted as two chunks more than it has: 1,500 + 300 + 200 tokens
         // 159 and 191, 1,300 + 517 + 231 160 and 176, 300 + 700 + 200 113 and 100, 4 x 512 168 and 151, 900 + 500 125 and 113, 8 x 1,024 556 and 508).
         const long long blocks = (long long)heads * num_segs * (V / VC), all = (long long)(T_ / C + 2 * num_segs) * heads * (V / VC);
-        const bool deep = blocks <= 148 || (blocks > 2 * 148 && 20ll * 148 * (longest / C + 2) >= 13 * all);
+        const long long sms = device_sms();
+        const bool deep = blocks <= sms || (blocks > 2 * sms && 20 * sms * (longest / C + 2) >= 13 * all);
         auto walk = deep ? pass_kernel<true> : pass_kernel<false>;
         walk<<<dim3(V / VC, heads, num_segs), 160, deep ? PASS_SMEM<true> : PASS_SMEM<false>, stream>>>((const unsigned char*)work, slots, L, state, state_stride, out, seg_q_start,
                                                                                                     seg_slot, H, h0, V, error_word);

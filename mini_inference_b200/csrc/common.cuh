@@ -43,6 +43,22 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// Sums NV values over the lanes of a warp; lane l ends with the sum of value l % NV
+template <int NV>
+__device__ __forceinline__ float sum_spread(float (&y)[NV], int l) {
+#pragma unroll
+    for (int w = 1; w < NV; w <<= 1)
+#pragma unroll
+        for (int e = 0; e < NV; e += 2 * w) {
+            const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
+            y[e] = (l & w ? y[e + w] : y[e]) + got;
+        }
+    float v = y[0];
+#pragma unroll
+    for (int w = NV; w < 32; w <<= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
+    return v;
+}
+
 // The gates of a feed-forward: act(g) * u.  The tanh form of gelu, 0.5 g (1 + tanh(y)) with y = sqrt(2 / pi) (g + 0.044715 g^3), is
 // g / (1 + e^(-2 y)).
 constexpr int GATE_RELU = 0, GATE_SILU = 1, GATE_GELU_TANH = 2;

@@ -172,7 +172,8 @@ constexpr int ROWS_AT_ONCE = 1024;             // rows per pass of a product tha
 // 1,024 x 1,024 15.0 / 16.5, 17.1 / 17.5, 81 / 23; from 256 x 4,096 on one row is faster here too); the error is a third everywhere.
 bool on_tensor_cores(int N, int K) { return K % 4 == 0 && K >= 512 && N >= 128 && (long long)N * K >= 1 << 20; }
 
-// Their K is cut until a tile of tokens alone gives about one block per SM, in pieces of at least 512
+// Their K is cut until a tile of tokens alone gives about one block per SM, in pieces of at least 512.  148 is a constant of the format here, like 512: a
+// row's bits go with it.
 int tc_segments(int N, int K, int* segment) {
     int S = K / 512 < 8 ? K / 512 : 8;
     if (S > 148 / ((N + 127) / 128)) S = 148 / ((N + 127) / 128);

@@ -20,7 +20,7 @@
 // an expert 110 / 108.  A product of 256 x 256 takes 0.85 us per 128 of K and hardly less with fewer columns (what gemm_tc2.cu takes too), so the
 // number of tiles counts.  Measured and left: tiles of up to 384 rows as two products on one piece of the matrix (165 us), stages of 64 of K
 // (177), tokens in boxes of 32 and 16 rows (157: the copying thread was the bound).
-#include "sm100.cuh"
+#include "pair.cuh"
 #include <math.h>
 
 using namespace mi;
@@ -34,43 +34,6 @@ constexpr int EPILOGUE_WARPS = 8, THREADS = 64 + 32 * EPILOGUE_WARPS, ACC_COLS =
 constexpr int TURN_BYTES = 4096;                                        // per epilogue warp: 32 x 32 bfloat16 to be stored, 16 x 32 float32 from its partner
 constexpr int SMEM = 1024 + STAGES * STAGE + EPILOGUE_WARPS * TURN_BYTES + 128;
 constexpr int TILE = 256, STEP = 32;                                    // most rows of a tile; rows of tiles come in steps
-
-__device__ __forceinline__ uint32_t cta_rank_in_cluster() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(local), "r"(rank));
-    return remote;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" :: "r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster) {
-    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n"
-                 :: "r"(dst), "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar_cluster) : "memory");
-}
-__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_slot, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" :: "r"(smem_slot), "r"(cols) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" :: "r"(taddr), "r"(cols) : "memory");
-}
-__device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, bool accumulate) {
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                 " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5, %5, %5, %5, %5}, p;\n}\n"
-                 :: "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"((uint32_t)accumulate), "r"(0u) : "memory");
-}
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
-                 :: "r"(bar), "h"(mask) : "memory");
-}
 
 __device__ __forceinline__ float gated(float g, float u, float limit, float slope, float shift) {
     g = fminf(g, limit);

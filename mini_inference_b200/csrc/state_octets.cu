@@ -43,22 +43,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 }
 __device__ __forceinline__ float silu(float x) { return x / (1.f + expf(-x)); }
 
-// Sums NV values over the lanes of a warp; lane l ends with the sum of value l % NV.
-template <int NV>
-__device__ __forceinline__ float sum_spread(float (&y)[NV], int l) {
-#pragma unroll
-    for (int w = 1; w < NV; w <<= 1)
-#pragma unroll
-        for (int e = 0; e < NV; e += 2 * w) {
-            const float got = __shfl_xor_sync(0xffffffffu, l & w ? y[e] : y[e + w], w);
-            y[e] = (l & w ? y[e + w] : y[e]) + got;
-        }
-    float v = y[0];
-#pragma unroll
-    for (int w = NV; w < 32; w <<= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
-    return v;
-}
-
 // R (2 or 4) neighbouring entries in one access
 template <int R> __device__ __forceinline__ void load_n(const float* p, float (&v)[R]) {
     if constexpr (R == 4) { const float4 t = *reinterpret_cast<const float4*>(p); v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; }
