@@ -172,14 +172,16 @@ constexpr int ROWS_AT_ONCE = 1024;             // rows per pass of a product tha
 // 1,024 x 1,024 15.0 / 16.5, 17.1 / 17.5, 81 / 23; from 256 x 4,096 on one row is faster here too); the error is a third everywhere.
 bool on_tensor_cores(int N, int K) { return K % 4 == 0 && K >= 512 && N >= 128 && (long long)N * K >= 1 << 20; }
 
-// Their K is cut until a tile of tokens alone gives about one block per SM, in pieces of at least 512.  148 is a constant of the format here, like 512: a
-// row's bits go with it.
+// Their K is cut until a tile of tokens alone gives about one block per SM, in pieces of at least 512 (148 is a
+// constant of the format here, like 512: a row's bits go with it).  The last piece takes the rest, at least three stages of 64: gemm_f32_tc.cu hands its
+// rows' maxima over between items of that length only.
 int tc_segments(int N, int K, int* segment) {
     int S = K / 512 < 8 ? K / 512 : 8;
     if (S > 148 / ((N + 127) / 128)) S = 148 / ((N + 127) / 128);
     if (S < 1) S = 1;
     *segment = ((K + S - 1) / S + BK_MAX - 1) / BK_MAX * BK_MAX;
-    return (K + *segment - 1) / *segment;
+    S = (K + *segment - 1) / *segment;
+    return S > 1 && K - (S - 1) * *segment <= 2 * BK_MAX ? S - 1 : S;
 }
 
 int add_up(const float* ws, float* C, int ldc, int M, int N, int S, cudaStream_t stream) {
@@ -229,6 +231,9 @@ MI_EXPORT long long mi_gemm_f32_workspace(int M, int N, int K) {
     const long long parts = mi::gemm_f32_tc_parts(rows, K) / 4 + (S > 1 ? (long long)S * rows * N : 0);
     return parts > plain ? parts : plain;
 }
+
+// Where K is cut for the tensor cores: the pieces, and how long all but the last are (0 pieces: multiply-adds)
+MI_EXPORT int mi_gemm_f32_pieces(int N, int K, int* length) { return on_tensor_cores(N, K) ? tc_segments(N, K, length) : 0; }
 
 // kernels that mi_gemm_f32_nt launches
 MI_EXPORT int mi_gemm_f32_launches(const float* W, int M, int N, int K) {

@@ -16,6 +16,9 @@
 //   warps 2-9    two groups that take turns: a thread reads a row's 64 numbers of a stage and writes their three parts to tensor memory
 //   warps 10-17  the sums: a thread has one row of W and half of the tile's tokens
 //   warp 18      the tokens' parts, made once by split_rows_kernel, by TMA
+// The rows' largest magnitudes go from the converting to the adding warps in two slots that take turns and are not handed back: an item has at least
+// three stages (tc_segments in gemm_f32.cu), so both groups have converted a stage that lies five or more behind item i before they end item i + 2, and
+// one four stages earlier, of a later item than i, was added up by then.
 // Tensor memory: two stages of W's parts (2 x 96 columns) and two accumulators (2 x NT columns).
 //
 // Against gemm_f32.cu's multiply-adds (microseconds; N x K = 6,144 x 2,560, 2,560 x 4,096, 19,456 x 2,560, 2,560 x 9,728): 501 rows 492, 332, 1,355, 668
@@ -88,7 +91,7 @@ __device__ __forceinline__ Item item_of(const Shape& sh, int i) {
     it.n0 = rest / sh.segments * BN;
     it.m0 = mt * NT;
     it.k_first = it.seg * sh.segment;
-    it.k_end = min(sh.K, it.k_first + sh.segment);
+    it.k_end = it.seg + 1 == sh.segments ? sh.K : it.k_first + sh.segment;
     it.stages = (it.k_end - it.k_first + BK - 1) / BK;
     return it;
 }
@@ -105,16 +108,15 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     uint64_t* bars = reinterpret_cast<uint64_t*>(row_max + 2 * 2 * BN);
     const uint32_t sW = smem_u32(base), sX = sW + WS * W_STAGE;
     const uint32_t w_full = smem_u32(bars), w_empty = w_full + 8 * WS, x_full = w_empty + 8 * WS, x_empty = x_full + 8 * XS,
-                   a_full = x_empty + 8 * XS, a_empty = a_full + 16, d_full = a_empty + 16, d_empty = d_full + 16, m_full = d_empty + 16,
-                   m_empty = m_full + 16;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * WS + 2 * XS + 12);
+                   a_full = x_empty + 8 * XS, a_empty = a_full + 16, d_full = a_empty + 16, d_empty = d_full + 16, m_full = d_empty + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * WS + 2 * XS + 10);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < WS; ++s) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 4); }
         for (int s = 0; s < XS; ++s) { mbar_init(x_full + 8 * s, 1); mbar_init(x_empty + 8 * s, 1); }
         for (int s = 0; s < 2; ++s) {
             mbar_init(a_full + 8 * s, 4); mbar_init(a_empty + 8 * s, 1); mbar_init(d_full + 8 * s, 1); mbar_init(d_empty + 8 * s, 8);
-            mbar_init(m_full + 8 * s, 8); mbar_init(m_empty + 8 * s, 8);
+            mbar_init(m_full + 8 * s, 8);
         }
         mbar_init_fence();
         tma_prefetch_desc(&wmap); tma_prefetch_desc(&xmap);
@@ -227,9 +229,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
                 }
                 if (++s == WS) { s = 0; ++turn; }
             }
-            if (!ok) break;
-            // An item may be one stage (the end of K), and a group none of it: the ring of stages alone does not keep it from the slot it wrote two items ago
-            if (turn_of_item >= 2 && !mbar_wait(m_empty + 8 * (turn_of_item & 1), ((turn_of_item >> 1) - 1) & 1)) { atomicExch(error_word, 80); break; }
             const float lo = __low2float(mx), hi = __high2float(mx);
             row_max[((turn_of_item & 1) * 2 + g) * BN + row] = lo == lo && hi == hi ? fmaxf(lo, hi) : INFINITY;
             __syncwarp();
@@ -272,8 +271,6 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             if (!mbar_wait(m_full + 8 * (turn_of_item & 1), (turn_of_item >> 1) & 1)) { atomicExch(error_word, 89); ok = false; break; }
             const float* rm = row_max + (turn_of_item & 1) * 2 * BN + row;
             const float most = fmaxf(rm[0], rm[BN]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(m_empty + 8 * (turn_of_item & 1));
             const bool odd_row = !(most <= MOST) || (most > 0.f && most < LEAST);
             const int mine = m_first + lane;
             const unsigned odd0 = __ballot_sync(0xffffffffu, lane < HALF && mine < sh.M && token_flag[mine]);

@@ -516,7 +516,7 @@ class CudaOps:
         if code != 0:
             self._stream_error.zero_()
             self._tc2_counters.zero_()
-            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-64 grouped expert product, 71-74 delta rule and constant decay in chunks, 80-89 float32 product, 91-92 channel decays in chunks)")
+            raise RuntimeError(f"a pipeline wait inside a kernel ran out (code {code}: 1-2 gemm_stream, 21-31 attention, 41-42 recurrences eight tokens at a time, 51-55 gemm_tc2, 61-64 grouped expert product, 71-74 delta rule and constant decay in chunks, 81-89 float32 product, 91-92 channel decays in chunks)")
 
     # ---------------------------------------------------------------- q/k norm, rotation, cache write
     def qk_norm_rope_cache(self, qkv, H, KV, D, q_weight, k_weight, eps, inv_freq, meta, k_cache, v_cache):

@@ -59,8 +59,8 @@ def test_gemm_f32_on_tensor_cores(ops, M, N, K):                # noqa: F811
 
 @pytest.mark.parametrize("M,N,K", [(652, 896, 4100), (700, 896, 4160), (768, 2048, 4100), (1030, 1152, 4132)])
 def test_gemm_f32_whose_last_segment_is_short(ops, M, N, K):    # noqa: F811
-    """K that leaves a last segment of one or two stages, so that a block has several such items in a row: which rows of W bfloat16 parts cannot hold is then
-    handed over faster than anything else (rows of infinities, NaN and 1e30 in every other tile, in the last segment's columns)."""
+    """K whose last 512th would be one or two stages, and blocks with several such items in a row: rows of infinities, NaN and 1e30 in every other tile, in the
+    last segment's columns, are handed from warp to warp as fast as it gets."""
     g = torch.Generator().manual_seed(M + K)
     x, w = torch.randn(M, K, generator=g).to(DEV), torch.randn(N, K, generator=g).to(DEV)
     plain = ops.linear(x, w)
