@@ -107,7 +107,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
     extern __shared__ float smem_raw[];  // [WARPS][16][D] outputs, then [WARPS][16] max and sum
     float* smem = smem_raw;
     pdl_trigger();
-    if (!BULK) pdl_wait();
+    if (!BULK) pdl_wait(q, k_cache, v_cache);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, c = lane & 3;
     const int G = H / KV;
@@ -170,7 +170,7 @@ attn_decode_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_co
         __syncwarp();
         for (; primed < DEC_STAGES && b0 + warp + primed * WARPS < min(b1, blk_hi - 1); ++primed)
             issue(b0 + warp + primed * WARPS, primed);
-        pdl_wait();
+        pdl_wait(q);
     }
     if (warp == 0) {
         const __nv_bfloat16* qrow = q + (size_t)tok * q_stride + (size_t)kvh * G * D;

@@ -154,7 +154,7 @@ __global__ void attn_decode_merge_kernel(const float* __restrict__ o_part, const
                                          T* __restrict__ out, const int* __restrict__ decode_segs,
                                          const int* __restrict__ seg_q_start, int H, int D, int S) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(o_part, lse_part);
     const int i = blockIdx.x, h = blockIdx.y;
     const int tok = seg_q_start[decode_segs[i]];
     const size_t base = ((size_t)i * H + h) * S;

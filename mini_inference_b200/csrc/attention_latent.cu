@@ -45,7 +45,7 @@ __global__ void latent_prepare_kernel(const T* __restrict__ p, int ldp, const T*
     const float pos = (float)positions[t];
     pdl_trigger();
     for (int i = threadIdx.x; i < nf; i += blockDim.x) sincosf(pos * inv_freq[i], turn + nf + i, turn + i);
-    pdl_wait();                                            // positions and frequencies were there before the step began
+    pdl_wait(row, qrow, q_abs);                                            // positions and frequencies were there before the step began
     __syncthreads();
     T* qo = q_out + (size_t)t * H * (C + R);
     const int parts = gridDim.y, mine = (H - (int)blockIdx.y + parts - 1) / parts;        // this part's heads

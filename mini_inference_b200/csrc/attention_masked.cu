@@ -262,7 +262,7 @@ __global__ void unit_qk_cache_kernel(T* __restrict__ p, int ldp, const T* __rest
         const float pos = (float)positions[t];
         for (int i = threadIdx.x; i < half; i += blockDim.x) sincosf(pos * inv_freq[i], turn + half + i, turn + i);
     }
-    pdl_wait();                                                 // positions and frequencies were there before the step began
+    pdl_wait(row, v_src);                                                 // positions and frequencies were there before the step began
     if (half > 0) __syncthreads();
     for (int u = warp; u < H + KV; u += nw) {                   // q heads, then k heads
         T* x = row + (size_t)u * D;
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(256) unit_qk_cache_vec_kernel(__nv_bfloat16* _
         const float pos = (float)positions[t];
         for (int i = threadIdx.x; i < half; i += 256) sincosf(pos * inv_freq[i], turn + half + i, turn + i);
     }
-    pdl_wait();                                                 // positions and frequencies were there before the step began
+    pdl_wait(row, v_src);                                                 // positions and frequencies were there before the step began
     if (half > 0) __syncthreads();
     const size_t base = ((size_t)(slot / ps) * KV * ps + slot % ps) * D + chunk * 8;        // + head * ps * D
     auto put = [&](__nv_bfloat16* dst, const float (&v)[8]) {

@@ -59,7 +59,7 @@ deferred_add_rmsnorm_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
     const long long U = (long long)NRT * NKC;
     for (int rt = threadIdx.x; rt < NRT; rt += blockDim.x) shares[rt] = shares_of(rt, NKC, U, G);
     __syncthreads();
-    pdl_wait();
+    pdl_wait(ws);
     const int t = blockIdx.x;
     float ss = 0.f;
     for (int i = threadIdx.x; i < N / 4; i += blockDim.x) {
@@ -97,7 +97,7 @@ deferred_add_rmsnorm_kernel(__nv_bfloat16* __restrict__ x, const float* __restri
 __global__ void deferred_reduce_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int N, int K, int G,
                                        int max_contrib, int tok) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(ws);
     const int NKC = K / KC, NRT = (N + TR - 1) / TR;
     const long long U = (long long)NRT * NKC;
     const int t = blockIdx.y;
@@ -114,7 +114,7 @@ __global__ void deferred_reduce_kernel(const float* __restrict__ ws, __nv_bfloat
 __global__ void deferred_glu_kernel(const float* __restrict__ ws, __nv_bfloat16* __restrict__ out, int inter, int K, int G,
                                     int max_contrib, int tok, int act) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(ws);
     const int N = 2 * inter;
     const int NKC = K / KC, NRT = (N + TR - 1) / TR;
     const long long U = (long long)NRT * NKC;

@@ -13,7 +13,7 @@ template <typename T>
 __global__ void embedding_kernel(const int* __restrict__ ids, const T* __restrict__ table, T* __restrict__ out,
                                  int hidden, int vocab) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(ids);
     const int t = blockIdx.x;
     int id = ids[t];
     if (id < 0 || id >= vocab) id = 0;       // the host refuses such ids; never read out of range
@@ -68,7 +68,7 @@ __global__ void add_rmsnorm_kernel(T* __restrict__ x, const T* __restrict__ delt
     __shared__ float scratch[32];
     pdl_trigger();
     if (l2_ahead_rides(ahead, ahead_bytes, work)) return;
-    pdl_wait();
+    pdl_wait(x, delta);
     const int r = blockIdx.x;
     const size_t src = (size_t)(rows ? rows[r] : r) * hidden;
     T* xr = x + src;
@@ -145,7 +145,7 @@ add_rmsnorm_vec_kernel(T* __restrict__ x, const T* __restrict__ delta, const WT*
     constexpr int V = Vec16<T>::N;
     pdl_trigger();
     if (l2_ahead_rides(ahead, ahead_bytes, work)) return;
-    pdl_wait();
+    pdl_wait(x, delta);
     const int r = blockIdx.x;
     const size_t src = (size_t)(rows ? rows[r] : r) * hidden;
     const int nvec = hidden / V;
@@ -191,7 +191,7 @@ add_rmsnorm_warp_kernel(T* __restrict__ x, const T* __restrict__ delta, const WT
     constexpr int V = Vec16<T>::N;
     pdl_trigger();
     if (l2_ahead_rides(ahead, ahead_bytes, work)) return;
-    pdl_wait();
+    pdl_wait(x, delta);
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (r >= num_rows) return;
@@ -283,7 +283,7 @@ MI_EXPORT int mi_add_rmsnorm(void* x, const void* delta, const void* w, void* y,
 template <typename T>
 __global__ void swiglu_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int rows, int inter) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(gate_up);
     const size_t n = (size_t)rows * inter;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const size_t r = i / inter, c = i % inter;
@@ -298,7 +298,7 @@ template <typename T>
 __global__ void swiglu_vec_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int rows, int inter) {
     constexpr int V = Vec16<T>::N;
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(gate_up);
     const int vec_per_row = inter / V;
     const size_t n = (size_t)rows * vec_per_row;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {

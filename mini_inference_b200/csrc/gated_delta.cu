@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) delta_step_kernel(const T* __restrict__ p
         early[k] = i < channels ? past(c) : 0.f;
         last_tap[k] = conv[(size_t)c * taps + taps - 1];
     }
-    pdl_wait();
+    pdl_wait(row);
     if (tid == 255) {
         gates[0] = 1.f / (1.f + expf(-to_f32(row[C + H * V + h])));
         gates[1] = decay_of(log_decay(to_f32(row[C + H * V + H + h]), dt_bias[h], rate[h]));

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(NT) stream_layernorm_vec_kernel(float* __restr
             wyv[k] = y && q < quads ? *reinterpret_cast<const float4*>(wy + 4 * q) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
-    pdl_wait();
+    pdl_wait(x, y);
 #pragma unroll
     for (int k = 0; k < VPT; ++k) {
         const int q = threadIdx.x + k * NT;
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(LOOP_NT) stream_layernorm_kernel(float* __rest
                                                               const int* __restrict__ rows, int hidden, float eps, int keep) {
     __shared__ float4 scratch[2][LOOP_NT / 32];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(x, y);
     const size_t r = (rows ? (size_t)rows[blockIdx.x] : (size_t)blockIdx.x) * hidden;
     Moments my{0.f, 0.f};
     if (y) my = loop_moments([&](int i) { return to_f32(y[r + i]); }, hidden, eps_y, scratch[0]);

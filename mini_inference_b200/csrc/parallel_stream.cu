@@ -143,7 +143,7 @@ template <typename T>
 __global__ void rows_rmsnorm_kernel(const T* __restrict__ x, long long ldx, const float* __restrict__ w, T* __restrict__ y, int cols, float eps) {
     __shared__ float scratch[32];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(x);
     const T* xr = x + (size_t)blockIdx.x * ldx;
     float ss = 0.f;
     for (int i = threadIdx.x; i < cols; i += NT) { const float v = to_f32(xr[i]); ss += v * v; }
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(NT) rows_rmsnorm_vec_kernel(const T* __restric
     float wv[VN], v[VN], ss = 0.f;
 #pragma unroll
     for (int e = 0; e < VN; ++e) { wv[e] = i < cols ? w[i + e] : 0.f; v[e] = 0.f; }
-    pdl_wait();
+    pdl_wait(x);
     if (i < cols) load16(x + (size_t)blockIdx.x * ldx + i, v);
 #pragma unroll
     for (int e = 0; e < VN; ++e) ss += v[e] * v[e];
@@ -186,7 +186,7 @@ template <typename T> __device__ __forceinline__ void store16v(T* p, const float
 template <typename T>
 __global__ void bias_glu_kernel(const T* __restrict__ gu, const float* __restrict__ bias, T* __restrict__ out, int inter, int act) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(gu);
     const T* g = gu + (size_t)blockIdx.x * 2 * inter;
     T* o = out + (size_t)blockIdx.x * inter;
     for (int i = blockIdx.y * NT + threadIdx.x; i < inter; i += gridDim.y * NT) {
@@ -201,7 +201,7 @@ template <typename T>
 __global__ void bias_glu_vec_kernel(const T* __restrict__ gu, const float* __restrict__ bias, T* __restrict__ out, int inter, int act) {
     constexpr int VN = Vec16<T>::N;
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(gu);
     const T* g = gu + (size_t)blockIdx.x * 2 * inter;
     T* o = out + (size_t)blockIdx.x * inter;
     for (int i = (blockIdx.y * NT + threadIdx.x) * VN; i < inter; i += gridDim.y * NT * VN) {

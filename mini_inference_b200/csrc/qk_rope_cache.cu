@@ -22,7 +22,7 @@ __global__ void qk_norm_rope_cache_kernel(T* __restrict__ qkv, const WT* __restr
                                           const int* __restrict__ slots, T* __restrict__ k_cache, T* __restrict__ v_cache,
                                           int H, int KV, int D, int page_size, float eps, int num_tokens) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(qkv);
     const int lane = threadIdx.x & 31;
     const int heads = H + 2 * KV;
     const int half = D / 2;
@@ -100,7 +100,7 @@ qk_norm_rope_cache_token_kernel(T* __restrict__ qkv, const WT* __restrict__ q_w,
                                 int H, int KV, int D, int page_size, float eps) {
     __shared__ float cs[MAX_HALF], sn[MAX_HALF];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(qkv);
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     const int half = D / 2, heads = H + 2 * KV;
     if (inv_freq) {
@@ -204,7 +204,7 @@ qk_norm_rope_cache_vec_kernel(T* __restrict__ qkv, const WT* __restrict__ q_w, c
     constexpr bool PACKED = sizeof(T) == 2 && sizeof(WT) == 2;     // bfloat16 rows and weights: two elements per register
     __shared__ __align__(16) float cs[HALF < 4 ? 4 : HALF], sn[HALF < 4 ? 4 : HALF];
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(qkv);
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int heads = H + 2 * KV;
     const int h = (blockIdx.y * 8 + warp) * HPW + lane / LPH, chunk = lane % LPH;

@@ -29,7 +29,7 @@ __global__ void sample_kernel(const float* __restrict__ logits, int ld, int voca
     __shared__ float best_v[NT / 32];
     __shared__ int best_i[NT / 32];
     mi::pdl_trigger();
-    mi::pdl_wait();
+    mi::pdl_wait(logits, temps, seeds, counters);
     const int r = blockIdx.x;
     const float* row = logits + (size_t)r * ld;
     const float temp = temps ? temps[r] : 0.f;
@@ -76,7 +76,7 @@ __global__ void sample_split_kernel(const float* __restrict__ logits, int ld, in
                                     int* __restrict__ arrivals) {
     __shared__ unsigned long long best[NT / 32];
     mi::pdl_trigger();
-    mi::pdl_wait();
+    mi::pdl_wait(logits, temps, seeds, counters);
     const int r = blockIdx.x;
     const float* row = logits + (size_t)r * ld;
     const float temp = temps ? temps[r] : 0.f;

@@ -202,7 +202,7 @@ __global__ void head_gate_vec_kernel(const T* __restrict__ o, const T* __restric
 template <typename T, int VN>
 __global__ void sigmoid_gate_kernel(T* __restrict__ rows, const T* __restrict__ gate, int gate_stride, int n) {
     pdl_trigger();
-    pdl_wait();
+    pdl_wait(rows, gate);
     T* r = rows + (size_t)blockIdx.x * n;
     const T* g = gate + (size_t)blockIdx.x * gate_stride;
     for (int i = (blockIdx.y * blockDim.x + threadIdx.x) * VN; i < n; i += gridDim.y * blockDim.x * VN) {
