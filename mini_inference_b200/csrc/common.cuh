@@ -19,8 +19,8 @@ namespace mi {
 // anything the predecessor produces (or still reads).  pdl_trigger() lets the NEXT kernel start
 // its own preamble early.  Both are no-ops for a kernel launched the ordinary way.
 // Pointers to what the predecessor writes are passed along: a kernel's __restrict__ pointer promises that nobody else writes there while the kernel runs, so
-// that the compiler may read by it ahead of the wait; what it knows of these begins anew here.  (A pointer that is also written by stays out: two that begin
-// anew may be the same to the compiler, and a loop that reads by one and writes by the other waits every time; deferred_sum.cu so: a decode step 8 % slower.)
+// that the compiler may read by it ahead of the wait; what it knows of these begins anew here.  (Two that begin anew may be the same to the compiler: where
+// a loop reads by one and writes by the other, only the first is passed.  deferred_sum.cu with both: a decode step 8 % slower.)
 template <typename P> __device__ __forceinline__ void begins_here(P& p) { asm volatile("" : "+l"(p) :: "memory"); }
 template <typename... P> __device__ __forceinline__ void pdl_wait(P&... written) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
