@@ -783,7 +783,7 @@ class CudaOps:
         """Whether a recurrence with a constant decay that _takes_octets goes 128 tokens at a time on the tensor cores instead (csrc/state_chunks.cu): keys
         of 128, values in blocks of 128 columns, a prompt of at least 320 tokens (three kernels of some 36 us in all against eight tokens at a time:
         192 tokens 27 us there, 256 31, 400 41, 2,048 167 against 73) and 100 tokens an entry on average, since a short entry takes a whole chunk
-        (16 prompts of 64 tokens 73 us there, 89 here; 192 tokens beside 40 decoded ones 92 and 256).  H heads: where the chunks are one wave of blocks
+        (16 prompts of 64 tokens 73 us there, 83 here; 192 tokens beside 40 decoded ones 92 and 256).  H heads: where the chunks are one wave of blocks
         that is all; beyond, both sides' times are weighed, a line through 2 to 64 heads of 128 to 512 columns (within a tenth): 64 heads 2,048 tokens 502 us
         there, 288 here, 1,024 beside 8 single ones 285 and 305, 400 beside 3 121 and 145; 32 heads 330 beside 2 65 and 71, 700 beside 3 125 and 80."""
         if not (D == 128 and V % 128 == 0 and getattr(batch, "max_q_len", 0) >= 320 and T >= 100 * batch.num_segs):
